@@ -98,6 +98,8 @@ __device__ __forceinline__ void close_step(Control* ctl, unsigned it, float rel,
     ctl->total_iters += it;
 }
 
+constexpr uint32_t kNearCap = 64;  // within-h list entries per particle
+
 // List skins (units of h) an adaptive scene chooses from, smallest first.
 constexpr int kSkinLevels = 3;
 __host__ __device__ inline float skin_level_value(int k) { return k <= 0 ? 0.25f : k == 1 ? 0.35f : 0.5f; }

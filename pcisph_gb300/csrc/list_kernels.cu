@@ -35,6 +35,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "list_kernels.cuh"
 #include "pair_terms.cuh"
@@ -52,29 +53,6 @@ constexpr unsigned kMarkBlocks = 152;  // the marking kernel's grid (grid-stride
 // chunk c as 1 KB of contiguous memory, and the builder writes whole 32-byte sectors.
 __device__ __forceinline__ uint4* list_chunk(uint32_t* list, uint32_t i, uint32_t c, uint32_t stride) {
     return reinterpret_cast<uint4*>(list) + 2 * ((size_t)c * stride + i);
-}
-
-// The builder stages each list's current chunk in shared memory, slot-major (buf[slot * kBlock + thread]:
-// conflict-free whatever slot each lane is at), and writes whole chunks.
-__device__ __forceinline__ void list_store_chunk(uint32_t* list, uint32_t i, uint32_t c, uint32_t stride,
-                                                 const uint32_t* buf) {
-    const uint32_t t = threadIdx.x;
-    uint4* p = list_chunk(list, i, c, stride);
-    __stcs(p, make_uint4(buf[t], buf[kBlock + t], buf[2 * kBlock + t], buf[3 * kBlock + t]));
-    __stcs(p + 1, make_uint4(buf[4 * kBlock + t], buf[5 * kBlock + t], buf[6 * kBlock + t], buf[7 * kBlock + t]));
-}
-
-// Append j as entry k of particle i's list.
-__device__ __forceinline__ void list_append(uint32_t* list, uint32_t i, uint32_t stride, uint32_t* buf, uint32_t k,
-                                            uint32_t j) {
-    buf[(k & 7u) * kBlock + threadIdx.x] = j;
-    if ((k & 7u) == 7u) list_store_chunk(list, i, k >> 3, stride, buf);
-}
-
-// Write the last, partial chunk of a list of n <= cap entries.
-__device__ __forceinline__ void list_finish(uint32_t* list, uint32_t i, uint32_t stride, const uint32_t* buf,
-                                            uint32_t n, uint32_t cap) {
-    if (n <= cap && (n & 7u)) list_store_chunk(list, i, n >> 3, stride, buf);
 }
 
 // One float4 of data that the step's kernels write: the read-only path, or (kCoherent) a plain load for data
@@ -138,25 +116,191 @@ __device__ __forceinline__ bool near_fast(const DevParams& P, const unsigned cha
     return any;
 }
 
-// The fluid particles within r_list of boundary particle k at the step's start, in the order of the walk
-// of pcisph.cl:212-263 with boundary_update = 1 (27 fluid buckets around the boundary particle's cell).
-__global__ void __launch_bounds__(kBlock) k_boundary_fluid_list(DevParams P, ListBuffers b) {
-    const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
-    if (k >= P.boundary_count) return;
-    const float4 xb = b.b_pos[k];
-    const Cell c = cell_of(xb.x, xb.y, xb.z, P);
-    __shared__ uint32_t staged[8 * kBlock];
-    const uint32_t stride = P.boundary_count;
-    uint32_t n = 0;
-    for_each_neighbour(b.cells, c, P, [&](uint32_t j) {
-        const float4 o = __ldg(&b.pos[j]);
-        if (dist2(xb.x - o.x, xb.y - o.y, xb.z - o.z) <= P.list_r2) {
-            if (n < P.bfl_cap) list_append(b.bfl, k, stride, staged, n, j);
-            ++n;
+// ------------------------------------------------------------------ list builders: one warp per few particles
+//
+// A warp serves W consecutive particles, cell by cell (consecutive particles mostly share one). The candidates of a
+// cell's 27 buckets, concatenated in walk order, sit in registers, 32 a round: every particle of the cell tests them
+// without loading them again, and the hits of a round are appended in walk order by ballot. Tests run with all lanes
+// busy, where a thread per particle walked with half of its lanes idle (buckets of unequal length, divergent appends),
+// and a small scene has 4 to 16 times more warps in flight. Builder per launch (CUDA events), thread per particle -> this:
+// 4,096 particles 72 -> 10 us, 32,768 96 -> 27, 156,244 138 -> 82, 1,048,576 649 -> 495, batch of 1.32M 815 -> 538;
+// the boundary's fluid lists (103,736 boundary particles) 61 -> 37. What bounds it at 1M: issue (73% of the slots; of
+// ~416 instructions a particle 145 are the tests, 90-120 the set-up of a cell's candidates, the rest the compaction
+// into the two lists); 613 instructions a particle before, with 15 of 32 lanes active.
+constexpr int kCellRounds = 10;   // candidate rounds in registers: 320, a full neighbourhood at rest density with its
+                                  // hash collisions holds ~270 (9 rounds: 508 us at 1M, more cells take two passes;
+                                  // 12: 614, fewer warps)
+constexpr int kCellBlock = 128;   // 4 warps a block, 20 resident per SM (24 spill: 501 us)
+constexpr uint32_t kAll = 0xffffffffu;
+
+// A warp's working set: the hits of one particle (index, |d|^2 bits), the cell's bucket offsets, the particles.
+template <int W>
+struct CellWarp {
+    uint2 hit[kCellRounds * 32 + 32];  // 32 entries beyond the last hit: no distance (+inf)
+    uint32_t delta[32];
+    float4 target[W];  // x, y, z, list radius^2
+};
+// The density builder also stages each particle's near list: (index, poly6 term), in walk order.
+template <int W>
+struct DensityWarp : CellWarp<W> {
+    uint2 near[W][kNearCap + 1];
+};
+
+__device__ __forceinline__ uint32_t lanes_below() {
+    uint32_t m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
+// A shared store where a <= b, predicated (a branch costs the warp a reconvergence per round).
+__device__ __forceinline__ void store_shared_le(float a, float b, uint32_t addr, uint32_t v0, uint32_t v1) {
+    asm volatile("{ .reg .pred q; setp.le.f32 q, %0, %1; @q st.shared.v2.b32 [%2], {%3, %4}; }" ::"f"(a), "f"(b),
+                 "r"(addr), "r"(v0), "r"(v1)
+                 : "memory");
+}
+
+// The candidates of one cell: the 27 buckets in the reference's walk order (grid_utils.cl:68-69), one per lane.
+// delta[k] turns a position in the concatenation into a particle index for the k-th bucket that is not empty.
+struct CellWalk {
+    uint32_t total;  // candidates of the cell
+    uint32_t off;    // where this lane's bucket begins in the concatenation (kAll: empty, or no bucket)
+    uint32_t rank;   // the last bucket begun before the next round
+};
+__device__ __forceinline__ CellWalk begin_cell(const uint2* __restrict__ cells, const DevParams& P, uint32_t cx,
+                                               uint32_t cy, uint32_t cz, uint32_t lane, uint32_t* delta) {
+    uint2 r = make_uint2(0u, 0u);
+    if (lane < 27u) {
+        const uint32_t dz = lane / 9u, dy = (lane / 3u) % 3u, dx = lane % 3u;
+        r = __ldg(&cells[P.bucket_base + hash_key(cx + dx - 1u, cy + dy - 1u, cz + dz - 1u, P)]);
+    }
+    const uint32_t len = r.y > r.x ? r.y - r.x : 0u;
+    uint32_t incl = len;
+#pragma unroll
+    for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(kAll, incl, o);
+        if (lane >= o) incl += y;
+    }
+    CellWalk w;
+    w.total = __shfl_sync(kAll, incl, 31);
+    w.rank = kAll;
+    const uint32_t filled = __ballot_sync(kAll, len != 0u);
+    w.off = len ? incl - len : kAll;
+    __syncwarp();  // the last cell's reads of delta are done
+    if (len) delta[__popc(filled & lanes_below())] = r.x - w.off;
+    __syncwarp();
+    return w;
+}
+
+// The next kCellRounds rounds of candidates from position base: index and position, NaN beyond the last (no test
+// accepts it). odd: some candidate has a coordinate that is not finite.
+struct Candidates {
+    uint32_t j[kCellRounds];
+    float x[kCellRounds], y[kCellRounds], z[kCellRounds];
+    uint32_t count;  // of these rounds
+    bool odd;
+};
+__device__ __forceinline__ void load_candidates(Candidates& c, CellWalk& w, uint32_t base, uint32_t lane,
+                                                const uint32_t* delta, const float4* __restrict__ src) {
+    const uint32_t at_or_below = 2u * lanes_below() + 1u;
+    const float nan = __uint_as_float(0x7fffffffu);
+    float zero = 0.f;  // stays 0 while every coordinate is finite
+    c.count = min(w.total - base, (uint32_t)kCellRounds * 32u);
+#pragma unroll
+    for (int u = 0; u < kCellRounds; ++u) {
+        // the buckets that begin in this round, as bits of their first position
+        const uint32_t rel = w.off - (base + u * 32u);
+        const uint32_t begun = __reduce_or_sync(kAll, rel < 32u ? 1u << rel : 0u);
+        const uint32_t f = base + u * 32u + lane;
+        const uint32_t k = w.rank + __popc(begun & at_or_below);
+        w.rank += __popc(begun);
+        c.j[u] = 0u;
+        c.x[u] = c.y[u] = c.z[u] = nan;
+        if (f < w.total) {
+            c.j[u] = f + delta[k & 31u];
+            const float4 o = __ldg(&src[c.j[u]]);
+            c.x[u] = o.x;
+            c.y[u] = o.y;
+            c.z[u] = o.z;
+            zero = __fmaf_rn(o.x, 0.f, __fmaf_rn(o.y, 0.f, __fmaf_rn(o.z, 0.f, zero)));
         }
-    });
-    list_finish(b.bfl, k, stride, staged, n, P.bfl_cap);
-    b.bfl_count[k] = n;
+    }
+    c.odd = __any_sync(kAll, !(zero == 0.f));
+}
+
+// The candidates within sqrt(q.w) of q, into hit[] in walk order; returns their number (the whole warp calls, with
+// the same q).
+__device__ __forceinline__ uint32_t collect_hits(const Candidates& c, const float4& q, uint2* hit, uint32_t lane) {
+    const uint32_t hit_addr = (uint32_t)__cvta_generic_to_shared(hit);
+    const uint32_t below = lanes_below();
+    uint32_t n = 0;
+    __syncwarp();  // the last particle's hits have been read
+#pragma unroll
+    for (int u = 0; u < kCellRounds; ++u) {
+        if (u < 6 || u * 32u < c.count) {
+            const float r2 = dist2(q.x - c.x[u], q.y - c.y[u], q.z - c.z[u]);
+            const uint32_t bits = __ballot_sync(kAll, r2 <= q.w);
+            store_shared_le(r2, q.w, hit_addr + 8u * (n + __popc(bits & below)), c.j[u], __float_as_uint(r2));
+            n += __popc(bits);
+        }
+    }
+    hit[n + lane] = make_uint2(0u, 0x7f800000u);
+    __syncwarp();
+    return n;
+}
+
+// Is the distance of q from some candidate NaN (a rare path: some candidate is not finite)?
+__device__ __forceinline__ bool nan_distance(const Candidates& c, const float4& q, uint32_t lane) {
+    bool nan = false;
+#pragma unroll
+    for (int u = 0; u < kCellRounds; ++u) {
+        const float r2 = dist2(q.x - c.x[u], q.y - c.y[u], q.z - c.z[u]);
+        nan |= u * 32u + lane < c.count && r2 != r2;
+    }
+    return __any_sync(kAll, nan);
+}
+
+// Entry s of particle i's list.
+__device__ __forceinline__ uint32_t* list_entry(uint32_t* list, uint32_t i, uint32_t s, uint32_t stride) {
+    return list + 8 * ((size_t)(s >> 3) * stride + i) + (s & 7u);
+}
+
+// The fluid particles within r_list of each boundary particle at the step's start, in the order of the walk of
+// pcisph.cl:212-263 with boundary_update = 1 (27 fluid buckets around the boundary particle's cell).
+__global__ void __launch_bounds__(kCellBlock, 5) k_boundary_fluid_list(DevParams P, ListBuffers b) {
+    constexpr int W = 8;
+    __shared__ CellWarp<W> warps[kCellBlock / 32];
+    CellWarp<W>& S = warps[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t k0 = (blockIdx.x * (kCellBlock / 32) + (threadIdx.x >> 5)) * W;
+    if (k0 >= P.boundary_count) return;
+    const uint32_t me = k0 + lane;
+    const bool own = lane < W && me < P.boundary_count;
+    const float4 xb = b.b_pos[own ? me : k0];
+    const Cell c = cell_of(xb.x, xb.y, xb.z, P);
+    if (lane < W) S.target[lane] = make_float4(xb.x, xb.y, xb.z, P.list_r2);
+    uint32_t n_own = 0;
+    uint32_t todo = __ballot_sync(kAll, own);
+    while (todo) {
+        const int lead = __ffs(todo) - 1;
+        const uint32_t cx = __shfl_sync(kAll, c.x, lead), cy = __shfl_sync(kAll, c.y, lead),
+                       cz = __shfl_sync(kAll, c.z, lead);
+        const uint32_t group = __ballot_sync(kAll, c.x == cx && c.y == cy && c.z == cz) & todo;
+        todo &= ~group;
+        CellWalk w = begin_cell(b.cells, P, cx, cy, cz, lane, S.delta);
+        for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
+            Candidates cand;
+            load_candidates(cand, w, base, lane, S.delta, b.pos);
+            for (uint32_t g = group; g; g &= g - 1u) {
+                const int t = __ffs(g) - 1;
+                const uint32_t n = collect_hits(cand, S.target[t], S.hit, lane);
+                const uint32_t n0 = __shfl_sync(kAll, n_own, t);
+                for (uint32_t k = lane; k < n; k += 32u)
+                    if (n0 + k < P.bfl_cap)
+                        __stcs(list_entry(b.bfl, k0 + t, n0 + k, P.boundary_count), S.hit[k].x);
+                if ((int)lane == t) n_own = n0 + n;
+            }
+        }
+    }
+    if (own) b.bfl_count[me] = n_own;
 }
 
 __global__ void __launch_bounds__(kBlock) k_boundary_cell_bounds(DevParams P, const float4* __restrict__ b_pos,
@@ -222,71 +366,172 @@ __global__ void __launch_bounds__(kBlock) k_boundary_pressure_list(DevParams P, 
     boundary_pressure_list_body(P, ctl, b, blockIdx.x * kBlock + threadIdx.x);
 }
 
-// pcisph.cl:65-92, and the neighbour list of the step. kBoundary: the scene has boundary particles (their
-// walk and list are compiled out otherwise: the fluid-only builder measured 5% slower with them present)
-template <class PS, bool kBoundary>
-// (at most 40 registers: 6 blocks, 48 warps per SM; 46 registers measured 5% slower at 1M)
-__global__ void __launch_bounds__(kBlock, 6) k_density_list(PS ps, ListBuffers b) {
-    const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-    if (i >= ps.count()) return;
-    const DevParams& P = ps.params(i);
-    const float4 xi = b.pos[i];  // xi.w: the particle's stored half skin
-    const Cell c = cell_of(xi.x, xi.y, xi.z, P);
-    const float sh_i = half_skin_of(P, xi.w);
-    const float list_r2 = particle_list_r2(P, sh_i), blist_r2 = boundary_list_r2(P, sh_i);
-    float acc = 0.f;
+// pcisph.cl:65-92, and the neighbour lists of the step (see the list builders above). kBoundary: the scene has boundary
+// particles (their walk is compiled out otherwise). A particle's density terms are staged in walk order and summed by
+// one lane in that order: the sum of the walk, whose other terms are zero.
+template <class PS, bool kBoundary, int W>
+__global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffers b) {
+    __shared__ DensityWarp<W> warps[kCellBlock / 32];
+    DensityWarp<W>& S = warps[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, below = lanes_below();
+    const uint32_t i0 = (blockIdx.x * (kCellBlock / 32) + (threadIdx.x >> 5)) * W;
+    const uint32_t N = ps.count();
+    if (i0 >= N) return;
+    const uint32_t me = i0 + lane;
+    const bool own = lane < W && me < N;
+    const DevParams& Pi = ps.params(own ? me : i0);
+    const float4 xi = b.pos[own ? me : i0];  // xi.w: the particle's stored half skin
+    const Cell c = cell_of(xi.x, xi.y, xi.z, Pi);
+    const float sh = half_skin_of(Pi, xi.w);
+    if (lane < W) S.target[lane] = make_float4(xi.x, xi.y, xi.z, particle_list_r2(Pi, sh));
+    const uint32_t near_addr = (uint32_t)__cvta_generic_to_shared(&S.near[0][0]);
     const uint32_t stride = b.nbr_stride;
-    // current chunk of each thread's skin and within-h lists; the boundary list's chunks go through the
-    // within-h buffer before the fluid walk starts (more shared memory would take it from the L1 cache)
-    __shared__ uint32_t staged[2][8 * kBlock];
-    uint32_t* fbuf = staged[0];
-    uint32_t* nbuf = staged[1];
-    if (kBoundary && P.boundary_count && b.b_zone && !in_boundary_zone(b, c)) {
-        b.b_near[i] = 0;  // every boundary particle is at least 2h away
-        if (b.bnbr) b.bnbr_count[i] = 0;
-    } else if (kBoundary && P.boundary_count) {
-        // boundary particles within r_list, in walk order: the later sweeps read them from the boundary list
-        // (all of them, or walk the boundary buckets when there are more than bnd_cap)
-        uint32_t nb = 0;
-        uint32_t* bbuf = staged[1];
-        for_each_neighbour(b.b_cells, c, P, [&](uint32_t j) {
-            const float4 o = __ldg(&b.b_pos[j]);
-            const float r2 = dist2(xi.x - o.x, xi.y - o.y, xi.z - o.z);
-            acc += poly6(r2, P.h2);  // density_term's expression
-            if (r2 <= blist_r2) {
-                if (b.bnbr && nb < P.bnd_cap) list_append(b.bnbr, i, stride, bbuf, nb, j);
-                ++nb;
+    // lane t < W: particle i0 + t's list lengths, the terms staged for it, their sum so far
+    uint32_t n_own = 0, near_own = 0, staged = 0;
+    float acc = 0.f;
+    bool nan_own = false;  // some pair distance is NaN: so is the sum
+    // where this lane stores the first of 32 entries of the skin list of particle i0
+    uint32_t* const out0 = list_entry(b.nbr, i0, lane, stride);
+    const size_t out_step = 32 * (size_t)stride;
+    auto flush = [&](int t, uint32_t count) {
+        __syncwarp();
+        if ((int)lane == t)
+            for (uint32_t k = 0; k < count; ++k) acc += __uint_as_float(S.near[t][k].y);
+        __syncwarp();
+    };
+    uint32_t todo = __ballot_sync(kAll, own);
+    while (todo) {
+        const int lead = __ffs(todo) - 1;
+        const DevParams& P = ps.params(i0 + lead);  // the same scene for the whole group: buckets do not overlap
+        const uint32_t cx = __shfl_sync(kAll, c.x, lead), cy = __shfl_sync(kAll, c.y, lead),
+                       cz = __shfl_sync(kAll, c.z, lead);
+        bool same = c.x == cx && c.y == cy && c.z == cz;
+        if (PS::kBatched) same = same && Pi.bucket_base == P.bucket_base;
+        const uint32_t group = __ballot_sync(kAll, same) & todo;
+        todo &= ~group;
+        const float near_r2 = P.near_r2, h2 = P.h2;
+        if (kBoundary && P.boundary_count) {
+            // boundary particles within r_list, in walk order: the later sweeps read them from the boundary list
+            // (all of them, or walk the boundary buckets when there are more than bnd_cap); a cell outside the
+            // boundary zone has every boundary particle at least 2h away
+            const bool in_zone = !b.b_zone || in_boundary_zone(b, Cell{cx, cy, cz});
+            uint32_t nb_own = 0;
+            if (in_zone) {
+                CellWalk w = begin_cell(b.b_cells, P, cx, cy, cz, lane, S.delta);
+                for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
+                    Candidates cand;
+                    load_candidates(cand, w, base, lane, S.delta, b.b_pos);
+                    for (uint32_t g = group; g; g &= g - 1u) {
+                        const int t = __ffs(g) - 1;
+                        float4 q = S.target[t];
+                        q.w = boundary_list_r2(P, __shfl_sync(kAll, sh, t));
+                        if (cand.odd) nan_own |= nan_distance(cand, q, lane) && (int)lane == t;
+                        const uint32_t n = collect_hits(cand, q, S.hit, lane);
+                        const uint32_t n0 = __shfl_sync(kAll, nb_own, t);
+                        uint32_t cnt = __shfl_sync(kAll, staged, t);
+                        for (uint32_t k0 = 0; k0 < n; k0 += 32u) {
+                            const uint32_t k = k0 + lane;
+                            const uint2 e = S.hit[k];
+                            const float r2 = __uint_as_float(e.y);
+                            if (b.bnbr && k < n && n0 + k < P.bnd_cap)
+                                __stcs(list_entry(b.bnbr, i0 + t, n0 + k, stride), e.x);
+                            const uint32_t bits = __ballot_sync(kAll, r2 <= h2);
+                            if (cnt + __popc(bits) > kNearCap) {
+                                flush(t, cnt);
+                                cnt = 0;
+                            }
+                            store_shared_le(r2, h2, near_addr + 8u * (t * (kNearCap + 1u) + cnt + __popc(bits & below)),
+                                            e.x, __float_as_uint(poly6(r2, h2)));
+                            cnt += __popc(bits);
+                        }
+                        if ((int)lane == t) {
+                            nb_own = n0 + n;
+                            staged = cnt;
+                        }
+                    }
+                }
+                for (uint32_t g = group; g; g &= g - 1u) {  // the staging area is for the fluid's near list from here
+                    const int t = __ffs(g) - 1;
+                    flush(t, __shfl_sync(kAll, staged, t));
+                    if ((int)lane == t) staged = 0;
+                }
             }
-        });
-        b.b_near[i] = nb ? 1 : 0;
-        if (b.bnbr) {
-            list_finish(b.bnbr, i, stride, bbuf, nb, P.bnd_cap);
-            b.bnbr_count[i] = nb;
+            if ((group >> lane) & 1u) {
+                b.b_near[me] = nb_own ? 1 : 0;
+                if (b.bnbr) b.bnbr_count[me] = nb_own;
+            }
+        }
+        CellWalk w = begin_cell(b.cells, P, cx, cy, cz, lane, S.delta);
+        for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
+            Candidates cand;
+            load_candidates(cand, w, base, lane, S.delta, b.pos);
+            for (uint32_t g = group; g; g &= g - 1u) {
+                const int t = __ffs(g) - 1;
+                const float4 q = S.target[t];
+                if (cand.odd) nan_own |= nan_distance(cand, q, lane) && (int)lane == t;
+                const uint32_t n = collect_hits(cand, q, S.hit, lane);
+                const uint32_t n0 = __shfl_sync(kAll, n_own, t);
+                uint32_t cnt = __shfl_sync(kAll, staged, t);
+                if (n0 != 0u)  // a cell of more than kCellRounds rounds: the list goes on
+                    for (uint32_t k = lane; k < n; k += 32u)
+                        if (n0 + k < P.list_cap) __stcs(list_entry(b.nbr, i0 + t, n0 + k, stride), S.hit[k].x);
+                const uint32_t stored = n0 == 0u ? min(n, P.list_cap) : 0u;
+                uint32_t* out = out0 + 8 * t;
+                const uint32_t stage_addr = near_addr + 8u * t * (kNearCap + 1u);
+                for (uint32_t k0 = 0; k0 < n; k0 += 32u) {
+                    const uint2 e = S.hit[k0 + lane];
+                    const float r2 = __uint_as_float(e.y);
+                    if (k0 + lane < stored) __stcs(out, e.x);
+                    out += out_step;
+                    const uint32_t bits = __ballot_sync(kAll, r2 <= near_r2);
+                    const uint32_t more = __popc(bits);
+                    if (cnt + more > kNearCap) {
+                        flush(t, cnt);
+                        if ((int)lane == t) near_own += cnt;
+                        cnt = 0;
+                    }
+                    const float dr = fmaxf(h2 - r2, 0.f);  // poly6 of a finite |d|^2
+                    store_shared_le(r2, near_r2, stage_addr + 8u * (cnt + __popc(bits & below)), e.x,
+                                    __float_as_uint(dr * dr * dr));
+                    cnt += more;
+                }
+                if ((int)lane == t) {
+                    n_own = n0 + n;  // > list_cap: this particle walks the buckets in the pressure sweeps
+                    staged = cnt;
+                }
+            }
         }
     }
-    uint32_t n = 0, nn = 0;
-    auto load = [&](uint32_t j) { return __ldg(&b.pos[j]); };
-    auto use = [&](uint32_t j, const float4& o) {
-        const float dx = xi.x - o.x, dy = xi.y - o.y, dz = xi.z - o.z;
-        const float r2 = dist2(dx, dy, dz);
-        acc += poly6(r2, P.h2);
-        if (r2 <= list_r2) {
-            if (n < P.list_cap) list_append(b.nbr, i, stride, fbuf, n, j);
-            ++n;
-            if (r2 <= P.near_r2) {
-                if (nn < P.near_cap) list_append(b.near, i, stride, nbuf, nn, j);
-                ++nn;
-            }
-        }
-    };
-    for_each_neighbour_prefetched(b.cells, c, P, load, use);
-    list_finish(b.nbr, i, stride, fbuf, n, P.list_cap);
-    list_finish(b.near, i, stride, nbuf, nn, P.near_cap);
-    b.nbr_count[i] = n;  // n > list_cap: this particle walks the buckets in the pressure sweeps
-    b.near_count[i] = nn;  // nn > near_cap: it walks them in the sweeps at the current positions
-    acc *= P.particle_mass * P.poly6_norm;
-    b.rho[i] = acc;
-    b.pr4[i] = make_float4(xi.x, xi.y, xi.z, acc);
+    near_own += staged;  // > near_cap: this particle walks the buckets in the sweeps at the current positions
+    __syncwarp();
+    if (own) {
+        for (uint32_t k = 0; k < staged; ++k) acc += __uint_as_float(S.near[lane][k].y);
+        if (nan_own) acc = __uint_as_float(0x7fffffffu);
+        b.nbr_count[me] = n_own;
+        b.near_count[me] = near_own;
+        acc *= Pi.particle_mass * Pi.poly6_norm;
+        b.rho[me] = acc;
+        b.pr4[me] = make_float4(xi.x, xi.y, xi.z, acc);
+    }
+    // the near lists, chunk by chunk: the W particles' chunks are contiguous. A list that outran the staging area
+    // (near_cap entries) is not read.
+    const uint32_t longest = __reduce_max_sync(kAll, near_own <= kNearCap ? near_own : 0u);
+    constexpr int kParts = (8 * W + 31) / 32;
+    uint32_t len[kParts];
+#pragma unroll
+    for (int h = 0; h < kParts; ++h) {
+        const uint32_t t = 4u * h + (lane >> 3);
+        const uint32_t nn = __shfl_sync(kAll, near_own, t & 31u);
+        len[h] = t < W && nn <= kNearCap ? nn : 0u;
+    }
+    uint32_t* out = b.near + 8 * (size_t)i0 + lane;
+    for (uint32_t k = 0; k < longest; k += 8u) {
+        const uint32_t e = k + (lane & 7u);
+#pragma unroll
+        for (int h = 0; h < kParts; ++h)
+            if (e < len[h]) __stcs(out + 32 * h, S.near[4 * h + (lane >> 3)][e].x);
+        out += 8 * (size_t)stride;
+    }
 }
 
 // pcisph.cl:94-112
@@ -745,9 +990,33 @@ __global__ void __launch_bounds__(kBlock) k_hash_scenes(SceneTable ps, const flo
 
 }  // namespace
 
+namespace {
+inline unsigned grid_cells(uint32_t n, int w) {
+    const uint32_t per = (kCellBlock / 32) * (uint32_t)w;
+    return (n + per - 1) / per;
+}
+template <class PS>
+void launch_density(const PS& ps, uint32_t n, bool boundary, const ListBuffers& b, cudaStream_t s) {
+    auto go = [&](auto w) {
+        constexpr int W = decltype(w)::value;
+        if constexpr (!PS::kBatched)
+            if (boundary) {
+                k_density_list<PS, true, W><<<grid_cells(n, W), kCellBlock, 0, s>>>(ps, b);
+                return;
+            }
+        k_density_list<PS, false, W><<<grid_cells(n, W), kCellBlock, 0, s>>>(ps, b);
+    };
+    // Fewer particles per warp where warps are few: with 8 / 4 / 2 a warp 32,768 particles take 28 / 27 / 32 us (4,096:
+    // 12 with 8, 10 with 2); from there on the set-up of a cell per warp costs more than it spreads (156,244 particles
+    // 82 / 95 / 129 us, 1,048,576 495 / 605 / 845).
+    if (n <= 8192u) go(std::integral_constant<int, 2>{});
+    else if (n <= 49152u) go(std::integral_constant<int, 4>{});
+    else go(std::integral_constant<int, 8>{});
+}
+}  // namespace
+
 void launch_density_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
-    if (P.boundary_count) k_density_list<OneScene, true><<<grid_for(P.fluid_count), kBlock, 0, s>>>(OneScene{P, ctl}, b);
-    else k_density_list<OneScene, false><<<grid_for(P.fluid_count), kBlock, 0, s>>>(OneScene{P, ctl}, b);
+    launch_density(OneScene{P, ctl}, P.fluid_count, P.boundary_count != 0, b, s);
 }
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     k_normal_list<<<grid_for(P.fluid_count), kBlock, 0, s>>>(OneScene{P, ctl}, b);
@@ -818,7 +1087,7 @@ void launch_boundary_zone(const DevParams& P, const float4* b_pos, const int* or
                                                                       dim[1], zone);
 }
 void launch_boundary_fluid_list(const DevParams& P, const ListBuffers& b, cudaStream_t s) {
-    if (P.boundary_count) k_boundary_fluid_list<<<grid_for(P.boundary_count), kBlock, 0, s>>>(P, b);
+    if (P.boundary_count) k_boundary_fluid_list<<<grid_cells(P.boundary_count, 8), kCellBlock, 0, s>>>(P, b);
 }
 void launch_boundary_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     if (P.boundary_count) k_boundary_pressure_list<<<grid_for(P.boundary_count), kBlock, 0, s>>>(P, ctl, b);
@@ -833,7 +1102,7 @@ void launch_hash_scenes(const SceneTable& t, const float4* pos, uint32_t* keys, 
     if (t.n) k_hash_scenes<<<grid_for(t.n), kBlock, 0, s>>>(t, pos, keys);
 }
 void launch_density_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s) {
-    if (t.n) k_density_list<SceneTable, false><<<grid_for(t.n), kBlock, 0, s>>>(t, b);  // no boundary in a batch
+    if (t.n) launch_density(t, t.n, false, b, s);  // no boundary in a batch
 }
 void launch_normal_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s) {
     if (t.n) k_normal_list<<<grid_for(t.n), kBlock, 0, s>>>(t, b);

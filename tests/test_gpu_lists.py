@@ -1,0 +1,71 @@
+"""GPU: the neighbour-list builder at the edges of its work split (particles per warp, candidate rounds, list and staging
+capacities), against the oracle and against the plain walk of the buckets (kernel variant 1)."""
+import numpy as np
+import pytest
+
+from gpu_util import RTOL, assert_close, fluid_like
+
+pytestmark = pytest.mark.gpu
+
+D = 0.02  # lattice spacing: h = 2 D, 8 particles a cell at rest
+
+
+def _cloud(n, per_cell, seed):
+    """n particles at uniform random places of a cube that holds per_cell of them per cell of size h."""
+    side = 2 * D * (n / per_cell) ** (1 / 3)
+    return (np.random.default_rng(seed).random((n, 3)) * side).astype(np.float32)
+
+
+# sizes around the particles of a warp and of a block for each of the three splits (2, 4 and 8 particles a warp: up to
+# 8,192, up to 49,152, beyond), and dense clouds: more candidates than the 320 of one pass, more neighbours than the
+# near list (64), the skin list (96) and the staging area hold
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("n,per_cell", [(1, 8), (2, 8), (7, 8), (9, 8), (33, 20), (1000, 40), (700, 300), (2000, 600),
+                                        (8191, 8), (8192, 8), (8193, 8), (49152, 8), (49153, 10), (60001, 8)])
+def test_lists_hold_the_walks_neighbours(oracle, n, per_cell, order):
+    pos = _cloud(n, per_cell, seed=n)
+    p = oracle.derive_params(0.5 * D, 1000.0, n, 0, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    got = {}
+    for variant in (2, 1):
+        f = fluid_like(p, kernel_variant=variant, spatial_order=order)
+        f.set_fluid_state(pos)
+        f.run_stage("sort")
+        f.run_stage("density")
+        f.run_stage("normal")
+        f.run_stage("force")
+        f.set_field("predicted_position", f.get_field("sorted_position"))
+        f.run_stage("pressure")
+        f.run_stage("pressure_force", 0)
+        got[variant] = {k: f.get_field(k) for k in ("density", "normal", "other_force", "density_variation",
+                                                    "pressure_force", "sorted_position", "cell_offsets")}
+        f.close()
+    a, w = got[2], got[1]
+    off = a["cell_offsets"].astype(np.int64).reshape(-1, 2)
+    rho = oracle.update_density(p, None, None, a["cell_offsets"], a["sorted_position"])
+    # sums of up to K terms in FP32, each side rounded on its own: 2 K ulp of the sum of the terms' magnitudes
+    k = min(n, 27 * int((off[:, 1] - off[:, 0]).max()))
+    tol = max(RTOL, 2 * k * 2.0 ** -24)
+    assert_close("density", a["density"], rho, rtol=tol)
+    assert_close("density_variation", a["density_variation"], np.maximum(rho - 1000.0, 0), scale=float(rho.max()), rtol=tol)
+    for name in ("density", "normal", "other_force", "pressure_force"):
+        assert_close(name, a[name], w[name], rtol=tol)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("n", [64, 9000])
+def test_nonfinite_particles_reach_the_same_sums(oracle, n, value):
+    pos = _cloud(n, 8, seed=3)
+    pos[n // 3, 1] = value
+    pos[n // 2] = value
+    p = oracle.derive_params(0.5 * D, 1000.0, n, 0, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    rho = []
+    for variant in (2, 1):
+        f = fluid_like(p, kernel_variant=variant, spatial_order=0)
+        f.set_fluid_state(pos)
+        f.run_stage("sort")
+        f.run_stage("density")
+        rho.append(f.get_field("density"))
+        f.close()
+    np.testing.assert_array_equal(np.isnan(rho[0]), np.isnan(rho[1]))
+    ok = ~np.isnan(rho[1])
+    assert_close("density", rho[0][ok], rho[1][ok])
