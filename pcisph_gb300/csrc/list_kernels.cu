@@ -93,6 +93,107 @@ __device__ __forceinline__ void for_each_listed(const uint32_t* __restrict__ lis
     }
 }
 
+// The same with the gathers of U chunks in flight before their first use (load(j), then use(value) in list order): for
+// scenes of few warps, where nothing else covers a gather's latency.
+template <int U, class Load, class Use>
+__device__ __forceinline__ void for_each_listed_deep(const uint32_t* __restrict__ list, uint32_t i, uint32_t n,
+                                                     uint32_t stride, Load&& load, Use&& use) {
+    const uint4* p = list_chunk(const_cast<uint32_t*>(list), i, 0, stride);
+    const size_t step = 2 * (size_t)stride;
+    uint32_t j[8 * U];
+    auto fetch = [&](uint32_t e) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (e + 8u * u < n) {
+                const uint4 a = __ldcs(p + u * step), b = __ldcs(p + u * step + 1);
+                j[8 * u] = a.x, j[8 * u + 1] = a.y, j[8 * u + 2] = a.z, j[8 * u + 3] = a.w;
+                j[8 * u + 4] = b.x, j[8 * u + 5] = b.y, j[8 * u + 6] = b.z, j[8 * u + 7] = b.w;
+            }
+        p += U * step;
+    };
+    fetch(0u);
+#pragma unroll 1
+    for (uint32_t e = 0; e < n; e += 8u * U) {
+        decltype(load(0u)) o[8 * U];
+#pragma unroll
+        for (uint32_t k = 0; k < 8u * U; ++k)
+            if (e + k < n) o[k] = load(j[k]);
+        fetch(e + 8u * U);
+#pragma unroll
+        for (uint32_t k = 0; k < 8u * U; ++k)
+            if (e + k < n) use(o[k]);
+    }
+}
+
+// ------------------------------------------------------------------ small scenes: eight lanes per particle
+//
+// A scene that fills less than a wave of threads is bound by each thread's chain of loads and sums (15 us a sweep from
+// 4,096 to 32,768 particles). There eight lanes share a particle: lane q takes entry 8c + q of chunk c, so a chunk is one
+// gather per lane instead of eight in a row, and the entries' terms are then summed in list order (the sum of the
+// one-lane sweep: entries that contribute nothing add zero).
+
+// The entries of this lane, chunk by chunk, in batches of U chunks whose gathers are in flight together: load(j) for
+// the lane's entry, then sum(value, valid) once per chunk by the whole warp. n: this particle's entries; most: the
+// warp's largest n.
+template <int L, int U, class Load, class Sum>
+__device__ __forceinline__ void for_each_shared(const uint32_t* __restrict__ list, uint32_t i, uint32_t n, uint32_t most,
+                                                uint32_t stride, uint32_t q, Load&& load, Sum&& sum) {
+    const uint32_t* p = list + 8 * (size_t)i;
+    auto entry = [&](uint32_t e) { return __ldcs(p + (e >> 3) * (8 * (size_t)stride) + (e & 7u)); };
+    uint32_t j[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) j[u] = q + L * u < n ? entry(q + L * u) : 0u;
+#pragma unroll 1
+    for (uint32_t e = q; e - q < most; e += L * U) {
+        decltype(load(0u)) o[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (e + L * u < n) o[u] = load(j[u]);
+#pragma unroll
+        for (int u = 0; u < U; ++u) j[u] = e + L * (U + u) < n ? entry(e + L * (U + u)) : 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (e - q + L * u < most) sum(o[u], e + L * u < n);
+    }
+}
+
+// The lane's candidates of a walk over the buckets around c, eight at a time: use(j, valid) by the eight lanes (mask).
+template <int L, class Use>
+__device__ __forceinline__ void walk_shared(const uint2* __restrict__ cells, const Cell& c, const DevParams& P, uint32_t q,
+                                            Use&& use) {
+    for_each_bucket(cells, c, P, [&](uint2 r) {
+        for (uint32_t j = r.x; j < r.y; j += L) use(j + q, j + q < r.y);
+    });
+}
+
+// The L lanes that share this lane's particle.
+template <int L>
+__device__ __forceinline__ uint32_t lanes_mask() {
+    return ((1u << L) - 1u) << (threadIdx.x & 31u & ~(L - 1u));
+}
+
+// acc plus the L lanes' terms in lane order.
+template <int L>
+__device__ __forceinline__ void add_lanes(float& acc, float term, uint32_t mask) {
+#pragma unroll
+    for (int k = 0; k < L; ++k) acc += __shfl_sync(mask, term, k, L);
+}
+
+// Vector terms of eight lanes, summed in lane order, one component per lane: lane q < 3 holds component q of the sum.
+template <int L>
+struct TermStage {
+    float4 t[L];
+};
+template <int L>
+__device__ __forceinline__ void add_lanes(float& acc, const PairTerm& term, TermStage<L>& s, uint32_t q, uint32_t mask) {
+    s.t[q] = make_float4(term.x, term.y, term.z, term.k);
+    __syncwarp(mask);
+    const float* v = reinterpret_cast<const float*>(s.t) + (q < 3u ? q : 0u);
+#pragma unroll
+    for (int k = 0; k < L; ++k) acc = __fmaf_rn(v[4 * k], s.t[k].w, acc);
+    __syncwarp(mask);
+}
+
 // Does any of the 27 buckets around c hold a fast particle this step?
 __device__ __forceinline__ bool near_fast(const DevParams& P, const unsigned char* __restrict__ bucket_fast,
                                           const Cell& c) {
@@ -535,7 +636,7 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
 }
 
 // pcisph.cl:94-112
-template <class PS>
+template <class PS, int DEEP = 1>
 __global__ void __launch_bounds__(kBlock) k_normal_list(PS ps, ListBuffers b) {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= ps.count()) return;
@@ -544,13 +645,38 @@ __global__ void __launch_bounds__(kBlock) k_normal_list(PS ps, ListBuffers b) {
     float3 n = make_float3(0.f, 0.f, 0.f);
     const uint32_t cnt = b.near_count[i];
     auto f = [&](uint32_t j) { normal_term(xi.x, xi.y, xi.z, __ldg(&b.pr4[j]), P.h2, n); };
-    if (cnt <= P.near_cap) for_each_listed(b.near, i, cnt, b.nbr_stride, f);
-    else for_each_neighbour(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, f);
+    if (cnt > P.near_cap)
+        for_each_neighbour(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, f);
+    else if constexpr (DEEP > 1)
+        for_each_listed_deep<DEEP>(
+            b.near, i, cnt, b.nbr_stride, [&](uint32_t j) { return __ldg(&b.pr4[j]); },
+            [&](const float4& o) { normal_term(xi.x, xi.y, xi.z, o, P.h2, n); });
+    else
+        for_each_listed(b.near, i, cnt, b.nbr_stride, f);
     const float scale = P.h * P.particle_mass * P.poly6_d1_norm;
     b.normal[i] = make_float4(n.x * scale, n.y * scale, n.z * scale, 0.f);
 }
 
-// pcisph.cl:121-173, then the first predict (pcisph.cl:175-193, F_p = 0)
+// The force sweep's epilogue from its three sums, and the first predict (pcisph.cl:175-193, F_p = 0).
+template <class PS>
+__device__ __forceinline__ void finish_force(const PS& ps, const ListBuffers& b, const DevParams& P, uint32_t i,
+                                             const float4& xi, const float3& vi, const float3& visc, const float3& coh,
+                                             const float3& curv) {
+    const float m = P.particle_mass;
+    const float3 fo = other_force(m, P.gravity, visc, P.viscosity * m * P.visc_d2_norm, coh,
+                                  -P.st_coeff * m * m * P.st_norm, curv, -P.st_coeff * m);
+    b.f_other[i] = f4(fo, 0.f);
+    b.press[i] = 0.f;
+    const float3 v = vi + (fo / m) * P.dt;
+    const float3 dx = v * P.dt;
+    const float4 xs = make_float4(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z, 0.f);
+    b.pred[i] = xs;
+    const float disp = note_displacement(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin,
+                                         PS::kBatched ? nullptr : b.fast_list, i);
+    if (P.particle_skin) b.disp_max[i] = disp;
+}
+
+// pcisph.cl:121-173, then the first predict
 template <class PS>
 __global__ void __launch_bounds__(kBlock) k_force_list(PS ps, ListBuffers b) {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
@@ -566,18 +692,89 @@ __global__ void __launch_bounds__(kBlock) k_force_list(PS ps, ListBuffers b) {
     };
     if (cnt <= P.near_cap) for_each_listed(b.near, i, cnt, b.nbr_stride, f);
     else for_each_neighbour(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, f);
-    const float m = P.particle_mass;
-    const float3 fo = other_force(m, P.gravity, fa.visc, P.viscosity * m * P.visc_d2_norm, fa.coh,
-                                  -P.st_coeff * m * m * P.st_norm, fa.curv, -P.st_coeff * m);
-    b.f_other[i] = f4(fo, 0.f);
-    b.press[i] = 0.f;
-    const float3 v = vi + (fo / m) * P.dt;
-    const float3 dx = v * P.dt;
-    const float4 xs = make_float4(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z, 0.f);
-    b.pred[i] = xs;
-    const float disp = note_displacement(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin,
-                                         PS::kBatched ? nullptr : b.fast_list, i);
-    if (P.particle_skin) b.disp_max[i] = disp;
+    finish_force(ps, b, P, i, xi, vi, fa.visc, fa.coh, fa.curv);
+}
+
+// The same two sweeps with eight lanes per particle (small scenes).
+template <class PS, int L>
+__global__ void __launch_bounds__(kBlock) k_normal_shared(PS ps, ListBuffers b) {
+    const uint32_t t = blockIdx.x * kBlock + threadIdx.x, i0 = t / L, q = t % L;
+    __shared__ TermStage<L> stage[kBlock / L];
+    TermStage<L>& S = stage[threadIdx.x / L];
+    const bool live = i0 < ps.count();
+    const uint32_t i = live ? i0 : ps.count() - 1u;
+    const DevParams& P = ps.params(i);
+    const uint32_t mask = lanes_mask<L>();
+    const float4 xi = b.pr4[i];
+    const uint32_t cnt = b.near_count[i];
+    const bool listed = cnt <= P.near_cap;
+    const uint32_t n = listed ? cnt : 0u;
+    float acc = 0.f;  // lane 0, 1, 2: x, y, z
+    auto sum = [&](const float4& o, bool valid, uint32_t m) {
+        PairTerm term{0.f, 0.f, 0.f, 0.f};
+        if (valid) normal_pair(xi.x, xi.y, xi.z, o, P.h2, [&](const PairTerm& p) { term = p; });
+        add_lanes(acc, term, S, q, m);
+    };
+    for_each_shared<L, 32 / L>(
+        b.near, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.pr4[j]); },
+        [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+    if (!listed)
+        walk_shared<L>(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, q, [&](uint32_t j, bool valid) {
+            float4 o = xi;
+            if (valid) o = __ldg(&b.pr4[j]);
+            sum(o, valid, mask);
+        });
+    acc *= P.h * P.particle_mass * P.poly6_d1_norm;
+    const float y = __shfl_sync(mask, acc, 1, L), z = __shfl_sync(mask, acc, 2, L);
+    if (live && q == 0) b.normal[i] = make_float4(acc, y, z, 0.f);
+}
+
+template <class PS, int L>
+__global__ void __launch_bounds__(kBlock) k_force_shared(PS ps, ListBuffers b) {
+    const uint32_t t = blockIdx.x * kBlock + threadIdx.x, i0 = t / L, q = t % L;
+    __shared__ TermStage<L> stage[kBlock / L];
+    TermStage<L>& S = stage[threadIdx.x / L];
+    const bool live = i0 < ps.count();
+    const uint32_t i = live ? i0 : ps.count() - 1u;
+    const DevParams& P = ps.params(i);
+    const uint32_t mask = lanes_mask<L>();
+    const float4 xi = b.pr4[i];
+    const float3 vi = f3(b.vel[i]), ni = f3(b.normal[i]);
+    const uint32_t cnt = b.near_count[i];
+    const bool listed = cnt <= P.near_cap;
+    const uint32_t n = listed ? cnt : 0u;
+    float visc = 0.f, coh = 0.f, curv = 0.f;  // lane 0, 1, 2: x, y, z
+    struct ForceOperand {
+        float4 x, v, n;
+    };
+    auto load = [&](uint32_t j) { return ForceOperand{__ldg(&b.pr4[j]), __ldg(&b.vel[j]), __ldg(&b.normal[j])}; };
+    auto sum = [&](const ForceOperand& o, bool valid, uint32_t m) {
+        const PairTerm none{0.f, 0.f, 0.f, 0.f};
+        PairTerm a = none, c = none, d = none;
+        if (valid)
+            force_pair(
+                xi, vi, ni, o.x, f3(o.v), f3(o.n), P, [&](const PairTerm& p) { a = p; },
+                [&](const PairTerm& p, const PairTerm& r) {
+                    c = p;
+                    d = r;
+                });
+        add_lanes(visc, a, S, q, m);
+        add_lanes(coh, c, S, q, m);
+        add_lanes(curv, d, S, q, m);
+    };
+    for_each_shared<L, 16 / L>(b.near, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, load,
+                       [&](const ForceOperand& o, bool valid) { sum(o, valid, kAll); });
+    if (!listed)
+        walk_shared<L>(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, q, [&](uint32_t j, bool valid) {
+            ForceOperand o{xi, xi, xi};
+            if (valid) o = load(j);
+            sum(o, valid, mask);
+        });
+    auto all = [&](float v) {
+        return make_float3(__shfl_sync(mask, v, 0, L), __shfl_sync(mask, v, 1, L), __shfl_sync(mask, v, 2, L));
+    };
+    const float3 sv = all(visc), sc = all(coh), su = all(curv);
+    if (live && q == 0) finish_force(ps, b, P, i, xi, vi, sv, sc, su);
 }
 
 // Partner marks after a prediction round (one scene). A pair of the reference's walk whose predictions are
@@ -644,6 +841,81 @@ __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Con
 }
 
 // pcisph.cl:212-263 (boundary_update = 0); one scene: also the stop decision in the last block
+
+// How one particle's pressure sweep finds its neighbours.
+struct PressurePlan {
+    uint32_t cnt, bcnt;              // entries of its skin list and of its boundary list
+    bool walk;                       // the fluid buckets instead of the skin list
+    bool walk_boundary, list_boundary;
+    Cell c;                          // set where it walks
+};
+template <class PS>
+__device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBuffers& b, const DevParams& P,
+                                                      const Control* ctl, uint32_t i, const float4& xi,
+                                                      const float4& xp) {
+    PressurePlan p;
+    // no particle of the scene moved more than half the skin: its lists are complete for x*
+    const bool all_lists_ok = ctl->fast_particles == ctl->fast_at_begin;
+    p.cnt = b.nbr_count[i];
+    const bool overflow = p.cnt > P.list_cap;
+    // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
+    // skin) may miss a pair: with per-particle skins it walks. Boundary terms: all zero unless a boundary
+    // particle was within r_list of x, or x* moved past the half skin (boundary particles do not move);
+    // within it, the boundary list (every boundary particle within r_list of x) holds every one that can
+    // be within h of x*.
+    bool self_fast = false;
+    if (P.particle_skin || P.boundary_count) {
+        const float dx = xp.x - xi.x, dy = xp.y - xi.y, dz = xp.z - xi.z;
+        self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w));
+    }
+    p.walk_boundary = p.list_boundary = false;
+    p.bcnt = 0;
+    if (P.boundary_count) {
+        if (self_fast) {
+            p.walk_boundary = true;
+        } else if (b.b_near[i] != 0) {
+            if (b.bnbr) p.bcnt = b.bnbr_count[i];
+            p.list_boundary = b.bnbr && p.bcnt <= P.bnd_cap;
+            p.walk_boundary = !p.list_boundary;
+        }
+    }
+    p.c = Cell{0u, 0u, 0u};  // the cell (three IEEE divisions) only where a walk may need it
+    const bool own_walk = overflow || (P.particle_skin && self_fast);
+    // partner marks of this round (one scene, after the marking kernel): the particles that may miss a
+    // pair of their walk are stamped with the round's number; a round past the cap (or no marks) takes
+    // the bucket flags: every particle near a fast one walks
+    const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
+    const bool marks = fast_round <= P.mark_cap;
+    if (marks) {
+        p.walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
+        if (p.walk || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
+    } else {
+        if (own_walk || !all_lists_ok || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
+        p.walk = own_walk || (!all_lists_ok && near_fast(P, b.bucket_fast, p.c));
+    }
+    return p;
+}
+
+// From a particle's density sum: its density variation (returned), pressure and packed operand.
+template <class PS>
+__device__ __forceinline__ float finish_pressure(const ListBuffers& b, const DevParams& P, Control* ctl, uint32_t i,
+                                                 const float4& xi, float acc) {
+    acc *= P.particle_mass * P.poly6_norm;
+    if (!isfinite(acc)) atomicOr(&ctl->status, 2u);
+    float dv = acc - P.rest_density;
+    dv = 0.f < dv ? dv : 0.f;
+    b.err[i] = dv;
+    float p = b.press[i];
+    if (dv != 0.f) {
+        p += dv * P.delta;
+        b.press[i] = p;
+    }
+    const float r = b.rho[i];
+    b.pf4[i] = make_float4(xi.x, xi.y, xi.z, p / (r * r));
+    if (PS::kBatched) warp_atomic_max(&ctl->max_err_bits, __float_as_uint(dv));
+    return dv;
+}
+
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range).
 template <class PS, bool kCoherent = false>
 __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i) {
@@ -728,10 +1000,53 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
     return dv;
 }
 
+// The same with eight lanes per particle, lane q; returned to each of them.
+template <class PS, int L>
+__device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers& b, uint32_t i0, uint32_t q) {
+    const bool live = i0 < ps.count() && !ps.skip_pressure(i0);
+    const uint32_t i = i0 < ps.count() ? i0 : ps.count() - 1u;
+    const uint32_t mask = lanes_mask<L>();
+    const DevParams& P = ps.params(i);
+    Control* ctl = ps.control(i);
+    const float4 xi = b.pos[i];
+    const float4 xp = b.pred[i];
+    PressurePlan p{};
+    if (live) p = plan_pressure(ps, b, P, ctl, i, xi, xp);
+    float acc = 0.f;
+    auto sum = [&](const float4& o, bool valid, uint32_t m) {
+        add_lanes<L>(acc, valid ? density_term(xp.x, xp.y, xp.z, o, P.h2) : 0.f, m);
+    };
+    auto walk = [&](const uint2* cells, const float4* src) {
+        walk_shared<L>(cells, p.c, P, q, [&](uint32_t j, bool valid) {
+            float4 o = xp;
+            if (valid) o = __ldg(&src[j]);
+            sum(o, valid, mask);
+        });
+    };
+    if (P.boundary_count) {
+        const uint32_t n = p.list_boundary ? p.bcnt : 0u;
+        for_each_shared<L, 32 / L>(
+            b.bnbr, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.b_pos[j]); },
+            [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+        if (p.walk_boundary) walk(b.b_cells, b.b_pos);
+    }
+    const uint32_t n = live && !p.walk ? p.cnt : 0u;
+    for_each_shared<L, 32 / L>(
+        b.nbr, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.pred[j]); },
+        [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+    if (p.walk) walk(b.cells, b.pred);
+    float dv = 0.f;
+    if (live && q == 0) dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
+    return dv;
+}
+
 // BS: threads per block (128, 256 or 512; the autotuner's choice for one scene)
-template <class PS, int BS = kBlock>
+template <class PS, int BS = kBlock, int LANES = 1>
 __global__ void __launch_bounds__(BS) k_pressure_list(PS ps, ListBuffers b) {
-    const float dv = pressure_body(ps, b, blockIdx.x * BS + threadIdx.x);
+    const uint32_t t = blockIdx.x * BS + threadIdx.x;
+    float dv;
+    if constexpr (LANES == 1) dv = pressure_body(ps, b, t);
+    else dv = pressure_shared<PS, LANES>(ps, b, t / LANES, t % LANES);
     if (PS::kBatched) return;
     // one scene: block max of dv, the last block decides (dv >= 0: bit patterns order like values)
     const unsigned bits = __reduce_max_sync(0xffffffffu, __float_as_uint(dv));
@@ -761,30 +1076,12 @@ __global__ void __launch_bounds__(BS) k_pressure_list(PS ps, ListBuffers b) {
 }
 
 // pcisph.cl:265-300, then predict (pcisph.cl:175-193) or integrate with optional walls
-// One particle's pressure-force sweep, then predict (mode 0 before the decision, 1) or integrate (mode 0
-// after it, 2) with optional walls.
-template <class PS, bool kCoherent = false>
-__device__ __forceinline__ void pressure_force_body(const PS& ps, const ListBuffers& b, uint32_t i, int mode) {
-    if (i >= ps.count() || ps.skip_force(i)) return;
-    const DevParams& P = ps.params(i);
-    Control* ctl = ps.control(i);
-    const float4 xi = b.pf4[i];
-    float3 f = make_float3(0.f, 0.f, 0.f);
-    const uint32_t cnt = b.near_count[i];
-    // boundary terms at x (within h): all zero unless a boundary particle was within r_list of x; the
-    // boundary list holds every one within r_list (terms beyond h are zero)
-    const bool near_b = P.boundary_count && b.b_near[i] != 0;
-    const uint32_t bcnt = near_b && b.bnbr ? b.bnbr_count[i] : 0u;
-    const bool list_boundary = near_b && b.bnbr && bcnt <= P.bnd_cap;
-    const bool walk_boundary = near_b && !list_boundary;
-    Cell c{0u, 0u, 0u};
-    if (cnt > P.near_cap || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
-    auto fb = [&](uint32_t j) { pressure_force_term(xi, load_slot<kCoherent>(&b.bpf[j]), P.h, P.h2, f); };
-    if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
-    else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
-    auto body = [&](uint32_t j) { pressure_force_term(xi, load_slot<kCoherent>(&b.pf4[j]), P.h, P.h2, f); };
-    if (cnt <= P.near_cap) for_each_listed(b.near, i, cnt, b.nbr_stride, body);
-    else for_each_neighbour(b.cells, c, P, body);
+// After the pressure-force sum f: predict (mode 0 before the decision, 1) or integrate (mode 0 after it, 2) with
+// optional walls.
+template <class PS>
+__device__ __forceinline__ void finish_pressure_force(const PS& ps, const ListBuffers& b, const DevParams& P,
+                                                      Control* ctl, uint32_t i, const float4& xi, const float3& f,
+                                                      int mode) {
     const float m = P.particle_mass;
     const float scale = -P.spiky_d1_norm * m * m;
     const float3 fp = make_float3(f.x * scale, f.y * scale, f.z * scale);
@@ -823,9 +1120,85 @@ __device__ __forceinline__ void pressure_force_body(const PS& ps, const ListBuff
         b.state_skin[o] = fminf(fmaxf(P.skin_factor * b.disp_max[i], P.skin_min_half), P.skin_max_half);
 }
 
-template <class PS, int BS = kBlock>
+// One particle's pressure-force sweep.
+template <class PS, bool kCoherent = false, int DEEP = 1>
+__device__ __forceinline__ void pressure_force_body(const PS& ps, const ListBuffers& b, uint32_t i, int mode) {
+    if (i >= ps.count() || ps.skip_force(i)) return;
+    const DevParams& P = ps.params(i);
+    Control* ctl = ps.control(i);
+    const float4 xi = b.pf4[i];
+    float3 f = make_float3(0.f, 0.f, 0.f);
+    const uint32_t cnt = b.near_count[i];
+    // boundary terms at x (within h): all zero unless a boundary particle was within r_list of x; the
+    // boundary list holds every one within r_list (terms beyond h are zero)
+    const bool near_b = P.boundary_count && b.b_near[i] != 0;
+    const uint32_t bcnt = near_b && b.bnbr ? b.bnbr_count[i] : 0u;
+    const bool list_boundary = near_b && b.bnbr && bcnt <= P.bnd_cap;
+    const bool walk_boundary = near_b && !list_boundary;
+    Cell c{0u, 0u, 0u};
+    if (cnt > P.near_cap || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
+    auto fb = [&](uint32_t j) { pressure_force_term(xi, load_slot<kCoherent>(&b.bpf[j]), P.h, P.h2, f); };
+    if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
+    else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
+    auto body = [&](uint32_t j) { pressure_force_term(xi, load_slot<kCoherent>(&b.pf4[j]), P.h, P.h2, f); };
+    if (cnt > P.near_cap) {
+        for_each_neighbour(b.cells, c, P, body);
+    } else if constexpr (DEEP > 1) {
+        for_each_listed_deep<DEEP>(
+            b.near, i, cnt, b.nbr_stride, [&](uint32_t j) { return load_slot<kCoherent>(&b.pf4[j]); },
+            [&](const float4& o) { pressure_force_term(xi, o, P.h, P.h2, f); });
+    } else {
+        for_each_listed(b.near, i, cnt, b.nbr_stride, body);
+    }
+    finish_pressure_force(ps, b, P, ctl, i, xi, f, mode);
+}
+
+// The same with eight lanes per particle, lane q.
+template <class PS, int L>
+__device__ __forceinline__ void pressure_force_shared(const PS& ps, const ListBuffers& b, uint32_t i0, uint32_t q,
+                                                      TermStage<L>& S, int mode) {
+    const bool live = i0 < ps.count() && !ps.skip_force(i0);
+    const uint32_t i = i0 < ps.count() ? i0 : ps.count() - 1u;
+    const uint32_t mask = lanes_mask<L>();
+    const DevParams& P = ps.params(i);
+    const float4 xi = b.pf4[i];
+    float acc = 0.f;  // lane 0, 1, 2: x, y, z
+    auto sum = [&](const float4& o, bool valid, uint32_t m) {
+        PairTerm term{0.f, 0.f, 0.f, 0.f};
+        if (valid) pressure_force_pair(xi, o, P.h, P.h2, [&](const PairTerm& t) { term = t; });
+        add_lanes(acc, term, S, q, m);
+    };
+    auto walk = [&](const uint2* cells, const float4* src) {
+        walk_shared<L>(cells, cell_of(xi.x, xi.y, xi.z, P), P, q, [&](uint32_t j, bool valid) {
+            float4 o = xi;
+            if (valid) o = __ldg(&src[j]);
+            sum(o, valid, mask);
+        });
+    };
+    if (P.boundary_count) {
+        const bool near_b = live && b.b_near[i] != 0;
+        const uint32_t bcnt = near_b && b.bnbr ? b.bnbr_count[i] : 0u;
+        const bool listed = b.bnbr && bcnt <= P.bnd_cap;
+        const uint32_t n = listed ? bcnt : 0u;
+        for_each_shared<L, 32 / L>(
+            b.bnbr, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.bpf[j]); },
+            [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+        if (near_b && !listed) walk(b.b_cells, b.bpf);
+    }
+    const uint32_t cnt = live ? b.near_count[i] : 0u;
+    const uint32_t n = cnt <= P.near_cap ? cnt : 0u;
+    for_each_shared<L, 32 / L>(
+        b.near, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.pf4[j]); },
+        [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+    if (cnt > P.near_cap) walk(b.cells, b.pf4);
+    const float y = __shfl_sync(mask, acc, 1, L), z = __shfl_sync(mask, acc, 2, L);
+    if (live && q == 0)
+        finish_pressure_force(ps, b, P, ps.control(i), i, xi, make_float3(acc, y, z), mode);
+}
+
+template <class PS, int BS = kBlock, int LANES = 1, int DEEP = 1>
 // (at most 40 registers: 48 resident warps per SM; 48 registers measured 10% slower at 1M)
-__global__ void __launch_bounds__(BS, 1536 / BS) k_pressure_force_list(PS ps, ListBuffers b, int mode,
+__global__ void __launch_bounds__(BS, LANES == 1 && DEEP == 1 ? 1536 / BS : 1) k_pressure_force_list(PS ps, ListBuffers b, int mode,
                                                             cudaGraphConditionalHandle cond, int use_cond) {
     const uint32_t i = blockIdx.x * BS + threadIdx.x;
     if (!PS::kBatched && use_cond && i == 0) {
@@ -835,7 +1208,12 @@ __global__ void __launch_bounds__(BS, 1536 / BS) k_pressure_force_list(PS ps, Li
         const bool stop = ctl->done != 0u || g >= (unsigned)ps.params(0).max_iters;
         cudaGraphSetConditional(cond, stop ? 0u : 1u);
     }
-    pressure_force_body(ps, b, i, mode);
+    if constexpr (LANES == 1) {
+        pressure_force_body<PS, false, DEEP>(ps, b, i, mode);
+    } else {
+        __shared__ TermStage<LANES> stage[BS / LANES];
+        pressure_force_shared<PS, LANES>(ps, b, i / LANES, i % LANES, stage[threadIdx.x / LANES], mode);
+    }
 }
 
 // The corrective loop of one step as one cooperative launch (every block resident, grid-stride over the
@@ -1018,16 +1396,34 @@ void launch_density(const PS& ps, uint32_t n, bool boundary, const ListBuffers& 
 void launch_density_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     launch_density(OneScene{P, ctl}, P.fluid_count, P.boundary_count != 0, b, s);
 }
+// Scenes of few threads, us per launch (CUDA events; about 5 of them the events' own) by one lane / two chunks in flight /
+// eight lanes per particle:
+//   particles   pressure             pressure force       normal               force
+//   4,096       15.2 / 15.7 / 11.3   14.2 / 10.1 / 8.0    14.7 / 10.4 / 8.5    19.0 / 18.9 / 11.4
+//   8,000       14.4 / 15.8 / 11.8   14.4 / 10.2 / 10.1   15.0 / 11.0 / 10.1   19.5 / 19.4 / 14.6
+//   15,625      14.8 / 15.4 / 13.3   15.3 / 10.7 / 12.2   15.0 / 10.9 / 12.7   19.2 / 20.2 / 22.2
+//   32,768      14.8 / 16.8 / 19.0   15.2 / 12.1 / 16.2   14.5 / 10.7 / 16.2   19.2 /  -   / 33
+//   64,000      19.5 / 21.0 / 29.8   16.2 / 16.3 / 26.4   15.1 / 16.2 / 25
+constexpr int kLanes = 8;
+constexpr uint32_t kSharedMax = 8192u;  // eight lanes
+constexpr uint32_t kDeepMax = 49152u;   // two chunks in flight, pressure force and normal
+
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
-    k_normal_list<<<grid_for(P.fluid_count), kBlock, 0, s>>>(OneScene{P, ctl}, b);
+    const uint32_t n = P.fluid_count;
+    if (n <= kSharedMax) k_normal_shared<OneScene, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(OneScene{P, ctl}, b);
+    else if (n <= kDeepMax) k_normal_list<OneScene, 2><<<grid_for(n), kBlock, 0, s>>>(OneScene{P, ctl}, b);
+    else k_normal_list<<<grid_for(n), kBlock, 0, s>>>(OneScene{P, ctl}, b);
 }
 void launch_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
-    k_force_list<<<grid_for(P.fluid_count), kBlock, 0, s>>>(OneScene{P, ctl}, b);
+    const uint32_t n = P.fluid_count;
+    if (n <= kSharedMax) k_force_shared<OneScene, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(OneScene{P, ctl}, b);
+    else k_force_list<<<grid_for(n), kBlock, 0, s>>>(OneScene{P, ctl}, b);
 }
 void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, cudaStream_t s) {
     const OneScene ps{P, ctl};
     const uint32_t n = P.fluid_count;
-    if (block == 128) k_pressure_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b);
+    if (n <= kSharedMax) k_pressure_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b);
+    else if (block == 128) k_pressure_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b);
     else if (block == 512) k_pressure_list<OneScene, 512><<<(n + 511) / 512, 512, 0, s>>>(ps, b);
     else k_pressure_list<OneScene, kBlock><<<grid_for(n), kBlock, 0, s>>>(ps, b);
 }
@@ -1039,7 +1435,11 @@ void launch_pressure_force_list(const DevParams& P, Control* ctl, const ListBuff
     const OneScene ps{P, ctl};
     const uint32_t n = P.fluid_count;
     const int uc = use_cond ? 1 : 0;
-    if (block == 128) k_pressure_force_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
+    if (n <= kSharedMax)
+        k_pressure_force_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b, mode, cond, uc);
+    else if (n <= kDeepMax)
+        k_pressure_force_list<OneScene, 128, 1, 2><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
+    else if (block == 128) k_pressure_force_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
     else if (block == 512) k_pressure_force_list<OneScene, 512><<<(n + 511) / 512, 512, 0, s>>>(ps, b, mode, cond, uc);
     else k_pressure_force_list<OneScene, kBlock><<<grid_for(n), kBlock, 0, s>>>(ps, b, mode, cond, uc);
 }

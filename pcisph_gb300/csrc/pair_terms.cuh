@@ -18,25 +18,38 @@ __device__ __forceinline__ float density_term(float xi, float yi, float zi, cons
     return poly6(dist2(dx, dy, dz), h2);
 }
 
+// A pair's vector term as a factor and the difference it scales: accumulated as one FMA per component everywhere (a
+// thread that sums its own pairs, or lanes that sum what others computed), so every sweep gives the same bits. The
+// _pair functions call add(term) where the pair contributes.
+struct PairTerm {
+    float x, y, z, k;
+};
+__device__ __forceinline__ void add_term(float3& a, const PairTerm& t) {
+    a.x = __fmaf_rn(t.x, t.k, a.x);
+    a.y = __fmaf_rn(t.y, t.k, a.y);
+    a.z = __fmaf_rn(t.z, t.k, a.z);
+}
+
 // poly6 gradient over the neighbour's density (pcisph.cl:18-26, :107); o = (x_j, rho_j)
-__device__ __forceinline__ void normal_term(float xi, float yi, float zi, const float4& o, float h2, float3& n) {
+template <class Add>
+__device__ __forceinline__ void normal_pair(float xi, float yi, float zi, const float4& o, float h2, Add&& add) {
     const float dx = xi - o.x, dy = yi - o.y, dz = zi - o.z;
     const float r2 = dist2(dx, dy, dz);
-    if (r2 <= h2) {
-        const float k = __fdividef((r2 - h2) * (r2 - h2), o.w);
-        n.x += dx * k;
-        n.y += dy * k;
-        n.z += dz * k;
-    }
+    if (r2 <= h2) add(PairTerm{dx, dy, dz, __fdividef((r2 - h2) * (r2 - h2), o.w)});
+}
+__device__ __forceinline__ void normal_term(float xi, float yi, float zi, const float4& o, float h2, float3& n) {
+    normal_pair(xi, yi, zi, o, h2, [&](const PairTerm& t) { add_term(n, t); });
 }
 
 // viscosity and Akinci cohesion + curvature (pcisph.cl:137-159); xi = (x_i, rho_i), o = (x_j, rho_j)
 struct ForceAccum {
     float3 visc, coh, curv;
 };
-__device__ __forceinline__ void force_term(const float4& xi, const float3& vi, const float3& ni, const float4& o,
-                                           const float3& vj, const float3& nj, const DevParams& P,
-                                           ForceAccum& a) {
+// viscous(term) and surface(cohesion, curvature) are called where the pair has them.
+template <class Viscous, class Surface>
+__device__ __forceinline__ void force_pair(const float4& xi, const float3& vi, const float3& ni, const float4& o,
+                                           const float3& vj, const float3& nj, const DevParams& P, Viscous&& viscous,
+                                           Surface&& surface) {
     const float dx = xi.x - o.x, dy = xi.y - o.y, dz = xi.z - o.z;
     const float r2 = dist2(dx, dy, dz);
     // The curvature term does not vanish at r = h: it jumps to zero there. Within a few ulp of the cut-off the
@@ -48,39 +61,41 @@ __device__ __forceinline__ void force_term(const float4& xi, const float3& vi, c
         const float inv_r = r2 > 0.f ? rsqrtf(r2) : 0.f;
         const float dist = __fmul_rn(r2, inv_r);  // rounded once: it has several uses
         const float rj = o.w;
-        if (r2 <= P.h2 && rj > 0.0001f) {
-            const float k = __fdividef(__fsub_rn(P.h, dist), rj);  // kernel_viscosity_d2 / rho_j
-            a.visc.x += (vj.x - vi.x) * k;
-            a.visc.y += (vj.y - vi.y) * k;
-            a.visc.z += (vj.z - vi.z) * k;
-        }
+        if (r2 <= P.h2 && rj > 0.0001f)  // times kernel_viscosity_d2 / rho_j
+            viscous(PairTerm{vj.x - vi.x, vj.y - vi.y, vj.z - vi.z, __fdividef(__fsub_rn(P.h, dist), rj)});
         const float d_cut =
             at_cut ? __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz))) : dist;
         if (dist > 0.0001f && d_cut < P.h) {
             const float corr = __fdividef(2.f * P.rest_density, xi.w + rj);
             const float c = corr * surface_tension_kernel(dist, P.h, P.st_term) * inv_r;  // * (x_i - x_j)/r
-            a.coh.x += c * dx;
-            a.coh.y += c * dy;
-            a.coh.z += c * dz;
-            a.curv.x += corr * (ni.x - nj.x);
-            a.curv.y += corr * (ni.y - nj.y);
-            a.curv.z += corr * (ni.z - nj.z);
+            surface(PairTerm{dx, dy, dz, c}, PairTerm{ni.x - nj.x, ni.y - nj.y, ni.z - nj.z, corr});
         }
     }
 }
+__device__ __forceinline__ void force_term(const float4& xi, const float3& vi, const float3& ni, const float4& o,
+                                           const float3& vj, const float3& nj, const DevParams& P,
+                                           ForceAccum& a) {
+    force_pair(
+        xi, vi, ni, o, vj, nj, P, [&](const PairTerm& t) { add_term(a.visc, t); },
+        [&](const PairTerm& t, const PairTerm& u) {
+            add_term(a.coh, t);
+            add_term(a.curv, u);
+        });
+}
 
 // spiky gradient times (p_i/rho_i^2 + p_j/rho_j^2) (pcisph.cl:28-37, :279-295); xi.w, o.w = p/rho^2
-__device__ __forceinline__ void pressure_force_term(const float4& xi, const float4& o, float h, float h2, float3& f) {
+template <class Add>
+__device__ __forceinline__ void pressure_force_pair(const float4& xi, const float4& o, float h, float h2, Add&& add) {
     const float dx = xi.x - o.x, dy = xi.y - o.y, dz = xi.z - o.z;
     const float r2 = dist2(dx, dy, dz);
     if (r2 <= h2 && r2 >= 1e-8f) {  // 1e-4 <= r <= h
         const float inv_r = rsqrtf(r2);
         const float dr = __fmaf_rn(-r2, inv_r, h);
-        const float k = dr * dr * inv_r * (xi.w + o.w);
-        f.x += dx * k;
-        f.y += dy * k;
-        f.z += dz * k;
+        add(PairTerm{dx, dy, dz, dr * dr * inv_r * (xi.w + o.w)});
     }
+}
+__device__ __forceinline__ void pressure_force_term(const float4& xi, const float4& o, float h, float h2, float3& f) {
+    pressure_force_pair(xi, o, h, h2, [&](const PairTerm& t) { add_term(f, t); });
 }
 
 // One fluid particle's term in a boundary particle's predicted density (pcisph.cl:240-250 from the boundary

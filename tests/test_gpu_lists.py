@@ -69,3 +69,34 @@ def test_nonfinite_particles_reach_the_same_sums(oracle, n, value):
     np.testing.assert_array_equal(np.isnan(rho[0]), np.isnan(rho[1]))
     ok = ~np.isnan(rho[1])
     assert_close("density", rho[0][ok], rho[1][ok])
+
+
+# one particle more takes the next split of the sweeps (eight lanes per particle up to 8,192, two chunks in flight up to
+# 49,152, then one); its own place is far away, and the bucket count is the same
+@pytest.mark.parametrize("boundary", [False, True])
+@pytest.mark.parametrize("n", [8192, 49152])
+def test_splits_of_the_sweeps_give_the_same_bits(oracle, n, boundary):
+    rng = np.random.default_rng(n)
+    pos = _cloud(n, 8, seed=n + 1) + np.float32(0.1)
+    pos[:90] = pos[0] + rng.random((90, 3)).astype(np.float32) * 0.5 * D  # a clump that overflows its lists
+    vel = (0.3 * rng.standard_normal((n, 3))).astype(np.float32)
+    vel[rng.choice(n, 30, replace=False)] *= 20.0  # predictions that outrun the lists
+    far = np.float32([[40.0, 40.0, 40.0]])
+    floor = np.stack(np.meshgrid(np.arange(20), [0.0], np.arange(20), indexing="ij"), -1).reshape(-1, 3) * D + 0.1
+    out = []
+    for extra in (False, True):
+        x = np.concatenate([pos, far]) if extra else pos
+        v = np.concatenate([vel, 0 * far]) if extra else vel
+        p = oracle.derive_params(0.5 * D, 1000.0, len(x), len(floor) if boundary else 0, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+        f = fluid_like(p, min_iters=3, max_iters=3, spatial_order=0)
+        f.set_fluid_state(x, v)
+        if boundary:
+            f.set_boundary_state(floor.astype(np.float32))
+        f.update()
+        keep = f.get_field("src") < n
+        out.append({k: f.get_field(k)[keep] for k in ("src", "density", "normal", "other_force", "predicted_position",
+                                                      "pressure", "pressure_force", "position", "velocity")})
+        assert f.stats().fast_particles > 0
+        f.close()
+    for k in out[0]:
+        np.testing.assert_array_equal(out[0][k], out[1][k], err_msg=k)
