@@ -42,6 +42,10 @@ struct DevParams {
     // them, and a kernel stamps the particles whose pressure sweep must walk because of them; 0: off (every
     // particle near a flagged bucket walks)
     uint32_t mark_cap;
+    // moving lists (one scene without boundary particles or per-particle skins): in a step that begins with more than
+    // 1 in kMovingShare particles that move kMovingSpeed of half the skin or more per step, the skin lists are built around y = x + v dt
+    // (moving_place) and a prediction is measured from there: a body that moves as a whole keeps its lists
+    int moving_lists;
     // batched scenes with an adaptive skin: each step picks one of kSkinLevels skins from the previous
     // step's count of predictions past each level's half skin (skin_half[k])
     int adaptive_skin;
@@ -80,6 +84,9 @@ struct Control {
     // the current round's pressure sweep, whose last block closes the round)
     unsigned long long fast_n;
     unsigned int round;
+    unsigned int moving;         // moving lists: the particles that fast (kMovingSpeed) when the step began
+    unsigned int lists_outrun;   // one scene: some prediction of this step was fast (1), measured from the place that
+                                 // the step's lists are built around; it flagged its bucket
 };
 
 // Close a step after its last corrective iteration `it` (Fluid.cpp:301-306 decides the same way): status
@@ -99,6 +106,21 @@ __device__ __forceinline__ void close_step(Control* ctl, unsigned it, float rel,
 }
 
 constexpr uint32_t kNearCap = 64;  // within-h list entries per particle
+
+// Moving lists (DevParams::moving_lists): the share of fast particles from which a step takes them. The two list radii then
+// test different places, which costs the list builder half again its time; a pressure sweep whose particles walk the
+// buckets takes 2 to 3 times one that reads lists.
+constexpr unsigned kMovingShare = 8;
+// A particle counts as fast from this share of half the skin per step: pressure and gravity move a prediction further
+// (a sphere falling at 0.11 h a step outran a half skin of 0.125 h in every prediction).
+constexpr float kMovingSpeed = 0.75f;
+__device__ __forceinline__ bool lists_move(const DevParams& P, const Control* ctl) {
+    return P.moving_lists && ctl->moving > P.fluid_count / kMovingShare;
+}
+// y = x + v dt, the same bits wherever it is formed
+__device__ __forceinline__ float4 moving_place(const DevParams& P, const float4& x, const float3& v) {
+    return make_float4(__fmaf_rn(v.x, P.dt, x.x), __fmaf_rn(v.y, P.dt, x.y), __fmaf_rn(v.z, P.dt, x.z), 0.f);
+}
 
 // List skins (units of h) an adaptive scene chooses from, smallest first.
 constexpr int kSkinLevels = 3;

@@ -358,6 +358,7 @@ struct pcisph_ctx {
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
         // cells (with a margin for the divisions of cell_of)
+        P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
         P.mark_cap = list_sweeps() && P.h + P.skin_max_half <= 1.9f * P.cell_size ? kMarkCap : 0u;
         graph_valid = false;
         order_age = kNoOrder;
@@ -392,8 +393,10 @@ struct pcisph_ctx {
 
     // ---------------------------------------------------------------- sort
     int sort_set(const float4* pos_in, uint32_t n, uint32_t* keys, uint32_t* ids, uint32_t** sk, uint32_t** sv,
-                 cudaStream_t s) {
-        timed("hash", s, [&] { launch_hash(reinterpret_cast<const float*>(pos_in), false, n, P, keys, nullptr, s); });
+                 cudaStream_t s, const float4* vel = nullptr) {
+        timed("hash", s, [&] {
+            launch_hash(reinterpret_cast<const float*>(pos_in), false, n, P, keys, nullptr, s, vel, b.ctl);
+        });
         int nl = 0;
         cudaError_t e = cudaSuccess;
         timed("radix_sort", s, [&] {
@@ -478,7 +481,7 @@ struct pcisph_ctx {
         if (cudaMemsetAsync(b.cells, 0, (size_t)params.bucket_count * 8, s) != cudaSuccess) return -1;
         if (list_sweeps() && cudaMemsetAsync(b.bucket_fast, 0, params.bucket_count, s) != cudaSuccess) return -1;
         uint32_t *sk = nullptr, *sv = nullptr;
-        int r = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s);
+        int r = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s, P.moving_lists ? b.state_vel : nullptr);
         if (r < 0) return -1;
         nl += r;
         sorted_keys = sk;
@@ -496,6 +499,10 @@ struct pcisph_ctx {
         const SweepArgs A = sweep_args();
         if (list_sweeps()) {
             timed("density", s, [&] { launch_density_list(P, b.ctl, list_buffers(), s); });
+            if (P.moving_lists) {
+                timed("moving_lists", s, [&] { launch_moving_lists(P, b.ctl, list_buffers(), s); });
+                ++nl;
+            }
             timed("normal", s, [&] { launch_normal_list(P, b.ctl, list_buffers(), s); });
             if (B) {
                 timed("boundary_list", s, [&] { launch_boundary_fluid_list(P, list_buffers(), s); });
@@ -727,7 +734,7 @@ struct pcisph_ctx {
                 CUDA_TRY(cudaMemsetAsync(b.cells, 0, (size_t)params.bucket_count * 8, s));
                 if (list_sweeps()) CUDA_TRY(cudaMemsetAsync(b.bucket_fast, 0, params.bucket_count, s));
                 uint32_t *sk = nullptr, *sv = nullptr;
-                int nl = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s);
+                int nl = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s, P.moving_lists ? b.state_vel : nullptr);
                 if (nl < 0) return PCISPH_ERR_CUDA;
                 sorted_keys = sk;
                 sorted_ids = sv;
@@ -743,8 +750,13 @@ struct pcisph_ctx {
                 break;
             }
             case PCISPH_STAGE_DENSITY:
-                if (list_sweeps()) launch_density_list(P, b.ctl, list_buffers(), s);
-                else if (warp_sweeps()) launch_density_sweep(P, b, sweep_args(), sweep_grid, s);
+                if (list_sweeps()) {
+                    launch_density_list(P, b.ctl, list_buffers(), s);
+                    if (P.moving_lists) {
+                        launch_moving_lists(P, b.ctl, list_buffers(), s);
+                        ++host_launches;
+                    }
+                } else if (warp_sweeps()) launch_density_sweep(P, b, sweep_args(), sweep_grid, s);
                 else launch_density(P, b, s);
                 ++host_launches;
                 break;

@@ -19,6 +19,8 @@
 //     whose 27 buckets include a flagged one walks the buckets instead of using its list: every pair with a
 //     fast particle j in i's walk (spatial neighbour or hash collision) is then summed by a walk. Flags
 //     last for the rest of the step;
+//   - in a step of moving lists (lists_move: many particles faster than half the skin per step) the skin lists are
+//     built around y = x + v dt instead of x, and a prediction is fast when it strays half the skin from there;
 //   - a particle with more than list_cap (near_cap) candidates is marked (count > cap) and walks the
 //     buckets in the sweeps that would use that list.
 // Boundary particles (B > 0, single scene) are summed by walking the boundary buckets. The density sweep
@@ -234,6 +236,8 @@ constexpr int kCellRounds = 10;   // candidate rounds in registers: 320, a full 
 constexpr int kCellBlock = 128;   // 4 warps a block, 20 resident per SM (24 spill: 501 us)
 constexpr uint32_t kAll = 0xffffffffu;
 
+constexpr unsigned long long kNoMarks = 1ull << 40;  // a round's count past any cap of the partner marks
+
 // A warp's working set: the hits of one particle (index, |d|^2 bits), the cell's bucket offsets, the particles.
 template <int W>
 struct CellWarp {
@@ -299,8 +303,9 @@ struct Candidates {
     uint32_t count;  // of these rounds
     bool odd;
 };
+template <class Place>
 __device__ __forceinline__ void load_candidates(Candidates& c, CellWalk& w, uint32_t base, uint32_t lane,
-                                                const uint32_t* delta, const float4* __restrict__ src) {
+                                                const uint32_t* delta, Place&& place) {
     const uint32_t at_or_below = 2u * lanes_below() + 1u;
     const float nan = __uint_as_float(0x7fffffffu);
     float zero = 0.f;  // stays 0 while every coordinate is finite
@@ -317,7 +322,7 @@ __device__ __forceinline__ void load_candidates(Candidates& c, CellWalk& w, uint
         c.x[u] = c.y[u] = c.z[u] = nan;
         if (f < w.total) {
             c.j[u] = f + delta[k & 31u];
-            const float4 o = __ldg(&src[c.j[u]]);
+            const float4 o = place(c.j[u]);
             c.x[u] = o.x;
             c.y[u] = o.y;
             c.z[u] = o.z;
@@ -389,7 +394,7 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_boundary_fluid_list(DevParams
         CellWalk w = begin_cell(b.cells, P, cx, cy, cz, lane, S.delta);
         for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
             Candidates cand;
-            load_candidates(cand, w, base, lane, S.delta, b.pos);
+            load_candidates(cand, w, base, lane, S.delta, [&](uint32_t j) { return __ldg(&b.pos[j]); });
             for (uint32_t g = group; g; g &= g - 1u) {
                 const int t = __ffs(g) - 1;
                 const uint32_t n = collect_hits(cand, S.target[t], S.hit, lane);
@@ -453,7 +458,7 @@ __device__ __forceinline__ void boundary_pressure_list_body(const DevParams& P, 
     const uint32_t cnt = b.bfl_count[k];
     bool walk = cnt > P.bfl_cap;
     Cell c{0u, 0u, 0u};
-    if (walk || ctl->fast_particles != ctl->fast_at_begin) {
+    if (walk || ctl->lists_outrun != 0u) {
         c = cell_of(xb.x, xb.y, xb.z, P);
         walk = walk || near_fast(P, b.bucket_fast, c);
     }
@@ -465,6 +470,54 @@ __device__ __forceinline__ void boundary_pressure_list_body(const DevParams& P, 
 
 __global__ void __launch_bounds__(kBlock) k_boundary_pressure_list(DevParams P, const Control* ctl, ListBuffers b) {
     boundary_pressure_list_body(P, ctl, b, blockIdx.x * kBlock + threadIdx.x);
+}
+
+// The skin lists of a step of moving lists (no work in any other step): the pairs of the walk (buckets around x) within
+// r_list at y = x + v dt. A kernel of its own: inside the density sweep its registers slowed every step (1M: 495 -> 517
+// us), as an early exit it costs 1-2 us. It also puts the round's count of fast predictions past any cap: no marks.
+__global__ void __launch_bounds__(kCellBlock, 5) k_moving_lists(DevParams P, Control* ctl, ListBuffers b) {
+    if (!lists_move(P, ctl)) return;
+    constexpr int W = 8;
+    __shared__ CellWarp<W> warps[kCellBlock / 32];
+    CellWarp<W>& S = warps[threadIdx.x >> 5];
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->fast_n = kNoMarks;
+    const uint32_t lane = threadIdx.x & 31u;
+    auto place = [&](uint32_t j) { return moving_place(P, __ldg(&b.pos[j]), f3(__ldg(&b.vel[j]))); };
+    for (uint32_t i0 = (blockIdx.x * (kCellBlock / 32) + (threadIdx.x >> 5)) * W; i0 < P.fluid_count;
+         i0 += gridDim.x * (kCellBlock / 32) * W) {
+        const uint32_t me = i0 + lane;
+        const bool own = lane < W && me < P.fluid_count;
+        const float4 xi = b.pos[own ? me : i0];
+        const Cell c = cell_of(xi.x, xi.y, xi.z, P);
+        if (lane < W) {
+            S.target[lane] = moving_place(P, xi, f3(b.vel[own ? me : i0]));
+            S.target[lane].w = P.list_r2;
+        }
+        uint32_t n_own = 0;
+        uint32_t todo = __ballot_sync(kAll, own);
+        while (todo) {
+            const int lead = __ffs(todo) - 1;
+            const uint32_t cx = __shfl_sync(kAll, c.x, lead), cy = __shfl_sync(kAll, c.y, lead),
+                           cz = __shfl_sync(kAll, c.z, lead);
+            const uint32_t group = __ballot_sync(kAll, c.x == cx && c.y == cy && c.z == cz) & todo;
+            todo &= ~group;
+            CellWalk w = begin_cell(b.cells, P, cx, cy, cz, lane, S.delta);
+            for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
+                Candidates cand;
+                load_candidates(cand, w, base, lane, S.delta, place);
+                for (uint32_t g = group; g; g &= g - 1u) {
+                    const int t = __ffs(g) - 1;
+                    const uint32_t n = collect_hits(cand, S.target[t], S.hit, lane);
+                    const uint32_t n0 = __shfl_sync(kAll, n_own, t);
+                    for (uint32_t k = lane; k < n; k += 32u)
+                        if (n0 + k < P.list_cap) __stcs(list_entry(b.nbr, i0 + t, n0 + k, b.nbr_stride), S.hit[k].x);
+                    if ((int)lane == t) n_own = n0 + n;
+                }
+            }
+        }
+        if (own) b.nbr_count[me] = n_own;
+        __syncwarp();
+    }
 }
 
 // pcisph.cl:65-92, and the neighbour lists of the step (see the list builders above). kBoundary: the scene has boundary
@@ -501,6 +554,9 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
         __syncwarp();
     };
     uint32_t todo = __ballot_sync(kAll, own);
+    // moving lists: k_moving_lists builds the skin lists, this pass at x only what lies within h of x
+    const bool moving = !PS::kBatched && !kBoundary && lists_move(Pi, ps.control(0));
+    if (moving && lane < W) S.target[lane].w = Pi.near_r2;
     while (todo) {
         const int lead = __ffs(todo) - 1;
         const DevParams& P = ps.params(i0 + lead);  // the same scene for the whole group: buckets do not overlap
@@ -521,7 +577,7 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
                 CellWalk w = begin_cell(b.b_cells, P, cx, cy, cz, lane, S.delta);
                 for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
                     Candidates cand;
-                    load_candidates(cand, w, base, lane, S.delta, b.b_pos);
+                    load_candidates(cand, w, base, lane, S.delta, [&](uint32_t j) { return __ldg(&b.b_pos[j]); });
                     for (uint32_t g = group; g; g &= g - 1u) {
                         const int t = __ffs(g) - 1;
                         float4 q = S.target[t];
@@ -565,7 +621,7 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
         CellWalk w = begin_cell(b.cells, P, cx, cy, cz, lane, S.delta);
         for (uint32_t base = 0; base < w.total; base += kCellRounds * 32u) {
             Candidates cand;
-            load_candidates(cand, w, base, lane, S.delta, b.pos);
+            load_candidates(cand, w, base, lane, S.delta, [&](uint32_t j) { return __ldg(&b.pos[j]); });
             for (uint32_t g = group; g; g &= g - 1u) {
                 const int t = __ffs(g) - 1;
                 const float4 q = S.target[t];
@@ -573,10 +629,10 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
                 const uint32_t n = collect_hits(cand, q, S.hit, lane);
                 const uint32_t n0 = __shfl_sync(kAll, n_own, t);
                 uint32_t cnt = __shfl_sync(kAll, staged, t);
-                if (n0 != 0u)  // a cell of more than kCellRounds rounds: the list goes on
+                if (n0 != 0u && !moving)  // a cell of more than kCellRounds rounds: the list goes on
                     for (uint32_t k = lane; k < n; k += 32u)
                         if (n0 + k < P.list_cap) __stcs(list_entry(b.nbr, i0 + t, n0 + k, stride), S.hit[k].x);
-                const uint32_t stored = n0 == 0u ? min(n, P.list_cap) : 0u;
+                const uint32_t stored = n0 == 0u && !moving ? min(n, P.list_cap) : 0u;
                 uint32_t* out = out0 + 8 * t;
                 const uint32_t stage_addr = near_addr + 8u * t * (kNearCap + 1u);
                 for (uint32_t k0 = 0; k0 < n; k0 += 32u) {
@@ -608,7 +664,7 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
     if (own) {
         for (uint32_t k = 0; k < staged; ++k) acc += __uint_as_float(S.near[lane][k].y);
         if (nan_own) acc = __uint_as_float(0x7fffffffu);
-        b.nbr_count[me] = n_own;
+        if (!moving) b.nbr_count[me] = n_own;
         b.near_count[me] = near_own;
         acc *= Pi.particle_mass * Pi.poly6_norm;
         b.rho[me] = acc;
@@ -671,8 +727,8 @@ __device__ __forceinline__ void finish_force(const PS& ps, const ListBuffers& b,
     const float3 dx = v * P.dt;
     const float4 xs = make_float4(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z, 0.f);
     b.pred[i] = xs;
-    const float disp = note_displacement(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin,
-                                         PS::kBatched ? nullptr : b.fast_list, i);
+    const float disp = note_displacement<!PS::kBatched>(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin, vi,
+                                                        PS::kBatched ? nullptr : b.fast_list, i);
     if (P.particle_skin) b.disp_max[i] = disp;
 }
 
@@ -788,7 +844,8 @@ __global__ void __launch_bounds__(kBlock) k_force_shared(PS ps, ListBuffers b) {
 // and |x_i - x_j| is beyond i's list radius (the builder's test, the same bits), and stamps j itself.
 // Stamping more than needed only makes a particle walk, which gives the walk's sum. The round is the one the
 // next pressure sweep reads (Control::round + 1); that sweep's last block closes it. A round with more than
-// mark_cap fast predictions stamps nothing (the sweep then uses the bucket flags).
+// mark_cap fast predictions stamps nothing (the sweep then uses the bucket flags), nor does a step of moving lists (no
+// fast prediction is listed).
 __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Control* ctl, ListBuffers b) {
     const unsigned long long n = ctl->fast_n;
     if (n == 0 || n > P.mark_cap) return;
@@ -842,6 +899,12 @@ __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Con
 
 // pcisph.cl:212-263 (boundary_update = 0); one scene: also the stop decision in the last block
 
+// No prediction of this step was fast: the scene's lists are complete for x*.
+template <class PS>
+__device__ __forceinline__ bool lists_hold(const Control* ctl) {
+    return PS::kBatched ? ctl->fast_particles == ctl->fast_at_begin : ctl->lists_outrun == 0u;
+}
+
 // How one particle's pressure sweep finds its neighbours.
 struct PressurePlan {
     uint32_t cnt, bcnt;              // entries of its skin list and of its boundary list
@@ -854,8 +917,7 @@ __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBu
                                                       const Control* ctl, uint32_t i, const float4& xi,
                                                       const float4& xp) {
     PressurePlan p;
-    // no particle of the scene moved more than half the skin: its lists are complete for x*
-    const bool all_lists_ok = ctl->fast_particles == ctl->fast_at_begin;
+    const bool all_lists_ok = lists_hold<PS>(ctl);
     p.cnt = b.nbr_count[i];
     const bool overflow = p.cnt > P.list_cap;
     // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
@@ -923,8 +985,7 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
     if (i < ps.count() && !ps.skip_pressure(i)) {
         const DevParams& P = ps.params(i);
         Control* ctl = ps.control(i);
-        // no particle of the scene moved more than half the skin: its lists are complete for x*
-        const bool all_lists_ok = ctl->fast_particles == ctl->fast_at_begin;
+        const bool all_lists_ok = lists_hold<PS>(ctl);
         const float4 xi = b.pos[i];
         const float4 xp = b.pred[i];
         float acc = 0.f;
@@ -1069,7 +1130,7 @@ __global__ void __launch_bounds__(BS) k_pressure_list(PS ps, ListBuffers b) {
         ctl->max_err_bits = atomicAdd(&ctl->max_err_bits, 0u);  // see every block's contribution
         if (b.walk_stamp) {  // close the prediction round of the partner marks: the next one starts empty
             ctl->round += 1u;
-            ctl->fast_n = 0;
+            ctl->fast_n = lists_move(ps.params(0), ctl) ? kNoMarks : 0ull;  // moving lists: no marks
         }
         decide(ps.params(0), ctl);
     }
@@ -1088,14 +1149,15 @@ __device__ __forceinline__ void finish_pressure_force(const PS& ps, const ListBu
     b.f_press[i] = f4(fp, 0.f);
     const bool integrate = mode == 0 ? (ctl->done != 0u) : mode == 2;
     const float3 a = (f3(b.f_other[i]) + fp) / m;
-    float3 v = f3(b.vel[i]) + a * P.dt;
+    const float3 vi = f3(b.vel[i]);
+    float3 v = vi + a * P.dt;
     const float3 dx = v * P.dt;
     float3 x = make_float3(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z);
     if (!integrate) {
         const float4 xs = f4(x, 0.f);
         b.pred[i] = xs;
-        const float disp = note_displacement(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin,
-                                             PS::kBatched ? nullptr : b.fast_list, i);
+        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin, vi,
+                                                            PS::kBatched ? nullptr : b.fast_list, i);
         if (P.particle_skin) b.disp_max[i] = fmaxf(b.disp_max[i], disp);
         return;
     }
@@ -1407,6 +1469,11 @@ void launch_density_list(const DevParams& P, Control* ctl, const ListBuffers& b,
 constexpr int kLanes = 8;
 constexpr uint32_t kSharedMax = 8192u;  // eight lanes
 constexpr uint32_t kDeepMax = 49152u;   // two chunks in flight, pressure force and normal
+
+void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
+    const unsigned blocks = std::min(grid_cells(P.fluid_count, 8), 5u * 152u);
+    if (P.fluid_count) k_moving_lists<<<blocks, kCellBlock, 0, s>>>(P, ctl, b);
+}
 
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     const uint32_t n = P.fluid_count;

@@ -99,6 +99,8 @@ void launch_boundary_cell_bounds(const DevParams& P, const float4* b_pos, int* b
 void launch_boundary_zone(const DevParams& P, const float4* b_pos, const int* org, const uint32_t* dim,
                           unsigned char* zone, cudaStream_t s);
 void launch_boundary_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
+// The skin lists of a step of moving lists (DevParams::moving_lists), after the density sweep; no work in other steps.
+void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 void launch_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 // Partner marks of the prediction round just completed (DevParams::mark_cap; b.fast_list and b.walk_stamp

@@ -27,8 +27,20 @@ inline unsigned grid_for(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 
 template <bool PACKED>
 __global__ void __launch_bounds__(kBlock) k_hash(const float* __restrict__ pos, uint32_t n, DevParams P,
-                                                 uint32_t* __restrict__ keys, uint32_t* __restrict__ ids) {
+                                                 uint32_t* __restrict__ keys, uint32_t* __restrict__ ids,
+                                                 const float4* __restrict__ vel, Control* ctl) {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+    if (vel) {
+        bool moves = false;
+        if (i < n) {
+            const float4 v = vel[i];
+            const float dx = v.x * P.dt, dy = v.y * P.dt, dz = v.z * P.dt;
+            const float slow = kMovingSpeed * P.list_half_skin;
+            moves = dist2(dx, dy, dz) > slow * slow;
+        }
+        const int m = __syncthreads_count(moves);  // one atomic per block that has any
+        if (m && threadIdx.x == 0) atomicAdd(&ctl->moving, (unsigned)m);
+    }
     if (i >= n) return;
     float x, y, z;
     if (PACKED) {
@@ -97,6 +109,8 @@ __global__ void k_begin(Control* ctl) {
     ctl->n_groups = 0;
     ctl->fast_at_begin = ctl->fast_particles;
     ctl->fast_n = 0;
+    ctl->moving = 0;
+    ctl->lists_outrun = 0;
 }
 
 // pcisph.cl:65-92
@@ -389,10 +403,10 @@ __global__ void __launch_bounds__(kBlock) k_unpack4_to3(const float4* __restrict
 }  // namespace
 
 void launch_hash(const float* pos, bool packed, uint32_t n, const DevParams& P, uint32_t* keys, uint32_t* ids,
-                 cudaStream_t s) {
+                 cudaStream_t s, const float4* vel, Control* ctl) {
     if (!n) return;
-    if (packed) k_hash<true><<<grid_for(n), kBlock, 0, s>>>(pos, n, P, keys, ids);
-    else k_hash<false><<<grid_for(n), kBlock, 0, s>>>(pos, n, P, keys, ids);
+    if (packed) k_hash<true><<<grid_for(n), kBlock, 0, s>>>(pos, n, P, keys, ids, vel, ctl);
+    else k_hash<false><<<grid_for(n), kBlock, 0, s>>>(pos, n, P, keys, ids, vel, ctl);
 }
 
 void launch_reorder(const uint32_t* keys, const uint32_t* ids, const float4* in_pos, const float4* in_vel,

@@ -47,8 +47,9 @@ struct StepBuffers {
 };
 
 // Kernels launched per call are reported through the return value (count), errors via cudaGetLastError.
+// vel and ctl (or null): also counts the fast particles of the moving lists (Control::moving).
 void launch_hash(const float* pos, bool packed, uint32_t n, const DevParams& P, uint32_t* keys, uint32_t* ids,
-                 cudaStream_t s);
+                 cudaStream_t s, const float4* vel = nullptr, Control* ctl = nullptr);
 // Also writes cell codes (if codes) and appends bucket-run starts to groups (if groups).
 void launch_reorder(const uint32_t* keys, const uint32_t* ids, const float4* in_pos, const float4* in_vel,
                     uint32_t n, float4* out_pos, float4* out_vel, uint2* cells, uint32_t* codes, uint32_t* groups,

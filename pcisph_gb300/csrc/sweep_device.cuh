@@ -30,15 +30,26 @@ __device__ __forceinline__ void warp_count(unsigned long long* addr, bool pred) 
 // past each adaptive skin level are counted. With a fast list (partner marks, one scene), a fast particle
 // also takes a slot of the round's list while the round holds at most P.mark_cap of them (one atomic per
 // warp that has one; none once the round is past the cap, which then falls back to the bucket flags).
-// Returns the displacement |x* - x|; threshold: the particle's fast_threshold.
+// Returns the displacement |x* - x|; threshold: the particle's fast_threshold. kOne: one scene, whose lists may move
+// with the particles (then the bucket is flagged when the prediction strays from y, and the round's count is past the
+// cap, so that nothing is listed); vi: the velocity at the step's start.
+template <bool kOne>
 __device__ __forceinline__ float note_displacement(const DevParams& P, Control* ctl,
                                                    unsigned char* __restrict__ bucket_fast, const float4& xi,
-                                                   const float4& xs, float threshold,
+                                                   const float4& xs, float threshold, const float3& vi,
                                                    uint32_t* __restrict__ fast_list = nullptr, uint32_t i = 0) {
     const float dx = xs.x - xi.x, dy = xs.y - xi.y, dz = xs.z - xi.z;  // exact: xs and xi are close
     const float disp = sqrtf(dist2(dx, dy, dz));
     const bool fast = disp > threshold;
     warp_count(&ctl->fast_particles, fast);
+    bool flag = fast;
+    if (kOne) {
+        if (lists_move(P, ctl)) {
+            const float4 y = moving_place(P, xi, vi);
+            flag = !(sqrtf(dist2(xs.x - y.x, xs.y - y.y, xs.z - y.z)) <= threshold);  // NaN strays
+        }
+        if (flag && ctl->lists_outrun == 0u) ctl->lists_outrun = 1u;
+    }
     if (fast_list) {
         const unsigned act = __activemask();
         const unsigned set = __ballot_sync(act, fast);
@@ -58,7 +69,7 @@ __device__ __forceinline__ float note_displacement(const DevParams& P, Control* 
 #pragma unroll
         for (int k = 0; k < kSkinLevels; ++k) warp_count(&ctl->over_level[k], disp > P.skin_half[k]);
     }
-    if (fast) {
+    if (flag) {
         const Cell c = cell_of(xi.x, xi.y, xi.z, P);
         bucket_fast[P.bucket_base + hash_key(c.x, c.y, c.z, P)] = 1;
     }

@@ -100,3 +100,57 @@ def test_splits_of_the_sweeps_give_the_same_bits(oracle, n, boundary):
         f.close()
     for k in out[0]:
         np.testing.assert_array_equal(out[0][k], out[1][k], err_msg=k)
+
+
+@pytest.mark.parametrize("loop_mode,order", [(0, 0), (0, 1), (1, 1), (2, 0)])
+@pytest.mark.parametrize("motion", ["fall", "shear", "random", "half"])
+def test_moving_lists_change_no_bits(oracle, motion, loop_mode, order):
+    """A scene of which many particles move faster than the skin allows builds its skin lists around y = x + v dt. The
+    same steps without that (per-particle skins build every list around x) give the same bits and the same counts."""
+    n = 12000
+    rng = np.random.default_rng(7)
+    pos = _cloud(n, 8, seed=11) + np.float32(0.2)
+    vel = np.zeros_like(pos)
+    if motion == "fall":
+        vel[:, 1] = -9.0  # 0.23 h per step, the whole body
+    elif motion == "shear":
+        vel[:, 0] = 20.0 * (pos[:, 1] - 0.2)
+    elif motion == "random":
+        vel = (6.0 * rng.standard_normal(pos.shape)).astype(np.float32)
+    else:
+        vel[pos[:, 0] < np.median(pos[:, 0]), 2] = 15.0  # one half slides past the other
+    p = oracle.derive_params(0.5 * D, 1000.0, n, 0, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    out = []
+    for skins in (0, 1):
+        f = fluid_like(p, min_iters=4, max_iters=4, loop_mode=loop_mode, spatial_order=order, walls=True,
+                       box_hi=(3.0, 3.0, 3.0))
+        f.set_options(particle_skin=skins)
+        f.set_fluid_state(pos, vel)
+        f.step(2)
+        st = f.stats()
+        out.append(({k: f.get_field(k) for k in ("src", "density", "normal", "pressure", "pressure_force", "position",
+                                                 "velocity", "predicted_position")},
+                    (st.fast_particles, st.list_fallbacks, st.status_all)))
+        f.close()
+    assert out[0][1] == out[1][1] and out[0][1][0] > n // 8
+    for k in out[0][0]:
+        np.testing.assert_array_equal(out[0][0][k], out[1][0][k], err_msg=k)
+
+
+def test_moving_lists_keep_nonfinite_velocities(oracle):
+    n = 9000
+    pos = _cloud(n, 8, seed=12)
+    vel = np.full_like(pos, 8.0)
+    vel[5, 0], vel[77] = np.nan, np.inf
+    p = oracle.derive_params(0.5 * D, 1000.0, n, 0, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    out = []
+    for skins in (0, 1):
+        f = fluid_like(p, min_iters=3, max_iters=3, spatial_order=0)
+        f.set_options(particle_skin=skins)
+        f.set_fluid_state(pos, vel)
+        f.update()
+        assert f.stats().status & 2
+        out.append([f.get_field(k) for k in ("density", "pressure", "density_variation")])
+        f.close()
+    for a, w in zip(*out):
+        np.testing.assert_array_equal(a, w)
