@@ -355,11 +355,15 @@ struct pcisph_ctx {
         P.particle_skin = skins && list_sweeps() ? 1 : 0;
         P.skin_min_half = std::min(kSkinMinHalf * P.h, P.skin_max_half);
         P.skin_factor = kSkinFactor;
+        P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
-        // cells (with a margin for the divisions of cell_of)
-        P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
-        P.mark_cap = list_sweeps() && P.h + P.skin_max_half <= 1.9f * P.cell_size ? kMarkCap : 0u;
+        // cells (with a margin for the divisions of cell_of). With more than 1 in 8 fast nearly every warp holds walkers
+        // whether marked or flagged, and the marks only cost (120,000 particles, half of them fast: 137 us a round
+        // against 56 us for the sweep that walks): such a round takes the flags.
+        P.mark_cap = list_sweeps() && P.h + P.skin_max_half <= 1.9f * P.cell_size
+                         ? std::min(kMarkCap, std::max(64u, params.fluid_count / 8u))
+                         : 0u;
         graph_valid = false;
         order_age = kNoOrder;
     }

@@ -48,7 +48,9 @@ namespace {
 
 constexpr int kBlock = 256;
 inline unsigned grid_for(uint32_t n) { return (n + kBlock - 1) / kBlock; }
-constexpr unsigned kMarkBlocks = 152;  // the marking kernel's grid (grid-stride over its items)
+// The marking kernel's grid (grid-stride over its items): 4 blocks an SM. A round of ~3,000 fast predictions at 1M takes
+// 13 us (21 with one block an SM), a round without any 2.5 either way.
+constexpr unsigned kMarkBlocks = 608;
 
 // List layout: entries k = 8c .. 8c+7 of particle i (chunk c) are 32 contiguous bytes at uint4 offset
 // 2 (c * stride + i); chunks are column-major over particles. A warp's 32 consecutive particles read
@@ -978,17 +980,94 @@ __device__ __forceinline__ float finish_pressure(const ListBuffers& b, const Dev
     return dv;
 }
 
-// One particle's pressure sweep; returns its density variation (0 when skipped or out of range).
+// The particles of a warp that walk, after their boundary terms (acc). A walk by one lane takes the warp ~400 steps of one
+// gather each, whatever its other lanes do; few walkers are therefore served one after another by all 32 lanes (27 bucket
+// ranges at once, 32 candidates a round, ~9 rounds), and their terms summed in walk order by their own lane. Each costs
+// ~500 instructions, a lane's share of a full warp's walk ~300: from kFewWalkers on each lane walks by itself.
+// Pressure sweep with few hundred to few thousand fast predictions: 1M jittered block 158 -> 144 us, a 98,904-particle drop
+// at 2.4 m/s 43 -> 32; from 6 to 32 the split makes no difference there. (A function of its own: the registers of the
+// walks stay out of the list path, which alone gained 137 -> 134 us at 1M, 42 -> 39 with 103,736 boundary particles.)
+constexpr int kFewWalkers = 12;
+struct WalkStage {
+    uint32_t delta[32];
+    float term[96];
+};
+template <class PS, bool kCoherent>
+__device__ __noinline__ float pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
+                                               uint32_t walkers, WalkStage& S) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const bool mine = (walkers >> lane) & 1u;
+    const uint32_t first = __shfl_sync(kAll, i, __ffs(walkers) - 1);
+    const uint32_t ii = mine ? i : first;  // a lane that does not walk stands in for the first that does
+    const DevParams& P = ps.params(ii);
+    const float4 xi = b.pos[ii];
+    const float4 xp = b.pred[ii];
+    const Cell c = cell_of(xi.x, xi.y, xi.z, P);
+    if (__popc(walkers) > kFewWalkers) {
+        if (mine) {
+            auto load = [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); };
+            auto use = [&](uint32_t, const float4& o) { acc += density_term(xp.x, xp.y, xp.z, o, P.h2); };
+            // a batch walks with two gathers in flight (terms still added in walk order): its walkers are latency-bound
+            // (256 batched scenes, 9.8M particles, over 500 steps: 26.8 -> 25.8 s); one scene walks plainly (8M
+            // particles all walking: 3.0 ms per sweep, 3.6 with the prefetch)
+            if constexpr (PS::kBatched) for_each_neighbour_prefetched(b.cells, c, P, load, use);
+            else for_each_neighbour(b.cells, c, P, [&](uint32_t j) { use(j, load(j)); });
+        }
+    } else {
+        const uint32_t below = lanes_below();
+        for (uint32_t todo = walkers; todo; todo &= todo - 1u) {
+            const int t = __ffs(todo) - 1;
+            const DevParams& Q = ps.params(__shfl_sync(kAll, ii, t));
+            const float x = __shfl_sync(kAll, xp.x, t), y = __shfl_sync(kAll, xp.y, t), z = __shfl_sync(kAll, xp.z, t);
+            CellWalk w = begin_cell(b.cells, Q, __shfl_sync(kAll, c.x, t), __shfl_sync(kAll, c.y, t),
+                                    __shfl_sync(kAll, c.z, t), lane, S.delta);
+            uint32_t n = 0;
+            auto sum = [&] {  // the staged terms, by the walker's own lane
+                __syncwarp();
+                if ((int)lane == t)
+                    for (uint32_t k = 0; k < n; ++k) acc += S.term[k];
+                n = 0;
+                __syncwarp();
+            };
+            constexpr int U = 3;  // rounds with their gathers in flight
+            for (uint32_t base = 0; base < w.total; base += 32u * U) {
+                float4 o[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t rel = w.off - (base + u * 32u);
+                    const uint32_t begun = __reduce_or_sync(kAll, rel < 32u ? 1u << rel : 0u);
+                    const uint32_t f = base + u * 32u + lane, k = w.rank + __popc(begun & (2u * below + 1u));
+                    w.rank += __popc(begun);
+                    if (f < w.total) o[u] = load_slot<kCoherent>(&b.pred[f + S.delta[k & 31u]]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    float term = 0.f;
+                    if (base + u * 32u + lane < w.total) term = density_term(x, y, z, o[u], Q.h2);
+                    const uint32_t bits = __ballot_sync(kAll, term != 0.f);  // NaN counts
+                    if (n + __popc(bits) > 96u) sum();
+                    if (term != 0.f) S.term[n + __popc(bits & below)] = term;
+                    n += __popc(bits);
+                }
+            }
+            sum();
+        }
+    }
+    return mine ? finish_pressure<PS>(b, P, ps.control(ii), ii, xi, acc) : 0.f;
+}
+
+// One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
+// stage: its WalkStage.
 template <class PS, bool kCoherent = false>
-__device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i) {
-    float dv = 0.f;
+__device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, WalkStage& stage) {
+    float dv = 0.f, acc = 0.f;
+    bool walk = false;
     if (i < ps.count() && !ps.skip_pressure(i)) {
         const DevParams& P = ps.params(i);
         Control* ctl = ps.control(i);
         const bool all_lists_ok = lists_hold<PS>(ctl);
         const float4 xi = b.pos[i];
         const float4 xp = b.pred[i];
-        float acc = 0.f;
         const uint32_t cnt = b.nbr_count[i];
         const bool overflow = cnt > P.list_cap;
         // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
@@ -1019,7 +1098,6 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         // the bucket flags: every particle near a fast one walks
         const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
         const bool marks = fast_round <= P.mark_cap;
-        bool walk;
         if (marks) {
             walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
             if (walk || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
@@ -1030,33 +1108,17 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         auto fb = [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, __ldg(&b.b_pos[j]), P.h2); };
         if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
         else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
-        auto f = [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2); };
-        if (walk) {
-            // a batch walks with two gathers in flight (terms still added in walk order): its walkers are
-            // few and latency-bound (256 batched scenes, 9.8M particles, over 500 steps: 26.8 -> 25.8 s); one scene walks plainly
-            // (8M particles all walking: 3.0 ms per sweep, 3.6 with the prefetch)
-            if constexpr (PS::kBatched)
-                for_each_neighbour_prefetched(
-                    b.cells, c, P, [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); },
-                    [&](uint32_t, const float4& o) { acc += density_term(xp.x, xp.y, xp.z, o, P.h2); });
-            else
-                for_each_neighbour(b.cells, c, P, f);
-        } else {
-            for_each_listed(b.nbr, i, cnt, b.nbr_stride, f);
+        if (!walk) {
+            for_each_listed(b.nbr, i, cnt, b.nbr_stride, [&](uint32_t j) {
+                acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
+            });
+            dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
         }
-        acc *= P.particle_mass * P.poly6_norm;
-        if (!isfinite(acc)) atomicOr(&ctl->status, 2u);
-        dv = acc - P.rest_density;
-        dv = 0.f < dv ? dv : 0.f;
-        b.err[i] = dv;
-        float p = b.press[i];
-        if (dv != 0.f) {
-            p += dv * P.delta;
-            b.press[i] = p;
-        }
-        const float r = b.rho[i];
-        b.pf4[i] = make_float4(xi.x, xi.y, xi.z, p / (r * r));
-        if (PS::kBatched) warp_atomic_max(&ctl->max_err_bits, __float_as_uint(dv));
+    }
+    const uint32_t walkers = __ballot_sync(kAll, walk);
+    if (walkers) {
+        const float w = pressure_walkers<PS, kCoherent>(ps, b, i, acc, walkers, stage);
+        if (walk) dv = w;
     }
     return dv;
 }
@@ -1106,7 +1168,8 @@ template <class PS, int BS = kBlock, int LANES = 1>
 __global__ void __launch_bounds__(BS) k_pressure_list(PS ps, ListBuffers b) {
     const uint32_t t = blockIdx.x * BS + threadIdx.x;
     float dv;
-    if constexpr (LANES == 1) dv = pressure_body(ps, b, t);
+    __shared__ WalkStage stage[LANES == 1 ? BS / 32 : 1];
+    if constexpr (LANES == 1) dv = pressure_body(ps, b, t, stage[threadIdx.x >> 5]);
     else dv = pressure_shared<PS, LANES>(ps, b, t / LANES, t % LANES);
     if (PS::kBatched) return;
     // one scene: block max of dv, the last block decides (dv >= 0: bit patterns order like values)
@@ -1290,6 +1353,7 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
     const uint32_t stride = gridDim.x * kBlock;
     const uint32_t rounds = (ps.count() + stride - 1) / stride;
     __shared__ int running;
+    __shared__ WalkStage stage[kBlock / 32];
     for (int it = 0; it < max_iters; ++it) {
         if constexpr (!PS::kBatched) {  // boundary pressures at the predicted positions (read by the force)
             const DevParams& P = ps.params(0);
@@ -1299,7 +1363,8 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
         unsigned local = 0;
         for (uint32_t r = 0; r < rounds; ++r)
             local = max(local, __float_as_uint(
-                                   pressure_body<PS, true>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x)));
+                                   pressure_body<PS, true>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
+                                                           stage[threadIdx.x >> 5])));
         if (!PS::kBatched) {  // batched scenes reduced per scene inside the body
             const unsigned m = __reduce_max_sync(0xffffffffu, local);
             if ((threadIdx.x & 31) == 0 && m) atomicMax(&ps.control(0)->max_err_bits, m);
