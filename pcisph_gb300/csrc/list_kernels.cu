@@ -984,16 +984,15 @@ __device__ __forceinline__ float finish_pressure(const ListBuffers& b, const Dev
 // gather each, whatever its other lanes do; few walkers are therefore served one after another by all 32 lanes (27 bucket
 // ranges at once, 32 candidates a round, ~9 rounds), and their terms summed in walk order by their own lane. Each costs
 // ~500 instructions, a lane's share of a full warp's walk ~300: from kFewWalkers on each lane walks by itself.
-// Pressure sweep with few hundred to few thousand fast predictions: 1M jittered block 158 -> 144 us, a 98,904-particle drop
-// at 2.4 m/s 43 -> 32; from 6 to 32 the split makes no difference there. (A function of its own: the registers of the
-// walks stay out of the list path, which alone gained 137 -> 134 us at 1M, 42 -> 39 with 103,736 boundary particles.)
+// Pressure sweep with few hundred to few thousand fast predictions: 1M jittered block 158 -> 146 us, a 98,904-particle drop
+// at 2.4 m/s 43 -> 31; from 6 to 32 the split makes no difference there. U: rounds with their gathers in flight.
 constexpr int kFewWalkers = 12;
 struct WalkStage {
     uint32_t delta[32];
     float term[96];
 };
-template <class PS, bool kCoherent>
-__device__ __noinline__ float pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
+template <class PS, bool kCoherent, int U>
+__device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
                                                uint32_t walkers, WalkStage& S) {
     const uint32_t lane = threadIdx.x & 31u;
     const bool mine = (walkers >> lane) & 1u;
@@ -1029,7 +1028,6 @@ __device__ __noinline__ float pressure_walkers(const PS& ps, const ListBuffers& 
                 n = 0;
                 __syncwarp();
             };
-            constexpr int U = 3;  // rounds with their gathers in flight
             for (uint32_t base = 0; base < w.total; base += 32u * U) {
                 float4 o[U];
 #pragma unroll
@@ -1056,9 +1054,15 @@ __device__ __noinline__ float pressure_walkers(const PS& ps, const ListBuffers& 
     return mine ? finish_pressure<PS>(b, P, ps.control(ii), ii, xi, acc) : 0.f;
 }
 
+template <class PS, bool kCoherent>
+__device__ __noinline__ float call_pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
+                                                    uint32_t walkers, WalkStage& S) {
+    return pressure_walkers<PS, kCoherent, 3>(ps, b, i, acc, walkers, S);
+}
+
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
-// stage: its WalkStage.
-template <class PS, bool kCoherent = false>
+// stage: its WalkStage. kWide: the walks as a function call.
+template <class PS, bool kCoherent, bool kWide>
 __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, WalkStage& stage) {
     float dv = 0.f, acc = 0.f;
     bool walk = false;
@@ -1117,7 +1121,9 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
     }
     const uint32_t walkers = __ballot_sync(kAll, walk);
     if (walkers) {
-        const float w = pressure_walkers<PS, kCoherent>(ps, b, i, acc, walkers, stage);
+        float w;
+        if constexpr (kWide) w = call_pressure_walkers<PS, kCoherent>(ps, b, i, acc, walkers, stage);
+        else w = pressure_walkers<PS, kCoherent, 2>(ps, b, i, acc, walkers, stage);
         if (walk) dv = w;
     }
     return dv;
@@ -1164,12 +1170,13 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
 }
 
 // BS: threads per block (128, 256 or 512; the autotuner's choice for one scene)
-template <class PS, int BS = kBlock, int LANES = 1>
-__global__ void __launch_bounds__(BS) k_pressure_list(PS ps, ListBuffers b) {
+// kWide: 32 warps per SM at 64 registers instead of 40 at 48, with more gathers in flight each (see launch_pressure_list)
+template <class PS, int BS = kBlock, int LANES = 1, bool kWide = true>
+__global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWide ? 1024 / BS : 1280 / BS) k_pressure_list(PS ps, ListBuffers b) {
     const uint32_t t = blockIdx.x * BS + threadIdx.x;
     float dv;
     __shared__ WalkStage stage[LANES == 1 ? BS / 32 : 1];
-    if constexpr (LANES == 1) dv = pressure_body(ps, b, t, stage[threadIdx.x >> 5]);
+    if constexpr (LANES == 1) dv = pressure_body<PS, false, kWide>(ps, b, t, stage[threadIdx.x >> 5]);
     else dv = pressure_shared<PS, LANES>(ps, b, t / LANES, t % LANES);
     if (PS::kBatched) return;
     // one scene: block max of dv, the last block decides (dv >= 0: bit patterns order like values)
@@ -1363,7 +1370,7 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
         unsigned local = 0;
         for (uint32_t r = 0; r < rounds; ++r)
             local = max(local, __float_as_uint(
-                                   pressure_body<PS, true>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
+                                   pressure_body<PS, true, true>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
                                                            stage[threadIdx.x >> 5])));
         if (!PS::kBatched) {  // batched scenes reduced per scene inside the body
             const unsigned m = __reduce_max_sync(0xffffffffu, local);
@@ -1554,10 +1561,19 @@ void launch_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, c
 void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, cudaStream_t s) {
     const OneScene ps{P, ctl};
     const uint32_t n = P.fluid_count;
+    auto go = [&](auto bs) {
+        constexpr int BS = decltype(bs)::value;
+        const unsigned blocks = (n + BS - 1) / BS;
+        // 64 registers a thread (4 blocks of 256 per SM) against 48 (5 blocks), us per launch: 201,600 particles 42 / 47,
+        // 286,720 44 / 52, 400,000 62 / 69, 600,000 80 / 91, 1,048,576 135 / 140, 1.6M and 2.6M equal, 4.2M 516 / 508,
+        // 8.4M 1071 / 1050; below, 48 as long as they hold the scene in one wave (156,244: 33 / 29).
+        if (n > 5u * 256u * 152u && n <= (1u << 21)) k_pressure_list<OneScene, BS, 1, true><<<blocks, BS, 0, s>>>(ps, b);
+        else k_pressure_list<OneScene, BS, 1, false><<<blocks, BS, 0, s>>>(ps, b);
+    };
     if (n <= kSharedMax) k_pressure_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b);
-    else if (block == 128) k_pressure_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b);
-    else if (block == 512) k_pressure_list<OneScene, 512><<<(n + 511) / 512, 512, 0, s>>>(ps, b);
-    else k_pressure_list<OneScene, kBlock><<<grid_for(n), kBlock, 0, s>>>(ps, b);
+    else if (block == 128) go(std::integral_constant<int, 128>{});
+    else if (block == 512) go(std::integral_constant<int, 512>{});
+    else go(std::integral_constant<int, kBlock>{});
 }
 void launch_mark_partners(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     k_mark_partners<<<kMarkBlocks, kBlock, 0, s>>>(P, ctl, b);
