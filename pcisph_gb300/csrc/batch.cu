@@ -144,6 +144,7 @@ struct pcisph_batch {
         BTRY(cudaMemset(tables.p, 0, tbytes));
         const size_t sbytes = RadixSorter::scratch_bytes(n, sorter.digit_bits());
         if (sort_block.ensure(sbytes) != cudaSuccess) return report_error(PCISPH_ERR_OOM, "device allocation of the sort scratch failed");
+        sorter.set_nearly_sorted();
         sorter.set_scratch(sort_block.p, sort_block.cap);
         BTRY(cudaMallocHost(&h_ctls, ns * sizeof(Control)));
         return PCISPH_OK;
@@ -469,7 +470,7 @@ int pcisph_batch_create(int device, void* stream, uint32_t max_particles, uint32
     if (device < 0 || device >= ndev) return report_error(PCISPH_ERR_INVALID_ARG, "no CUDA device " + std::to_string(device));
     DeviceGuard g(device);
     BTRY(cudaFree(nullptr));
-    BTRY(radix_configure_kernels());
+    BTRY(radix_configure_kernels(8));
     pcisph_batch* b = new pcisph_batch();
     b->device = device;
     b->max_particles = max_particles;
@@ -595,6 +596,7 @@ int pcisph_batch_autotune(pcisph_batch* b, uint32_t steps, pcisph_batch_tune_res
         if (!b->adaptive_skin) b->list_skin = skin;
         b->loop_mode = mode;
         b->sorter.set_digit_bits(bits);
+        BTRY(radix_configure_kernels(bits));
         b->sort_block.release();
         const size_t sbytes = RadixSorter::scratch_bytes(b->max_particles, bits);
         if (b->sort_block.ensure(sbytes) != cudaSuccess)

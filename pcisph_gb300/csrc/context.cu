@@ -375,6 +375,7 @@ struct pcisph_ctx {
         // (70.6 -> 60.5 us at 1M); other widths keep 8-bit digits. The autotuner may choose again.
         const int kb = key_bits(params.bucket_count);
         sorter.set_digit_bits(kb > 16 && kb <= 20 ? 10 : 8);
+        CUDA_TRY(radix_configure_kernels(sorter.digit_bits()));
         int rc = ensure_fluid(params.fluid_count, params.bucket_count);
         if (rc) return rc;
         rc = ensure_boundary(params.boundary_count, params.bucket_count);
@@ -1037,7 +1038,7 @@ int pcisph_create(int device, void* stream, pcisph_ctx** out) {
     if (device < 0 || device >= ndev) return fail(PCISPH_ERR_INVALID_ARG, "no CUDA device " + std::to_string(device));
     DeviceGuard g(device);
     CUDA_TRY(cudaFree(nullptr));  // create the primary context
-    CUDA_TRY(radix_configure_kernels());
+    CUDA_TRY(radix_configure_kernels(8));
     SweepGrid sg{};
     CUDA_TRY(sweep_configure(&sg));
     pcisph_ctx* c = new pcisph_ctx();
@@ -1055,6 +1056,7 @@ int pcisph_create(int device, void* stream, pcisph_ctx** out) {
         return fail(PCISPH_ERR_CUDA, std::string("context setup: ") + cudaGetErrorString(e));
     }
     c->user_stream = stream ? static_cast<cudaStream_t>(stream) : c->own_stream;
+    c->sorter.set_nearly_sorted();
     c->b.ctl = c->ctl = static_cast<Control*>(c->misc_block.p);
     std::memset(c->host_ctl, 0, sizeof(Control));
     *out = c;
@@ -1451,6 +1453,7 @@ int pcisph_autotune(pcisph_ctx* ctx, uint32_t steps, pcisph_tune_result* out) {
         int r = pcisph_set_options(ctx, &o);
         if (r) return r;
         ctx->sorter.set_digit_bits(bits);
+        CUDA_TRY(radix_configure_kernels(bits));
         ctx->sort_block.release();  // scratch size depends on the digit width
         ctx->sorted_keys = ctx->f_keys;  // no view into the released scratch survives
         ctx->sorted_ids = ctx->f_ids;
@@ -1616,7 +1619,7 @@ int pcisph_radixsort_create(int device, pcisph_radixsort** out) {
     if (!out) return fail(PCISPH_ERR_INVALID_ARG, "out is NULL");
     DeviceGuard g(device);
     CUDA_TRY(cudaFree(nullptr));
-    CUDA_TRY(radix_configure_kernels());
+    CUDA_TRY(radix_configure_kernels(8));
     *out = new pcisph_radixsort{device, {}};
     return PCISPH_OK;
 }
@@ -1631,6 +1634,8 @@ int pcisph_radixsort_set_digit_bits(pcisph_radixsort* s, int bits) {
     if (!s) return fail(PCISPH_ERR_INVALID_ARG, "sorter is NULL");
     if (bits == 0) bits = 8;
     if (bits < 4 || bits > 11) return fail(PCISPH_ERR_INVALID_ARG, "digit bits must be in 4..11");
+    DeviceGuard g(s->device);
+    CUDA_TRY(radix_configure_kernels(bits));
     s->sorter.set_digit_bits(bits);
     return PCISPH_OK;
 }

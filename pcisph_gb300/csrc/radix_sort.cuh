@@ -3,9 +3,11 @@
 // Replaces clogs::Radixsort (libs/clogs/include/clogs/radixsort.h:176-191), whose
 // contract is a stable key/value sort with an optional bound on key bits. Each
 // digit pass is reduce-then-scan: per-tile digit counts (upsweep), a scan of
-// every digit's tile counts (one CTA per digit), and a downsweep that ranks the
-// tile's keys stably (warp match + per-warp counters, in element order), stages
-// them in shared memory in digit order and writes each digit run coalesced.
+// every digit's tile counts (one warp per digit, or by the next kernel where the
+// tiles are few), and a downsweep that ranks the tile's keys stably (warp match or
+// ballots + per-warp counters, in element order), stages them in shared memory in
+// digit order and writes each digit run coalesced. Up to 8,192 keys are sorted by
+// one block in one launch.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -13,7 +15,7 @@
 
 namespace pcisph {
 
-// Keys per tile of the sort kernels (256 threads x 16 keys).
+// Keys per tile that the scratch holds digit counts for (512 threads x 8 keys).
 constexpr size_t kRadixTile = 4096;
 
 constexpr size_t radix_align256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -26,22 +28,16 @@ constexpr size_t radix_scratch_bytes(size_t n, int digit_bits) {
            radix_align256(((size_t)1 << digit_bits) * sizeof(uint32_t));
 }
 
-// Dynamic shared memory of the downsweep kernel for bits-wide digits (8 warps' 16-bit digit counters, two
+// Dynamic shared memory of the downsweep kernel for bits-wide digits (16 warps' 16-bit digit counters, two
 // digit tables, the tile's keys and values). Above 48 KB the kernel needs radix_configure_kernels().
 constexpr size_t radix_downsweep_smem(int bits) {
-    return (size_t)8 * ((size_t)1 << bits) * sizeof(unsigned short) + 2 * ((size_t)1 << bits) * sizeof(uint32_t) +
+    return (size_t)16 * ((size_t)1 << bits) * sizeof(unsigned short) + 2 * ((size_t)1 << bits) * sizeof(uint32_t) +
            2 * kRadixTile * sizeof(uint32_t);
 }
 
-// Raise the dynamic shared-memory limit of the wide-digit kernels on the current device.
-// Call once per device before the first sort (outside stream capture).
-cudaError_t radix_configure_kernels();
-
-struct RadixSortPlan {
-    int digit_bits = 8;
-    int passes = 0;
-    size_t tiles = 0;
-};
+// Raise the dynamic shared-memory limit of the kernels that sorts with digits of at most digit_bits bits take, on the
+// current device. Call before the first such sort (outside stream capture); again costs a few microseconds.
+cudaError_t radix_configure_kernels(int digit_bits);
 
 class RadixSorter {
    public:
@@ -56,6 +52,10 @@ class RadixSorter {
     void set_scratch(void* ptr, size_t bytes);
     void set_digit_bits(int bits) { digit_bits_ = bits; }
     int digit_bits() const { return digit_bits_; }
+    // Keep to kernels within the default 48 KB of shared memory (radix_configure_kernels() may not have run).
+    void set_small_smem() { small_smem_ = true; }
+    // The keys will come nearly sorted (a time step's, in the last step's order); any keys are sorted either way.
+    void set_nearly_sorted() { nearly_sorted_ = true; }
 
     // Sorts keys/values in place (result copied back if the pass count is odd, unless out_* are given).
     // If values_in_identity, the input values are taken as 0..n-1 and `values` is write-only.
@@ -70,6 +70,8 @@ class RadixSorter {
     void* scratch_ = nullptr;
     size_t scratch_cap_ = 0;
     bool owns_ = false;
+    bool small_smem_ = false;
+    bool nearly_sorted_ = false;
     int digit_bits_ = 8;
     int last_launches_ = 0;
 };

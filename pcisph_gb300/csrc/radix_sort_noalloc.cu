@@ -71,6 +71,7 @@ extern "C" int pcisph_radixsort_enqueue_noalloc(uint32_t* keys, uint32_t* values
     // and race; order them on one stream or with events.
     pcisph::RadixSorter sorter;
     sorter.set_digit_bits(kDigitBits);
+    sorter.set_small_smem();
     sorter.set_scratch(scratch, kScratchBytes);
     cudaError_t e = sorter.sort(keys, values, elements, max_bits == 0 ? 32 : (int)max_bits, false,
                                 static_cast<cudaStream_t>(stream));
