@@ -1061,8 +1061,9 @@ __device__ __noinline__ float call_pressure_walkers(const PS& ps, const ListBuff
 }
 
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
-// stage: its WalkStage. kWide: the walks as a function call.
-template <class PS, bool kCoherent, bool kWide>
+// stage: its WalkStage.
+enum class Walks { kLane, kInline, kCall };  // each lane by itself; pressure_walkers inline; or as a function call
+template <class PS, bool kCoherent, Walks kWalks>
 __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, WalkStage& stage) {
     float dv = 0.f, acc = 0.f;
     bool walk = false;
@@ -1112,17 +1113,23 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         auto fb = [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, __ldg(&b.b_pos[j]), P.h2); };
         if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
         else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
-        if (!walk) {
+        if (kWalks == Walks::kLane && walk) {
+            for_each_neighbour(b.cells, c, P, [&](uint32_t j) {
+                acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
+            });
+            walk = false;
+        } else if (!walk) {
             for_each_listed(b.nbr, i, cnt, b.nbr_stride, [&](uint32_t j) {
                 acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
             });
-            dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
         }
+        if (!walk) dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
     }
+    if constexpr (kWalks == Walks::kLane) return dv;
     const uint32_t walkers = __ballot_sync(kAll, walk);
     if (walkers) {
         float w;
-        if constexpr (kWide) w = call_pressure_walkers<PS, kCoherent>(ps, b, i, acc, walkers, stage);
+        if constexpr (kWalks == Walks::kCall) w = call_pressure_walkers<PS, kCoherent>(ps, b, i, acc, walkers, stage);
         else w = pressure_walkers<PS, kCoherent, 2>(ps, b, i, acc, walkers, stage);
         if (walk) dv = w;
     }
@@ -1170,13 +1177,14 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
 }
 
 // BS: threads per block (128, 256 or 512; the autotuner's choice for one scene)
-// kWide: 32 warps per SM at 64 registers instead of 40 at 48, with more gathers in flight each (see launch_pressure_list)
-template <class PS, int BS = kBlock, int LANES = 1, bool kWide = true>
-__global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWide ? 1024 / BS : 1280 / BS) k_pressure_list(PS ps, ListBuffers b) {
+// Walks::kCall: 32 warps per SM at 64 registers instead of 40 at 48, with more gathers in flight each (see
+// launch_pressure_list)
+template <class PS, int BS = kBlock, int LANES = 1, Walks kWalks = Walks::kCall>
+__global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1024 / BS : 1280 / BS) k_pressure_list(PS ps, ListBuffers b) {
     const uint32_t t = blockIdx.x * BS + threadIdx.x;
     float dv;
     __shared__ WalkStage stage[LANES == 1 ? BS / 32 : 1];
-    if constexpr (LANES == 1) dv = pressure_body<PS, false, kWide>(ps, b, t, stage[threadIdx.x >> 5]);
+    if constexpr (LANES == 1) dv = pressure_body<PS, false, kWalks>(ps, b, t, stage[threadIdx.x >> 5]);
     else dv = pressure_shared<PS, LANES>(ps, b, t / LANES, t % LANES);
     if (PS::kBatched) return;
     // one scene: block max of dv, the last block decides (dv >= 0: bit patterns order like values)
@@ -1370,7 +1378,7 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
         unsigned local = 0;
         for (uint32_t r = 0; r < rounds; ++r)
             local = max(local, __float_as_uint(
-                                   pressure_body<PS, true, true>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
+                                   pressure_body<PS, true, Walks::kCall>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
                                                            stage[threadIdx.x >> 5])));
         if (!PS::kBatched) {  // batched scenes reduced per scene inside the body
             const unsigned m = __reduce_max_sync(0xffffffffu, local);
@@ -1567,8 +1575,11 @@ void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b
         // 64 registers a thread (4 blocks of 256 per SM) against 48 (5 blocks), us per launch: 201,600 particles 42 / 47,
         // 286,720 44 / 52, 400,000 62 / 69, 600,000 80 / 91, 1,048,576 135 / 140, 1.6M and 2.6M equal, 4.2M 516 / 508,
         // 8.4M 1071 / 1050; below, 48 as long as they hold the scene in one wave (156,244: 33 / 29).
-        if (n > 5u * 256u * 152u && n <= (1u << 21)) k_pressure_list<OneScene, BS, 1, true><<<blocks, BS, 0, s>>>(ps, b);
-        else k_pressure_list<OneScene, BS, 1, false><<<blocks, BS, 0, s>>>(ps, b);
+        // Past 2M the walks in lane form, which need none of the spills of the inline form: 2.6M 321 -> 313 us, 8.4M
+        // 1050 -> 1036.
+        if (n > (1u << 21)) k_pressure_list<OneScene, BS, 1, Walks::kLane><<<blocks, BS, 0, s>>>(ps, b);
+        else if (n > 5u * 256u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall><<<blocks, BS, 0, s>>>(ps, b);
+        else k_pressure_list<OneScene, BS, 1, Walks::kInline><<<blocks, BS, 0, s>>>(ps, b);
     };
     if (n <= kSharedMax) k_pressure_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b);
     else if (block == 128) go(std::integral_constant<int, 128>{});
