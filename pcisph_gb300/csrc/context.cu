@@ -115,8 +115,8 @@ struct pcisph_ctx {
     bool working_order() const {
         return list_sweeps() && (opts.spatial_order == 1 || (opts.spatial_order == 2 && params.fluid_count >= (1u << 17)));
     }
-    // marks: the launch follows the partner-marking kernel of its round (the graph's and the host-driven
-    // loop's pressure sweeps, and that kernel itself): the pressure sweep may read the stamps
+    // marks: a pressure sweep of the graph or the host-driven loop (it reads the stamps), the marking kernel, or a
+    // predicting sweep that marks by itself
     ListBuffers list_buffers(bool marks = false) const {
         const bool w = working_order();
         const bool m = P.mark_cap != 0;
@@ -126,10 +126,11 @@ struct pcisph_ctx {
                            w ? d_of_w : nullptr, b.disp_max, b.state_skin, b.b_init, b.b_press, b.b_near, b.bnbr,
                            b.bnbr_count, b.bfl,
                            b.bfl_count, zone_map, {zone_org[0], zone_org[1], zone_org[2]},
-                           {zone_dim[0], zone_dim[1], zone_dim[2]}, m ? b.fast_list : nullptr,
+                           {zone_dim[0], zone_dim[1], zone_dim[2]},
+                           m && !marks_inline(P.fluid_count) ? b.fast_list : nullptr,
                            m && marks ? b.walk_stamp : nullptr};
     }
-    // the partner-marking kernel runs after each prediction round of the graph and the host-driven loop
+    // the partners of fast predictions are marked in the graph and the host-driven loop
     bool partner_marks() const { return list_sweeps() && P.mark_cap != 0 && opts.loop_mode != 2; }
 
     // Working-order buffers for n particles and bk buckets; the index maps start as the identity.
@@ -521,11 +522,12 @@ struct pcisph_ctx {
             timed("normal", s, [&] { launch_normal(P, b, s); });
         }
         if (B && cudaMemsetAsync(b.b_press, 0, (size_t)B * 4, s) != cudaSuccess) return -1;
-        if (list_sweeps()) timed("force", s, [&] { launch_force_list(P, b.ctl, list_buffers(), s); });
+        if (list_sweeps())
+            timed("force", s, [&] { launch_force_list(P, b.ctl, list_buffers(partner_marks() && marks_inline(N)), s); });
         else if (warp_sweeps()) timed("force", s, [&] { launch_force_sweep(P, b, A, sweep_grid, s); });
         else timed("force", s, [&] { launch_force(P, b, s); });
         nl += 4;
-        if (partner_marks()) {
+        if (partner_marks() && !marks_inline(N)) {
             timed("mark", s, [&] { launch_mark_partners(P, b.ctl, list_buffers(true), s); });
             ++nl;
         }
@@ -543,12 +545,12 @@ struct pcisph_ctx {
             ++nl;
         }
         if (list_sweeps()) {
-            const bool marks = partner_marks();
+            const bool marks = partner_marks(), inline_marks = marks && marks_inline(params.fluid_count);
             timed("pressure", s, [&] { launch_pressure_list(P, b.ctl, list_buffers(marks), opts.sweep_block, s); });
             timed("pressure_force", s, [&] {
-                launch_pressure_force_list(P, b.ctl, list_buffers(), 0, cond, use_cond, opts.sweep_block, s);
+                launch_pressure_force_list(P, b.ctl, list_buffers(inline_marks), 0, cond, use_cond, opts.sweep_block, s);
             });
-            if (marks) {
+            if (marks && !inline_marks) {
                 timed("mark", s, [&] { launch_mark_partners(P, b.ctl, list_buffers(true), s); });
                 ++nl;
             }

@@ -48,9 +48,6 @@ namespace {
 
 constexpr int kBlock = 256;
 inline unsigned grid_for(uint32_t n) { return (n + kBlock - 1) / kBlock; }
-// The marking kernel's grid (grid-stride over its items): 4 blocks an SM. A round of ~3,000 fast predictions at 1M takes
-// 13 us (21 with one block an SM), a round without any 2.5 either way.
-constexpr unsigned kMarkBlocks = 608;
 
 // List layout: entries k = 8c .. 8c+7 of particle i (chunk c) are 32 contiguous bytes at uint4 offset
 // 2 (c * stride + i); chunks are column-major over particles. A warp's 32 consecutive particles read
@@ -272,13 +269,8 @@ struct CellWalk {
     uint32_t off;    // where this lane's bucket begins in the concatenation (kAll: empty, or no bucket)
     uint32_t rank;   // the last bucket begun before the next round
 };
-__device__ __forceinline__ CellWalk begin_cell(const uint2* __restrict__ cells, const DevParams& P, uint32_t cx,
-                                               uint32_t cy, uint32_t cz, uint32_t lane, uint32_t* delta) {
-    uint2 r = make_uint2(0u, 0u);
-    if (lane < 27u) {
-        const uint32_t dz = lane / 9u, dy = (lane / 3u) % 3u, dx = lane % 3u;
-        r = __ldg(&cells[P.bucket_base + hash_key(cx + dx - 1u, cy + dy - 1u, cz + dz - 1u, P)]);
-    }
+// The lanes' ranges concatenated in lane order.
+__device__ __forceinline__ CellWalk concatenate(const uint2& r, uint32_t lane, uint32_t* delta) {
     const uint32_t len = r.y > r.x ? r.y - r.x : 0u;
     uint32_t incl = len;
 #pragma unroll
@@ -291,10 +283,29 @@ __device__ __forceinline__ CellWalk begin_cell(const uint2* __restrict__ cells, 
     w.rank = kAll;
     const uint32_t filled = __ballot_sync(kAll, len != 0u);
     w.off = len ? incl - len : kAll;
-    __syncwarp();  // the last cell's reads of delta are done
+    __syncwarp();  // the last reads of delta are done
     if (len) delta[__popc(filled & lanes_below())] = r.x - w.off;
     __syncwarp();
     return w;
+}
+__device__ __forceinline__ CellWalk begin_cell(const uint2* __restrict__ cells, const DevParams& P, uint32_t cx,
+                                               uint32_t cy, uint32_t cz, uint32_t lane, uint32_t* delta) {
+    uint2 r = make_uint2(0u, 0u);
+    if (lane < 27u) {
+        const uint32_t dz = lane / 9u, dy = (lane / 3u) % 3u, dx = lane % 3u;
+        r = __ldg(&cells[P.bucket_base + hash_key(cx + dx - 1u, cy + dy - 1u, cz + dz - 1u, P)]);
+    }
+    return concatenate(r, lane, delta);
+}
+
+// The particle at position base + lane of the concatenation (kAll past its end); base goes up by 32 from 0.
+__device__ __forceinline__ uint32_t next_candidate(CellWalk& w, uint32_t base, uint32_t lane, const uint32_t* delta) {
+    // the buckets that begin in this round, as bits of their first position
+    const uint32_t rel = w.off - base;
+    const uint32_t begun = __reduce_or_sync(kAll, rel < 32u ? 1u << rel : 0u);
+    const uint32_t f = base + lane, k = w.rank + __popc(begun & (2u * lanes_below() + 1u));
+    w.rank += __popc(begun);
+    return f < w.total ? f + delta[k & 31u] : kAll;
 }
 
 // The next kCellRounds rounds of candidates from position base: index and position, NaN beyond the last (no test
@@ -314,7 +325,7 @@ __device__ __forceinline__ void load_candidates(Candidates& c, CellWalk& w, uint
     c.count = min(w.total - base, (uint32_t)kCellRounds * 32u);
 #pragma unroll
     for (int u = 0; u < kCellRounds; ++u) {
-        // the buckets that begin in this round, as bits of their first position
+        // next_candidate, written out: as a call with its end test on the result the builder took 490 us at 1M, not 482
         const uint32_t rel = w.off - (base + u * 32u);
         const uint32_t begun = __reduce_or_sync(kAll, rel < 32u ? 1u << rel : 0u);
         const uint32_t f = base + u * 32u + lane;
@@ -715,9 +726,125 @@ __global__ void __launch_bounds__(kBlock) k_normal_list(PS ps, ListBuffers b) {
     b.normal[i] = make_float4(n.x * scale, n.y * scale, n.z * scale, 0.f);
 }
 
-// The force sweep's epilogue from its three sums, and the first predict (pcisph.cl:175-193, F_p = 0).
+// Partner marks of a prediction round (one scene). A pair of the reference's walk whose predictions are within h is in the
+// skin list unless one of the two predictions is fast (moved more than half the skin), so the pressure sweep of particle
+// i can use its list unless i is fast or some fast j has x*_j within h of x*_i while j is not in i's list. For every fast
+// j, particle i is stamped with the round's number when |x_i - x_j| is beyond i's list radius (the builder's test, the
+// same bits) and x*_j comes close enough, and j itself is stamped. Stamping more than needed only makes a particle walk,
+// which gives the walk's sum. The round is the one the next pressure sweep reads (Control::round + 1); that sweep's last
+// block closes it.
+//
+// Cell o of the 5 x 5 x 5 cells around x*_j's cell c0, if particles in it can be partners: a particle that is not fast
+// lies within D = h + skin_max_half (< 2 cells, checked on the host) of such an x*_j, so its cell is among them, and its
+// box comes within D of x*_j (with a margin for the divisions of cell_of). Within 2^14 cells of the origin the rounding of
+// the box bounds and of cell_of's division is far below that margin; farther out (or saturated, or NaN) every cell counts.
+__device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& pj, const Cell& c0, uint32_t o, Cell& c) {
+    c = Cell{c0.x + o % 5u - 2u, c0.y + o / 5u % 5u - 2u, c0.z + o / 25u - 2u};
+    auto inner = [](uint32_t v) { return v + 16384u < 32768u; };  // -2^14 < (int)v < 2^14, wrapping
+    if (!(inner(c0.x) && inner(c0.y) && inner(c0.z))) return true;
+    auto gap = [&](uint32_t v, float x) {  // distance from x to the cell along an axis
+        const float lo = (float)(int)v * P.cell_size, hi = lo + P.cell_size;
+        return fmaxf(fmaxf(lo - x, x - hi), 0.f);
+    };
+    const float gx = gap(c.x, pj.x), gy = gap(c.y, pj.y), gz = gap(c.z, pj.z);
+    const float reach = P.h + P.skin_max_half + 0.01f * P.cell_size;
+    return !(gx * gx + gy * gy + gz * gz > reach * reach);
+}
+__device__ __forceinline__ bool beyond_list(const DevParams& P, const float4& xi, const float4& xj) {
+    return !(dist2(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z) <= particle_list_r2(P, half_skin_of(P, xi.w)));
+}
+
+// After a prediction round: a thread per (fast prediction that the round listed, cell). Close enough: |x*_i - x*_j| <= h
+// (the pressure sweep's |d|^2, with d negated: the same bits). A round with more than mark_cap fast predictions stamps
+// nothing (the sweep then uses the bucket flags), nor does a step of moving lists. Grid-stride over the items, 4 blocks an
+// SM: a round of ~3,000 fast predictions at 1M takes 13 us (21 with one block an SM; 14 with a warp per prediction), a
+// round without any 2.5.
+constexpr unsigned kMarkBlocks = 608;
+__global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Control* ctl, ListBuffers b) {
+    const unsigned long long n = ctl->fast_n;
+    if (n == 0 || n > P.mark_cap) return;
+    const unsigned round = ctl->round + 1u;
+    const unsigned long long items = n * 125ull;
+    for (unsigned long long t = (unsigned long long)blockIdx.x * kBlock + threadIdx.x; t < items;
+         t += (unsigned long long)gridDim.x * kBlock) {
+        const uint32_t j = b.fast_list[t / 125ull];
+        const uint32_t o = (uint32_t)(t % 125ull);
+        if (o == 62u) b.walk_stamp[j] = round;  // the centre cell's thread: j itself walks
+        const float4 pj = b.pred[j];
+        const float4 xj = b.pos[j];
+        Cell c;
+        if (!partner_cell(P, pj, cell_of(pj.x, pj.y, pj.z, P), o, c)) continue;
+        const uint2 r = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
+#pragma unroll 1
+        for (uint32_t i0 = r.x; i0 < r.y; i0 += 4) {
+            float4 pi[4], xi[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u < r.y) {
+                    pi[u] = b.pred[i0 + u];
+                    xi[u] = b.pos[i0 + u];
+                }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (i0 + u < r.y && dist2(pj.x - pi[u].x, pj.y - pi[u].y, pj.z - pi[u].z) <= P.h2 &&
+                    beyond_list(P, xi[u], xj))
+                    b.walk_stamp[i0 + u] = round;
+        }
+    }
+}
+
+// The same by the warp that predicts, for the fast predictions set of its lanes' particles i (the whole warp calls). Close
+// enough: |x_i - x*_j| <= D, which needs no other prediction of the round. It saves the launch after each round (4,096
+// particles, 7 rounds: 182 -> 166 us a step). Larger scenes lose: the fast predictions of a warp follow one another (120K
+// particles, up to 1 in 8 fast: pressure force 26 -> 108 us against 26 + 15 with the kernel).
+__device__ __noinline__ void mark_partners_inline(const DevParams& P, Control* ctl, const ListBuffers& b, uint32_t i,
+                                                  unsigned set, uint32_t* delta) {
+    const uint32_t lane = threadIdx.x & 31u;
+    unsigned long long base = ~0ull;
+    if (lane == 0 && *(volatile unsigned long long*)&ctl->fast_n <= P.mark_cap)
+        base = atomicAdd(&ctl->fast_n, (unsigned long long)__popc(set));
+    base = __shfl_sync(kAll, base, 0);
+    if (base >= P.mark_cap) return;  // past the cap: the sweep takes the bucket flags
+    __syncwarp();                    // the lanes' predictions are stored
+    const unsigned round = ctl->round + 1u;
+    const float far = P.h + P.skin_max_half + 1e-4f * P.h;  // D, past the rounding of the distances
+    for (; set; set &= set - 1u) {
+        const uint32_t j = __shfl_sync(kAll, i, __ffs(set) - 1);
+        const float4 pj = b.pred[j], xj = b.pos[j];
+        const Cell c0 = cell_of(pj.x, pj.y, pj.z, P);
+        if (lane == 0) b.walk_stamp[j] = round;
+        uint2 r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t o = lane + 32u * q;
+            Cell c;
+            r[q] = make_uint2(0u, 0u);
+            if (o < 125u && partner_cell(P, pj, c0, o, c)) r[q] = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            CellWalk w = concatenate(r[q], lane, delta);
+            for (uint32_t at = 0; at < w.total; at += 32u) {
+                const uint32_t k = next_candidate(w, at, lane, delta);
+                if (k == kAll) continue;
+                const float4 x = b.pos[k];
+                if (dist2(pj.x - x.x, pj.y - x.y, pj.z - x.z) <= far * far && beyond_list(P, x, xj))
+                    b.walk_stamp[k] = round;
+            }
+        }
+    }
+}
 template <class PS>
-__device__ __forceinline__ void finish_force(const PS& ps, const ListBuffers& b, const DevParams& P, uint32_t i,
+__device__ __forceinline__ void close_round(const PS& ps, const ListBuffers& b, uint32_t i, bool fast, uint32_t* delta) {
+    if (PS::kBatched || !b.walk_stamp) return;
+    const unsigned set = __ballot_sync(kAll, fast);
+    if (set) mark_partners_inline(ps.params(0), ps.control(0), b, i, set, delta);
+}
+
+// The force sweep's epilogue from its three sums, and the first predict (pcisph.cl:175-193, F_p = 0); returns whether the
+// prediction is fast.
+template <class PS>
+__device__ __forceinline__ bool finish_force(const PS& ps, const ListBuffers& b, const DevParams& P, uint32_t i,
                                              const float4& xi, const float3& vi, const float3& visc, const float3& coh,
                                              const float3& curv) {
     const float m = P.particle_mass;
@@ -729,9 +856,11 @@ __device__ __forceinline__ void finish_force(const PS& ps, const ListBuffers& b,
     const float3 dx = v * P.dt;
     const float4 xs = make_float4(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z, 0.f);
     b.pred[i] = xs;
+    bool fast;
     const float disp = note_displacement<!PS::kBatched>(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin, vi,
-                                                        PS::kBatched ? nullptr : b.fast_list, i);
+                                                        fast, PS::kBatched ? nullptr : b.fast_list, i);
     if (P.particle_skin) b.disp_max[i] = disp;
+    return fast;
 }
 
 // pcisph.cl:121-173, then the first predict
@@ -832,71 +961,10 @@ __global__ void __launch_bounds__(kBlock) k_force_shared(PS ps, ListBuffers b) {
         return make_float3(__shfl_sync(mask, v, 0, L), __shfl_sync(mask, v, 1, L), __shfl_sync(mask, v, 2, L));
     };
     const float3 sv = all(visc), sc = all(coh), su = all(curv);
-    if (live && q == 0) finish_force(ps, b, P, i, xi, vi, sv, sc, su);
-}
-
-// Partner marks after a prediction round (one scene). A pair of the reference's walk whose predictions are
-// within h is in the skin list unless one of the two predictions is fast (moved more than half the skin), so
-// the pressure sweep of particle i can use its list unless i is fast or some fast j has x*_j within h of
-// x*_i while j is not in i's list. For every fast j of the round (the fast list), thread (j, o) takes cell o
-// of the 5 x 5 x 5 cells around x*_j's cell: a particle i that is not fast lies within
-// D = h + skin_max_half (< 2 cells, checked on the host) of x*_j, so its cell is among them, and only the
-// cells whose box comes within D of x*_j (with a margin for the divisions of cell_of) are scanned. It stamps i
-// with the round's number when |x*_i - x*_j| <= h (the pressure sweep's |d|^2, with d negated: the same bits)
-// and |x_i - x_j| is beyond i's list radius (the builder's test, the same bits), and stamps j itself.
-// Stamping more than needed only makes a particle walk, which gives the walk's sum. The round is the one the
-// next pressure sweep reads (Control::round + 1); that sweep's last block closes it. A round with more than
-// mark_cap fast predictions stamps nothing (the sweep then uses the bucket flags), nor does a step of moving lists (no
-// fast prediction is listed).
-__global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Control* ctl, ListBuffers b) {
-    const unsigned long long n = ctl->fast_n;
-    if (n == 0 || n > P.mark_cap) return;
-    const unsigned round = ctl->round + 1u;
-    const float reach = P.h + P.skin_max_half + 0.01f * P.cell_size;
-    const unsigned long long items = n * 125ull;
-    for (unsigned long long t = (unsigned long long)blockIdx.x * kBlock + threadIdx.x; t < items;
-         t += (unsigned long long)gridDim.x * kBlock) {
-        const uint32_t j = b.fast_list[t / 125ull];
-        const uint32_t o = (uint32_t)(t % 125ull);
-        if (o == 62u) b.walk_stamp[j] = round;  // the centre cell's thread: j itself walks
-        const float4 pj = b.pred[j];
-        const float4 xj = b.pos[j];
-        const Cell c0 = cell_of(pj.x, pj.y, pj.z, P);
-        const int off[3] = {(int)(o % 5u) - 2, (int)(o / 5u % 5u) - 2, (int)(o / 25u) - 2};
-        const uint32_t cc[3] = {c0.x + (uint32_t)off[0], c0.y + (uint32_t)off[1], c0.z + (uint32_t)off[2]};
-        // Skip a cell whose box is farther than the reach from x*_j. Within 2^14 cells of the origin the
-        // rounding of the box bounds and of cell_of's division is far below the margin in the reach; farther
-        // out (or saturated, or NaN) every cell is scanned.
-        auto inner = [](uint32_t c) { return c + 16384u < 32768u; };  // -2^14 < (int)c < 2^14, wrapping
-        if (inner(c0.x) && inner(c0.y) && inner(c0.z)) {
-            const float pc[3] = {pj.x, pj.y, pj.z};
-            float gap2 = 0.f;  // squared distance from x*_j to the cell's box
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float lo = (float)(int)cc[a] * P.cell_size, hi = lo + P.cell_size;
-                const float g = fmaxf(fmaxf(lo - pc[a], pc[a] - hi), 0.f);
-                gap2 += g * g;
-            }
-            if (gap2 > reach * reach) continue;
-        }
-        const uint2 r = b.cells[P.bucket_base + hash_key(cc[0], cc[1], cc[2], P)];
-#pragma unroll 1
-        for (uint32_t i0 = r.x; i0 < r.y; i0 += 4) {
-            float4 pi[4], xi[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (i0 + u < r.y) {
-                    pi[u] = b.pred[i0 + u];
-                    xi[u] = b.pos[i0 + u];
-                }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (i0 + u < r.y && dist2(pj.x - pi[u].x, pj.y - pi[u].y, pj.z - pi[u].z) <= P.h2 &&
-                    !(dist2(xi[u].x - xj.x, xi[u].y - xj.y, xi[u].z - xj.z) <=
-                      particle_list_r2(P, half_skin_of(P, xi[u].w))))
-                    b.walk_stamp[i0 + u] = round;
-        }
-    }
+    bool fast = false;
+    if (live && q == 0) fast = finish_force(ps, b, P, i, xi, vi, sv, sc, su);
+    __shared__ uint32_t delta[kBlock];
+    close_round(ps, b, i, fast, delta + (threadIdx.x & ~31u));
 }
 
 // pcisph.cl:212-263 (boundary_update = 0); one scene: also the stop decision in the last block
@@ -1032,11 +1100,8 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
                 float4 o[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const uint32_t rel = w.off - (base + u * 32u);
-                    const uint32_t begun = __reduce_or_sync(kAll, rel < 32u ? 1u << rel : 0u);
-                    const uint32_t f = base + u * 32u + lane, k = w.rank + __popc(begun & (2u * below + 1u));
-                    w.rank += __popc(begun);
-                    if (f < w.total) o[u] = load_slot<kCoherent>(&b.pred[f + S.delta[k & 31u]]);
+                    const uint32_t j = next_candidate(w, base + u * 32u, lane, S.delta);
+                    if (j != kAll) o[u] = load_slot<kCoherent>(&b.pred[j]);
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
@@ -1216,9 +1281,9 @@ __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1
 
 // pcisph.cl:265-300, then predict (pcisph.cl:175-193) or integrate with optional walls
 // After the pressure-force sum f: predict (mode 0 before the decision, 1) or integrate (mode 0 after it, 2) with
-// optional walls.
+// optional walls. Returns whether a prediction is fast.
 template <class PS>
-__device__ __forceinline__ void finish_pressure_force(const PS& ps, const ListBuffers& b, const DevParams& P,
+__device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBuffers& b, const DevParams& P,
                                                       Control* ctl, uint32_t i, const float4& xi, const float3& f,
                                                       int mode) {
     const float m = P.particle_mass;
@@ -1234,10 +1299,11 @@ __device__ __forceinline__ void finish_pressure_force(const PS& ps, const ListBu
     if (!integrate) {
         const float4 xs = f4(x, 0.f);
         b.pred[i] = xs;
-        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin, vi,
+        bool fast;
+        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin, vi, fast,
                                                             PS::kBatched ? nullptr : b.fast_list, i);
         if (P.particle_skin) b.disp_max[i] = fmaxf(b.disp_max[i], disp);
-        return;
+        return fast;
     }
     if (P.walls) {
 #pragma unroll
@@ -1258,6 +1324,7 @@ __device__ __forceinline__ void finish_pressure_force(const PS& ps, const ListBu
     b.state_vel[o] = f4(v, 0.f);
     if (P.particle_skin)  // the next step's half skin: twice this step's largest predicted displacement
         b.state_skin[o] = fminf(fmaxf(P.skin_factor * b.disp_max[i], P.skin_min_half), P.skin_max_half);
+    return false;
 }
 
 // One particle's pressure-force sweep.
@@ -1293,9 +1360,9 @@ __device__ __forceinline__ void pressure_force_body(const PS& ps, const ListBuff
     finish_pressure_force(ps, b, P, ctl, i, xi, f, mode);
 }
 
-// The same with eight lanes per particle, lane q.
+// The same with eight lanes per particle, lane q; lane 0 returns whether the prediction is fast.
 template <class PS, int L>
-__device__ __forceinline__ void pressure_force_shared(const PS& ps, const ListBuffers& b, uint32_t i0, uint32_t q,
+__device__ __forceinline__ bool pressure_force_shared(const PS& ps, const ListBuffers& b, uint32_t i0, uint32_t q,
                                                       TermStage<L>& S, int mode) {
     const bool live = i0 < ps.count() && !ps.skip_force(i0);
     const uint32_t i = i0 < ps.count() ? i0 : ps.count() - 1u;
@@ -1332,8 +1399,8 @@ __device__ __forceinline__ void pressure_force_shared(const PS& ps, const ListBu
         [&](const float4& o, bool valid) { sum(o, valid, kAll); });
     if (cnt > P.near_cap) walk(b.cells, b.pf4);
     const float y = __shfl_sync(mask, acc, 1, L), z = __shfl_sync(mask, acc, 2, L);
-    if (live && q == 0)
-        finish_pressure_force(ps, b, P, ps.control(i), i, xi, make_float3(acc, y, z), mode);
+    if (live && q == 0) return finish_pressure_force(ps, b, P, ps.control(i), i, xi, make_float3(acc, y, z), mode);
+    return false;
 }
 
 template <class PS, int BS = kBlock, int LANES = 1, int DEEP = 1>
@@ -1352,7 +1419,10 @@ __global__ void __launch_bounds__(BS, LANES == 1 && DEEP == 1 ? 1536 / BS : 1) k
         pressure_force_body<PS, false, DEEP>(ps, b, i, mode);
     } else {
         __shared__ TermStage<LANES> stage[BS / LANES];
-        pressure_force_shared<PS, LANES>(ps, b, i / LANES, i % LANES, stage[threadIdx.x / LANES], mode);
+        const bool fast =
+            pressure_force_shared<PS, LANES>(ps, b, i / LANES, i % LANES, stage[threadIdx.x / LANES], mode);
+        __shared__ uint32_t delta[BS];
+        close_round(ps, b, i / LANES, fast, delta + (threadIdx.x & ~31u));
     }
 }
 
@@ -1586,6 +1656,7 @@ void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b
     else if (block == 512) go(std::integral_constant<int, 512>{});
     else go(std::integral_constant<int, kBlock>{});
 }
+bool marks_inline(uint32_t n) { return n <= kSharedMax; }
 void launch_mark_partners(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     k_mark_partners<<<kMarkBlocks, kBlock, 0, s>>>(P, ctl, b);
 }

@@ -43,8 +43,9 @@ struct ListBuffers {
     int zone_org[3];
     uint32_t zone_dim[3];
     // partner marks (one scene, or null): the fast predictions of the round (DevParams::mark_cap entries), and
-    // per particle the last round in which the marking kernel stamped it to walk. walk_stamp is null in the
-    // launches that do not follow a marking kernel (the stage runner, the persistent loop).
+    // per particle the last round that stamped it to walk. walk_stamp is null in the launches whose pressure sweeps
+    // take the bucket flags (the stage runner, the persistent loop) and in predicting sweeps that a marking kernel
+    // follows.
     uint32_t* fast_list;
     uint32_t* walk_stamp;
 };
@@ -103,6 +104,8 @@ void launch_boundary_pressure_list(const DevParams& P, Control* ctl, const ListB
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 void launch_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
+// Do the force and pressure-force sweeps of n particles mark by themselves (given b.walk_stamp; b.fast_list null)?
+bool marks_inline(uint32_t n);
 // Partner marks of the prediction round just completed (DevParams::mark_cap; b.fast_list and b.walk_stamp
 // set): the particles whose next pressure sweep must walk. That sweep (launched with b.walk_stamp) closes
 // the round.

@@ -30,17 +30,17 @@ __device__ __forceinline__ void warp_count(unsigned long long* addr, bool pred) 
 // past each adaptive skin level are counted. With a fast list (partner marks, one scene), a fast particle
 // also takes a slot of the round's list while the round holds at most P.mark_cap of them (one atomic per
 // warp that has one; none once the round is past the cap, which then falls back to the bucket flags).
-// Returns the displacement |x* - x|; threshold: the particle's fast_threshold. kOne: one scene, whose lists may move
+// Returns the displacement |x* - x|; threshold: the particle's fast_threshold; fast: whether it is past it. kOne: one scene, whose lists may move
 // with the particles (then the bucket is flagged when the prediction strays from y, and the round's count is past the
 // cap, so that nothing is listed); vi: the velocity at the step's start.
 template <bool kOne>
 __device__ __forceinline__ float note_displacement(const DevParams& P, Control* ctl,
                                                    unsigned char* __restrict__ bucket_fast, const float4& xi,
-                                                   const float4& xs, float threshold, const float3& vi,
+                                                   const float4& xs, float threshold, const float3& vi, bool& fast,
                                                    uint32_t* __restrict__ fast_list = nullptr, uint32_t i = 0) {
     const float dx = xs.x - xi.x, dy = xs.y - xi.y, dz = xs.z - xi.z;  // exact: xs and xi are close
     const float disp = sqrtf(dist2(dx, dy, dz));
-    const bool fast = disp > threshold;
+    fast = disp > threshold;
     warp_count(&ctl->fast_particles, fast);
     bool flag = fast;
     if (kOne) {
