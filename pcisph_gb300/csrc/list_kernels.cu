@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_density_list(PS ps, ListBuffe
 
 // pcisph.cl:94-112
 template <class PS, int DEEP = 1>
-__global__ void __launch_bounds__(kBlock) k_normal_list(PS ps, ListBuffers b) {
+__global__ void __launch_bounds__(kBlock, DEEP == 1 ? 1 : 2) k_normal_list(PS ps, ListBuffers b) {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i >= ps.count()) return;
     const DevParams& P = ps.params(i);
@@ -1405,7 +1405,7 @@ __device__ __forceinline__ bool pressure_force_shared(const PS& ps, const ListBu
 
 template <class PS, int BS = kBlock, int LANES = 1, int DEEP = 1>
 // (at most 40 registers: 48 resident warps per SM; 48 registers measured 10% slower at 1M)
-__global__ void __launch_bounds__(BS, LANES == 1 && DEEP == 1 ? 1536 / BS : 1) k_pressure_force_list(PS ps, ListBuffers b, int mode,
+__global__ void __launch_bounds__(BS, LANES > 1 ? 1 : DEEP == 1 ? 1536 / BS : 512 / BS) k_pressure_force_list(PS ps, ListBuffers b, int mode,
                                                             cudaGraphConditionalHandle cond, int use_cond) {
     const uint32_t i = blockIdx.x * BS + threadIdx.x;
     if (!PS::kBatched && use_cond && i == 0) {
@@ -1596,11 +1596,11 @@ void launch_density(const PS& ps, uint32_t n, bool boundary, const ListBuffers& 
             }
         k_density_list<PS, false, W><<<grid_cells(n, W), kCellBlock, 0, s>>>(ps, b);
     };
-    // Fewer particles per warp where warps are few: with 8 / 4 / 2 a warp 32,768 particles take 28 / 27 / 32 us (4,096:
-    // 12 with 8, 10 with 2); from there on the set-up of a cell per warp costs more than it spreads (156,244 particles
+    // Fewer particles per warp where warps are few: 4,096 particles take 12 us with 8, 10 with 2 (32,768: 28 / 27 / 32 us
+    // with 8 / 4 / 2, and 8 scenes at once 7% less time each with 8); from there on the set-up of a cell per warp costs more than it spreads (156,244 particles
     // 82 / 95 / 129 us, 1,048,576 495 / 605 / 845).
     if (n <= 8192u) go(std::integral_constant<int, 2>{});
-    else if (n <= 49152u) go(std::integral_constant<int, 4>{});
+    else if (n <= 16384u) go(std::integral_constant<int, 4>{});
     else go(std::integral_constant<int, 8>{});
 }
 }  // namespace
