@@ -46,6 +46,10 @@ struct DevParams {
     // 1 in kMovingShare particles that move kMovingSpeed of half the skin or more per step, the skin lists are built around y = x + v dt
     // (moving_place) and a prediction is measured from there: a body that moves as a whole keeps its lists
     int moving_lists;
+    // tight lists (the list sweeps without per-particle skins; see the list sweeps): the distance that a prediction may
+    // move from where the tight lists were built (0: none are built), the same less a margin for rounding, and the
+    // lists' radius^2, (h + 2 tight_margin)^2
+    float tight_margin, tight_reach, tight_r2;
     // batched scenes with an adaptive skin: each step picks one of kSkinLevels skins from the previous
     // step's count of predictions past each level's half skin (skin_half[k])
     int adaptive_skin;
@@ -85,6 +89,10 @@ struct Control {
     unsigned long long fast_n;
     unsigned int round;
     unsigned int moving;         // moving lists: the particles that fast (kMovingSpeed) when the step began
+    // tight lists: how the next pressure sweep finds its neighbours (kTightOff, kTightBuild or kTightUse), whether a
+    // prediction left their reach since they were built, the sweeps that used them, and how long the next sweeps do
+    // without after a building that served none
+    unsigned int tight_next, tight_stray, tight_age, tight_wait, tight_backoff;
     unsigned int lists_outrun;   // one scene: some prediction of this step was fast (1), measured from the place that
                                  // the step's lists are built around; it flagged its bucket
 };
@@ -105,6 +113,10 @@ __device__ __forceinline__ void close_step(Control* ctl, unsigned it, float rel,
     ctl->total_iters += it;
 }
 
+constexpr uint32_t kTightCap = 64;      // tight list entries per particle
+constexpr float kTightMargin = 0.035f;  // of h
+constexpr unsigned kTightAgain = 6;     // tight lists that were left behind are rebuilt from this iteration on
+constexpr unsigned kTightOff = 0, kTightBuild = 1, kTightUse = 2;
 constexpr uint32_t kNearCap = 64;  // within-h list entries per particle
 
 // Moving lists (DevParams::moving_lists): the share of fast particles from which a step takes them. The two list radii then
@@ -133,6 +145,13 @@ __host__ __device__ inline void set_list_skin(DevParams* d, float skin) {
     d->list_r2 = d->list_r * d->list_r;
     d->list_half_skin = 0.5f * d->h * skin - 1e-6f * d->h;
     d->skin_max_half = 0.5f * d->h * skin;
+}
+
+__host__ __device__ inline void set_tight_lists(DevParams* d, bool on) {
+    d->tight_margin = on ? kTightMargin * d->h : 0.f;
+    d->tight_reach = on ? kTightMargin * d->h - 1e-6f * d->h : 0.f;
+    const float r = d->h + 2.f * d->tight_margin;
+    d->tight_r2 = r * r;
 }
 
 // Particle k's half skin from its stored value w (the largest, skin_max_half, without per-particle skins or

@@ -102,6 +102,10 @@ struct pcisph_ctx {
     RadixSorter sorter;
     DevParams P{};
     SweepGrid sweep_grid{};
+    uint32_t *tight_list = nullptr, *tight_count = nullptr;  // null: no tight lists
+    float4* tight_ref = nullptr;
+    size_t tight_n = 0;
+    DeviceBlock tight_block;
     size_t list_n = 0;
     size_t list_b_n = 0;  // boundary particles the list block holds lists for
 
@@ -117,7 +121,7 @@ struct pcisph_ctx {
     }
     // marks: a pressure sweep of the graph or the host-driven loop (it reads the stamps), the marking kernel, or a
     // predicting sweep that marks by itself
-    ListBuffers list_buffers(bool marks = false) const {
+    ListBuffers list_buffers(bool marks = false, bool tight = false) const {
         const bool w = working_order();
         const bool m = P.mark_cap != 0;
         return ListBuffers{b.pos, b.vel, b.pr4, b.normal, b.f_other, b.f_press, b.pred, b.pf4, b.state_pos,
@@ -128,7 +132,8 @@ struct pcisph_ctx {
                            b.bfl_count, zone_map, {zone_org[0], zone_org[1], zone_org[2]},
                            {zone_dim[0], zone_dim[1], zone_dim[2]},
                            m && !marks_inline(P.fluid_count) ? b.fast_list : nullptr,
-                           m && marks ? b.walk_stamp : nullptr};
+                           m && marks ? b.walk_stamp : nullptr,
+                           tight ? tight_list : nullptr, tight_count, tight_ref};
     }
     // the partners of fast predictions are marked in the graph and the host-driven loop
     bool partner_marks() const { return list_sweeps() && P.mark_cap != 0 && opts.loop_mode != 2; }
@@ -214,6 +219,32 @@ struct pcisph_ctx {
         if (!list_sweeps()) return PCISPH_OK;
         const size_t n = params.fluid_count;
         if (n >= (1u << 31)) return fail(PCISPH_ERR_INVALID_ARG, "kernel variant 2 takes fewer than 2^31 particles");
+        if (int rc = ensure_base_lists()) return rc;
+        return ensure_tight_lists();
+    }
+    // A scene whose tight lists find no memory does without.
+    int ensure_tight_lists() {
+        const size_t n = params.fluid_count;
+        const bool want = P.tight_margin > 0.f && opts.loop_mode != 2;
+        if (want && tight_list && tight_n == n) return PCISPH_OK;
+        if (!want && !tight_list) return PCISPH_OK;
+        CUDA_TRY(cudaStreamSynchronize(stream()));
+        tight_list = nullptr;
+        graph_valid = false;
+        if (!want) return PCISPH_OK;
+        if (tight_block.ensure(align256(n * kTightCap * 4) + align256(n * 4) + align256(n * 16)) != cudaSuccess) {
+            cudaGetLastError();
+            return PCISPH_OK;
+        }
+        Carver c{static_cast<unsigned char*>(tight_block.p)};
+        tight_list = c.take<uint32_t>(n * kTightCap);
+        tight_count = c.take<uint32_t>(n);
+        tight_ref = c.take<float4>(n);
+        tight_n = n;
+        return PCISPH_OK;
+    }
+    int ensure_base_lists() {
+        const size_t n = params.fluid_count;
         const size_t nb = params.boundary_count;
         const bool bnd = nb > 0;
         const size_t bytes = align256(n * P.list_cap * 4) + align256(n * 4) + align256(n * P.near_cap * 4) +
@@ -255,6 +286,7 @@ struct pcisph_ctx {
     // and reused in between: any placement of whole buckets keeps every sum, only locality ages as
     // particles change cells. order_age: steps since the last bucket sort ran, kNoOrder when none ran for
     // the current buffers and graphs.
+    static constexpr int kUnrolled = 3;  // iterations of the graph before its loop, at most
     static constexpr uint32_t kOrderRefresh = 8;
     static constexpr uint32_t kNoOrder = 0xFFFFFFFFu;
     uint32_t order_age = kNoOrder;
@@ -357,6 +389,8 @@ struct pcisph_ctx {
         P.skin_min_half = std::min(kSkinMinHalf * P.h, P.skin_max_half);
         P.skin_factor = kSkinFactor;
         P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
+        set_tight_lists(&P, list_sweeps() && !P.particle_skin && !marks_inline(params.fluid_count) &&
+                                P.h + P.skin_max_half + kTightMargin * P.h <= 1.9f * P.cell_size);
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
         // cells (with a margin for the divisions of cell_of). With more than 1 in 8 fast nearly every warp holds walkers
@@ -523,19 +557,20 @@ struct pcisph_ctx {
         }
         if (B && cudaMemsetAsync(b.b_press, 0, (size_t)B * 4, s) != cudaSuccess) return -1;
         if (list_sweeps())
-            timed("force", s, [&] { launch_force_list(P, b.ctl, list_buffers(partner_marks() && marks_inline(N)), s); });
+            timed("force", s, [&] { launch_force_list(P, b.ctl, list_buffers(partner_marks() && marks_inline(N), true), s); });
         else if (warp_sweeps()) timed("force", s, [&] { launch_force_sweep(P, b, A, sweep_grid, s); });
         else timed("force", s, [&] { launch_force(P, b, s); });
         nl += 4;
         if (partner_marks() && !marks_inline(N)) {
-            timed("mark", s, [&] { launch_mark_partners(P, b.ctl, list_buffers(true), s); });
+            timed("mark", s, [&] { launch_mark_partners(P, b.ctl, list_buffers(true, true), s); });
             ++nl;
         }
         if (cudaGetLastError() != cudaSuccess) return -1;
         return nl;
     }
 
-    int record_iteration(cudaStream_t s, cudaGraphConditionalHandle cond, bool use_cond) {
+    // k: the iteration within the step, as far as it is known (0: the first, or one of the loop)
+    int record_iteration(cudaStream_t s, cudaGraphConditionalHandle cond, bool use_cond, int k) {
         int nl = 0;
         if (params.boundary_count) {
             if (list_sweeps())
@@ -546,12 +581,12 @@ struct pcisph_ctx {
         }
         if (list_sweeps()) {
             const bool marks = partner_marks(), inline_marks = marks && marks_inline(params.fluid_count);
-            timed("pressure", s, [&] { launch_pressure_list(P, b.ctl, list_buffers(marks), opts.sweep_block, s); });
+            timed("pressure", s, [&] { launch_pressure_list(P, b.ctl, list_buffers(marks, true), opts.sweep_block, k == 1, s); });
             timed("pressure_force", s, [&] {
-                launch_pressure_force_list(P, b.ctl, list_buffers(inline_marks), 0, cond, use_cond, opts.sweep_block, s);
+                launch_pressure_force_list(P, b.ctl, list_buffers(inline_marks, true), 0, cond, use_cond, opts.sweep_block, s);
             });
             if (marks && !inline_marks) {
-                timed("mark", s, [&] { launch_mark_partners(P, b.ctl, list_buffers(true), s); });
+                timed("mark", s, [&] { launch_mark_partners(P, b.ctl, list_buffers(true, true), s); });
                 ++nl;
             }
         } else if (warp_sweeps()) {
@@ -591,7 +626,13 @@ struct pcisph_ctx {
         profiling = false;
         cudaStream_t s = capture_stream;
         cudaGraph_t graph = nullptr;
-        CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        CUDA_TRY(cudaGraphCreate(&graph, 0));
+        cudaError_t be = cudaStreamBeginCaptureToGraph(s, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (be != cudaSuccess) {
+            cudaGraphDestroy(graph);
+            profiling = prof;
+            return fail(PCISPH_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(be));
+        }
         int nl = record_prefix(s);
         if (opts.loop_mode == 2) {  // persistent loop: prefix + one cooperative kernel, no conditional node
             cudaError_t le = nl < 0 ? cudaSuccess : launch_corrective_loop(P, b.ctl, list_buffers(), s);
@@ -609,6 +650,12 @@ struct pcisph_ctx {
             if (ie != cudaSuccess) return fail(PCISPH_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ie));
             return PCISPH_OK;
         }
+        // The iterations that every step runs come before the loop's node: a launch each less than in the loop, and the
+        // sweep that builds the tight lists (the second) is a kernel of its own.
+        cudaGraphConditionalHandle handle;
+        cudaError_t he = cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault);
+        const int before = std::max(1, std::min({kUnrolled, opts.min_iterations, opts.max_iterations}));
+        for (int k = 0; k < before && nl >= 0 && he == cudaSuccess; ++k) record_iteration(s, handle, k + 1 == before, k);
         cudaStreamCaptureStatus st;
         const cudaGraphNode_t* deps = nullptr;
         size_t ndeps = 0;
@@ -616,14 +663,13 @@ struct pcisph_ctx {
         std::vector<cudaGraphNode_t> leaves(deps, deps + (e == cudaSuccess ? ndeps : 0));
         cudaError_t e2 = cudaStreamEndCapture(s, &graph);
         profiling = prof;
+        if (he != cudaSuccess) e = he;
         if (nl < 0 || e != cudaSuccess || e2 != cudaSuccess) {
             if (graph) cudaGraphDestroy(graph);
             return fail(PCISPH_ERR_CUDA, std::string("graph capture of the step failed: ") +
                                              cudaGetErrorString(e != cudaSuccess ? e : e2));
         }
         *prefix_nl = nl;
-        cudaGraphConditionalHandle handle;
-        CUDA_TRY(cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault));
         cudaGraphNodeParams cp{};
         cp.type = cudaGraphNodeTypeConditional;
         cp.conditional.handle = handle;
@@ -634,7 +680,7 @@ struct pcisph_ctx {
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         CUDA_TRY(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
         profiling = false;
-        iter_launches = record_iteration(s, handle, true);
+        iter_launches = record_iteration(s, handle, true, 0);
         profiling = prof;
         cudaGraph_t body_out = nullptr;
         CUDA_TRY(cudaStreamEndCapture(s, &body_out));
@@ -706,7 +752,7 @@ struct pcisph_ctx {
         }
         const int lim = std::max(1, opts.max_iterations);
         for (int i = 0; i < lim; ++i) {
-            host_launches += record_iteration(s, 0, false);
+            host_launches += record_iteration(s, 0, false, i);
             ++host_mode_iters;
             CUDA_TRY(cudaGetLastError());
             if (i + 1 >= std::min(opts.min_iterations, lim)) {
@@ -781,7 +827,7 @@ struct pcisph_ctx {
                 break;
             case PCISPH_STAGE_BOUNDARY_PRESSURE: launch_boundary_pressure(P, b, working_order() ? cells_w : b.cells, s); ++host_launches; break;
             case PCISPH_STAGE_PRESSURE:
-                if (list_sweeps()) launch_pressure_list(P, b.ctl, list_buffers(), opts.sweep_block, s);
+                if (list_sweeps()) launch_pressure_list(P, b.ctl, list_buffers(), opts.sweep_block, false, s);
                 else if (warp_sweeps()) launch_pressure_sweep(P, b, sweep_args(), sweep_grid, s);
                 else launch_pressure(P, b, s);
                 ++host_launches;
@@ -974,6 +1020,7 @@ struct pcisph_ctx {
         sort_block.release();
         staging_block.release();
         list_block.release();
+        tight_block.release();
         zone_block.release();
         order_block.release();
         bucket_sort_block.release();

@@ -21,6 +21,8 @@
 //     last for the rest of the step;
 //   - in a step of moving lists (lists_move: many particles faster than half the skin per step) the skin lists are
 //     built around y = x + v dt instead of x, and a prediction is fast when it strays half the skin from there;
+//   - from the third pressure sweep of a step on, one scene's sweeps read tight lists rebuilt at the second one's
+//     predictions, as long as no prediction has moved past their margin from there (see tight_mode);
 //   - a particle with more than list_cap (near_cap) candidates is marked (count > cap) and walks the
 //     buckets in the sweeps that would use that list.
 // Boundary particles (B > 0, single scene) are summed by walking the boundary buckets. The density sweep
@@ -82,6 +84,12 @@ __device__ __forceinline__ Chunk load_chunk(const uint4* p) {
     return r;
 }
 
+__device__ __forceinline__ void store_chunk(uint4* p, const Chunk& r) {
+    asm volatile("st.global.v8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};" ::"r"(r.e[0]), "r"(r.e[1]), "r"(r.e[2]),
+                 "r"(r.e[3]), "r"(r.e[4]), "r"(r.e[5]), "r"(r.e[6]), "r"(r.e[7]), "l"(p)
+                 : "memory");
+}
+
 // Call f(j) for the n listed neighbours of particle i in list order. The next chunk's indices are loaded
 // while the current chunk's eight gathers are in flight, so the list stream and the gathers overlap.
 template <class F>
@@ -103,6 +111,33 @@ __device__ __forceinline__ void for_each_listed(const uint32_t* __restrict__ lis
 #pragma unroll
         for (int u = 0; u < 8; ++u)
             if ((uint32_t)u < left) f(a.e[u]);
+        a = next;
+    }
+}
+
+// The same where f has side effects that the compiler does not move loads across: a chunk's values first, then
+// use(j, value(j)) for each; after each chunk, done().
+template <class Value, class Use, class Done>
+__device__ __forceinline__ void for_each_listed_ahead(const uint32_t* __restrict__ list, uint32_t i, uint32_t n,
+                                                      uint32_t stride, Value&& value, Use&& use, Done&& done) {
+    if (!n) return;
+    const uint4* p = list_chunk(const_cast<uint32_t*>(list), i, 0, stride);
+    Chunk a = load_chunk(p);
+#pragma unroll 1
+    for (uint32_t e = 0; e < n; e += 8u) {
+        decltype(value(0u)) o[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; ++u)
+            if (e + u < n) o[u] = value(a.e[u]);
+        Chunk next{};
+        if (e + 8u < n) {
+            p += 2 * (size_t)stride;
+            next = load_chunk(p);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; ++u)
+            if (e + u < n) use(a.e[u], o[u]);
+        done();
         a = next;
     }
 }
@@ -247,6 +282,87 @@ constexpr int kCellRounds = 10;   // candidate rounds in registers: 320, a full 
                                   // 12: 614, fewer warps)
 constexpr int kCellBlock = 128;   // 4 warps a block, 20 resident per SM (24 spill: 501 us)
 constexpr uint32_t kAll = 0xffffffffu;
+
+// ------------------------------------------------------------------ tight lists
+//
+// The first correction moves a prediction most (0.05 h and more), the later ones little: from the second prediction x*_2 on
+// no particle of a collapsing column, a tank or a falling drop moves 0.035 h within a step of 7 iterations, and within one
+// of 50 they pass that a few times. So the second pressure sweep of a step also writes, per particle and in walk order, the
+// entries within h + 2 m of it (m = tight_margin; 40 of the skin list's 65 at rest density), and the later sweeps read
+// those: 1,048,576 particles 126 us a sweep -> 82, 8,388,608 957 -> 544, 98,904 falling 21 -> 11; the building sweep costs
+// 186, 1420 and 26. A step of 50 iterations of 8.4M particles 83.2 -> 68.2 ms, one of 6 at 1M 2060 -> 1990 us.
+//
+// Exact: a pair within h at later predictions, neither of which has moved more than m since, was within h + 2 m at the
+// building. A building sweep finds all such pairs: a prediction is flagged already past half the skin less m (in rounds
+// that a building sweep may follow, marks reach h + 2 m), so that a particle that is not flagged then stays within half the
+// skin, and its later partners are in the skin list; and the partners of one that is flagged walk. A particle with
+// more than kTightCap entries walks in every sweep that would read them. One prediction out of reach (or NaN) puts the whole
+// scene back on the skin lists, and from iteration kTightAgain on rebuilds: a building sweep in the loop (it stores entry by
+// entry, 1670 us at 8.4M) pays from three sweeps that use it, which a loop of fewer iterations need not have left.
+// Margins at 1M / 8.4M / a 98,904-particle drop / a violently jittered block of 110,592, us a step: 0.02 2284 / 70510 /
+// 1880 / 5075, 0.03 1998 / 68148 / 1840 / 4793, 0.04 2018 / 67244 / 1821 / 4556.
+//
+// How far flags and marks reach ahead of half the skin in this round.
+__device__ __forceinline__ float tight_margin(const DevParams& P, const Control* ctl, const ListBuffers& b) {
+    return b.tight && ctl->tight_next != kTightOff ? P.tight_margin : 0.f;
+}
+// How this pressure sweep finds its neighbours: constant while it runs.
+__device__ __forceinline__ unsigned tight_mode(const DevParams& P, const Control* ctl, const ListBuffers& b) {
+    if (!b.tight) return kTightOff;
+    const unsigned m = ctl->tight_next;
+    if (m != kTightUse || ctl->tight_stray == 0u) return m;
+    return ctl->tight_age != 0u && ctl->iter >= kTightAgain && (int)ctl->iter + 1 < P.max_iters ? kTightBuild : kTightOff;
+}
+// After a pressure sweep (before the decision): what the next one does.
+__device__ __forceinline__ void tight_advance(const DevParams& P, Control* ctl, const ListBuffers& b) {
+    if (!b.tight) return;
+    const unsigned m = tight_mode(P, ctl, b);
+    if (m == kTightUse) {
+        ctl->tight_age += 1;
+    } else if (m == kTightBuild) {
+        ctl->tight_next = kTightUse;
+        ctl->tight_age = 0;
+        ctl->tight_stray = 0;
+    } else if (ctl->tight_next == kTightUse) {  // left behind
+        if (ctl->tight_age == 0u) {  // before they served a sweep: do without for a while
+            ctl->tight_backoff = min(2u * ctl->tight_backoff + 1u, 15u);
+            ctl->tight_wait = ctl->tight_backoff;
+        }
+        ctl->tight_next = kTightOff;
+    } else if (ctl->tight_wait != 0u) {
+        ctl->tight_wait -= 1;
+    } else if ((ctl->iter == 0u || ctl->iter + 1u >= kTightAgain) && (int)ctl->iter + 2 < P.max_iters) {
+        ctl->tight_next = kTightBuild;
+    }
+}
+// A lane's tight list in the making. kShared: two chunks staged in shared memory, a chunk written out when it is full (whole
+// sectors; 188 us at 1M). Otherwise entry by entry: the sweeps of the loop, which seldom build, keep the L1 (16 KB of
+// staging a block cost each of them 5 to 10%).
+template <bool kShared>
+struct TightWriter {
+    uint32_t* list;
+    uint32_t i, stride, n;
+    uint32_t* column;  // kShared: the lane's column of [16][32]
+    __device__ __forceinline__ TightWriter(uint32_t* list, uint32_t i, uint32_t stride, uint32_t* stage)
+        : list(list), i(i), stride(stride), n(0), column(kShared ? stage + (threadIdx.x & 31u) : nullptr) {}
+    __device__ __forceinline__ void add(uint32_t j) {
+        if constexpr (kShared) column[(n & 15u) * 32u] = j;
+        else if (n < kTightCap) reinterpret_cast<uint32_t*>(list_chunk(list, i, n >> 3, stride))[n & 7u] = j;
+        ++n;
+    }
+    __device__ __forceinline__ void flush(uint32_t c) const {
+        if constexpr (kShared) {
+            if (c >= kTightCap / 8u) return;
+            Chunk k;
+#pragma unroll
+            for (uint32_t u = 0; u < 8u; ++u) k.e[u] = column[((c & 1u) * 8u + u) * 32u];
+            store_chunk(list_chunk(list, i, c, stride), k);
+        }
+    }
+    __device__ __forceinline__ void finish() const {
+        if (n & 7u) flush(n >> 3);
+    }
+};
 
 constexpr unsigned long long kNoMarks = 1ull << 40;  // a round's count past any cap of the partner marks
 
@@ -751,7 +867,8 @@ __global__ void __launch_bounds__(kBlock, DEEP == 1 ? 1 : 2) k_normal_list(PS ps
 // lies within D = h + skin_max_half (< 2 cells, checked on the host) of such an x*_j, so its cell is among them, and its
 // box comes within D of x*_j (with a margin for the divisions of cell_of). Within 2^14 cells of the origin the rounding of
 // the box bounds and of cell_of's division is far below that margin; farther out (or saturated, or NaN) every cell counts.
-__device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& pj, const Cell& c0, uint32_t o, Cell& c) {
+__device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& pj, const Cell& c0, uint32_t o, float margin,
+                                             Cell& c) {
     c = Cell{c0.x + o % 5u - 2u, c0.y + o / 5u % 5u - 2u, c0.z + o / 25u - 2u};
     auto inner = [](uint32_t v) { return v + 16384u < 32768u; };  // -2^14 < (int)v < 2^14, wrapping
     if (!(inner(c0.x) && inner(c0.y) && inner(c0.z))) return true;
@@ -760,7 +877,7 @@ __device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& p
         return fmaxf(fmaxf(lo - x, x - hi), 0.f);
     };
     const float gx = gap(c.x, pj.x), gy = gap(c.y, pj.y), gz = gap(c.z, pj.z);
-    const float reach = P.h + P.skin_max_half + 0.01f * P.cell_size;
+    const float reach = P.h + P.skin_max_half + margin + 0.01f * P.cell_size;
     return !(gx * gx + gy * gy + gz * gz > reach * reach);
 }
 __device__ __forceinline__ bool beyond_list(const DevParams& P, const float4& xi, const float4& xj) {
@@ -776,6 +893,8 @@ constexpr unsigned kMarkBlocks = 608;
 __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Control* ctl, ListBuffers b) {
     const unsigned long long n = ctl->fast_n;
     if (n == 0 || n > P.mark_cap) return;
+    if (b.tight && ctl->tight_next == kTightUse && ctl->tight_stray == 0u) return;  // the next sweep asks no marks
+    const float margin = tight_margin(P, ctl, b), far2 = margin > 0.f ? P.tight_r2 : P.h2;
     const unsigned round = ctl->round + 1u;
     const unsigned long long items = n * 125ull;
     for (unsigned long long t = (unsigned long long)blockIdx.x * kBlock + threadIdx.x; t < items;
@@ -786,7 +905,7 @@ __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Con
         const float4 pj = b.pred[j];
         const float4 xj = b.pos[j];
         Cell c;
-        if (!partner_cell(P, pj, cell_of(pj.x, pj.y, pj.z, P), o, c)) continue;
+        if (!partner_cell(P, pj, cell_of(pj.x, pj.y, pj.z, P), o, margin, c)) continue;
         const uint2 r = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
 #pragma unroll 1
         for (uint32_t i0 = r.x; i0 < r.y; i0 += 4) {
@@ -799,7 +918,7 @@ __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Con
                 }
 #pragma unroll
             for (int u = 0; u < 4; ++u)
-                if (i0 + u < r.y && dist2(pj.x - pi[u].x, pj.y - pi[u].y, pj.z - pi[u].z) <= P.h2 &&
+                if (i0 + u < r.y && dist2(pj.x - pi[u].x, pj.y - pi[u].y, pj.z - pi[u].z) <= far2 &&
                     beyond_list(P, xi[u], xj))
                     b.walk_stamp[i0 + u] = round;
         }
@@ -820,7 +939,8 @@ __device__ __noinline__ void mark_partners_inline(const DevParams& P, Control* c
     if (base >= P.mark_cap) return;  // past the cap: the sweep takes the bucket flags
     __syncwarp();                    // the lanes' predictions are stored
     const unsigned round = ctl->round + 1u;
-    const float far = P.h + P.skin_max_half + 1e-4f * P.h;  // D, past the rounding of the distances
+    const float margin = tight_margin(P, ctl, b);
+    const float far = P.h + P.skin_max_half + margin + 1e-4f * P.h;  // D, past the rounding of the distances
     for (; set; set &= set - 1u) {
         const uint32_t j = __shfl_sync(kAll, i, __ffs(set) - 1);
         const float4 pj = b.pred[j], xj = b.pos[j];
@@ -832,7 +952,7 @@ __device__ __noinline__ void mark_partners_inline(const DevParams& P, Control* c
             const uint32_t o = lane + 32u * q;
             Cell c;
             r[q] = make_uint2(0u, 0u);
-            if (o < 125u && partner_cell(P, pj, c0, o, c)) r[q] = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
+            if (o < 125u && partner_cell(P, pj, c0, o, margin, c)) r[q] = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -870,8 +990,8 @@ __device__ __forceinline__ bool finish_force(const PS& ps, const ListBuffers& b,
     const float4 xs = make_float4(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z, 0.f);
     b.pred[i] = xs;
     bool fast;
-    const float disp = note_displacement<!PS::kBatched>(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin, vi,
-                                                        fast, PS::kBatched ? nullptr : b.fast_list, i);
+    const float disp = note_displacement<!PS::kBatched>(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin,
+                                                        tight_margin(P, ps.control(i), b), vi, fast, PS::kBatched ? nullptr : b.fast_list, i);
     if (P.particle_skin) b.disp_max[i] = disp;
     return fast;
 }
@@ -985,7 +1105,7 @@ __global__ void __launch_bounds__(kBlock) k_force_shared(PS ps, ListBuffers b) {
 // No prediction of this step was fast: the scene's lists are complete for x*.
 template <class PS>
 __device__ __forceinline__ bool lists_hold(const Control* ctl) {
-    return PS::kBatched ? ctl->fast_particles == ctl->fast_at_begin : ctl->lists_outrun == 0u;
+    return ctl->lists_outrun == 0u;
 }
 
 // How one particle's pressure sweep finds its neighbours.
@@ -1072,9 +1192,21 @@ struct WalkStage {
     uint32_t delta[32];
     float term[96];
 };
-template <class PS, bool kCoherent, int U>
+// With room to stage the tight lists of a warp's lanes (before its walkers are served, or by them).
+union BuildStage {
+    WalkStage walk;
+    uint32_t tight[16 * 32];
+};
+template <bool kShared>
+using Stage = std::conditional_t<kShared, BuildStage, WalkStage>;
+__device__ __forceinline__ uint32_t* stage_tight(WalkStage&) { return nullptr; }
+__device__ __forceinline__ uint32_t* stage_tight(BuildStage& s) { return s.tight; }
+__device__ __forceinline__ WalkStage& stage_walk(WalkStage& s) { return s; }
+__device__ __forceinline__ WalkStage& stage_walk(BuildStage& s) { return s.walk; }
+template <class PS, bool kCoherent, int U, bool kShared>
 __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
-                                               uint32_t walkers, WalkStage& S) {
+                                               uint32_t walkers, bool build, Stage<kShared>& stage) {
+    WalkStage& S = stage_walk(stage);
     const uint32_t lane = threadIdx.x & 31u;
     const bool mine = (walkers >> lane) & 1u;
     const uint32_t first = __shfl_sync(kAll, i, __ffs(walkers) - 1);
@@ -1086,12 +1218,24 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
     if (__popc(walkers) > kFewWalkers) {
         if (mine) {
             auto load = [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); };
-            auto use = [&](uint32_t, const float4& o) { acc += density_term(xp.x, xp.y, xp.z, o, P.h2); };
+            TightWriter<kShared> w(b.tight, ii, b.nbr_stride, stage_tight(stage));
+            auto use = [&](uint32_t j, const float4& o) {
+                const float d2 = dist2(xp.x - o.x, xp.y - o.y, xp.z - o.z);
+                acc += poly6(d2, P.h2);
+                if (build && !(d2 > P.tight_r2)) {
+                    w.add(j);
+                    if ((w.n & 7u) == 0u) w.flush((w.n >> 3) - 1u);
+                }
+            };
             // a batch walks with two gathers in flight (terms still added in walk order): its walkers are latency-bound
             // (256 batched scenes, 9.8M particles, over 500 steps: 26.8 -> 25.8 s); one scene walks plainly (8M
             // particles all walking: 3.0 ms per sweep, 3.6 with the prefetch)
             if constexpr (PS::kBatched) for_each_neighbour_prefetched(b.cells, c, P, load, use);
             else for_each_neighbour(b.cells, c, P, [&](uint32_t j) { use(j, load(j)); });
+            if (build) {
+                w.finish();
+                b.tight_count[ii] = w.n;
+            }
         }
     } else {
         const uint32_t below = lanes_below();
@@ -1101,7 +1245,9 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
             const float x = __shfl_sync(kAll, xp.x, t), y = __shfl_sync(kAll, xp.y, t), z = __shfl_sync(kAll, xp.z, t);
             CellWalk w = begin_cell(b.cells, Q, __shfl_sync(kAll, c.x, t), __shfl_sync(kAll, c.y, t),
                                     __shfl_sync(kAll, c.z, t), lane, S.delta);
-            uint32_t n = 0;
+            const uint32_t it = __shfl_sync(kAll, ii, t);
+            const bool keep = __shfl_sync(kAll, (int)build, t) != 0;
+            uint32_t n = 0, kept = 0;
             auto sum = [&] {  // the staged terms, by the walker's own lane
                 __syncwarp();
                 if ((int)lane == t)
@@ -1111,15 +1257,27 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
             };
             for (uint32_t base = 0; base < w.total; base += 32u * U) {
                 float4 o[U];
+                uint32_t js[U];
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const uint32_t j = next_candidate(w, base + u * 32u, lane, S.delta);
-                    if (j != kAll) o[u] = load_slot<kCoherent>(&b.pred[j]);
+                    js[u] = next_candidate(w, base + u * 32u, lane, S.delta);
+                    if (js[u] != kAll) o[u] = load_slot<kCoherent>(&b.pred[js[u]]);
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     float term = 0.f;
-                    if (base + u * 32u + lane < w.total) term = density_term(x, y, z, o[u], Q.h2);
+                    bool tight = false;
+                    if (base + u * 32u + lane < w.total) {
+                        const float d2 = dist2(x - o[u].x, y - o[u].y, z - o[u].z);
+                        term = poly6(d2, Q.h2);
+                        tight = keep && !(d2 > Q.tight_r2);
+                    }
+                    const uint32_t set = __ballot_sync(kAll, tight);
+                    if (tight) {
+                        const uint32_t e = kept + __popc(set & below);
+                        if (e < kTightCap) reinterpret_cast<uint32_t*>(list_chunk(b.tight, it, e >> 3, b.nbr_stride))[e & 7u] = js[u];
+                    }
+                    kept += __popc(set);
                     const uint32_t bits = __ballot_sync(kAll, term != 0.f);  // NaN counts
                     if (n + __popc(bits) > 96u) sum();
                     if (term != 0.f) S.term[n + __popc(bits & below)] = term;
@@ -1127,32 +1285,64 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
                 }
             }
             sum();
+            if (keep && (int)lane == t) b.tight_count[it] = kept;
         }
     }
     return mine ? finish_pressure<PS>(b, P, ps.control(ii), ii, xi, acc) : 0.f;
 }
 
-template <class PS, bool kCoherent>
+template <class PS, bool kCoherent, bool kShared>
 __device__ __noinline__ float call_pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
-                                                    uint32_t walkers, WalkStage& S) {
-    return pressure_walkers<PS, kCoherent, 3>(ps, b, i, acc, walkers, S);
+                                                    uint32_t walkers, bool build, Stage<kShared>& S) {
+    return pressure_walkers<PS, kCoherent, 3, kShared>(ps, b, i, acc, walkers, build, S);
 }
 
+// A particle's fluid terms added to acc by its own lane, from its skin list (cnt entries) or a walk, building its tight
+// list. (A chunk's distances before its entries are kept: 218 -> 186 us at 1M, the gathers in flight together.)
+template <bool kCoherent, bool kShared>
+__device__ __forceinline__ float build_tight_list(const ListBuffers& b, const DevParams& P, uint32_t i, const float4& xp,
+                                                  uint32_t cnt, float acc, bool walk, const Cell& c, uint32_t* stage) {
+    TightWriter<kShared> w(b.tight, i, b.nbr_stride, stage);
+    uint32_t written = 0;  // entries at the last look
+    auto away2 = [&](uint32_t j) {
+        const float4 o = load_slot<kCoherent>(&b.pred[j]);
+        return dist2(xp.x - o.x, xp.y - o.y, xp.z - o.z);
+    };
+    auto keep = [&](uint32_t j, float d2) {
+        acc += poly6(d2, P.h2);
+        if (!(d2 > P.tight_r2)) w.add(j);
+    };
+    auto flush = [&] {
+        if ((written ^ w.n) & 8u) w.flush(written >> 3);
+        written = w.n;
+    };
+    if (walk)
+        for_each_neighbour(b.cells, c, P, [&](uint32_t j) {
+            keep(j, away2(j));
+            flush();
+        });
+    else for_each_listed_ahead(b.nbr, i, cnt, b.nbr_stride, away2, keep, flush);
+    w.finish();
+    b.tight_count[i] = w.n;
+    return acc;
+}
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
 // stage: its WalkStage.
 enum class Walks { kLane, kInline, kCall };  // each lane by itself; pressure_walkers inline; or as a function call
-template <class PS, bool kCoherent, Walks kWalks>
-__device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, WalkStage& stage) {
+template <class PS, bool kCoherent, Walks kWalks, bool kShared>
+__device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, Stage<kShared>& stage) {
     float dv = 0.f, acc = 0.f;
-    bool walk = false;
+    bool walk = false, build = false;
     if (i < ps.count() && !ps.skip_pressure(i)) {
         const DevParams& P = ps.params(i);
         Control* ctl = ps.control(i);
         const bool all_lists_ok = lists_hold<PS>(ctl);
         const float4 xi = b.pos[i];
         const float4 xp = b.pred[i];
-        const uint32_t cnt = b.nbr_count[i];
-        const bool overflow = cnt > P.list_cap;
+        const unsigned mode = tight_mode(P, ctl, b);
+        build = mode == kTightBuild;
+        const uint32_t cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
+        const bool overflow = cnt > (mode == kTightUse ? kTightCap : P.list_cap);
         // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
         // skin) may miss a pair: with per-particle skins it walks. Boundary terms: all zero unless a boundary
         // particle was within r_list of x, or x* moved past the half skin (boundary particles do not move);
@@ -1181,7 +1371,10 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         // the bucket flags: every particle near a fast one walks
         const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
         const bool marks = fast_round <= P.mark_cap;
-        if (marks) {
+        if (mode == kTightUse) {
+            walk = overflow;
+            if (walk || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
+        } else if (marks) {
             walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
             if (walk || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
         } else {
@@ -1191,24 +1384,28 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         auto fb = [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, __ldg(&b.b_pos[j]), P.h2); };
         if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
         else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
-        if (kWalks == Walks::kLane && walk) {
-            for_each_neighbour(b.cells, c, P, [&](uint32_t j) {
-                acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
-            });
+        auto add = [&](uint32_t j) {
+            acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
+        };
+        if (build) b.tight_ref[i] = xp;
+        if (build && (kWalks == Walks::kLane || !walk)) {
+            acc = build_tight_list<kCoherent, kShared>(b, P, i, xp, cnt, acc, walk, c, stage_tight(stage));
+            walk = false;
+        } else if (kWalks == Walks::kLane && walk) {
+            for_each_neighbour(b.cells, c, P, add);
             walk = false;
         } else if (!walk) {
-            for_each_listed(b.nbr, i, cnt, b.nbr_stride, [&](uint32_t j) {
-                acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
-            });
+            for_each_listed(mode == kTightUse ? b.tight : b.nbr, i, cnt, b.nbr_stride, add);
         }
         if (!walk) dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
     }
     if constexpr (kWalks == Walks::kLane) return dv;
     const uint32_t walkers = __ballot_sync(kAll, walk);
     if (walkers) {
+        __syncwarp();  // the stage changes hands
         float w;
-        if constexpr (kWalks == Walks::kCall) w = call_pressure_walkers<PS, kCoherent>(ps, b, i, acc, walkers, stage);
-        else w = pressure_walkers<PS, kCoherent, 2>(ps, b, i, acc, walkers, stage);
+        if constexpr (kWalks == Walks::kCall) w = call_pressure_walkers<PS, kCoherent, kShared>(ps, b, i, acc, walkers, build, stage);
+        else w = pressure_walkers<PS, kCoherent, 2, kShared>(ps, b, i, acc, walkers, build, stage);
         if (walk) dv = w;
     }
     return dv;
@@ -1257,12 +1454,12 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
 // BS: threads per block (128, 256 or 512; the autotuner's choice for one scene)
 // Walks::kCall: 32 warps per SM at 64 registers instead of 40 at 48, with more gathers in flight each (see
 // launch_pressure_list)
-template <class PS, int BS = kBlock, int LANES = 1, Walks kWalks = Walks::kCall>
+template <class PS, int BS = kBlock, int LANES = 1, Walks kWalks = Walks::kCall, bool kShared = false>
 __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1024 / BS : 1280 / BS) k_pressure_list(PS ps, ListBuffers b) {
     const uint32_t t = blockIdx.x * BS + threadIdx.x;
     float dv;
-    __shared__ WalkStage stage[LANES == 1 ? BS / 32 : 1];
-    if constexpr (LANES == 1) dv = pressure_body<PS, false, kWalks>(ps, b, t, stage[threadIdx.x >> 5]);
+    __shared__ Stage<kShared> stage[LANES == 1 ? BS / 32 : 1];
+    if constexpr (LANES == 1) dv = pressure_body<PS, false, kWalks, kShared>(ps, b, t, stage[threadIdx.x >> 5]);
     else dv = pressure_shared<PS, LANES>(ps, b, t / LANES, t % LANES);
     if (PS::kBatched) return;
     // one scene: block max of dv, the last block decides (dv >= 0: bit patterns order like values)
@@ -1288,6 +1485,7 @@ __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1
             ctl->round += 1u;
             ctl->fast_n = lists_move(ps.params(0), ctl) ? kNoMarks : 0ull;  // moving lists: no marks
         }
+        tight_advance(ps.params(0), ctl, b);
         decide(ps.params(0), ctl);
     }
 }
@@ -1304,6 +1502,9 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
     const float3 fp = make_float3(f.x * scale, f.y * scale, f.z * scale);
     b.f_press[i] = f4(fp, 0.f);
     const bool integrate = mode == 0 ? (ctl->done != 0u) : mode == 2;
+    const bool watch = b.tight && ctl->tight_next == kTightUse;
+    float4 r = xi;
+    if (watch) r = b.tight_ref[i];  // with the loads below, not after them
     const float3 a = (f3(b.f_other[i]) + fp) / m;
     const float3 vi = f3(b.vel[i]);
     float3 v = vi + a * P.dt;
@@ -1313,8 +1514,13 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
         const float4 xs = f4(x, 0.f);
         b.pred[i] = xs;
         bool fast;
-        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin, vi, fast,
+        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin,
+                                                            tight_margin(P, ctl, b), vi, fast,
                                                             PS::kBatched ? nullptr : b.fast_list, i);
+        if (watch) {
+            if (!(sqrtf(dist2(xs.x - r.x, xs.y - r.y, xs.z - r.z)) <= P.tight_reach) && ctl->tight_stray == 0u)
+                ctl->tight_stray = 1u;  // NaN strays
+        }
         if (P.particle_skin) b.disp_max[i] = fmaxf(b.disp_max[i], disp);
         return fast;
     }
@@ -1461,7 +1667,7 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
         unsigned local = 0;
         for (uint32_t r = 0; r < rounds; ++r)
             local = max(local, __float_as_uint(
-                                   pressure_body<PS, true, Walks::kCall>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
+                                   pressure_body<PS, true, Walks::kCall, false>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
                                                            stage[threadIdx.x >> 5])));
         if (!PS::kBatched) {  // batched scenes reduced per scene inside the body
             const unsigned m = __reduce_max_sync(0xffffffffu, local);
@@ -1558,6 +1764,12 @@ __global__ void k_batch_begin(DevParams* table, Control* ctls, uint32_t n_scenes
         c->finished = 0;
         c->max_err_bits = 0;
         c->fast_at_begin = c->fast_particles;
+        c->lists_outrun = 0;
+        c->tight_next = kTightOff;
+        c->tight_stray = 0;
+        c->tight_age = 0;
+        c->tight_wait = 0;
+        c->tight_backoff = 0;
         c->status = 0;
     }
     if (threadIdx.x == 0) {
@@ -1632,6 +1844,9 @@ void launch_density_list(const DevParams& P, Control* ctl, const ListBuffers& b,
 constexpr int kLanes = 8;
 constexpr uint32_t kSharedMax = 8192u;  // eight lanes
 constexpr uint32_t kDeepMax = 49152u;   // two chunks in flight, pressure force and normal
+// Past 2M particles the default block of the corrective sweeps is 128 threads instead of 256 (8.4M: pressure force 614 -> 588
+// us, pressure 663 -> 658; equal at 1M).
+constexpr uint32_t kLargeScene = 1u << 21;
 
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     const unsigned blocks = std::min(grid_cells(P.fluid_count, 8), 5u * 152u);
@@ -1649,25 +1864,31 @@ void launch_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, c
     if (n <= kSharedMax) k_force_shared<OneScene, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(OneScene{P, ctl}, b);
     else k_force_list<<<grid_for(n), kBlock, 0, s>>>(OneScene{P, ctl}, b);
 }
-void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, cudaStream_t s) {
+void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, bool builds,
+                          cudaStream_t s) {
     const OneScene ps{P, ctl};
     const uint32_t n = P.fluid_count;
-    auto go = [&](auto bs) {
+    auto go = [&](auto bs, auto shared) {
         constexpr int BS = decltype(bs)::value;
+        constexpr bool S = decltype(shared)::value;
         const unsigned blocks = (n + BS - 1) / BS;
         // 64 registers a thread (4 blocks of 256 per SM) against 48 (5 blocks), us per launch: 201,600 particles 42 / 47,
         // 286,720 44 / 52, 400,000 62 / 69, 600,000 80 / 91, 1,048,576 135 / 140, 1.6M and 2.6M equal, 4.2M 516 / 508,
         // 8.4M 1071 / 1050; below, 48 as long as they hold the scene in one wave (156,244: 33 / 29).
         // Past 2M the walks in lane form, which need none of the spills of the inline form: 2.6M 321 -> 313 us, 8.4M
         // 1050 -> 1036.
-        if (n > (1u << 21)) k_pressure_list<OneScene, BS, 1, Walks::kLane><<<blocks, BS, 0, s>>>(ps, b);
-        else if (n > 5u * 256u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall><<<blocks, BS, 0, s>>>(ps, b);
-        else k_pressure_list<OneScene, BS, 1, Walks::kInline><<<blocks, BS, 0, s>>>(ps, b);
+        // The building sweep with 64 registers, too, but where a wave of them just misses the scene: 156,244 particles 37
+        // us with 48, 43 with 64; 32,768 29 and 21.
+        if (S && n <= 8u * 128u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall, S><<<blocks, BS, 0, s>>>(ps, b);
+        else if (n > kLargeScene) k_pressure_list<OneScene, BS, 1, Walks::kLane, S><<<blocks, BS, 0, s>>>(ps, b);
+        else if (n > 5u * 256u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall, S><<<blocks, BS, 0, s>>>(ps, b);
+        else k_pressure_list<OneScene, BS, 1, Walks::kInline, S><<<blocks, BS, 0, s>>>(ps, b);
     };
     if (n <= kSharedMax) k_pressure_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b);
-    else if (block == 128) go(std::integral_constant<int, 128>{});
-    else if (block == 512) go(std::integral_constant<int, 512>{});
-    else go(std::integral_constant<int, kBlock>{});
+    else if (builds && b.tight) go(std::integral_constant<int, 128>{}, std::true_type{});
+    else if (block == 128 || (block == kBlock && n > kLargeScene)) go(std::integral_constant<int, 128>{}, std::false_type{});
+    else if (block == 512) go(std::integral_constant<int, 512>{}, std::false_type{});
+    else go(std::integral_constant<int, kBlock>{}, std::false_type{});
 }
 bool marks_inline(uint32_t n) { return n <= kSharedMax; }
 void launch_mark_partners(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
@@ -1682,7 +1903,8 @@ void launch_pressure_force_list(const DevParams& P, Control* ctl, const ListBuff
         k_pressure_force_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b, mode, cond, uc);
     else if (n <= kDeepMax)
         k_pressure_force_list<OneScene, 128, 1, 2><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
-    else if (block == 128) k_pressure_force_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
+    else if (block == 128 || (block == kBlock && n > kLargeScene))
+        k_pressure_force_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
     else if (block == 512) k_pressure_force_list<OneScene, 512><<<(n + 511) / 512, 512, 0, s>>>(ps, b, mode, cond, uc);
     else k_pressure_force_list<OneScene, kBlock><<<grid_for(n), kBlock, 0, s>>>(ps, b, mode, cond, uc);
 }

@@ -48,6 +48,11 @@ struct ListBuffers {
     // follows.
     uint32_t* fast_list;
     uint32_t* walk_stamp;
+    // tight lists (or null): kTightCap entries per particle laid out like nbr, the entries per particle (> kTightCap: walk
+    // the buckets), and the predictions they were built at
+    uint32_t* tight;
+    uint32_t* tight_count;
+    float4* tight_ref;
 };
 
 // Is the cell in the boundary zone (ListBuffers::b_zone)? Cells are the signed integers the reference's
@@ -110,8 +115,10 @@ bool marks_inline(uint32_t n);
 // set): the particles whose next pressure sweep must walk. That sweep (launched with b.walk_stamp) closes
 // the round.
 void launch_mark_partners(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
-// block: threads per block of the two corrective-loop sweeps (128, 256 or 512)
-void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, cudaStream_t s);
+// block: threads per block of the two corrective-loop sweeps (128, 256 or 512). builds: this sweep is expected to build
+// the tight lists.
+void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, bool builds,
+                          cudaStream_t s);
 // mode 0: the loop decision picks predict or integrate; 1: predict; 2: integrate
 void launch_pressure_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, int mode,
                                 cudaGraphConditionalHandle cond, bool use_cond, int block, cudaStream_t s);

@@ -111,6 +111,11 @@ __global__ void k_begin(Control* ctl) {
     ctl->fast_n = 0;
     ctl->moving = 0;
     ctl->lists_outrun = 0;
+    ctl->tight_next = kTightOff;
+    ctl->tight_stray = 0;
+    ctl->tight_age = 0;
+    ctl->tight_wait = 0;
+    ctl->tight_backoff = 0;
 }
 
 // pcisph.cl:65-92

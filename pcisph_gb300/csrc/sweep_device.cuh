@@ -36,30 +36,29 @@ __device__ __forceinline__ void warp_count(unsigned long long* addr, bool pred) 
 template <bool kOne>
 __device__ __forceinline__ float note_displacement(const DevParams& P, Control* ctl,
                                                    unsigned char* __restrict__ bucket_fast, const float4& xi,
-                                                   const float4& xs, float threshold, const float3& vi, bool& fast,
+                                                   const float4& xs, float threshold, float margin, const float3& vi, bool& flag,
                                                    uint32_t* __restrict__ fast_list = nullptr, uint32_t i = 0) {
     const float dx = xs.x - xi.x, dy = xs.y - xi.y, dz = xs.z - xi.z;  // exact: xs and xi are close
     const float disp = sqrtf(dist2(dx, dy, dz));
-    fast = disp > threshold;
-    warp_count(&ctl->fast_particles, fast);
-    bool flag = fast;
+    warp_count(&ctl->fast_particles, disp > threshold);
+    flag = disp > threshold - margin;
     if (kOne) {
         if (lists_move(P, ctl)) {
             const float4 y = moving_place(P, xi, vi);
-            flag = !(sqrtf(dist2(xs.x - y.x, xs.y - y.y, xs.z - y.z)) <= threshold);  // NaN strays
+            flag = !(sqrtf(dist2(xs.x - y.x, xs.y - y.y, xs.z - y.z)) <= threshold - margin);  // NaN strays
         }
-        if (flag && ctl->lists_outrun == 0u) ctl->lists_outrun = 1u;
     }
+    if (flag && ctl->lists_outrun == 0u) ctl->lists_outrun = 1u;
     if (fast_list) {
         const unsigned act = __activemask();
-        const unsigned set = __ballot_sync(act, fast);
+        const unsigned set = __ballot_sync(act, flag);
         if (set) {
             const int lane = (int)(threadIdx.x & 31), leader = __ffs(set) - 1;
             unsigned long long base = ~0ull;
             if (lane == leader && *(volatile unsigned long long*)&ctl->fast_n <= P.mark_cap)
                 base = atomicAdd(&ctl->fast_n, (unsigned long long)__popc(set));
             base = __shfl_sync(act, base, leader);
-            if (fast && base != ~0ull) {
+            if (flag && base != ~0ull) {
                 const unsigned long long slot = base + __popc(set & ((1u << lane) - 1u));
                 if (slot < P.mark_cap) fast_list[slot] = i;
             }

@@ -154,3 +154,46 @@ def test_moving_lists_keep_nonfinite_velocities(oracle):
         f.close()
     for a, w in zip(*out):
         np.testing.assert_array_equal(a, w)
+
+
+# The pressure sweeps from the third iteration on read lists rebuilt at the second one's predictions. Sizes at the edges of
+# their launches (from 8,193; 155,648 and 194,560 where the building sweep changes its form; past 2M); loops that end before
+# a list is built, before it is used and long after it was left behind; a block that overflows them; predictions that
+# outrun every list at once or keep leaving the rebuilt ones; boundary particles; skins of other sizes; NaN
+@pytest.mark.parametrize("n,gap,jitter,speed,iters,options", [
+    (8193, 1.0, 0.1, 0.0, (3, 3), {}), (9001, 1.0, 0.1, 0.0, (1, 1), {}), (9001, 1.0, 0.1, 0.0, (2, 2), {}),
+    (9001, 1.0, 0.2, 0.0, (1, 9), {}), (20000, 1.0, 0.3, 0.0, (40, 40), {}), (30000, 0.8, 0.1, 0.0, (12, 12), {}),
+    (30000, 0.75, 0.4, 8.0, (30, 30), {}), (12000, 1.0, 0.1, 4.0, (8, 8), {"list_skin": 0.0}),
+    (12000, 1.0, 0.3, 1.0, (25, 25), {"list_skin": 0.5}), (16000, 1.0, 0.2, 0.0, (20, 20), {"particle_skin": 0, "boundary": 1}),
+    (16000, 1.0, 0.2, 3.0, (20, 20), {"nan": 1}), (155648, 1.0, 0.2, 0.0, (12, 12), {}),
+    (155649, 1.0, 0.15, 0.0, (8, 8), {"sweep_block": 512}), (194561, 1.0, 0.2, 0.5, (9, 9), {"sweep_block": 128}),
+    (2097153, 1.0, 0.2, 0.0, (9, 9), {})])
+def test_rebuilt_lists_change_no_bits(oracle, n, gap, jitter, speed, iters, options):
+    """The persistent loop builds no such lists: the same bits and the same counts."""
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    at = np.stack(np.unravel_index(np.arange(n), (side, side, side)), -1) + 0.5
+    pos = ((at + jitter * (2 * rng.random((n, 3)) - 1)) * gap * D).astype(np.float32)
+    vel = (speed * rng.standard_normal((n, 3))).astype(np.float32)
+    if options.get("nan"):
+        vel[n // 2] = np.nan
+    floor = np.stack(np.meshgrid(np.arange(side), [-0.5], np.arange(side), indexing="ij"), -1).reshape(-1, 3) * D
+    walls = len(floor) if options.get("boundary") else 0
+    p = oracle.derive_params(0.5 * D, 1000.0, n, walls, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    out = []
+    for loop_mode in (0, 1, 2):
+        f = fluid_like(p, min_iters=iters[0], max_iters=iters[1], loop_mode=loop_mode, spatial_order=2)
+        f.set_options(**{k: v for k, v in options.items() if k not in ("nan", "boundary")})
+        f.set_fluid_state(pos, vel)
+        if walls:
+            f.set_boundary_state(floor.astype(np.float32))
+        f.step(2)
+        st = f.stats()
+        out.append(({k: f.get_field(k) for k in ("src", "density", "density_variation", "pressure", "pressure_force",
+                                                 "position", "velocity", "predicted_position")},
+                    (st.fast_particles, st.list_fallbacks, st.status_all, st.total_iterations)))
+        f.close()
+    for got in out[:2]:
+        assert got[1] == out[2][1]
+        for k in got[0]:
+            np.testing.assert_array_equal(got[0][k], out[2][0][k], err_msg=k)
