@@ -68,6 +68,7 @@ struct pcisph_batch {
     int32_t next_id = 1;
     uint32_t n_particles = 0, n_buckets = 0;
     int max_iters = 1;
+    int sure_iters = 1;  // iterations that every step runs: some scene does
     int loop_mode = 0;   // 0: conditional WHILE node; 2: one persistent cooperative kernel
     float list_skin = 0.25f;   // the skin of every scene when adaptive_skin is off
     bool adaptive_skin = true;  // each scene picks its skin every step (k_batch_begin)
@@ -153,10 +154,18 @@ struct pcisph_batch {
     SceneTable scene_table() const {
         return SceneTable{d_table, d_ctls, scene_of, n_particles, (uint32_t)scenes.size()};
     }
-    ListBuffers list_buffers() const {
-        return ListBuffers{pos, vel, pr4, normal, f_other, f_press, pred, pf4, state_pos, state_vel, rho, press, err,
+    ListBuffers list_buffers(bool tight = false) const {
+        ListBuffers b{pos, vel, pr4, normal, f_other, f_press, pred, pf4, state_pos, state_vel, rho, press, err,
                            cells, cells, nullptr, nullptr, nbr, nbr_count, near, near_count, bucket_fast,
                            n_particles, /*out_index*/ nullptr, /*disp_max*/ nullptr, /*state_skin*/ nullptr};
+        if (tight) {  // in the pool's own memory: the last chunks of the skin lists, which few particles fill, and
+                      // arrays that rest between the reorder and the step's end
+            b.tight = nbr + (size_t)(kListCapWide - kTightCap) * n_particles;
+            b.tight_below = kListCapWide - kTightCap;
+            b.tight_count = keys;
+            b.tight_ref = staging;
+        }
+        return b;
     }
 
     uint32_t pool_end() const { return scenes.empty() ? 0u : scenes.back().offset + scenes.back().count; }
@@ -217,7 +226,7 @@ struct pcisph_batch {
         std::vector<DevParams> table(scenes.size());
         std::vector<uint32_t> offsets(scenes.size() + 1);
         uint32_t base = 0, off = 0;
-        max_iters = 1;
+        max_iters = sure_iters = 1;
         for (size_t k = 0; k < scenes.size(); ++k) {
             SceneSlot& s = scenes[k];
             s.offset = off;
@@ -226,6 +235,8 @@ struct pcisph_batch {
             make_devparams(s.params, d.min_iterations, d.max_iterations, d.walls, d.box_lo, d.box_hi, d.restitution,
                            d.density_variation_threshold, adaptive_skin ? skin_level_value(0) : list_skin, base,
                            &table[k], kListCapWide, adaptive_skin ? 1 : 0);
+            set_tight_lists(&table[k], true);
+            sure_iters = std::max(sure_iters, std::min(d.min_iterations, d.max_iterations));
             offsets[k] = off;
             off += s.count;
             base += s.params.bucket_count;
@@ -269,7 +280,7 @@ struct pcisph_batch {
         timed("reorder", s, [&] {
             launch_reorder(sk, sv, state_pos, state_vel, n_particles, pos, vel, cells, nullptr, nullptr, R, d_batch, s);
         });
-        const ListBuffers b = list_buffers();
+        const ListBuffers b = list_buffers(loop_mode != 2);
         timed("density", s, [&] { launch_density_scenes(t, b, s); });
         timed("normal", s, [&] { launch_normal_scenes(t, b, s); });
         timed("force", s, [&] { launch_force_scenes(t, b, s); });
@@ -283,7 +294,12 @@ struct pcisph_batch {
     int capture(cudaGraph_t* out) {
         cudaStream_t s = capture_stream;
         cudaGraph_t graph = nullptr;
-        BTRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+        BTRY(cudaGraphCreate(&graph, 0));
+        const cudaError_t be = cudaStreamBeginCaptureToGraph(s, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
+        if (be != cudaSuccess) {
+            cudaGraphDestroy(graph);
+            return report_error(PCISPH_ERR_CUDA, std::string("graph capture of the batch step: ") + cudaGetErrorString(be));
+        }
         const int nl = record_prefix(s);
         if (loop_mode == 2) {  // the corrective loop as one cooperative kernel after the prefix
             const cudaError_t le = nl < 0 ? cudaSuccess
@@ -300,12 +316,23 @@ struct pcisph_batch {
             *out = graph;
             return PCISPH_OK;
         }
+        const SceneTable t = scene_table();
+        const ListBuffers b = list_buffers(true);
+        cudaGraphConditionalHandle handle;
+        const cudaError_t he = cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault);
+        const int ahead = std::min(kIterationsAhead, sure_iters);
+        for (int k = 0; k < ahead && nl >= 0 && he == cudaSuccess; ++k) {
+            launch_pressure_scenes(t, b, k == 1, s);
+            launch_batch_decide(t, b, d_batch, max_iters, handle, k + 1 == ahead, s);
+            launch_pressure_force_scenes(t, b, s);
+        }
         cudaStreamCaptureStatus st;
         const cudaGraphNode_t* deps = nullptr;
         size_t ndeps = 0;
         cudaError_t e = cudaStreamGetCaptureInfo(s, &st, nullptr, nullptr, &deps, nullptr, &ndeps);
         std::vector<cudaGraphNode_t> leaves(deps, deps + (e == cudaSuccess ? ndeps : 0));
         cudaError_t e2 = cudaStreamEndCapture(s, &graph);
+        if (he != cudaSuccess) e = he;
         if (nl < 0 || e != cudaSuccess || e2 != cudaSuccess) {
             if (graph) cudaGraphDestroy(graph);
             return report_error(PCISPH_ERR_CUDA, std::string("graph capture of the batch step failed: ") +
@@ -313,10 +340,8 @@ struct pcisph_batch {
         }
         prefix_launches = nl;
         iter_launches = 3;
-        cudaGraphConditionalHandle handle;
         cudaGraphNodeParams cp{};
         cudaGraphNode_t loop_node;
-        e = cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault);
         if (e == cudaSuccess) {
             cp.type = cudaGraphNodeTypeConditional;
             cp.conditional.handle = handle;
@@ -331,10 +356,8 @@ struct pcisph_batch {
             cudaGraphDestroy(graph);
             return report_error(PCISPH_ERR_CUDA, std::string("graph loop node: ") + cudaGetErrorString(e));
         }
-        const SceneTable t = scene_table();
-        const ListBuffers b = list_buffers();
-        launch_pressure_scenes(t, b, s);
-        launch_batch_decide(t, d_batch, max_iters, handle, true, s);
+        launch_pressure_scenes(t, b, false, s);
+        launch_batch_decide(t, b, d_batch, max_iters, handle, true, s);
         launch_pressure_force_scenes(t, b, s);
         cudaGraph_t body = nullptr;
         e = cudaStreamEndCapture(s, &body);
@@ -402,7 +425,7 @@ struct pcisph_batch {
         if (nl < 0) return report_error(PCISPH_ERR_CUDA, std::string("batch step: ") + cudaGetErrorString(cudaGetLastError()));
         host_launches += nl;
         const SceneTable t = scene_table();
-        const ListBuffers b = list_buffers();
+        const ListBuffers b = list_buffers(loop_mode != 2);
         iter_launches = loop_mode == 2 ? 0 : 3;  // counted on the device per iteration (total_iters)
         if (loop_mode == 2) {
             cudaError_t le = cudaSuccess;
@@ -411,8 +434,8 @@ struct pcisph_batch {
             ++host_launches;
         } else {
             for (int it = 0; it < max_iters; ++it) {
-                timed("pressure", s, [&] { launch_pressure_scenes(t, b, s); });
-                timed("decide", s, [&] { launch_batch_decide(t, d_batch, max_iters, 0, false, s); });
+                timed("pressure", s, [&] { launch_pressure_scenes(t, b, it == 1, s); });
+                timed("decide", s, [&] { launch_batch_decide(t, b, d_batch, max_iters, 0, false, s); });
                 timed("pressure_force", s, [&] { launch_pressure_force_scenes(t, b, s); });
                 unsigned running = 0;
                 BTRY(cudaMemcpyAsync(&running, &d_batch->any_running, sizeof(unsigned), cudaMemcpyDeviceToHost, s));

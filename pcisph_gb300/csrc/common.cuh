@@ -113,8 +113,10 @@ __device__ __forceinline__ void close_step(Control* ctl, unsigned it, float rel,
     ctl->total_iters += it;
 }
 
-constexpr uint32_t kTightCap = 64;      // tight list entries per particle
+constexpr uint32_t kTightCap = 64;      // tight list entries per particle (a multiple of 8)
+constexpr uint32_t kTightSkin = 0xffffffffu;
 constexpr float kTightMargin = 0.035f;  // of h
+constexpr int kTightFrom = 4;           // iterations of the previous step (if there was one) from which a step builds them
 constexpr unsigned kTightAgain = 6;     // tight lists that were left behind are rebuilt from this iteration on
 constexpr unsigned kTightOff = 0, kTightBuild = 1, kTightUse = 2;
 constexpr uint32_t kNearCap = 64;  // within-h list entries per particle

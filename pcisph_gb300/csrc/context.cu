@@ -133,7 +133,7 @@ struct pcisph_ctx {
                            {zone_dim[0], zone_dim[1], zone_dim[2]},
                            m && !marks_inline(P.fluid_count) ? b.fast_list : nullptr,
                            m && marks ? b.walk_stamp : nullptr,
-                           tight ? tight_list : nullptr, tight_count, tight_ref};
+                           tight ? tight_list : nullptr, 0u, tight_count, tight_ref};
     }
     // the partners of fast predictions are marked in the graph and the host-driven loop
     bool partner_marks() const { return list_sweeps() && P.mark_cap != 0 && opts.loop_mode != 2; }
@@ -220,11 +220,7 @@ struct pcisph_ctx {
         const size_t n = params.fluid_count;
         if (n >= (1u << 31)) return fail(PCISPH_ERR_INVALID_ARG, "kernel variant 2 takes fewer than 2^31 particles");
         if (int rc = ensure_base_lists()) return rc;
-        return ensure_tight_lists();
-    }
-    // A scene whose tight lists find no memory does without.
-    int ensure_tight_lists() {
-        const size_t n = params.fluid_count;
+        // a scene whose tight lists find no memory does without
         const bool want = P.tight_margin > 0.f && opts.loop_mode != 2;
         if (want && tight_list && tight_n == n) return PCISPH_OK;
         if (!want && !tight_list) return PCISPH_OK;
@@ -232,7 +228,14 @@ struct pcisph_ctx {
         tight_list = nullptr;
         graph_valid = false;
         if (!want) return PCISPH_OK;
-        if (tight_block.ensure(align256(n * kTightCap * 4) + align256(n * 4) + align256(n * 16)) != cudaSuccess) {
+        const size_t bytes = align256(n * kTightCap * 4) + align256(n * 4) + align256(n * 16);
+        size_t room = 0, total = 0;
+        if (bytes > tight_block.cap) {  // never the last of the memory: a scene that just fits keeps room for its exports
+            tight_block.release();
+            CUDA_TRY(cudaMemGetInfo(&room, &total));
+            if (room < bytes + total / 8) return PCISPH_OK;
+        }
+        if (tight_block.ensure(bytes) != cudaSuccess) {
             cudaGetLastError();
             return PCISPH_OK;
         }
@@ -286,7 +289,6 @@ struct pcisph_ctx {
     // and reused in between: any placement of whole buckets keeps every sum, only locality ages as
     // particles change cells. order_age: steps since the last bucket sort ran, kNoOrder when none ran for
     // the current buffers and graphs.
-    static constexpr int kUnrolled = 3;  // iterations of the graph before its loop, at most
     static constexpr uint32_t kOrderRefresh = 8;
     static constexpr uint32_t kNoOrder = 0xFFFFFFFFu;
     uint32_t order_age = kNoOrder;
@@ -654,7 +656,7 @@ struct pcisph_ctx {
         // sweep that builds the tight lists (the second) is a kernel of its own.
         cudaGraphConditionalHandle handle;
         cudaError_t he = cudaGraphConditionalHandleCreate(&handle, graph, 1, cudaGraphCondAssignDefault);
-        const int before = std::max(1, std::min({kUnrolled, opts.min_iterations, opts.max_iterations}));
+        const int before = std::max(1, std::min({kIterationsAhead, opts.min_iterations, opts.max_iterations}));
         for (int k = 0; k < before && nl >= 0 && he == cudaSuccess; ++k) record_iteration(s, handle, k + 1 == before, k);
         cudaStreamCaptureStatus st;
         const cudaGraphNode_t* deps = nullptr;

@@ -21,7 +21,7 @@
 //     last for the rest of the step;
 //   - in a step of moving lists (lists_move: many particles faster than half the skin per step) the skin lists are
 //     built around y = x + v dt instead of x, and a prediction is fast when it strays half the skin from there;
-//   - from the third pressure sweep of a step on, one scene's sweeps read tight lists rebuilt at the second one's
+//   - from the third pressure sweep of a step on, the sweeps (past 8,192 particles, or of a batch) read tight lists rebuilt at the second one's
 //     predictions, as long as no prediction has moved past their margin from there (see tight_mode);
 //   - a particle with more than list_cap (near_cap) candidates is marked (count > cap) and walks the
 //     buckets in the sweeps that would use that list.
@@ -302,21 +302,25 @@ constexpr uint32_t kAll = 0xffffffffu;
 // Margins at 1M / 8.4M / a 98,904-particle drop / a violently jittered block of 110,592, us a step: 0.02 2284 / 70510 /
 // 1880 / 5075, 0.03 1998 / 68148 / 1840 / 4793, 0.04 2018 / 67244 / 1821 / 4556.
 //
+// A step of 3 iterations gains nothing (378 us of sweeps at 1M, 399 with them): the lists are built where the previous step
+// took 4 or more. Batch of 32 scenes, 1.32M particles: 46.4 -> 44.6 ms for 16 steps (46.3 without that rule: its falling
+// spheres walk in the building sweep, 456 us, for loops of 3).
+//
 // How far flags and marks reach ahead of half the skin in this round.
 __device__ __forceinline__ float tight_margin(const DevParams& P, const Control* ctl, const ListBuffers& b) {
     return b.tight && ctl->tight_next != kTightOff ? P.tight_margin : 0.f;
 }
 // How this pressure sweep finds its neighbours: constant while it runs.
-__device__ __forceinline__ unsigned tight_mode(const DevParams& P, const Control* ctl, const ListBuffers& b) {
-    if (!b.tight) return kTightOff;
+__device__ __forceinline__ unsigned tight_mode(const DevParams& P, const Control* ctl, bool on) {
+    if (!on) return kTightOff;
     const unsigned m = ctl->tight_next;
     if (m != kTightUse || ctl->tight_stray == 0u) return m;
     return ctl->tight_age != 0u && ctl->iter >= kTightAgain && (int)ctl->iter + 1 < P.max_iters ? kTightBuild : kTightOff;
 }
 // After a pressure sweep (before the decision): what the next one does.
-__device__ __forceinline__ void tight_advance(const DevParams& P, Control* ctl, const ListBuffers& b) {
-    if (!b.tight) return;
-    const unsigned m = tight_mode(P, ctl, b);
+__device__ __forceinline__ void tight_advance(const DevParams& P, Control* ctl, bool on) {
+    if (!on) return;
+    const unsigned m = tight_mode(P, ctl, on);
     if (m == kTightUse) {
         ctl->tight_age += 1;
     } else if (m == kTightBuild) {
@@ -331,7 +335,9 @@ __device__ __forceinline__ void tight_advance(const DevParams& P, Control* ctl, 
         ctl->tight_next = kTightOff;
     } else if (ctl->tight_wait != 0u) {
         ctl->tight_wait -= 1;
-    } else if ((ctl->iter == 0u || ctl->iter + 1u >= kTightAgain) && (int)ctl->iter + 2 < P.max_iters) {
+    } else if ((ctl->iter == 0u ? ctl->iterations_last == 0 || ctl->iterations_last >= kTightFrom
+                                : ctl->iter + 1u >= kTightAgain) &&
+               (int)ctl->iter + 2 < P.max_iters) {
         ctl->tight_next = kTightBuild;
     }
 }
@@ -1339,10 +1345,15 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         const bool all_lists_ok = lists_hold<PS>(ctl);
         const float4 xi = b.pos[i];
         const float4 xp = b.pred[i];
-        const unsigned mode = tight_mode(P, ctl, b);
+        const unsigned mode = tight_mode(P, ctl, b.tight != nullptr);
         build = mode == kTightBuild;
-        const uint32_t cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
-        const bool overflow = cnt > (mode == kTightUse ? kTightCap : P.list_cap);
+        uint32_t cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
+        bool tight = mode == kTightUse;
+        if (PS::kBatched && tight && cnt == kTightSkin) {
+            cnt = b.nbr_count[i];
+            tight = false;
+        }
+        const bool overflow = cnt > (tight ? kTightCap : P.list_cap);
         // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
         // skin) may miss a pair: with per-particle skins it walks. Boundary terms: all zero unless a boundary
         // particle was within r_list of x, or x* moved past the half skin (boundary particles do not move);
@@ -1387,7 +1398,13 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         auto add = [&](uint32_t j) {
             acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
         };
-        if (build) b.tight_ref[i] = xp;
+        if (build) {
+            b.tight_ref[i] = xp;
+            if (PS::kBatched && cnt > b.tight_below) {
+                b.tight_count[i] = walk ? kTightCap + 1u : kTightSkin;
+                build = false;
+            }
+        }
         if (build && (kWalks == Walks::kLane || !walk)) {
             acc = build_tight_list<kCoherent, kShared>(b, P, i, xp, cnt, acc, walk, c, stage_tight(stage));
             walk = false;
@@ -1395,7 +1412,7 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
             for_each_neighbour(b.cells, c, P, add);
             walk = false;
         } else if (!walk) {
-            for_each_listed(mode == kTightUse ? b.tight : b.nbr, i, cnt, b.nbr_stride, add);
+            for_each_listed(tight ? b.tight : b.nbr, i, cnt, b.nbr_stride, add);
         }
         if (!walk) dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
     }
@@ -1485,7 +1502,7 @@ __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1
             ctl->round += 1u;
             ctl->fast_n = lists_move(ps.params(0), ctl) ? kNoMarks : 0ull;  // moving lists: no marks
         }
-        tight_advance(ps.params(0), ctl, b);
+        tight_advance(ps.params(0), ctl, b.tight != nullptr);
         decide(ps.params(0), ctl);
     }
 }
@@ -1713,7 +1730,7 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
 // condition: continue while some scene iterates. A scene decided done here is integrated by the
 // pressure-force sweep that follows; the next call marks it finished. Every scene is done by its
 // max_iters, so the loop ends; the guard bounds it by the largest max_iters on its own.
-__global__ void k_batch_decide(const DevParams* __restrict__ table, Control* ctls, uint32_t n_scenes, Control* batch,
+__global__ void k_batch_decide(const DevParams* __restrict__ table, Control* ctls, uint32_t n_scenes, bool tight, Control* batch,
                                int max_iters, cudaGraphConditionalHandle cond, int use_cond) {
     __shared__ int running;
     if (threadIdx.x == 0) running = 0;
@@ -1724,6 +1741,7 @@ __global__ void k_batch_decide(const DevParams* __restrict__ table, Control* ctl
             c->finished = 1;
             continue;
         }
+        tight_advance(table[s], c, tight);
         decide(table[s], c);
         if (!c->done) atomicOr(&running, 1);
     }
@@ -1975,15 +1993,18 @@ void launch_normal_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_
 void launch_force_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s) {
     if (t.n) k_force_list<<<grid_for(t.n), kBlock, 0, s>>>(t, b);
 }
-void launch_pressure_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s) {
-    if (t.n) k_pressure_list<<<grid_for(t.n), kBlock, 0, s>>>(t, b);
+void launch_pressure_scenes(const SceneTable& t, const ListBuffers& b, bool builds, cudaStream_t s) {
+    if (!t.n) return;
+    if (builds && b.tight)
+        k_pressure_list<SceneTable, 128, 1, Walks::kCall, true><<<(t.n + 127) / 128, 128, 0, s>>>(t, b);
+    else k_pressure_list<<<grid_for(t.n), kBlock, 0, s>>>(t, b);
 }
 void launch_pressure_force_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s) {
     if (t.n) k_pressure_force_list<<<grid_for(t.n), kBlock, 0, s>>>(t, b, 0, 0, 0);
 }
-void launch_batch_decide(const SceneTable& t, Control* batch, int max_iters, cudaGraphConditionalHandle cond,
+void launch_batch_decide(const SceneTable& t, const ListBuffers& b, Control* batch, int max_iters, cudaGraphConditionalHandle cond,
                          bool use_cond, cudaStream_t s) {
-    k_batch_decide<<<1, 256, 0, s>>>(t.table, t.ctls, t.n_scenes, batch, max_iters, cond, use_cond ? 1 : 0);
+    k_batch_decide<<<1, 256, 0, s>>>(t.table, t.ctls, t.n_scenes, b.tight != nullptr, batch, max_iters, cond, use_cond ? 1 : 0);
 }
 
 }  // namespace pcisph

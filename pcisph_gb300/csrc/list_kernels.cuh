@@ -49,8 +49,10 @@ struct ListBuffers {
     uint32_t* fast_list;
     uint32_t* walk_stamp;
     // tight lists (or null): kTightCap entries per particle laid out like nbr, the entries per particle (> kTightCap: walk
-    // the buckets), and the predictions they were built at
+    // the buckets; kTightSkin: read the skin list), and the predictions they were built at. In a batch they lie where the
+    // skin list entries from tight_below on do: a particle with more keeps its skin list.
     uint32_t* tight;
+    uint32_t tight_below;
     uint32_t* tight_count;
     float4* tight_ref;
 };
@@ -129,7 +131,7 @@ void launch_hash_scenes(const SceneTable& t, const float4* pos, uint32_t* keys, 
 void launch_density_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s);
 void launch_normal_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s);
 void launch_force_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s);
-void launch_pressure_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s);
+void launch_pressure_scenes(const SceneTable& t, const ListBuffers& b, bool builds, cudaStream_t s);
 void launch_pressure_force_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s);
 // The whole corrective loop of a step in one cooperative launch (loop_mode 2); errors if the device cannot
 // run it (cooperative launch unsupported).
@@ -137,7 +139,7 @@ cudaError_t launch_corrective_loop(const DevParams& P, Control* ctl, const ListB
 cudaError_t launch_corrective_loop_scenes(const SceneTable& t, const ListBuffers& b, Control* batch, int max_iters,
                                           cudaStream_t s);
 // per-scene loop decision; sets the while-loop condition (continue while a scene iterates)
-void launch_batch_decide(const SceneTable& t, Control* batch, int max_iters, cudaGraphConditionalHandle cond,
+void launch_batch_decide(const SceneTable& t, const ListBuffers& b, Control* batch, int max_iters, cudaGraphConditionalHandle cond,
                          bool use_cond, cudaStream_t s);
 
 }  // namespace pcisph
