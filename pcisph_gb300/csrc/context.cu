@@ -388,11 +388,10 @@ struct pcisph_ctx {
                        opts.restitution, threshold, opts.list_skin, 0, &P);
         const bool skins = opts.particle_skin == 1 || (opts.particle_skin == 2 && params.boundary_count > 0);
         P.particle_skin = skins && list_sweeps() ? 1 : 0;
-        P.skin_min_half = std::min(kSkinMinHalf * P.h, P.skin_max_half);
         P.skin_factor = kSkinFactor;
         P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
-        set_tight_lists(&P, list_sweeps() && !P.particle_skin && !marks_inline(params.fluid_count) &&
-                                P.h + P.skin_max_half + kTightMargin * P.h <= 1.9f * P.cell_size);
+        set_tight_lists(&P, list_sweeps() && P.h + P.skin_max_half + kTightMargin * P.h <= 1.9f * P.cell_size);
+        P.skin_min_half = std::min(kSkinMinHalf * P.h + P.tight_margin, P.skin_max_half);
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
         // cells (with a margin for the divisions of cell_of). With more than 1 in 8 fast nearly every warp holds walkers

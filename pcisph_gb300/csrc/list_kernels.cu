@@ -21,7 +21,7 @@
 //     last for the rest of the step;
 //   - in a step of moving lists (lists_move: many particles faster than half the skin per step) the skin lists are
 //     built around y = x + v dt instead of x, and a prediction is fast when it strays half the skin from there;
-//   - from the third pressure sweep of a step on, the sweeps (past 8,192 particles, or of a batch) read tight lists rebuilt at the second one's
+//   - from the third pressure sweep of a step on, the sweeps read tight lists rebuilt at the second one's
 //     predictions, as long as no prediction has moved past their margin from there (see tight_mode);
 //   - a particle with more than list_cap (near_cap) candidates is marked (count > cap) and walks the
 //     buckets in the sweeps that would use that list.
@@ -182,7 +182,7 @@ __device__ __forceinline__ void for_each_listed_deep(const uint32_t* __restrict_
 // one-lane sweep: entries that contribute nothing add zero).
 
 // The entries of this lane, chunk by chunk, in batches of U chunks whose gathers are in flight together: load(j) for
-// the lane's entry, then sum(value, valid) once per chunk by the whole warp. n: this particle's entries; most: the
+// the lane's entry, then sum(value, entry, valid) once per chunk by the whole warp. n: this particle's entries; most: the
 // warp's largest n.
 template <int L, int U, class Load, class Sum>
 __device__ __forceinline__ void for_each_shared(const uint32_t* __restrict__ list, uint32_t i, uint32_t n, uint32_t most,
@@ -195,14 +195,17 @@ __device__ __forceinline__ void for_each_shared(const uint32_t* __restrict__ lis
 #pragma unroll 1
     for (uint32_t e = q; e - q < most; e += L * U) {
         decltype(load(0u)) o[U];
+        uint32_t k[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u)
+        for (int u = 0; u < U; ++u) {
             if (e + L * u < n) o[u] = load(j[u]);
+            k[u] = j[u];
+        }
 #pragma unroll
         for (int u = 0; u < U; ++u) j[u] = e + L * (U + u) < n ? entry(e + L * (U + u)) : 0u;
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (e - q + L * u < most) sum(o[u], e + L * u < n);
+            if (e - q + L * u < most) sum(o[u], k[u], e + L * u < n);
     }
 }
 
@@ -305,6 +308,10 @@ constexpr uint32_t kAll = 0xffffffffu;
 // A step of 3 iterations gains nothing (378 us of sweeps at 1M, 399 with them): the lists are built where the previous step
 // took 4 or more. Batch of 32 scenes, 1.32M particles: 46.4 -> 44.6 ms for 16 steps (46.3 without that rule: its falling
 // spheres walk in the building sweep, 456 us, for loops of 3).
+//
+// Per-particle skins (scenes with boundary particles): each skin is m wider, so that a particle within its skin less m at
+// the building stays within it: 1,048,576 fluid particles in a tank 2454 -> 2382 us a step, 279,936 862 -> 840.
+// Eight lanes per particle: 4,096 particles at rest 159 -> 157 us, 8,000 violently jittered 985 -> 667.
 //
 // How far flags and marks reach ahead of half the skin in this round.
 __device__ __forceinline__ float tight_margin(const DevParams& P, const Control* ctl, const ListBuffers& b) {
@@ -1043,7 +1050,7 @@ __global__ void __launch_bounds__(kBlock) k_normal_shared(PS ps, ListBuffers b) 
     };
     for_each_shared<L, 32 / L>(
         b.near, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.pr4[j]); },
-        [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+        [&](const float4& o, uint32_t, bool valid) { sum(o, valid, kAll); });
     if (!listed)
         walk_shared<L>(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, q, [&](uint32_t j, bool valid) {
             float4 o = xi;
@@ -1089,7 +1096,7 @@ __global__ void __launch_bounds__(kBlock) k_force_shared(PS ps, ListBuffers b) {
         add_lanes(curv, d, S, q, m);
     };
     for_each_shared<L, 16 / L>(b.near, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, load,
-                       [&](const ForceOperand& o, bool valid) { sum(o, valid, kAll); });
+                       [&](const ForceOperand& o, uint32_t, bool valid) { sum(o, valid, kAll); });
     if (!listed)
         walk_shared<L>(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, q, [&](uint32_t j, bool valid) {
             ForceOperand o{xi, xi, xi};
@@ -1124,11 +1131,11 @@ struct PressurePlan {
 template <class PS>
 __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBuffers& b, const DevParams& P,
                                                       const Control* ctl, uint32_t i, const float4& xi,
-                                                      const float4& xp) {
+                                                      const float4& xp, unsigned mode) {
     PressurePlan p;
     const bool all_lists_ok = lists_hold<PS>(ctl);
-    p.cnt = b.nbr_count[i];
-    const bool overflow = p.cnt > P.list_cap;
+    p.cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
+    const bool overflow = p.cnt > (mode == kTightUse ? kTightCap : P.list_cap);
     // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
     // skin) may miss a pair: with per-particle skins it walks. Boundary terms: all zero unless a boundary
     // particle was within r_list of x, or x* moved past the half skin (boundary particles do not move);
@@ -1137,7 +1144,8 @@ __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBu
     bool self_fast = false;
     if (P.particle_skin || P.boundary_count) {
         const float dx = xp.x - xi.x, dy = xp.y - xi.y, dz = xp.z - xi.z;
-        self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w));
+        const float ahead = mode == kTightBuild && P.particle_skin ? P.tight_margin : 0.f;
+        self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w)) - ahead;
     }
     p.walk_boundary = p.list_boundary = false;
     p.bcnt = 0;
@@ -1157,7 +1165,10 @@ __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBu
     // the bucket flags: every particle near a fast one walks
     const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
     const bool marks = fast_round <= P.mark_cap;
-    if (marks) {
+    if (mode == kTightUse) {
+        p.walk = overflow;
+        if (p.walk || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
+    } else if (marks) {
         p.walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
         if (p.walk || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
     } else {
@@ -1362,7 +1373,8 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         bool self_fast = false;
         if (P.particle_skin || P.boundary_count) {
             const float dx = xp.x - xi.x, dy = xp.y - xi.y, dz = xp.z - xi.z;
-            self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w));
+            const float ahead = build && P.particle_skin ? P.tight_margin : 0.f;
+            self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w)) - ahead;
         }
         bool walk_boundary = false, list_boundary = false;
         uint32_t bcnt = 0;
@@ -1439,7 +1451,8 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
     const float4 xi = b.pos[i];
     const float4 xp = b.pred[i];
     PressurePlan p{};
-    if (live) p = plan_pressure(ps, b, P, ctl, i, xi, xp);
+    const unsigned mode = tight_mode(P, ctl, b.tight != nullptr);
+    if (live) p = plan_pressure(ps, b, P, ctl, i, xi, xp, mode);
     float acc = 0.f;
     auto sum = [&](const float4& o, bool valid, uint32_t m) {
         add_lanes<L>(acc, valid ? density_term(xp.x, xp.y, xp.z, o, P.h2) : 0.f, m);
@@ -1455,14 +1468,39 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
         const uint32_t n = p.list_boundary ? p.bcnt : 0u;
         for_each_shared<L, 32 / L>(
             b.bnbr, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.b_pos[j]); },
-            [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+            [&](const float4& o, uint32_t, bool valid) { sum(o, valid, kAll); });
         if (p.walk_boundary) walk(b.b_cells, b.b_pos);
     }
     const uint32_t n = live && !p.walk ? p.cnt : 0u;
-    for_each_shared<L, 32 / L>(
-        b.nbr, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.pred[j]); },
-        [&](const float4& o, bool valid) { sum(o, valid, kAll); });
-    if (p.walk) walk(b.cells, b.pred);
+    const uint32_t most = __reduce_max_sync(kAll, n);
+    auto load = [&](uint32_t j) { return __ldg(&b.pred[j]); };
+    if (mode == kTightBuild) {
+        uint32_t kept = 0;
+        auto keep = [&](const float4& o, uint32_t j, bool valid, uint32_t m) {
+            const float d2 = dist2(xp.x - o.x, xp.y - o.y, xp.z - o.z);
+            add_lanes<L>(acc, valid ? poly6(d2, P.h2) : 0.f, m);
+            const bool in = valid && !(d2 > P.tight_r2);
+            const uint32_t set = __ballot_sync(m, in) & mask, e = kept + __popc(set & lanes_below());
+            if (in && e < kTightCap) reinterpret_cast<uint32_t*>(list_chunk(b.tight, i, e >> 3, b.nbr_stride))[e & 7u] = j;
+            kept += __popc(set);
+        };
+        for_each_shared<L, 32 / L>(b.nbr, i, n, most, b.nbr_stride, q, load,
+                                   [&](const float4& o, uint32_t j, bool valid) { keep(o, j, valid, kAll); });
+        if (p.walk)
+            walk_shared<L>(b.cells, p.c, P, q, [&](uint32_t j, bool valid) {
+                float4 o = xp;
+                if (valid) o = load(j);
+                keep(o, j, valid, mask);
+            });
+        if (live && q == 0) {
+            b.tight_count[i] = kept;
+            b.tight_ref[i] = xp;
+        }
+    } else {
+        for_each_shared<L, 32 / L>(mode == kTightUse ? b.tight : b.nbr, i, n, most, b.nbr_stride, q, load,
+                                   [&](const float4& o, uint32_t, bool valid) { sum(o, valid, kAll); });
+        if (p.walk) walk(b.cells, b.pred);
+    }
     float dv = 0.f;
     if (live && q == 0) dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
     return dv;
@@ -1498,11 +1536,14 @@ __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1
     if (is_last && threadIdx.x == 0) {
         __threadfence();
         ctl->max_err_bits = atomicAdd(&ctl->max_err_bits, 0u);  // see every block's contribution
+        tight_advance(ps.params(0), ctl, b.tight != nullptr);
         if (b.walk_stamp) {  // close the prediction round of the partner marks: the next one starts empty
             ctl->round += 1u;
-            ctl->fast_n = lists_move(ps.params(0), ctl) ? kNoMarks : 0ull;  // moving lists: no marks
+            // no marks with moving lists, nor by a predicting sweep that expects the next to read tight lists (one that
+            // then does not takes the bucket flags)
+            const bool none = lists_move(ps.params(0), ctl) || (!b.fast_list && b.tight && ctl->tight_next == kTightUse);
+            ctl->fast_n = none ? kNoMarks : 0ull;
         }
-        tight_advance(ps.params(0), ctl, b.tight != nullptr);
         decide(ps.params(0), ctl);
     }
 }
@@ -1559,7 +1600,7 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
     b.state_pos[o] = f4(x, 0.f);
     b.state_vel[o] = f4(v, 0.f);
     if (P.particle_skin)  // the next step's half skin: twice this step's largest predicted displacement
-        b.state_skin[o] = fminf(fmaxf(P.skin_factor * b.disp_max[i], P.skin_min_half), P.skin_max_half);
+        b.state_skin[o] = fminf(fmaxf(P.skin_factor * b.disp_max[i] + P.tight_margin, P.skin_min_half), P.skin_max_half);
     return false;
 }
 
@@ -1625,14 +1666,14 @@ __device__ __forceinline__ bool pressure_force_shared(const PS& ps, const ListBu
         const uint32_t n = listed ? bcnt : 0u;
         for_each_shared<L, 32 / L>(
             b.bnbr, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.bpf[j]); },
-            [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+            [&](const float4& o, uint32_t, bool valid) { sum(o, valid, kAll); });
         if (near_b && !listed) walk(b.b_cells, b.bpf);
     }
     const uint32_t cnt = live ? b.near_count[i] : 0u;
     const uint32_t n = cnt <= P.near_cap ? cnt : 0u;
     for_each_shared<L, 32 / L>(
         b.near, i, n, __reduce_max_sync(kAll, n), b.nbr_stride, q, [&](uint32_t j) { return __ldg(&b.pf4[j]); },
-        [&](const float4& o, bool valid) { sum(o, valid, kAll); });
+        [&](const float4& o, uint32_t, bool valid) { sum(o, valid, kAll); });
     if (cnt > P.near_cap) walk(b.cells, b.pf4);
     const float y = __shfl_sync(mask, acc, 1, L), z = __shfl_sync(mask, acc, 2, L);
     if (live && q == 0) return finish_pressure_force(ps, b, P, ps.control(i), i, xi, make_float3(acc, y, z), mode);

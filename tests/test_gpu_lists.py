@@ -157,14 +157,18 @@ def test_moving_lists_keep_nonfinite_velocities(oracle):
 
 
 # The pressure sweeps from the third iteration on read lists rebuilt at the second one's predictions. Sizes at the edges of
-# their launches (from 8,193; 155,648 and 194,560 where the building sweep changes its form; past 2M); loops that end before
+# their launches (8,192; 155,648 and 194,560 where the building sweep changes its form; past 2M); loops that end before
 # a list is built, before it is used and long after it was left behind; a block that overflows them; predictions that
 # outrun every list at once or keep leaving the rebuilt ones; boundary particles; skins of other sizes; NaN
 @pytest.mark.parametrize("n,gap,jitter,speed,iters,options", [
+    (1, 1.0, 0.1, 0.0, (5, 5), {}), (4097, 1.0, 0.3, 1.0, (25, 25), {}), (8192, 0.75, 0.4, 8.0, (12, 12), {}),
+    (5000, 1.0, 0.2, 0.0, (20, 20), {"boundary": 1}), (5001, 1.0, 0.1, 4.0, (8, 8), {"list_skin": 0.0}),
+    (7777, 1.0, 0.2, 3.0, (9, 9), {"nan": 1}),
     (8193, 1.0, 0.1, 0.0, (3, 3), {}), (9001, 1.0, 0.1, 0.0, (1, 1), {}), (9001, 1.0, 0.1, 0.0, (2, 2), {}),
     (9001, 1.0, 0.2, 0.0, (1, 9), {}), (20000, 1.0, 0.3, 0.0, (40, 40), {}), (30000, 0.8, 0.1, 0.0, (12, 12), {}),
     (30000, 0.75, 0.4, 8.0, (30, 30), {}), (12000, 1.0, 0.1, 4.0, (8, 8), {"list_skin": 0.0}),
     (12000, 1.0, 0.3, 1.0, (25, 25), {"list_skin": 0.5}), (16000, 1.0, 0.2, 0.0, (20, 20), {"particle_skin": 0, "boundary": 1}),
+    (16000, 1.0, 0.2, 0.0, (20, 20), {"boundary": 1}), (16000, 1.0, 0.3, 1.0, (9, 9), {"particle_skin": 1}),
     (16000, 1.0, 0.2, 3.0, (20, 20), {"nan": 1}), (155648, 1.0, 0.2, 0.0, (12, 12), {}),
     (155649, 1.0, 0.15, 0.0, (8, 8), {"sweep_block": 512}), (194561, 1.0, 0.2, 0.5, (9, 9), {"sweep_block": 128}),
     (2097153, 1.0, 0.2, 0.0, (9, 9), {})])
