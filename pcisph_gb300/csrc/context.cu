@@ -197,7 +197,7 @@ struct pcisph_ctx {
             launch_permute(sk, sv, b.state_pos, b.state_vel, N, BK, b.cells, cells_w, b.pos, b.vel, d_of_w, w_of_d,
                            b.ctl, s, P.particle_skin ? b.state_skin : nullptr);
         });
-        nl += 4;
+        nl += 3;
         return cudaGetLastError() == cudaSuccess ? nl : -1;
     }
 
@@ -517,10 +517,8 @@ struct pcisph_ctx {
     int record_prefix(cudaStream_t s) {
         const uint32_t N = params.fluid_count, B = params.boundary_count;
         int nl = 0;
-        launch_begin(b.ctl, s);
+        launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, s);
         ++nl;
-        if (cudaMemsetAsync(b.cells, 0, (size_t)params.bucket_count * 8, s) != cudaSuccess) return -1;
-        if (list_sweeps() && cudaMemsetAsync(b.bucket_fast, 0, params.bucket_count, s) != cudaSuccess) return -1;
         uint32_t *sk = nullptr, *sv = nullptr;
         int r = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s, P.moving_lists ? b.state_vel : nullptr);
         if (r < 0) return -1;
@@ -784,9 +782,7 @@ struct pcisph_ctx {
                     rc = boundary_sort(s);
                     if (rc) return rc;
                 }
-                launch_begin(b.ctl, s);
-                CUDA_TRY(cudaMemsetAsync(b.cells, 0, (size_t)params.bucket_count * 8, s));
-                if (list_sweeps()) CUDA_TRY(cudaMemsetAsync(b.bucket_fast, 0, params.bucket_count, s));
+                launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, s);
                 uint32_t *sk = nullptr, *sv = nullptr;
                 int nl = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s, P.moving_lists ? b.state_vel : nullptr);
                 if (nl < 0) return PCISPH_ERR_CUDA;

@@ -25,7 +25,7 @@ void launch_bucket_codes(const uint32_t* sorted_keys, const uint32_t* sorted_ids
 // Elements of scan scratch for bk buckets.
 size_t working_ranges_scratch(uint32_t bk);
 // order = bucket ids sorted by code; lengths from cells_d; cells_w[b] = range of bucket b in working order
-// (exclusive scan of the lengths in `order`, clamped to [0, n]). Three launches.
+// (exclusive scan of the lengths in `order`, clamped to [0, n]). Two launches.
 void launch_working_ranges(const uint32_t* order, uint32_t bk, const uint2* cells_d, uint2* cells_w,
                            uint32_t* scratch, uint32_t n, cudaStream_t s);
 

