@@ -908,6 +908,33 @@ struct pcisph_ctx {
         return PCISPH_OK;
     }
 
+    // Where the device reads or writes a packed array of the caller: itself, its pinned host memory, or null (staged).
+    static float* direct_view(const float* p, int memory) {
+        if (memory == PCISPH_MEM_DEVICE) return const_cast<float*>(p);
+        return const_cast<float*>(static_cast<const float*>(host::pinned_device_view(p)));
+    }
+
+    // Positions and velocities in one launch, where both are packed and reach the device without staging.
+    // false: not this case, nothing done.
+    bool copy_state_in(const float* pos, const float* vel, size_t n, int layout, int memory) {
+        if (!vel || !n || layout != PCISPH_LAYOUT_PACKED3) return false;
+        const float *p = direct_view(pos, memory), *v = p ? direct_view(vel, memory) : nullptr;
+        if (!p || !v) return false;
+        launch_pack3_to4(p, b.state_pos, (uint32_t)n, stream(), v, b.state_vel);
+        ++host_launches;
+        return true;
+    }
+    bool copy_state_out(float* pos, float* vel, size_t n, int layout, int memory) {
+        if (!pos || !vel || !n || !b.state_pos || layout != PCISPH_LAYOUT_PACKED3) return false;
+        const uintptr_t a = (uintptr_t)pos, c = (uintptr_t)vel;
+        if (a < c + n * 12 && c < a + n * 12) return false;  // overlapping: one after the other
+        float *p = direct_view(pos, memory), *v = p ? direct_view(vel, memory) : nullptr;
+        if (!p || !v) return false;
+        launch_unpack4_to3(b.state_pos, p, (uint32_t)n, stream(), b.state_vel, v);
+        ++host_launches;
+        return true;
+    }
+
     // sync = false: a HOST copy is left queued (the caller synchronises)
     int get_field(int field, void* dst, size_t dst_bytes, int layout, int memory, bool sync = true) {
         FieldView v;
@@ -1195,9 +1222,13 @@ int pcisph_get_fluid_state(pcisph_ctx* ctx, float* pos, float* vel, uint32_t cou
     DeviceGuard g(ctx->device);
     const size_t bytes = (size_t)count * (layout == PCISPH_LAYOUT_PACKED3 ? 12 : 16);
     int rc = PCISPH_OK;
-    if (pos) rc = ctx->get_field(PCISPH_FIELD_POSITION, pos, bytes, layout, memory, false);
-    if (!rc && vel) rc = ctx->get_field(PCISPH_FIELD_VELOCITY, vel, bytes, layout, memory, false);
-    if (rc) return rc;
+    if (ctx->copy_state_out(pos, vel, count, layout, memory)) {
+        CUDA_TRY(cudaGetLastError());
+    } else {
+        if (pos) rc = ctx->get_field(PCISPH_FIELD_POSITION, pos, bytes, layout, memory, false);
+        if (!rc && vel) rc = ctx->get_field(PCISPH_FIELD_VELOCITY, vel, bytes, layout, memory, false);
+        if (rc) return rc;
+    }
     if (memory == PCISPH_MEM_HOST) CUDA_TRY(cudaStreamSynchronize(ctx->stream()));
     return PCISPH_OK;
 }
@@ -1218,11 +1249,15 @@ int pcisph_set_fluid_state(pcisph_ctx* ctx, const float* pos, const float* vel, 
     bk = std::max(64u, bk);
     int rc = ctx->ensure_fluid(count, bk);
     if (rc) return rc;
-    rc = ctx->copy_vectors_in(ctx->b.state_pos, pos, count, layout, memory);
-    if (rc) return rc;
-    if (vel) rc = ctx->copy_vectors_in(ctx->b.state_vel, vel, count, layout, memory);
-    else if (count) CUDA_TRY(cudaMemsetAsync(ctx->b.state_vel, 0, (size_t)count * 16, ctx->stream()));
-    if (rc) return rc;
+    if (ctx->copy_state_in(pos, vel, count, layout, memory)) {
+        CUDA_TRY(cudaGetLastError());
+    } else {
+        rc = ctx->copy_vectors_in(ctx->b.state_pos, pos, count, layout, memory);
+        if (rc) return rc;
+        if (vel) rc = ctx->copy_vectors_in(ctx->b.state_vel, vel, count, layout, memory);
+        else if (count) CUDA_TRY(cudaMemsetAsync(ctx->b.state_vel, 0, (size_t)count * 16, ctx->stream()));
+        if (rc) return rc;
+    }
     if (memory == PCISPH_MEM_HOST) CUDA_TRY(cudaStreamSynchronize(ctx->stream()));
     ctx->fluid_loaded = count;
     return PCISPH_OK;

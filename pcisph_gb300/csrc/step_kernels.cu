@@ -372,8 +372,11 @@ __global__ void __launch_bounds__(kBlock) k_pack_boundary(DevParams P, const flo
 // rows (thread t: floats t, t + 256, t + 512) through shared memory (stride-3 element access there is
 // conflict-free), so every request covers whole 128-byte lines: this matters most when the packed side is
 // pinned host memory read or written over the host link.
+// Positions and velocities go together, blockIdx.y picking the array: one launch less on either side of a step.
 __global__ void __launch_bounds__(kBlock) k_pack3_to4(const float* __restrict__ in3, float4* __restrict__ out,
+                                                      const float* __restrict__ in3b, float4* __restrict__ outb,
                                                       uint32_t n) {
+    if (blockIdx.y) in3 = in3b, out = outb;
     __shared__ float tile[3 * kBlock];
     const size_t base = (size_t)blockIdx.x * kBlock;
     const size_t total = 3 * (size_t)n;
@@ -391,7 +394,9 @@ __global__ void __launch_bounds__(kBlock) k_pack3_to4(const float* __restrict__ 
 }
 
 __global__ void __launch_bounds__(kBlock) k_unpack4_to3(const float4* __restrict__ in, float* __restrict__ out3,
+                                                        const float4* __restrict__ inb, float* __restrict__ out3b,
                                                         uint32_t n) {
+    if (blockIdx.y) in = inb, out3 = out3b;
     __shared__ float tile[3 * kBlock];
     const size_t base = (size_t)blockIdx.x * kBlock;
     const size_t i = base + threadIdx.x;
@@ -474,12 +479,12 @@ void launch_pack(const DevParams& P, const StepBuffers& b, cudaStream_t s) {
         k_pack_boundary<<<grid_for(P.boundary_count), kBlock, 0, s>>>(P, b.b_pos, b.b_press, b.bpf);
 }
 
-void launch_pack3_to4(const float* in3, float4* out, uint32_t n, cudaStream_t s) {
-    if (n) k_pack3_to4<<<grid_for(n), kBlock, 0, s>>>(in3, out, n);
+void launch_pack3_to4(const float* in3, float4* out, uint32_t n, cudaStream_t s, const float* in3b, float4* outb) {
+    if (n) k_pack3_to4<<<dim3(grid_for(n), in3b ? 2 : 1), kBlock, 0, s>>>(in3, out, in3b, outb, n);
 }
 
-void launch_unpack4_to3(const float4* in, float* out3, uint32_t n, cudaStream_t s) {
-    if (n) k_unpack4_to3<<<grid_for(n), kBlock, 0, s>>>(in, out3, n);
+void launch_unpack4_to3(const float4* in, float* out3, uint32_t n, cudaStream_t s, const float4* inb, float* out3b) {
+    if (n) k_unpack4_to3<<<dim3(grid_for(n), inb ? 2 : 1), kBlock, 0, s>>>(in, out3, inb, out3b, n);
 }
 
 }  // namespace pcisph

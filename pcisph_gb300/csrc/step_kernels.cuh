@@ -86,7 +86,10 @@ void launch_pressure_sweep(const DevParams& P, const StepBuffers& b, const Sweep
 void launch_pressure_force_sweep(const DevParams& P, const StepBuffers& b, const SweepArgs& A, const SweepGrid& g,
                                  int mode, cudaGraphConditionalHandle cond, bool use_cond, cudaStream_t s);
 
-void launch_pack3_to4(const float* in3, float4* out, uint32_t n, cudaStream_t s);
-void launch_unpack4_to3(const float4* in, float* out3, uint32_t n, cudaStream_t s);
+// One array, or (in3b, outb; inb, out3b) two of n in one launch.
+void launch_pack3_to4(const float* in3, float4* out, uint32_t n, cudaStream_t s, const float* in3b = nullptr,
+                      float4* outb = nullptr);
+void launch_unpack4_to3(const float4* in, float* out3, uint32_t n, cudaStream_t s, const float4* inb = nullptr,
+                        float* out3b = nullptr);
 
 }  // namespace pcisph

@@ -851,3 +851,30 @@ def test_rederive_after_autotune_keeps_a_valid_sort_scratch():
     st = f.stats()
     assert st.steps == 5 and (st.status_all & 4) == 0
     f.close()
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 5000])
+@pytest.mark.parametrize("memory", ["device", "pinned", "host"])
+def test_state_goes_in_and_out_unchanged(oracle, n, memory):
+    """Positions and velocities travel in one launch where neither is staged; alone, and into overlapping outputs, each by
+    itself."""
+    import torch
+    rng = np.random.default_rng(n)
+    p = oracle.derive_params(0.01, 1000.0, n, 0, 1e-3, -9.81, 0.0, 0.0)
+    f = fluid_like(p)
+    host = [torch.from_numpy(rng.standard_normal((n, 3)).astype(np.float32)) for _ in range(2)]
+    place = {"device": lambda t: t.cuda(), "pinned": lambda t: t.pin_memory(), "host": lambda t: t.clone()}[memory]
+    arg = (lambda t: t) if memory == "device" else (lambda t: t.numpy())
+    x, v = (place(t) for t in host)
+    f.set_fluid_state(arg(x), arg(v))
+    a, b = (place(torch.zeros((n, 3))) for _ in range(2))
+    f.get_fluid_state(arg(a), arg(b))
+    f.sync()
+    assert torch.equal(a.cpu(), host[0]) and torch.equal(b.cpu(), host[1])
+    both = place(torch.zeros((n + 1, 3)))  # the second output begins one particle into the first
+    f.get_fluid_state(arg(both[:n]), arg(both[1:]))
+    f.sync()
+    assert torch.equal(both[:1].cpu(), host[0][:1]) and torch.equal(both[1:].cpu(), host[1])
+    f.set_fluid_state(arg(v))
+    assert np.array_equal(f.get_field("position"), host[1].numpy()) and not f.get_field("velocity").any()
+    f.close()
