@@ -42,3 +42,24 @@ def test_record_writes_frames(tmp_path):
         img = render.read_png(p)
         assert img.shape == (48, 64, 3) and img.max() > 0
     f.close()
+
+
+# one sphere more, out of sight, takes the next split of a sphere's rows over lanes
+@pytest.mark.parametrize("n", [32768, 131072, 524288])
+def test_splits_of_the_rows_draw_the_same_image(n):
+    rng = np.random.default_rng(n)
+    pos = rng.random((n, 3)).astype(np.float32)
+    pos[:200] += np.float32([0.0, 0.0, 1.0])  # nearer and larger
+    cam = render.camera(eye=(0.5, 0.6, 3.0), target=(0.5, 0.5, 0.5), fov_x_degrees=40.0)
+    images = []
+    for extra in (False, True):
+        x = np.concatenate([pos, np.float32([[0.5, 0.5, 40.0]])]) if extra else pos
+        f = Fluid(0)
+        f.set_particle_radius(0.01)
+        f.set_fluid_count(len(x))
+        f.prepare()
+        f.set_fluid_state(x)
+        images.append(render.render(f, cam, 322, 241))
+        f.close()
+    assert images[0].any()
+    np.testing.assert_array_equal(images[0], images[1])
