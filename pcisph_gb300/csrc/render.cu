@@ -71,7 +71,8 @@ __device__ __forceinline__ float hit_ray(float rx, float ry, float3 s, float out
 // Bound by the pixel tests (~50 a sphere of the 1M scene at 1280 x 720). The rays of kStrip columns are set up once and stay in
 // registers for all rows (a division a column and a row instead of one a pixel). The rows of a sphere are dealt to kLanes
 // lanes: few spheres are large ones, and do not fill the chip. A frame of 1,048,576 spheres 147 -> 119 us (2 lanes 123, 4
-// 145), of 262,144 95 -> 89 (1 lane 97, 8 108), of 64,000 83 -> 71 (1 lane 83), of 4,096 at 1920 x 721 311 -> 85 (1 lane 275).
+// 145), of 262,144 95 -> 87 (1 lane 97, 8 108), of 64,000 82 -> 71 (1 lane 83), of 4,096 at 1920 x 721 312 -> 85 (1 lane 275); small
+// spheres keep one lane (262,144 at 320 x 240 43 -> 41).
 // The image depends on each sum's last bit where a sphere is grazed: as before, the first (columns mod 4) columns of a sphere
 // add rounded products, the others fuse.
 constexpr int kStrip = 8;
@@ -201,9 +202,12 @@ extern "C" int pcisph_render(const float* pos4, const float* density, uint32_t n
             constexpr uint32_t L = decltype(lanes)::value, per = kBlock / L;
             k_splat<L><<<(n + per - 1) / per, kBlock, 0, s>>>(reinterpret_cast<const float4*>(pos4), n, c, z);
         };
-        if (n <= 32768u) splat(std::integral_constant<uint32_t, 8>{});
-        else if (n <= 131072u) splat(std::integral_constant<uint32_t, 4>{});
-        else if (n <= 524288u) splat(std::integral_constant<uint32_t, 2>{});
+        // lanes by the number of spheres, and 2.5 rows a lane at least for a sphere as far away as the target
+        const float rows = 2.f * (c.radius / (fl * c.tan_half_x) * 0.5f * width + 1.f) + 1.f;
+        const float most = rows / 2.5f;
+        if (n <= 32768u && most >= 8.f) splat(std::integral_constant<uint32_t, 8>{});
+        else if (n <= 131072u && most >= 4.f) splat(std::integral_constant<uint32_t, 4>{});
+        else if (n <= 524288u && most >= 2.f) splat(std::integral_constant<uint32_t, 2>{});
         else splat(std::integral_constant<uint32_t, 1>{});
     }
     const uint32_t pixels = (uint32_t)width * (uint32_t)height;
