@@ -222,10 +222,10 @@ struct pcisph_ctx {
         if (int rc = ensure_base_lists()) return rc;
         // a scene whose tight lists find no memory does without
         const bool want = P.tight_margin > 0.f && opts.loop_mode != 2;
-        if (want && tight_list && tight_n == n) return PCISPH_OK;
-        if (!want && !tight_list) return PCISPH_OK;
+        if (want ? tight_n == n : !tight_list) return PCISPH_OK;  // tried once for a particle count
         CUDA_TRY(cudaStreamSynchronize(stream()));
         tight_list = nullptr;
+        tight_n = want ? n : 0;
         graph_valid = false;
         if (!want) return PCISPH_OK;
         const size_t bytes = align256(n * kTightCap * 4) + align256(n * 4) + align256(n * 16);
@@ -243,7 +243,6 @@ struct pcisph_ctx {
         tight_list = c.take<uint32_t>(n * kTightCap);
         tight_count = c.take<uint32_t>(n);
         tight_ref = c.take<float4>(n);
-        tight_n = n;
         return PCISPH_OK;
     }
     int ensure_base_lists() {

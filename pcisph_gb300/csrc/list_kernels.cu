@@ -313,7 +313,7 @@ constexpr uint32_t kAll = 0xffffffffu;
 // the building stays within it: 1,048,576 fluid particles in a tank 2454 -> 2382 us a step, 279,936 862 -> 840.
 // Eight lanes per particle: 4,096 particles at rest 159 -> 157 us, 8,000 violently jittered 985 -> 667.
 //
-// How far flags and marks reach ahead of half the skin in this round.
+// How far flags and marks reach ahead of half the skin in this prediction round.
 __device__ __forceinline__ float tight_margin(const DevParams& P, const Control* ctl, const ListBuffers& b) {
     return b.tight && ctl->tight_next != kTightOff ? P.tight_margin : 0.f;
 }
@@ -1931,11 +1931,11 @@ void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b
         constexpr int BS = decltype(bs)::value;
         constexpr bool S = decltype(shared)::value;
         const unsigned blocks = (n + BS - 1) / BS;
-        // 64 registers a thread (4 blocks of 256 per SM) against 48 (5 blocks), us per launch: 201,600 particles 42 / 47,
-        // 286,720 44 / 52, 400,000 62 / 69, 600,000 80 / 91, 1,048,576 135 / 140, 1.6M and 2.6M equal, 4.2M 516 / 508,
-        // 8.4M 1071 / 1050; below, 48 as long as they hold the scene in one wave (156,244: 33 / 29).
-        // Past 2M the walks in lane form, which need none of the spills of the inline form: 2.6M 321 -> 313 us, 8.4M
-        // 1050 -> 1036.
+        // 64 registers a thread (4 blocks of 256 per SM) against 48 (5 blocks), us per launch over the sweeps of a step (skin,
+        // building and tight): 200,704 particles 35.5 / 36.8, 287,496 37.5 / 42.4, 405,224 52.5 / 55.8, 592,704 67.0 / 70.9,
+        // 1,048,576 112.3 / 113.5, 2.6M equal; below, 48 as long as they hold the scene in one wave (156,244: 27.6 / 23.9).
+        // Past 2M the walks in lane form, which need none of the spills of the inline form (skin list, before the lists were
+        // read past L1: 8.4M 1050 -> 1036).
         // The building sweep with 64 registers, too, but where a wave of them just misses the scene: 156,244 particles 37
         // us with 48, 43 with 64; 32,768 29 and 21.
         if (S && n <= 8u * 128u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall, S><<<blocks, BS, 0, s>>>(ps, b);
