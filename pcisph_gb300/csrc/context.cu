@@ -783,7 +783,8 @@ struct pcisph_ctx {
                 }
                 launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, s);
                 uint32_t *sk = nullptr, *sv = nullptr;
-                int nl = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s, P.moving_lists ? b.state_vel : nullptr);
+                // no velocities: no moving lists. A caller may set the predictions between the stages, anywhere around x.
+                int nl = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s);
                 if (nl < 0) return PCISPH_ERR_CUDA;
                 sorted_keys = sk;
                 sorted_ids = sv;
@@ -800,11 +801,8 @@ struct pcisph_ctx {
             }
             case PCISPH_STAGE_DENSITY:
                 if (list_sweeps()) {
+                    if (P.moving_lists) CUDA_TRY(cudaMemsetAsync(&b.ctl->moving, 0, sizeof(b.ctl->moving), s));  // nor after a step's
                     launch_density_list(P, b.ctl, list_buffers(), s);
-                    if (P.moving_lists) {
-                        launch_moving_lists(P, b.ctl, list_buffers(), s);
-                        ++host_launches;
-                    }
                 } else if (warp_sweeps()) launch_density_sweep(P, b, sweep_args(), sweep_grid, s);
                 else launch_density(P, b, s);
                 ++host_launches;
@@ -823,7 +821,13 @@ struct pcisph_ctx {
                 break;
             case PCISPH_STAGE_BOUNDARY_PRESSURE: launch_boundary_pressure(P, b, working_order() ? cells_w : b.cells, s); ++host_launches; break;
             case PCISPH_STAGE_PRESSURE:
-                if (list_sweeps()) launch_pressure_list(P, b.ctl, list_buffers(), opts.sweep_block, false, s);
+                if (list_sweeps()) {
+                    if (P.moving_lists) {
+                        launch_distrust_moving_lists(P, b.ctl, list_buffers(), s);
+                        ++host_launches;
+                    }
+                    launch_pressure_list(P, b.ctl, list_buffers(), opts.sweep_block, false, s);
+                }
                 else if (warp_sweeps()) launch_pressure_sweep(P, b, sweep_args(), sweep_grid, s);
                 else launch_pressure(P, b, s);
                 ++host_launches;

@@ -675,6 +675,14 @@ __global__ void __launch_bounds__(kCellBlock, 5) k_moving_lists(DevParams P, Con
     }
 }
 
+// Flags every bucket if the lists of the step are moving lists (see launch_distrust_moving_lists).
+__global__ void __launch_bounds__(kBlock) k_distrust_moving_lists(DevParams P, Control* ctl, unsigned char* __restrict__ fast) {
+    if (!lists_move(P, ctl)) return;
+    const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
+    if (k < P.bucket_count) fast[k] = 1;
+    if (k == 0) ctl->lists_outrun = 1u;
+}
+
 // pcisph.cl:65-92, and the neighbour lists of the step (see the list builders above). kBoundary: the scene has boundary
 // particles (their walk is compiled out otherwise). A particle's density terms are staged in walk order and summed by
 // one lane in that order: the sum of the walk, whose other terms are zero.
@@ -1910,6 +1918,10 @@ constexpr uint32_t kLargeScene = 1u << 21;
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     const unsigned blocks = std::min(grid_cells(P.fluid_count, 8), 5u * 152u);
     if (P.fluid_count) k_moving_lists<<<blocks, kCellBlock, 0, s>>>(P, ctl, b);
+}
+
+void launch_distrust_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
+    k_distrust_moving_lists<<<grid_for(P.bucket_count), kBlock, 0, s>>>(P, ctl, b.bucket_fast);
 }
 
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {

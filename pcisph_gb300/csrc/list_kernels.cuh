@@ -109,6 +109,9 @@ void launch_boundary_zone(const DevParams& P, const float4* b_pos, const int* or
 void launch_boundary_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 // The skin lists of a step of moving lists (DevParams::moving_lists), after the density sweep; no work in other steps.
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
+// After a step of moving lists (no work after any other): every bucket is flagged, so that the next pressure sweep walks. For
+// predictions that a caller set, which need not lie near the places that the lists are built around.
+void launch_distrust_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 void launch_normal_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 void launch_force_list(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
 // Do the force and pressure-force sweeps of n particles mark by themselves (given b.walk_stamp; b.fast_list null)?

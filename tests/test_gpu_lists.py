@@ -201,3 +201,33 @@ def test_rebuilt_lists_change_no_bits(oracle, n, gap, jitter, speed, iters, opti
         assert got[1] == out[2][1]
         for k in got[0]:
             np.testing.assert_array_equal(got[0][k], out[2][0][k], err_msg=k)
+
+
+# Predictions that a caller sets between the stages lie where the caller puts them, here at x: lists around y = x + v dt, which
+# a step of fast particles builds, do not hold their pairs (neighbours of opposite velocities are 2 h apart there)
+@pytest.mark.parametrize("after", ["sort", "step", "step, density"])
+@pytest.mark.parametrize("n,order", [(4000, 0), (12000, 0), (12000, 1)])
+def test_set_predictions_find_every_pair(oracle, n, order, after):
+    rng = np.random.default_rng(n)
+    pos = _cloud(n, 8, seed=n) + np.float32(1.0)
+    vel = np.zeros_like(pos)
+    vel[:, 2] = rng.choice([-40.0, 40.0], n)
+    p = oracle.derive_params(0.5 * D, 1000.0, n, 0, 1e-3, 0.0, 0.0, 0.0)
+    f = fluid_like(p, min_iters=1, max_iters=1, spatial_order=order)
+    f.set_fluid_state(pos, vel)
+    if after == "sort":
+        f.run_stage("sort")
+    else:
+        f.update()
+    if after != "step":
+        f.run_stage("density")
+    x, cells = f.get_field("sorted_position"), f.get_field("cell_offsets")
+    f.set_field("predicted_position", x)
+    f.run_stage("pressure")
+    got = f.get_field("density_variation")
+    f.close()
+    rho = oracle.update_density(p, None, None, cells, x)
+    off = cells.astype(np.int64).reshape(-1, 2)
+    tol = max(RTOL, 2 * min(n, 27 * int((off[:, 1] - off[:, 0]).max())) * 2.0 ** -24)
+    assert rho.max() > 1000.0
+    assert_close("density_variation", got, np.maximum(rho - 1000.0, 0), scale=float(rho.max()), rtol=tol)
