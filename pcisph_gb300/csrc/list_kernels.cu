@@ -1354,7 +1354,8 @@ __device__ __forceinline__ float build_tight_list(const ListBuffers& b, const De
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
 // stage: its WalkStage.
 enum class Walks { kLane, kInline, kCall };  // each lane by itself; pressure_walkers inline; or as a function call
-template <class PS, bool kCoherent, Walks kWalks, bool kShared>
+// kTight: the launch may have tight lists
+template <class PS, bool kCoherent, Walks kWalks, bool kShared, bool kTight = true>
 __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, Stage<kShared>& stage) {
     float dv = 0.f, acc = 0.f;
     bool walk = false, build = false;
@@ -1364,7 +1365,7 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         const bool all_lists_ok = lists_hold<PS>(ctl);
         const float4 xi = b.pos[i];
         const float4 xp = b.pred[i];
-        const unsigned mode = tight_mode(P, ctl, b.tight != nullptr);
+        const unsigned mode = kTight ? tight_mode(P, ctl, b.tight != nullptr) : kTightOff;
         build = mode == kTightBuild;
         uint32_t cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
         bool tight = mode == kTightUse;
@@ -1429,7 +1430,11 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
             acc = build_tight_list<kCoherent, kShared>(b, P, i, xp, cnt, acc, walk, c, stage_tight(stage));
             walk = false;
         } else if (kWalks == Walks::kLane && walk) {
-            for_each_neighbour(b.cells, c, P, add);
+            if constexpr (PS::kBatched)  // two gathers in flight (see pressure_walkers)
+                for_each_neighbour_prefetched(
+                    b.cells, c, P, [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); },
+                    [&](uint32_t, const float4& o) { acc += density_term(xp.x, xp.y, xp.z, o, P.h2); });
+            else for_each_neighbour(b.cells, c, P, add);
             walk = false;
         } else if (!walk) {
             for_each_listed(tight ? b.tight : b.nbr, i, cnt, b.nbr_stride, add);
@@ -1716,14 +1721,17 @@ __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : DEEP == 1 ? 1536 / BS : 51
 // batch with its own convergence flags), grid barrier, pressure-force sweep, grid barrier; until no scene
 // iterates, at most max_iters times. Same sweeps and decisions as the graph's while loop, so the same bits.
 // Every thread takes every barrier: the bodies return to the loop, never out of the kernel.
+// The form of few registers throughout (48, a batch 64: 5 or 4 blocks per SM): what the graph's sweeps gain by walks served by
+// a whole warp and by tight lists costs this kernel, whose registers are the largest of its parts', more than half of its warps
+// (103 and 123 registers, 2 blocks: 1,000,000 particles at rest 2334 -> 2990 us a step, 16 scenes of 65,000 3119 -> 3610).
 template <class PS>
-__global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b, Control* loop, int max_iters) {
+__global__ void __launch_bounds__(kBlock, PS::kBatched ? 4 : 5) k_corrective_loop(PS ps, ListBuffers b, Control* loop, int max_iters) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
     const uint32_t stride = gridDim.x * kBlock;
     const uint32_t rounds = (ps.count() + stride - 1) / stride;
     __shared__ int running;
-    __shared__ WalkStage stage[kBlock / 32];
+    __shared__ WalkStage unused;
     for (int it = 0; it < max_iters; ++it) {
         if constexpr (!PS::kBatched) {  // boundary pressures at the predicted positions (read by the force)
             const DevParams& P = ps.params(0);
@@ -1733,8 +1741,8 @@ __global__ void __launch_bounds__(kBlock) k_corrective_loop(PS ps, ListBuffers b
         unsigned local = 0;
         for (uint32_t r = 0; r < rounds; ++r)
             local = max(local, __float_as_uint(
-                                   pressure_body<PS, true, Walks::kCall, false>(ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x,
-                                                           stage[threadIdx.x >> 5])));
+                                   pressure_body<PS, true, Walks::kLane, false, false>(
+                                       ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x, unused)));
         if (!PS::kBatched) {  // batched scenes reduced per scene inside the body
             const unsigned m = __reduce_max_sync(0xffffffffu, local);
             if ((threadIdx.x & 31) == 0 && m) atomicMax(&ps.control(0)->max_err_bits, m);
