@@ -1206,12 +1206,12 @@ __device__ __forceinline__ float finish_pressure(const ListBuffers& b, const Dev
     return dv;
 }
 
-// The particles of a warp that walk, after their boundary terms (acc). A walk by one lane takes the warp ~400 steps of one
-// gather each, whatever its other lanes do; few walkers are therefore served one after another by all 32 lanes (27 bucket
-// ranges at once, 32 candidates a round, ~9 rounds), and their terms summed in walk order by their own lane. Each costs
-// ~500 instructions, a lane's share of a full warp's walk ~300: from kFewWalkers on each lane walks by itself.
+// The few particles of a warp that walk, after their boundary terms (acc). A walk by one lane takes the warp ~400 steps of one
+// gather each, whatever its other lanes do; up to kFewWalkers are therefore served one after another by all 32 lanes (27
+// bucket ranges at once, 32 candidates a round, ~9 rounds), and their terms summed in walk order by their own lane. Each costs
+// ~500 instructions, a lane's share of a full warp's walk ~300: with more, each lane walks by itself (pressure_body).
 // Pressure sweep with few hundred to few thousand fast predictions: 1M jittered block 158 -> 146 us, a 98,904-particle drop
-// at 2.4 m/s 43 -> 31; from 6 to 32 the split makes no difference there. U: rounds with their gathers in flight.
+// at 2.4 m/s 43 -> 31; from 6 to 32 the split makes no difference there.
 constexpr int kFewWalkers = 12;
 struct WalkStage {
     uint32_t delta[32];
@@ -1228,9 +1228,10 @@ __device__ __forceinline__ uint32_t* stage_tight(WalkStage&) { return nullptr; }
 __device__ __forceinline__ uint32_t* stage_tight(BuildStage& s) { return s.tight; }
 __device__ __forceinline__ WalkStage& stage_walk(WalkStage& s) { return s; }
 __device__ __forceinline__ WalkStage& stage_walk(BuildStage& s) { return s.walk; }
-template <class PS, bool kCoherent, int U, bool kShared>
+template <class PS, bool kCoherent, bool kShared>
 __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
                                                uint32_t walkers, bool build, Stage<kShared>& stage) {
+    constexpr int U = 2;  // rounds with their gathers in flight
     WalkStage& S = stage_walk(stage);
     const uint32_t lane = threadIdx.x & 31u;
     const bool mine = (walkers >> lane) & 1u;
@@ -1240,93 +1241,63 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
     const float4 xi = b.pos[ii];
     const float4 xp = b.pred[ii];
     const Cell c = cell_of(xi.x, xi.y, xi.z, P);
-    if (__popc(walkers) > kFewWalkers) {
-        if (mine) {
-            auto load = [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); };
-            TightWriter<kShared> w(b.tight, ii, b.nbr_stride, stage_tight(stage));
-            auto use = [&](uint32_t j, const float4& o) {
-                const float d2 = dist2(xp.x - o.x, xp.y - o.y, xp.z - o.z);
-                acc += poly6(d2, P.h2);
-                if (build && !(d2 > P.tight_r2)) {
-                    w.add(j);
-                    if ((w.n & 7u) == 0u) w.flush((w.n >> 3) - 1u);
+    const uint32_t below = lanes_below();
+    for (uint32_t todo = walkers; todo; todo &= todo - 1u) {
+        const int t = __ffs(todo) - 1;
+        const DevParams& Q = ps.params(__shfl_sync(kAll, ii, t));
+        const float x = __shfl_sync(kAll, xp.x, t), y = __shfl_sync(kAll, xp.y, t), z = __shfl_sync(kAll, xp.z, t);
+        CellWalk w = begin_cell(b.cells, Q, __shfl_sync(kAll, c.x, t), __shfl_sync(kAll, c.y, t),
+                                __shfl_sync(kAll, c.z, t), lane, S.delta);
+        const uint32_t it = __shfl_sync(kAll, ii, t);
+        const bool keep = __shfl_sync(kAll, (int)build, t) != 0;
+        uint32_t n = 0, kept = 0;
+        auto sum = [&] {  // the staged terms, by the walker's own lane
+            __syncwarp();
+            if ((int)lane == t)
+                for (uint32_t k = 0; k < n; ++k) acc += S.term[k];
+            n = 0;
+            __syncwarp();
+        };
+        for (uint32_t base = 0; base < w.total; base += 32u * U) {
+            float4 o[U];
+            uint32_t js[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                js[u] = next_candidate(w, base + u * 32u, lane, S.delta);
+                if (js[u] != kAll) o[u] = load_slot<kCoherent>(&b.pred[js[u]]);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                float term = 0.f;
+                bool tight = false;
+                if (base + u * 32u + lane < w.total) {
+                    const float d2 = dist2(x - o[u].x, y - o[u].y, z - o[u].z);
+                    term = poly6(d2, Q.h2);
+                    tight = keep && !(d2 > Q.tight_r2);
                 }
-            };
-            // a batch walks with two gathers in flight (terms still added in walk order): its walkers are latency-bound
-            // (256 batched scenes, 9.8M particles, over 500 steps: 26.8 -> 25.8 s); one scene walks plainly (8M
-            // particles all walking: 3.0 ms per sweep, 3.6 with the prefetch)
-            if constexpr (PS::kBatched) for_each_neighbour_prefetched(b.cells, c, P, load, use);
-            else for_each_neighbour(b.cells, c, P, [&](uint32_t j) { use(j, load(j)); });
-            if (build) {
-                w.finish();
-                b.tight_count[ii] = w.n;
+                const uint32_t set = __ballot_sync(kAll, tight);
+                if (tight) {
+                    const uint32_t e = kept + __popc(set & below);
+                    if (e < kTightCap) reinterpret_cast<uint32_t*>(list_chunk(b.tight, it, e >> 3, b.nbr_stride))[e & 7u] = js[u];
+                }
+                kept += __popc(set);
+                const uint32_t bits = __ballot_sync(kAll, term != 0.f);  // NaN counts
+                if (n + __popc(bits) > 96u) sum();
+                if (term != 0.f) S.term[n + __popc(bits & below)] = term;
+                n += __popc(bits);
             }
         }
-    } else {
-        const uint32_t below = lanes_below();
-        for (uint32_t todo = walkers; todo; todo &= todo - 1u) {
-            const int t = __ffs(todo) - 1;
-            const DevParams& Q = ps.params(__shfl_sync(kAll, ii, t));
-            const float x = __shfl_sync(kAll, xp.x, t), y = __shfl_sync(kAll, xp.y, t), z = __shfl_sync(kAll, xp.z, t);
-            CellWalk w = begin_cell(b.cells, Q, __shfl_sync(kAll, c.x, t), __shfl_sync(kAll, c.y, t),
-                                    __shfl_sync(kAll, c.z, t), lane, S.delta);
-            const uint32_t it = __shfl_sync(kAll, ii, t);
-            const bool keep = __shfl_sync(kAll, (int)build, t) != 0;
-            uint32_t n = 0, kept = 0;
-            auto sum = [&] {  // the staged terms, by the walker's own lane
-                __syncwarp();
-                if ((int)lane == t)
-                    for (uint32_t k = 0; k < n; ++k) acc += S.term[k];
-                n = 0;
-                __syncwarp();
-            };
-            for (uint32_t base = 0; base < w.total; base += 32u * U) {
-                float4 o[U];
-                uint32_t js[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    js[u] = next_candidate(w, base + u * 32u, lane, S.delta);
-                    if (js[u] != kAll) o[u] = load_slot<kCoherent>(&b.pred[js[u]]);
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    float term = 0.f;
-                    bool tight = false;
-                    if (base + u * 32u + lane < w.total) {
-                        const float d2 = dist2(x - o[u].x, y - o[u].y, z - o[u].z);
-                        term = poly6(d2, Q.h2);
-                        tight = keep && !(d2 > Q.tight_r2);
-                    }
-                    const uint32_t set = __ballot_sync(kAll, tight);
-                    if (tight) {
-                        const uint32_t e = kept + __popc(set & below);
-                        if (e < kTightCap) reinterpret_cast<uint32_t*>(list_chunk(b.tight, it, e >> 3, b.nbr_stride))[e & 7u] = js[u];
-                    }
-                    kept += __popc(set);
-                    const uint32_t bits = __ballot_sync(kAll, term != 0.f);  // NaN counts
-                    if (n + __popc(bits) > 96u) sum();
-                    if (term != 0.f) S.term[n + __popc(bits & below)] = term;
-                    n += __popc(bits);
-                }
-            }
-            sum();
-            if (keep && (int)lane == t) b.tight_count[it] = kept;
-        }
+        sum();
+        if (keep && (int)lane == t) b.tight_count[it] = kept;
     }
     return mine ? finish_pressure<PS>(b, P, ps.control(ii), ii, xi, acc) : 0.f;
-}
-
-template <class PS, bool kCoherent, bool kShared>
-__device__ __noinline__ float call_pressure_walkers(const PS& ps, const ListBuffers& b, uint32_t i, float acc,
-                                                    uint32_t walkers, bool build, Stage<kShared>& S) {
-    return pressure_walkers<PS, kCoherent, 3, kShared>(ps, b, i, acc, walkers, build, S);
 }
 
 // A particle's fluid terms added to acc by its own lane, from its skin list (cnt entries) or a walk, building its tight
 // list. (A chunk's distances before its entries are kept: 218 -> 186 us at 1M, the gathers in flight together.)
 template <bool kCoherent, bool kShared>
-__device__ __forceinline__ float build_tight_list(const ListBuffers& b, const DevParams& P, uint32_t i, const float4& xp,
-                                                  uint32_t cnt, float acc, bool walk, const Cell& c, uint32_t* stage) {
+__device__ __forceinline__ float build_tight_list(const ListBuffers& b, const DevParams& P, uint32_t i, const float4& xi,
+                                                  const float4& xp, uint32_t cnt, float acc, bool walk, uint32_t* stage) {
     TightWriter<kShared> w(b.tight, i, b.nbr_stride, stage);
     uint32_t written = 0;  // entries at the last look
     auto away2 = [&](uint32_t j) {
@@ -1342,7 +1313,7 @@ __device__ __forceinline__ float build_tight_list(const ListBuffers& b, const De
         written = w.n;
     };
     if (walk)
-        for_each_neighbour(b.cells, c, P, [&](uint32_t j) {
+        for_each_neighbour(b.cells, cell_of(xi.x, xi.y, xi.z, P), P, [&](uint32_t j) {
             keep(j, away2(j));
             flush();
         });
@@ -1352,23 +1323,32 @@ __device__ __forceinline__ float build_tight_list(const ListBuffers& b, const De
     return acc;
 }
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
-// stage: its WalkStage.
-enum class Walks { kLane, kInline, kCall };  // each lane by itself; pressure_walkers inline; or as a function call
-// kTight: the launch may have tight lists
-template <class PS, bool kCoherent, Walks kWalks, bool kShared, bool kTight = true>
+// stage: its WalkStage. The decisions are plan_pressure's (a struct returned to this form slowed it: 286,720 particles with
+// boundary 42.5 -> 48.7 us), and kTightSkin's for a batch.
+//
+// Where more than kFewWalkers lanes of a warp walk, each does so by itself, here and not in pressure_walkers: with that walk
+// there, as a function whose parameters lie in memory or inlined at 48 registers, a sweep in which most particles walk took
+// 1.2 to 2.2 times as long. us a step with most predictions fast, without walks by warps / so / now: 110,592 particles 677 /
+// 811 / 636, 1,000,000 3620 / 5270 / 3990, 16 batched scenes of 65,000 9690 / 12780 / 10670.
+//
+// kFew: few walkers of a warp go to pressure_walkers (or each walks by itself, too). kTight: the launch may have tight lists.
+template <class PS, bool kCoherent, bool kFew, bool kShared, bool kTight = true>
 __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& b, uint32_t i, Stage<kShared>& stage) {
     float dv = 0.f, acc = 0.f;
-    bool walk = false, build = false;
-    if (i < ps.count() && !ps.skip_pressure(i)) {
-        const DevParams& P = ps.params(i);
-        Control* ctl = ps.control(i);
+    bool walk = false, build = false, tight = false;
+    uint32_t cnt = 0;
+    float4 xi{}, xp{};
+    const bool live = i < ps.count() && !ps.skip_pressure(i);
+    const DevParams& P = ps.params(live ? i : 0u);
+    Control* ctl = ps.control(live ? i : 0u);
+    if (live) {
         const bool all_lists_ok = lists_hold<PS>(ctl);
-        const float4 xi = b.pos[i];
-        const float4 xp = b.pred[i];
+        xi = b.pos[i];
+        xp = b.pred[i];
         const unsigned mode = kTight ? tight_mode(P, ctl, b.tight != nullptr) : kTightOff;
         build = mode == kTightBuild;
-        uint32_t cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
-        bool tight = mode == kTightUse;
+        cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
+        tight = mode == kTightUse;
         if (PS::kBatched && tight && cnt == kTightSkin) {
             cnt = b.nbr_count[i];
             tight = false;
@@ -1405,20 +1385,17 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         const bool marks = fast_round <= P.mark_cap;
         if (mode == kTightUse) {
             walk = overflow;
-            if (walk || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
+            if (walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
         } else if (marks) {
             walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
-            if (walk || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
+            if (walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
         } else {
-            if (own_walk || !all_lists_ok || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
+            if (!all_lists_ok || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
             walk = own_walk || (!all_lists_ok && near_fast(P, b.bucket_fast, c));
         }
         auto fb = [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, __ldg(&b.b_pos[j]), P.h2); };
         if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
         else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
-        auto add = [&](uint32_t j) {
-            acc += density_term(xp.x, xp.y, xp.z, load_slot<kCoherent>(&b.pred[j]), P.h2);
-        };
         if (build) {
             b.tight_ref[i] = xp;
             if (PS::kBatched && cnt > b.tight_below) {
@@ -1426,29 +1403,40 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
                 build = false;
             }
         }
-        if (build && (kWalks == Walks::kLane || !walk)) {
-            acc = build_tight_list<kCoherent, kShared>(b, P, i, xp, cnt, acc, walk, c, stage_tight(stage));
-            walk = false;
-        } else if (kWalks == Walks::kLane && walk) {
-            if constexpr (PS::kBatched)  // two gathers in flight (see pressure_walkers)
-                for_each_neighbour_prefetched(
-                    b.cells, c, P, [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); },
-                    [&](uint32_t, const float4& o) { acc += density_term(xp.x, xp.y, xp.z, o, P.h2); });
-            else for_each_neighbour(b.cells, c, P, add);
-            walk = false;
-        } else if (!walk) {
-            for_each_listed(tight ? b.tight : b.nbr, i, cnt, b.nbr_stride, add);
-        }
-        if (!walk) dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
     }
-    if constexpr (kWalks == Walks::kLane) return dv;
-    const uint32_t walkers = __ballot_sync(kAll, walk);
-    if (walkers) {
-        __syncwarp();  // the stage changes hands
-        float w;
-        if constexpr (kWalks == Walks::kCall) w = call_pressure_walkers<PS, kCoherent, kShared>(ps, b, i, acc, walkers, build, stage);
-        else w = pressure_walkers<PS, kCoherent, 2, kShared>(ps, b, i, acc, walkers, build, stage);
-        if (walk) dv = w;
+    const auto load = [&](uint32_t j) { return load_slot<kCoherent>(&b.pred[j]); };
+    const auto by_lane = [&] {  // this lane's walk
+        if (build) {
+            acc = build_tight_list<kCoherent, kShared>(b, P, i, xi, xp, cnt, acc, true, stage_tight(stage));
+        } else {
+            const Cell c = cell_of(xi.x, xi.y, xi.z, P);
+            auto use = [&](uint32_t, const float4& o) { acc += density_term(xp.x, xp.y, xp.z, o, P.h2); };
+            // a batch walks with two gathers in flight (terms still added in walk order): its walkers are latency-bound
+            // (256 batched scenes, 9.8M particles, over 500 steps: 26.8 -> 25.8 s); one scene walks plainly (8M
+            // particles all walking: 3.0 ms per sweep, 3.6 with the prefetch)
+            if constexpr (PS::kBatched) for_each_neighbour_prefetched(b.cells, c, P, load, use);
+            else for_each_neighbour(b.cells, c, P, [&](uint32_t j) { use(j, load(j)); });
+        }
+        dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
+    };
+    if (live && !walk) {
+        if (build) acc = build_tight_list<kCoherent, kShared>(b, P, i, xi, xp, cnt, acc, false, stage_tight(stage));
+        else
+            for_each_listed(tight ? b.tight : b.nbr, i, cnt, b.nbr_stride,
+                            [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, load(j), P.h2); });
+        dv = finish_pressure<PS>(b, P, ctl, i, xi, acc);
+    } else if (!kFew && walk) {
+        by_lane();
+    }
+    if constexpr (kFew) {
+        const uint32_t walkers = __ballot_sync(kAll, walk);
+        if (__popc(walkers) > kFewWalkers) {
+            if (walk) by_lane();
+        } else if (walkers) {
+            __syncwarp();  // the stage changes hands
+            const float w = pressure_walkers<PS, kCoherent, kShared>(ps, b, i, acc, walkers, build, stage);
+            if (walk) dv = w;
+        }
     }
     return dv;
 }
@@ -1520,14 +1508,13 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
 }
 
 // BS: threads per block (128, 256 or 512; the autotuner's choice for one scene)
-// Walks::kCall: 32 warps per SM at 64 registers instead of 40 at 48, with more gathers in flight each (see
-// launch_pressure_list)
-template <class PS, int BS = kBlock, int LANES = 1, Walks kWalks = Walks::kCall, bool kShared = false>
-__global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kWalks == Walks::kCall ? 1024 / BS : 1280 / BS) k_pressure_list(PS ps, ListBuffers b) {
+// kThreads: resident threads per SM, 1024 at 64 registers or 1280 at 48 (see launch_pressure_list)
+template <class PS, int BS = kBlock, int LANES = 1, bool kFew = true, bool kShared = false, int kThreads = 1024>
+__global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kThreads / BS) k_pressure_list(PS ps, ListBuffers b) {
     const uint32_t t = blockIdx.x * BS + threadIdx.x;
     float dv;
     __shared__ Stage<kShared> stage[LANES == 1 ? BS / 32 : 1];
-    if constexpr (LANES == 1) dv = pressure_body<PS, false, kWalks, kShared>(ps, b, t, stage[threadIdx.x >> 5]);
+    if constexpr (LANES == 1) dv = pressure_body<PS, false, kFew, kShared>(ps, b, t, stage[threadIdx.x >> 5]);
     else dv = pressure_shared<PS, LANES>(ps, b, t / LANES, t % LANES);
     if (PS::kBatched) return;
     // one scene: block max of dv, the last block decides (dv >= 0: bit patterns order like values)
@@ -1741,7 +1728,7 @@ __global__ void __launch_bounds__(kBlock, PS::kBatched ? 4 : 5) k_corrective_loo
         unsigned local = 0;
         for (uint32_t r = 0; r < rounds; ++r)
             local = max(local, __float_as_uint(
-                                   pressure_body<PS, true, Walks::kLane, false, false>(
+                                   pressure_body<PS, true, false, false, false>(
                                        ps, b, r * stride + blockIdx.x * kBlock + threadIdx.x, unused)));
         if (!PS::kBatched) {  // batched scenes reduced per scene inside the body
             const unsigned m = __reduce_max_sync(0xffffffffu, local);
@@ -1922,6 +1909,7 @@ constexpr uint32_t kDeepMax = 49152u;   // two chunks in flight, pressure force 
 // Past 2M particles the default block of the corrective sweeps is 128 threads instead of 256 (8.4M: pressure force 614 -> 588
 // us, pressure 663 -> 658; equal at 1M).
 constexpr uint32_t kLargeScene = 1u << 21;
+constexpr uint32_t kSms = 152u;  // of a GB300; launch shapes that fill it (results do not depend on them)
 
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
     const unsigned blocks = std::min(grid_cells(P.fluid_count, 8), 5u * 152u);
@@ -1958,10 +1946,9 @@ void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b
         // read past L1: 8.4M 1050 -> 1036).
         // The building sweep with 64 registers, too, but where a wave of them just misses the scene: 156,244 particles 37
         // us with 48, 43 with 64; 32,768 29 and 21.
-        if (S && n <= 8u * 128u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall, S><<<blocks, BS, 0, s>>>(ps, b);
-        else if (n > kLargeScene) k_pressure_list<OneScene, BS, 1, Walks::kLane, S><<<blocks, BS, 0, s>>>(ps, b);
-        else if (n > 5u * 256u * 152u) k_pressure_list<OneScene, BS, 1, Walks::kCall, S><<<blocks, BS, 0, s>>>(ps, b);
-        else k_pressure_list<OneScene, BS, 1, Walks::kInline, S><<<blocks, BS, 0, s>>>(ps, b);
+        if (n > kLargeScene) k_pressure_list<OneScene, BS, 1, false, S, 1280><<<blocks, BS, 0, s>>>(ps, b);
+        else if (n > 1024u * kSms && n <= 1280u * kSms) k_pressure_list<OneScene, BS, 1, true, S, 1280><<<blocks, BS, 0, s>>>(ps, b);
+        else k_pressure_list<OneScene, BS, 1, true, S><<<blocks, BS, 0, s>>>(ps, b);
     };
     if (n <= kSharedMax) k_pressure_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b);
     else if (builds && b.tight) go(std::integral_constant<int, 128>{}, std::true_type{});
@@ -2057,7 +2044,7 @@ void launch_force_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t
 void launch_pressure_scenes(const SceneTable& t, const ListBuffers& b, bool builds, cudaStream_t s) {
     if (!t.n) return;
     if (builds && b.tight)
-        k_pressure_list<SceneTable, 128, 1, Walks::kCall, true><<<(t.n + 127) / 128, 128, 0, s>>>(t, b);
+        k_pressure_list<SceneTable, 128, 1, true, true><<<(t.n + 127) / 128, 128, 0, s>>>(t, b);
     else k_pressure_list<<<grid_for(t.n), kBlock, 0, s>>>(t, b);
 }
 void launch_pressure_force_scenes(const SceneTable& t, const ListBuffers& b, cudaStream_t s) {
