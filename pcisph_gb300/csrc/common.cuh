@@ -46,9 +46,8 @@ struct DevParams {
     // 1 in kMovingShare particles that move kMovingSpeed of half the skin or more per step, the skin lists are built around y = x + v dt
     // (moving_place) and a prediction is measured from there: a body that moves as a whole keeps its lists
     int moving_lists;
-    // tight lists (the list sweeps without per-particle skins; see the list sweeps): the distance that a prediction may
-    // move from where the tight lists were built (0: none are built), the same less a margin for rounding, and the
-    // lists' radius^2, (h + 2 tight_margin)^2
+    // tight lists (see the list sweeps): the distance that a prediction may move from where they were built (0: none are),
+    // the same less a margin for rounding, and their radius^2, (h + 2 tight_margin)^2
     float tight_margin, tight_reach, tight_r2;
     // batched scenes with an adaptive skin: each step picks one of kSkinLevels skins from the previous
     // step's count of predictions past each level's half skin (skin_half[k])
@@ -89,12 +88,22 @@ struct Control {
     unsigned long long fast_n;
     unsigned int round;
     unsigned int moving;         // moving lists: the particles that fast (kMovingSpeed) when the step began
-    // tight lists: how the next pressure sweep finds its neighbours (kTightOff, kTightBuild or kTightUse), whether a
-    // prediction left their reach since they were built, the sweeps that used them, and how long the next sweeps do
-    // without after a building that served none
-    unsigned int tight_next, tight_stray, tight_age, tight_wait, tight_backoff;
-    unsigned int lists_outrun;   // one scene: some prediction of this step was fast (1), measured from the place that
-                                 // the step's lists are built around; it flagged its bucket
+    // Every particle's pressure sweep reads these four, as one vector (list_state). Tight lists: how the next sweep finds its
+    // neighbours (kTightOff, kTightBuild or kTightUse), whether a prediction left their reach since they were built
+    alignas(16) unsigned int tight_next;
+    unsigned int tight_stray;
+    unsigned int lists_outrun;   // some prediction of this step was fast (1), measured from the place that the step's
+                                 // lists are built around; it flagged its bucket
+    unsigned int tight_outrun;   // some prediction since the tight lists were built was fast and was not so there (nor, if
+                                 // flags were taken then, was its bucket flagged)
+    // the sweeps that used the tight lists, and how long the next sweeps (of later steps, too) do without after a building
+    // that served none
+    unsigned int tight_age, tight_wait, tight_backoff;
+    // moving lists: the particles that a step of such lists left half a skin away from its y, and the steps that do without
+    // after one that left many there
+    unsigned int strays, moving_wait, moving_backoff;
+    unsigned long long fast_before;  // fast_particles without those of the current round
+    unsigned int tight_marked;   // the tight lists were built by a sweep that took marks, not flags
 };
 
 // Close a step after its last corrective iteration `it` (Fluid.cpp:301-306 decides the same way): status
@@ -114,12 +123,17 @@ __device__ __forceinline__ void close_step(Control* ctl, unsigned it, float rel,
 }
 
 constexpr uint32_t kTightCap = 64;      // tight list entries per particle (a multiple of 8)
-constexpr uint32_t kTightSkin = 0xffffffffu;
+// Beside the number of entries: built by a walk, or (for the number itself) the skin list is read instead.
+constexpr uint32_t kTightWalked = 0x80000000u, kTightSkin = 0x7fffffffu;
 constexpr float kTightMargin = 0.035f;  // of h
 constexpr int kTightFrom = 4;           // iterations of the previous step (if there was one) from which a step builds them
 constexpr unsigned kTightAgain = 6;     // tight lists that were left behind are rebuilt from this iteration on
+// Tight lists are built in a round in which at most 1 in kTightShare predictions outran the lists: of more, some leave the
+// tight lists, too, before these have paid for a building sweep in which as many walk.
+constexpr unsigned kTightShare = 16;
 constexpr unsigned kTightOff = 0, kTightBuild = 1, kTightUse = 2;
 constexpr uint32_t kNearCap = 64;  // within-h list entries per particle
+constexpr uint32_t kSharedMax = 8192u;  // a scene of at most so many particles: eight lanes a particle in the list sweeps
 
 // Moving lists (DevParams::moving_lists): the share of fast particles from which a step takes them. The two list radii then
 // test different places, which costs the list builder half again its time; a pressure sweep whose particles walk the

@@ -389,7 +389,8 @@ struct pcisph_ctx {
         P.particle_skin = skins && list_sweeps() ? 1 : 0;
         P.skin_factor = kSkinFactor;
         P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
-        set_tight_lists(&P, list_sweeps() && P.h + P.skin_max_half + kTightMargin * P.h <= 1.9f * P.cell_size);
+        // (marks reach up to 2 kTightMargin h further where tight lists are built, see below)
+        set_tight_lists(&P, list_sweeps() && P.h + P.skin_max_half + 2.f * kTightMargin * P.h <= 1.9f * P.cell_size);
         P.skin_min_half = std::min(kSkinMinHalf * P.h + P.tight_margin, P.skin_max_half);
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
@@ -516,7 +517,7 @@ struct pcisph_ctx {
     int record_prefix(cudaStream_t s) {
         const uint32_t N = params.fluid_count, B = params.boundary_count;
         int nl = 0;
-        launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, s);
+        launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, N, s);
         ++nl;
         uint32_t *sk = nullptr, *sv = nullptr;
         int r = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s, P.moving_lists ? b.state_vel : nullptr);
@@ -781,7 +782,7 @@ struct pcisph_ctx {
                     rc = boundary_sort(s);
                     if (rc) return rc;
                 }
-                launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, s);
+                launch_begin(b.ctl, b.cells, list_sweeps() ? b.bucket_fast : nullptr, params.bucket_count, N, s);
                 uint32_t *sk = nullptr, *sv = nullptr;
                 // no velocities: no moving lists. A caller may set the predictions between the stages, anywhere around x.
                 int nl = sort_set(b.state_pos, N, f_keys, f_ids, &sk, &sv, s);

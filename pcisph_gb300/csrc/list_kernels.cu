@@ -22,7 +22,7 @@
 //   - in a step of moving lists (lists_move: many particles faster than half the skin per step) the skin lists are
 //     built around y = x + v dt instead of x, and a prediction is fast when it strays half the skin from there;
 //   - from the third pressure sweep of a step on, the sweeps read tight lists rebuilt at the second one's
-//     predictions, as long as no prediction has moved past their margin from there (see tight_mode);
+//     predictions, as long as no prediction has moved past their margin from there (see the tight lists);
 //   - a particle with more than list_cap (near_cap) candidates is marked (count > cap) and walks the
 //     buckets in the sweeps that would use that list.
 // Boundary particles (B > 0, single scene) are summed by walking the boundary buckets. The density sweep
@@ -291,14 +291,16 @@ constexpr uint32_t kAll = 0xffffffffu;
 // The first correction moves a prediction most (0.05 h and more), the later ones little: from the second prediction x*_2 on
 // no particle of a collapsing column, a tank or a falling drop moves 0.035 h within a step of 7 iterations, and within one
 // of 50 they pass that a few times. So the second pressure sweep of a step also writes, per particle and in walk order, the
-// entries within h + 2 m of it (m = tight_margin; 40 of the skin list's 65 at rest density), and the later sweeps read
+// entries within h + 2 m of it (m = kTightMargin h; 40 of the skin list's 65 at rest density), and the later sweeps read
 // those: 1,048,576 particles 126 us a sweep -> 82, 8,388,608 957 -> 544, 98,904 falling 21 -> 11; the building sweep costs
 // 186, 1420 and 26. A step of 50 iterations of 8.4M particles 83.2 -> 68.2 ms, one of 6 at 1M 2060 -> 1990 us.
 //
 // Exact: a pair within h at later predictions, neither of which has moved more than m since, was within h + 2 m at the
-// building. A building sweep finds all such pairs: a prediction is flagged already past half the skin less m (in rounds
-// that a building sweep may follow, marks reach h + 2 m), so that a particle that is not flagged then stays within half the
-// skin, and its later partners are in the skin list; and the partners of one that is flagged walk. A particle with
+// building. So the tight list of a particle that walked then holds every pair of its walk that comes within h; and that of
+// one that read its skin list holds every such pair of the skin list, which is all of them unless the particle has to
+// walk by the rules of the skin lists (fast predictions' flags or marks). It does walk where these say so, and did not in the
+// building sweep. A fast prediction that was fast at the building, too, asks nobody again: there its partners within h + 2 m
+// were marked (or all near its bucket flagged), and walked. A particle with
 // more than kTightCap entries walks in every sweep that would read them. One prediction out of reach (or NaN) puts the whole
 // scene back on the skin lists, and from iteration kTightAgain on rebuilds: a building sweep in the loop (it stores entry by
 // entry, 1670 us at 8.4M) pays from three sweeps that use it, which a loop of fewer iterations need not have left.
@@ -309,44 +311,72 @@ constexpr uint32_t kAll = 0xffffffffu;
 // took 4 or more. Batch of 32 scenes, 1.32M particles: 46.4 -> 44.6 ms for 16 steps (46.3 without that rule: its falling
 // spheres walk in the building sweep, 456 us, for loops of 3).
 //
-// Per-particle skins (scenes with boundary particles): each skin is m wider, so that a particle within its skin less m at
-// the building stays within it: 1,048,576 fluid particles in a tank 2454 -> 2382 us a step, 279,936 862 -> 840.
-// Eight lanes per particle: 4,096 particles at rest 159 -> 157 us, 8,000 violently jittered 985 -> 667.
+// With per-particle skins (scenes with boundary particles) 1,048,576 fluid particles in a tank 2454 -> 2382 us a step, 279,936
+// 862 -> 840. Eight lanes per particle: 4,096 particles at rest 159 -> 157 us, 8,000 violently jittered 985 -> 667.
 //
-// How far flags and marks reach ahead of half the skin in this prediction round.
-__device__ __forceinline__ float tight_margin(const DevParams& P, const Control* ctl, const ListBuffers& b) {
-    return b.tight && ctl->tight_next != kTightOff ? P.tight_margin : 0.f;
+// Skin lists narrower than this hold too few of the later pairs: the building sweep walks throughout, and every tight list is
+// complete. (list_skin 0.05, 4,096 particles 350 -> 183 us a step; from 0.07 on the lists are read, 182 -> 139.)
+__device__ __forceinline__ bool tight_by_walks(const DevParams& P) { return P.skin_max_half < 1.05f * P.tight_margin; }
+// The control fields that decide over the tight lists, loaded together: one thread decides at the end of a sweep, and small
+// scenes wait for it.
+struct TightState {
+    unsigned next, stray, age, wait, backoff, iter;
+    int last;
+    bool moves;
+    unsigned long long fast, before;
+    __device__ __forceinline__ TightState(const DevParams& P, const Control* c)
+        : next(c->tight_next), stray(c->tight_stray), age(c->tight_age), wait(c->tight_wait), backoff(c->tight_backoff),
+          iter(c->iter), last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before) {}
+    __device__ __forceinline__ unsigned mode(const DevParams& P) const {
+        if (next == kTightOff || (next == kTightUse && stray == 0u)) return next;
+        const bool again = age != 0u && iter >= kTightAgain && (int)iter + 1 < P.max_iters;
+        // many fast predictions of a scene that moving lists do not serve go apart (kTightShare); elsewhere they may go together
+        const bool few = !P.moving_lists || moves || tight_by_walks(P) || P.fluid_count <= kSharedMax ||
+                         fast - before <= P.fluid_count / kTightShare;
+        return (next == kTightBuild || again) && few ? kTightBuild : kTightOff;
+    }
+};
+// How this pressure sweep finds its neighbours (constant while it runs), and whether some prediction outran the lists that it
+// reads.
+struct ListState {
+    unsigned mode;
+    bool outrun;
+};
+template <bool kTight>
+__device__ __forceinline__ ListState list_state(const DevParams& P, const Control* ctl, bool on) {
+    const uint4 s = *reinterpret_cast<const uint4*>(&ctl->tight_next);  // next, stray, outrun, outrun since the building
+    if (!kTight || !on) return ListState{kTightOff, s.z != 0u};
+    unsigned mode = s.x;
+    if (mode == kTightBuild || (mode == kTightUse && s.y != 0u)) mode = TightState(P, ctl).mode(P);
+    return ListState{mode, (mode == kTightUse ? s.w : s.z) != 0u};
 }
-// How this pressure sweep finds its neighbours: constant while it runs.
-__device__ __forceinline__ unsigned tight_mode(const DevParams& P, const Control* ctl, bool on) {
+// After a pressure sweep (before the decision): what the next one does (returned, too). marks: the sweep took marks, not flags.
+__device__ __forceinline__ unsigned tight_advance(const DevParams& P, Control* ctl, bool on, bool marks) {
     if (!on) return kTightOff;
-    const unsigned m = ctl->tight_next;
-    if (m != kTightUse || ctl->tight_stray == 0u) return m;
-    return ctl->tight_age != 0u && ctl->iter >= kTightAgain && (int)ctl->iter + 1 < P.max_iters ? kTightBuild : kTightOff;
-}
-// After a pressure sweep (before the decision): what the next one does.
-__device__ __forceinline__ void tight_advance(const DevParams& P, Control* ctl, bool on) {
-    if (!on) return;
-    const unsigned m = tight_mode(P, ctl, on);
+    const TightState t(P, ctl);
+    const unsigned m = t.mode(P);
+    unsigned next = t.next;
     if (m == kTightUse) {
-        ctl->tight_age += 1;
+        ctl->tight_age = t.age + 1u;
+        if (t.age != 0u && t.backoff != 0u) ctl->tight_backoff = 0;
     } else if (m == kTightBuild) {
-        ctl->tight_next = kTightUse;
+        next = kTightUse;
         ctl->tight_age = 0;
         ctl->tight_stray = 0;
-    } else if (ctl->tight_next == kTightUse) {  // left behind
-        if (ctl->tight_age == 0u) {  // before they served a sweep: do without for a while
-            ctl->tight_backoff = min(2u * ctl->tight_backoff + 1u, 15u);
-            ctl->tight_wait = ctl->tight_backoff;
-        }
-        ctl->tight_next = kTightOff;
-    } else if (ctl->tight_wait != 0u) {
-        ctl->tight_wait -= 1;
-    } else if ((ctl->iter == 0u ? ctl->iterations_last == 0 || ctl->iterations_last >= kTightFrom
-                                : ctl->iter + 1u >= kTightAgain) &&
-               (int)ctl->iter + 2 < P.max_iters) {
-        ctl->tight_next = kTightBuild;
+        ctl->tight_marked = marks ? 1u : 0u;
+        ctl->tight_outrun = 0;
+    } else if (t.next != kTightOff) {  // left behind, or not built
+        if (t.age == 0u) ctl->tight_wait = ctl->tight_backoff = min(2u * t.backoff + 1u, 63u);  // they served no sweep
+        next = kTightOff;
+    } else if (t.wait != 0u) {
+        ctl->tight_wait = t.wait - 1u;
+    } else if ((t.iter == 0u ? t.last == 0 || t.last >= kTightFrom : t.iter + 1u >= kTightAgain) && (int)t.iter + 2 < P.max_iters) {
+        next = kTightBuild;
+        ctl->tight_age = 0;
     }
+    if (next != t.next) ctl->tight_next = next;
+    ctl->fast_before = t.fast;
+    return next;
 }
 // A lane's tight list in the making. kShared: two chunks staged in shared memory, a chunk written out when it is full (whole
 // sectors; 188 us at 1M). Otherwise entry by entry: the sweeps of the loop, which seldom build, keep the L1 (16 KB of
@@ -884,11 +914,15 @@ __global__ void __launch_bounds__(kBlock, DEEP == 1 ? 1 : 2) k_normal_list(PS ps
 // which gives the walk's sum. The round is the one the next pressure sweep reads (Control::round + 1); that sweep's last
 // block closes it.
 //
+// Where the next sweep may build tight lists, or reads some, partners count within h + 2 m.
+__device__ __forceinline__ float marks_ahead(const DevParams& P, const Control* ctl, const ListBuffers& b) {
+    return b.tight && ctl->tight_next != kTightOff ? 2.f * P.tight_margin : 0.f;
+}
 // Cell o of the 5 x 5 x 5 cells around x*_j's cell c0, if particles in it can be partners: a particle that is not fast
 // lies within D = h + skin_max_half (< 2 cells, checked on the host) of such an x*_j, so its cell is among them, and its
 // box comes within D of x*_j (with a margin for the divisions of cell_of). Within 2^14 cells of the origin the rounding of
 // the box bounds and of cell_of's division is far below that margin; farther out (or saturated, or NaN) every cell counts.
-__device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& pj, const Cell& c0, uint32_t o, float margin,
+__device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& pj, const Cell& c0, uint32_t o, float ahead,
                                              Cell& c) {
     c = Cell{c0.x + o % 5u - 2u, c0.y + o / 5u % 5u - 2u, c0.z + o / 25u - 2u};
     auto inner = [](uint32_t v) { return v + 16384u < 32768u; };  // -2^14 < (int)v < 2^14, wrapping
@@ -898,7 +932,7 @@ __device__ __forceinline__ bool partner_cell(const DevParams& P, const float4& p
         return fmaxf(fmaxf(lo - x, x - hi), 0.f);
     };
     const float gx = gap(c.x, pj.x), gy = gap(c.y, pj.y), gz = gap(c.z, pj.z);
-    const float reach = P.h + P.skin_max_half + margin + 0.01f * P.cell_size;
+    const float reach = P.h + P.skin_max_half + ahead + 0.01f * P.cell_size;
     return !(gx * gx + gy * gy + gz * gz > reach * reach);
 }
 __device__ __forceinline__ bool beyond_list(const DevParams& P, const float4& xi, const float4& xj) {
@@ -914,19 +948,22 @@ constexpr unsigned kMarkBlocks = 608;
 __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Control* ctl, ListBuffers b) {
     const unsigned long long n = ctl->fast_n;
     if (n == 0 || n > P.mark_cap) return;
-    if (b.tight && ctl->tight_next == kTightUse && ctl->tight_stray == 0u) return;  // the next sweep asks no marks
-    const float margin = tight_margin(P, ctl, b), far2 = margin > 0.f ? P.tight_r2 : P.h2;
+    const bool watch = b.tight && ctl->tight_next == kTightUse && ctl->tight_stray == 0u;  // the next sweep reads tight lists
+    if (watch && ctl->tight_outrun == 0u) return;  // and asks no marks
+    const float ahead = marks_ahead(P, ctl, b), far2 = ahead > 0.f ? P.tight_r2 : P.h2;
     const unsigned round = ctl->round + 1u;
     const unsigned long long items = n * 125ull;
     for (unsigned long long t = (unsigned long long)blockIdx.x * kBlock + threadIdx.x; t < items;
          t += (unsigned long long)gridDim.x * kBlock) {
         const uint32_t j = b.fast_list[t / 125ull];
         const uint32_t o = (uint32_t)(t % 125ull);
-        if (o == 62u) b.walk_stamp[j] = round;  // the centre cell's thread: j itself walks
         const float4 pj = b.pred[j];
         const float4 xj = b.pos[j];
+        float disp;
+        if (watch && outruns<false>(P, ctl, xj, b.tight_ref[j], P.list_half_skin, make_float3(0.f, 0.f, 0.f), disp)) continue;
+        if (o == 62u) b.walk_stamp[j] = round;  // the centre cell's thread: j itself walks
         Cell c;
-        if (!partner_cell(P, pj, cell_of(pj.x, pj.y, pj.z, P), o, margin, c)) continue;
+        if (!partner_cell(P, pj, cell_of(pj.x, pj.y, pj.z, P), o, ahead, c)) continue;
         const uint2 r = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
 #pragma unroll 1
         for (uint32_t i0 = r.x; i0 < r.y; i0 += 4) {
@@ -960,8 +997,8 @@ __device__ __noinline__ void mark_partners_inline(const DevParams& P, Control* c
     if (base >= P.mark_cap) return;  // past the cap: the sweep takes the bucket flags
     __syncwarp();                    // the lanes' predictions are stored
     const unsigned round = ctl->round + 1u;
-    const float margin = tight_margin(P, ctl, b);
-    const float far = P.h + P.skin_max_half + margin + 1e-4f * P.h;  // D, past the rounding of the distances
+    const float ahead = marks_ahead(P, ctl, b);
+    const float far = P.h + P.skin_max_half + ahead + 1e-4f * P.h;  // D, past the rounding of the distances
     for (; set; set &= set - 1u) {
         const uint32_t j = __shfl_sync(kAll, i, __ffs(set) - 1);
         const float4 pj = b.pred[j], xj = b.pos[j];
@@ -973,7 +1010,7 @@ __device__ __noinline__ void mark_partners_inline(const DevParams& P, Control* c
             const uint32_t o = lane + 32u * q;
             Cell c;
             r[q] = make_uint2(0u, 0u);
-            if (o < 125u && partner_cell(P, pj, c0, o, margin, c)) r[q] = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
+            if (o < 125u && partner_cell(P, pj, c0, o, ahead, c)) r[q] = b.cells[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1011,8 +1048,8 @@ __device__ __forceinline__ bool finish_force(const PS& ps, const ListBuffers& b,
     const float4 xs = make_float4(xi.x + dx.x, xi.y + dx.y, xi.z + dx.z, 0.f);
     b.pred[i] = xs;
     bool fast;
-    const float disp = note_displacement<!PS::kBatched>(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin,
-                                                        tight_margin(P, ps.control(i), b), vi, fast, PS::kBatched ? nullptr : b.fast_list, i);
+    const float disp = note_displacement<!PS::kBatched>(P, ps.control(i), b.bucket_fast, xi, xs, P.list_half_skin, vi, nullptr,
+                                                        fast, PS::kBatched ? nullptr : b.fast_list, i);
     if (P.particle_skin) b.disp_max[i] = disp;
     return fast;
 }
@@ -1123,12 +1160,6 @@ __global__ void __launch_bounds__(kBlock) k_force_shared(PS ps, ListBuffers b) {
 
 // pcisph.cl:212-263 (boundary_update = 0); one scene: also the stop decision in the last block
 
-// No prediction of this step was fast: the scene's lists are complete for x*.
-template <class PS>
-__device__ __forceinline__ bool lists_hold(const Control* ctl) {
-    return ctl->lists_outrun == 0u;
-}
-
 // How one particle's pressure sweep finds its neighbours.
 struct PressurePlan {
     uint32_t cnt, bcnt;              // entries of its skin list and of its boundary list
@@ -1139,10 +1170,13 @@ struct PressurePlan {
 template <class PS>
 __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBuffers& b, const DevParams& P,
                                                       const Control* ctl, uint32_t i, const float4& xi,
-                                                      const float4& xp, unsigned mode) {
+                                                      const float4& xp, const ListState& state) {
     PressurePlan p;
-    const bool all_lists_ok = lists_hold<PS>(ctl);
-    p.cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
+    const unsigned mode = state.mode;
+    const bool all_lists_ok = !state.outrun;
+    const uint32_t listed = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
+    const bool complete = mode == kTightUse && (listed & kTightWalked) != 0u;  // its tight list was built by a walk
+    p.cnt = mode == kTightUse ? listed & ~kTightWalked : listed;
     const bool overflow = p.cnt > (mode == kTightUse ? kTightCap : P.list_cap);
     // self_fast: x* moved more than the particle's own half skin from x, so its lists (built for that
     // skin) may miss a pair: with per-particle skins it walks. Boundary terms: all zero unless a boundary
@@ -1152,8 +1186,7 @@ __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBu
     bool self_fast = false;
     if (P.particle_skin || P.boundary_count) {
         const float dx = xp.x - xi.x, dy = xp.y - xi.y, dz = xp.z - xi.z;
-        const float ahead = mode == kTightBuild && P.particle_skin ? P.tight_margin : 0.f;
-        self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w)) - ahead;
+        self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w));
     }
     p.walk_boundary = p.list_boundary = false;
     p.bcnt = 0;
@@ -1167,22 +1200,23 @@ __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBu
         }
     }
     p.c = Cell{0u, 0u, 0u};  // the cell (three IEEE divisions) only where a walk may need it
-    const bool own_walk = overflow || (P.particle_skin && self_fast);
-    // partner marks of this round (one scene, after the marking kernel): the particles that may miss a
-    // pair of their walk are stamped with the round's number; a round past the cap (or no marks) takes
-    // the bucket flags: every particle near a fast one walks
-    const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
-    const bool marks = fast_round <= P.mark_cap;
-    if (mode == kTightUse) {
+    const bool own_walk = overflow || (P.particle_skin && self_fast) || (mode == kTightBuild && tight_by_walks(P));
+    if (complete || (mode == kTightUse && all_lists_ok && !own_walk)) {
         p.walk = overflow;
-        if (p.walk || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
-    } else if (marks) {
-        p.walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
-        if (p.walk || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
     } else {
-        if (own_walk || !all_lists_ok || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
-        p.walk = own_walk || (!all_lists_ok && near_fast(P, b.bucket_fast, p.c));
+        // partner marks of this round (one scene, after the marking kernel): the particles that may miss a
+        // pair of their walk are stamped with the round's number; a round past the cap (or no marks) takes
+        // the bucket flags: every particle near a fast one walks (marks by a predicting sweep that expected
+        // tight lists to be read lack the predictions that were fast at their building)
+        const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
+        if (fast_round <= P.mark_cap && (mode == kTightUse || b.fast_list || !b.tight || ctl->tight_next != kTightUse)) {
+            p.walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
+        } else {
+            if (!all_lists_ok) p.c = cell_of(xi.x, xi.y, xi.z, P);
+            p.walk = own_walk || (!all_lists_ok && near_fast(P, b.bucket_fast, p.c));
+        }
     }
+    if (p.walk || p.walk_boundary) p.c = cell_of(xi.x, xi.y, xi.z, P);
     return p;
 }
 
@@ -1288,7 +1322,7 @@ __device__ __forceinline__ float pressure_walkers(const PS& ps, const ListBuffer
             }
         }
         sum();
-        if (keep && (int)lane == t) b.tight_count[it] = kept;
+        if (keep && (int)lane == t) b.tight_count[it] = kept | kTightWalked;
     }
     return mine ? finish_pressure<PS>(b, P, ps.control(ii), ii, xi, acc) : 0.f;
 }
@@ -1319,7 +1353,7 @@ __device__ __forceinline__ float build_tight_list(const ListBuffers& b, const De
         });
     else for_each_listed_ahead(b.nbr, i, cnt, b.nbr_stride, away2, keep, flush);
     w.finish();
-    b.tight_count[i] = w.n;
+    b.tight_count[i] = w.n | (walk ? kTightWalked : 0u);
     return acc;
 }
 // One particle's pressure sweep; returns its density variation (0 when skipped or out of range). The whole warp calls;
@@ -1342,13 +1376,16 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
     const DevParams& P = ps.params(live ? i : 0u);
     Control* ctl = ps.control(live ? i : 0u);
     if (live) {
-        const bool all_lists_ok = lists_hold<PS>(ctl);
         xi = b.pos[i];
         xp = b.pred[i];
-        const unsigned mode = kTight ? tight_mode(P, ctl, b.tight != nullptr) : kTightOff;
+        const ListState state = list_state<kTight>(P, ctl, b.tight != nullptr);
+        const unsigned mode = state.mode;
+        const bool all_lists_ok = !state.outrun;
         build = mode == kTightBuild;
-        cnt = mode == kTightUse ? b.tight_count[i] : b.nbr_count[i];
         tight = mode == kTightUse;
+        cnt = tight ? b.tight_count[i] : b.nbr_count[i];
+        const bool complete = tight && (cnt & kTightWalked) != 0u;  // its tight list was built by a walk
+        if (tight) cnt &= ~kTightWalked;
         if (PS::kBatched && tight && cnt == kTightSkin) {
             cnt = b.nbr_count[i];
             tight = false;
@@ -1362,8 +1399,7 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
         bool self_fast = false;
         if (P.particle_skin || P.boundary_count) {
             const float dx = xp.x - xi.x, dy = xp.y - xi.y, dz = xp.z - xi.z;
-            const float ahead = build && P.particle_skin ? P.tight_margin : 0.f;
-            self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w)) - ahead;
+            self_fast = sqrtf(dist2(dx, dy, dz)) > fast_threshold(P, half_skin_of(P, xi.w));
         }
         bool walk_boundary = false, list_boundary = false;
         uint32_t bcnt = 0;
@@ -1377,22 +1413,19 @@ __device__ __forceinline__ float pressure_body(const PS& ps, const ListBuffers& 
             }
         }
         Cell c{0u, 0u, 0u};  // the cell (three IEEE divisions) only where a walk may need it
-        const bool own_walk = overflow || (P.particle_skin && self_fast);
-        // partner marks of this round (one scene, after the marking kernel): the particles that may miss a
-        // pair of their walk are stamped with the round's number; a round past the cap (or no marks) takes
-        // the bucket flags: every particle near a fast one walks
-        const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
-        const bool marks = fast_round <= P.mark_cap;
-        if (mode == kTightUse) {
+        const bool own_walk = overflow || (P.particle_skin && self_fast) || (build && tight_by_walks(P));
+        if (complete || (tight && all_lists_ok && !own_walk)) {
             walk = overflow;
-            if (walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
-        } else if (marks) {
-            walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
-            if (walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
-        } else {
-            if (!all_lists_ok || walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
-            walk = own_walk || (!all_lists_ok && near_fast(P, b.bucket_fast, c));
+        } else {  // by marks or flags (see plan_pressure)
+            const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
+            if (fast_round <= P.mark_cap) {
+                walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
+            } else {
+                if (!all_lists_ok) c = cell_of(xi.x, xi.y, xi.z, P);
+                walk = own_walk || (!all_lists_ok && near_fast(P, b.bucket_fast, c));
+            }
         }
+        if (walk_boundary) c = cell_of(xi.x, xi.y, xi.z, P);
         auto fb = [&](uint32_t j) { acc += density_term(xp.x, xp.y, xp.z, __ldg(&b.b_pos[j]), P.h2); };
         if (walk_boundary) for_each_neighbour(b.b_cells, c, P, fb);
         else if (list_boundary) for_each_listed(b.bnbr, i, bcnt, b.nbr_stride, fb);
@@ -1452,8 +1485,9 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
     const float4 xi = b.pos[i];
     const float4 xp = b.pred[i];
     PressurePlan p{};
-    const unsigned mode = tight_mode(P, ctl, b.tight != nullptr);
-    if (live) p = plan_pressure(ps, b, P, ctl, i, xi, xp, mode);
+    const ListState state = list_state<true>(P, ctl, b.tight != nullptr);
+    const unsigned mode = state.mode;
+    if (live) p = plan_pressure(ps, b, P, ctl, i, xi, xp, state);
     float acc = 0.f;
     auto sum = [&](const float4& o, bool valid, uint32_t m) {
         add_lanes<L>(acc, valid ? density_term(xp.x, xp.y, xp.z, o, P.h2) : 0.f, m);
@@ -1494,7 +1528,7 @@ __device__ __forceinline__ float pressure_shared(const PS& ps, const ListBuffers
                 keep(o, j, valid, mask);
             });
         if (live && q == 0) {
-            b.tight_count[i] = kept;
+            b.tight_count[i] = kept | (p.walk ? kTightWalked : 0u);
             b.tight_ref[i] = xp;
         }
     } else {
@@ -1535,15 +1569,16 @@ __global__ void __launch_bounds__(BS, LANES > 1 ? 1 : kThreads / BS) k_pressure_
     __syncthreads();
     if (is_last && threadIdx.x == 0) {
         __threadfence();
-        ctl->max_err_bits = atomicAdd(&ctl->max_err_bits, 0u);  // see every block's contribution
-        tight_advance(ps.params(0), ctl, b.tight != nullptr);
+        const DevParams& P = ps.params(0);
+        const bool marks = b.walk_stamp && ctl->fast_n <= P.mark_cap, moves = lists_move(P, ctl);
+        const unsigned round = ctl->round;
+        const unsigned next = tight_advance(P, ctl, b.tight != nullptr, marks);
         if (b.walk_stamp) {  // close the prediction round of the partner marks: the next one starts empty
-            ctl->round += 1u;
-            // no marks with moving lists, nor by a predicting sweep that expects the next to read tight lists (one that
-            // then does not takes the bucket flags)
-            const bool none = lists_move(ps.params(0), ctl) || (!b.fast_list && b.tight && ctl->tight_next == kTightUse);
-            ctl->fast_n = none ? kNoMarks : 0ull;
+            ctl->round = round + 1u;
+            // no marks with moving lists, nor where nobody needs them
+            ctl->fast_n = moves || (next != kTightOff && tight_by_walks(P)) ? kNoMarks : 0ull;
         }
+        ctl->max_err_bits = atomicAdd(&ctl->max_err_bits, 0u);  // see every block's contribution
         decide(ps.params(0), ctl);
     }
 }
@@ -1572,9 +1607,8 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
         const float4 xs = f4(x, 0.f);
         b.pred[i] = xs;
         bool fast;
-        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin,
-                                                            tight_margin(P, ctl, b), vi, fast,
-                                                            PS::kBatched ? nullptr : b.fast_list, i);
+        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin, vi,
+                                                            watch ? &r : nullptr, fast, PS::kBatched ? nullptr : b.fast_list, i);
         if (watch) {
             if (!(sqrtf(dist2(xs.x - r.x, xs.y - r.y, xs.z - r.z)) <= P.tight_reach) && ctl->tight_stray == 0u)
                 ctl->tight_stray = 1u;  // NaN strays
@@ -1594,6 +1628,13 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
                 *xs = P.box_hi[ax];
                 if (*vs > 0.f) *vs = -P.restitution * *vs;
             }
+        }
+    }
+    if constexpr (!PS::kBatched) {
+        if (lists_move(P, ctl)) {
+            float disp;
+            const unsigned set = __ballot_sync(__activemask(), outruns<true>(P, ctl, xi, f4(x, 0.f), P.list_half_skin, vi, disp));
+            if (set && (int)(threadIdx.x & 31u) == __ffs(set) - 1) atomicAdd(&ctl->strays, (unsigned)__popc(set));
         }
     }
     const uint32_t o = b.out_index ? b.out_index[i] : i;  // working order -> sorted order
@@ -1785,7 +1826,7 @@ __global__ void k_batch_decide(const DevParams* __restrict__ table, Control* ctl
             c->finished = 1;
             continue;
         }
-        tight_advance(table[s], c, tight);
+        tight_advance(table[s], c, tight, false);
         decide(table[s], c);
         if (!c->done) atomicOr(&running, 1);
     }
@@ -1830,8 +1871,8 @@ __global__ void k_batch_begin(DevParams* table, Control* ctls, uint32_t n_scenes
         c->tight_next = kTightOff;
         c->tight_stray = 0;
         c->tight_age = 0;
-        c->tight_wait = 0;
-        c->tight_backoff = 0;
+        c->tight_outrun = 0;
+        c->fast_before = c->fast_particles;
         c->status = 0;
     }
     if (threadIdx.x == 0) {
@@ -1904,7 +1945,6 @@ void launch_density_list(const DevParams& P, Control* ctl, const ListBuffers& b,
 //   32,768      14.8 / 16.8 / 19.0   15.2 / 12.1 / 16.2   14.5 / 10.7 / 16.2   19.2 /  -   / 33
 //   64,000      19.5 / 21.0 / 29.8   16.2 / 16.3 / 26.4   15.1 / 16.2 / 25
 constexpr int kLanes = 8;
-constexpr uint32_t kSharedMax = 8192u;  // eight lanes
 constexpr uint32_t kDeepMax = 49152u;   // two chunks in flight, pressure force and normal
 // Past 2M particles the default block of the corrective sweeps is 128 threads instead of 256 (8.4M: pressure force 614 -> 588
 // us, pressure 663 -> 658; equal at 1M).

@@ -49,7 +49,7 @@ struct ListBuffers {
     uint32_t* fast_list;
     uint32_t* walk_stamp;
     // tight lists (or null): kTightCap entries per particle laid out like nbr, the entries per particle (> kTightCap: walk
-    // the buckets; kTightSkin: read the skin list), and the predictions they were built at. In a batch they lie where the
+    // the buckets; kTightSkin: read the skin list; kTightWalked beside them), and the predictions they were built at. In a batch they lie where the
     // skin list entries from tight_below on do: a particle with more keeps its skin list.
     uint32_t* tight;
     uint32_t tight_below;

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(kBlock) k_hash(const float* __restrict__ pos, 
             moves = dist2(dx, dy, dz) > slow * slow;
         }
         const int m = __syncthreads_count(moves);  // one atomic per block that has any
-        if (m && threadIdx.x == 0) atomicAdd(&ctl->moving, (unsigned)m);
+        if (m && threadIdx.x == 0 && ctl->moving_wait == 0u) atomicAdd(&ctl->moving, (unsigned)m);
     }
     if (i >= n) return;
     float x, y, z;
@@ -101,11 +101,13 @@ __global__ void __launch_bounds__(kBlock) k_reorder(const uint32_t* __restrict__
 
 // The step's start: its control fields, empty buckets and no bucket flags, in one launch (two memset nodes before: a step of
 // 4,096 particles 159 -> 157 us).
-__global__ void __launch_bounds__(kBlock) k_begin(Control* ctl, uint2* cells, uint32_t* fast, uint32_t bk) {
+__global__ void __launch_bounds__(kBlock) k_begin(Control* ctl, uint2* cells, uint32_t* fast, uint32_t bk, uint32_t n) {
     const uint32_t t = blockIdx.x * kBlock + threadIdx.x;
     if (t < bk) cells[t] = make_uint2(0u, 0u);
     if (fast && t < (bk + 3u) / 4u) fast[t] = 0u;
     if (t != 0) return;
+    const unsigned moving = ctl->moving, strays = ctl->strays, wait = ctl->moving_wait, backoff = ctl->moving_backoff;
+    const unsigned long long fast_particles = ctl->fast_particles;
     ctl->iter = 0;
     ctl->done = 0;
     ctl->max_err_bits = 0;
@@ -113,15 +115,20 @@ __global__ void __launch_bounds__(kBlock) k_begin(Control* ctl, uint2* cells, ui
     ctl->status = 0;
     ctl->guard_iters = 0;
     ctl->n_groups = 0;
-    ctl->fast_at_begin = ctl->fast_particles;
+    ctl->fast_at_begin = fast_particles;
     ctl->fast_n = 0;
+    if (moving > n / kMovingShare)  // the last step took moving lists
+        ctl->moving_wait = ctl->moving_backoff =
+            n > kSharedMax && strays > n / kMovingShare ? min(2u * backoff + 1u, 15u) : 0u;
+    else if (wait != 0u) ctl->moving_wait = wait - 1u;
     ctl->moving = 0;
+    ctl->strays = 0;
     ctl->lists_outrun = 0;
     ctl->tight_next = kTightOff;
     ctl->tight_stray = 0;
     ctl->tight_age = 0;
-    ctl->tight_wait = 0;
-    ctl->tight_backoff = 0;
+    ctl->tight_outrun = 0;
+    ctl->fast_before = fast_particles;
 }
 
 // pcisph.cl:65-92
@@ -433,8 +440,8 @@ void launch_reorder(const uint32_t* keys, const uint32_t* ids, const float4* in_
                                              ctl, in_skin);
 }
 
-void launch_begin(Control* ctl, uint2* cells, unsigned char* bucket_fast, uint32_t buckets, cudaStream_t s) {
-    k_begin<<<std::max(1u, grid_for(buckets)), kBlock, 0, s>>>(ctl, cells, reinterpret_cast<uint32_t*>(bucket_fast), buckets);
+void launch_begin(Control* ctl, uint2* cells, unsigned char* bucket_fast, uint32_t buckets, uint32_t n, cudaStream_t s) {
+    k_begin<<<std::max(1u, grid_for(buckets)), kBlock, 0, s>>>(ctl, cells, reinterpret_cast<uint32_t*>(bucket_fast), buckets, n);
 }
 
 void launch_density(const DevParams& P, const StepBuffers& b, cudaStream_t s) {

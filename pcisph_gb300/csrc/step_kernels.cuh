@@ -54,8 +54,8 @@ void launch_hash(const float* pos, bool packed, uint32_t n, const DevParams& P, 
 void launch_reorder(const uint32_t* keys, const uint32_t* ids, const float4* in_pos, const float4* in_vel,
                     uint32_t n, float4* out_pos, float4* out_vel, uint2* cells, uint32_t* codes, uint32_t* groups,
                     const DevParams& P, Control* ctl, cudaStream_t s, const float* in_skin = nullptr);
-// buckets entries of cells and (or null) bucket_fast are cleared, the latter to a multiple of 4 bytes.
-void launch_begin(Control* ctl, uint2* cells, unsigned char* bucket_fast, uint32_t buckets, cudaStream_t s);
+// buckets entries of cells and (or null) bucket_fast are cleared, the latter to a multiple of 4 bytes. n: particles.
+void launch_begin(Control* ctl, uint2* cells, unsigned char* bucket_fast, uint32_t buckets, uint32_t n, cudaStream_t s);
 void launch_density(const DevParams& P, const StepBuffers& b, cudaStream_t s);
 void launch_normal(const DevParams& P, const StepBuffers& b, cudaStream_t s);
 void launch_force(const DevParams& P, const StepBuffers& b, cudaStream_t s);

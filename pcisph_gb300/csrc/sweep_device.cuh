@@ -24,30 +24,39 @@ __device__ __forceinline__ void warp_count(unsigned long long* addr, bool pred) 
     if (c && (int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(addr, (unsigned long long)c);
 }
 
+// Did xs leave the lists of the particle at xi behind (a move past the threshold from x, or from y with moving lists)? disp:
+// its displacement.
+template <bool kOne>
+__device__ __forceinline__ bool outruns(const DevParams& P, const Control* ctl, const float4& xi, const float4& xs,
+                                        float threshold, const float3& vi, float& disp) {
+    disp = sqrtf(dist2(xs.x - xi.x, xs.y - xi.y, xs.z - xi.z));  // exact differences: xs and xi are close
+    if (kOne) {
+        if (lists_move(P, ctl)) {
+            const float4 y = moving_place(P, xi, vi);
+            return !(sqrtf(dist2(xs.x - y.x, xs.y - y.y, xs.z - y.z)) <= threshold);  // NaN strays
+        }
+    }
+    return disp > threshold;
+}
+
 // After predicting x*_i (stored as xs): a fast particle (moved more than half the skin) flags its bucket
 // and is counted (one atomic per warp that has one; no store otherwise: in a splash most predictions are
 // fast, and a flag stored by each of their warps measured slower than the counts alone); the predictions
 // past each adaptive skin level are counted. With a fast list (partner marks, one scene), a fast particle
 // also takes a slot of the round's list while the round holds at most P.mark_cap of them (one atomic per
 // warp that has one; none once the round is past the cap, which then falls back to the bucket flags).
-// Returns the displacement |x* - x|; threshold: the particle's fast_threshold; fast: whether it is past it. kOne: one scene, whose lists may move
-// with the particles (then the bucket is flagged when the prediction strays from y, and the round's count is past the
-// cap, so that nothing is listed); vi: the velocity at the step's start.
+// Returns the displacement |x* - x|; threshold: the particle's fast_threshold; flag: whether it is past it. kOne: one
+// scene, whose lists may move with the particles (then the bucket is flagged when the prediction strays from y, and the
+// round's count is past the cap, so that nothing is listed); vi: the velocity at the step's start. ref (or null): the
+// prediction that the tight lists in use were built at; flag is then whether xs outran the lists and that one did not.
 template <bool kOne>
 __device__ __forceinline__ float note_displacement(const DevParams& P, Control* ctl,
                                                    unsigned char* __restrict__ bucket_fast, const float4& xi,
-                                                   const float4& xs, float threshold, float margin, const float3& vi, bool& flag,
-                                                   uint32_t* __restrict__ fast_list = nullptr, uint32_t i = 0) {
-    const float dx = xs.x - xi.x, dy = xs.y - xi.y, dz = xs.z - xi.z;  // exact: xs and xi are close
-    const float disp = sqrtf(dist2(dx, dy, dz));
+                                                   const float4& xs, float threshold, const float3& vi, const float4* ref,
+                                                   bool& flag, uint32_t* __restrict__ fast_list = nullptr, uint32_t i = 0) {
+    float disp;
+    flag = outruns<kOne>(P, ctl, xi, xs, threshold, vi, disp);
     warp_count(&ctl->fast_particles, disp > threshold);
-    flag = disp > threshold - margin;
-    if (kOne) {
-        if (lists_move(P, ctl)) {
-            const float4 y = moving_place(P, xi, vi);
-            flag = !(sqrtf(dist2(xs.x - y.x, xs.y - y.y, xs.z - y.z)) <= threshold - margin);  // NaN strays
-        }
-    }
     if (flag && ctl->lists_outrun == 0u) ctl->lists_outrun = 1u;
     if (fast_list) {
         const unsigned act = __activemask();
@@ -70,7 +79,13 @@ __device__ __forceinline__ float note_displacement(const DevParams& P, Control* 
     }
     if (flag) {
         const Cell c = cell_of(xi.x, xi.y, xi.z, P);
-        bucket_fast[P.bucket_base + hash_key(c.x, c.y, c.z, P)] = 1;
+        unsigned char* mine = &bucket_fast[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
+        if (ref) {
+            float at_ref;
+            flag = !outruns<kOne>(P, ctl, xi, *ref, threshold, vi, at_ref);
+            if (flag && (*mine == 0 || ctl->tight_marked) && ctl->tight_outrun == 0u) ctl->tight_outrun = 1u;
+        }
+        *mine = 1;
     }
     return disp;
 }

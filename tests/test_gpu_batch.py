@@ -259,3 +259,37 @@ def test_batch_rebuilt_lists_change_no_bits():
     for a, b in zip(*out):
         for k, (x, y) in enumerate(zip(a, b)):
             _assert_same("scene %d" % k, x, y)
+
+
+@pytest.mark.parametrize("skin", ["adaptive", 0.03, 0.25])
+def test_batch_outrun_lists_change_no_bits(skin):
+    """Scenes whose predictions outrun the skin lists before, at and after the building of the rebuilt ones: few fast
+    particles around half the skin per step, a corner, most of them, a dense scene whose skin lists fill the rebuilt ones'
+    place; beside them one at rest."""
+    rng = np.random.default_rng(17)
+    sc = []
+    for n_side, motion, speed, gap in ((12, "rest", 0.0, 1.0), (17, "few", 2.2, 1.0), (20, "few", 4.0, 1.0), (16, "corner", 6.0, 1.0),
+                                       (18, "all", 1.5, 1.0), (14, "few", 2.0, 0.72)):
+        s = scenes.small_dam(n_side, seed=n_side)
+        n = s.fluid_count
+        pos = np.asarray(s.fluid_pos)
+        s.fluid_pos = (pos * gap).astype(np.float32)
+        way = rng.standard_normal((n, 3))
+        who = {"rest": np.zeros(n, bool), "few": rng.random(n) < 0.01, "all": np.ones(n, bool),
+               "corner": (pos < np.median(pos, 0)).all(1)}[motion]
+        v = np.zeros((n, 3), np.float32)
+        v[who] = (speed * way / np.linalg.norm(way, axis=1)[:, None]).astype(np.float32)[who]
+        s.fluid_vel = v
+        s.min_iters = s.max_iters = 12
+        sc.append(s)
+    out = []
+    for mode in (0, 2):
+        bt = Batch(0, max_particles=sum(s.fluid_count for s in sc), max_scenes=8, loop_mode=mode)
+        if skin != "adaptive":
+            bt.set_list_skin(skin)
+        ids = [bt.add_scene(s) for s in sc]
+        bt.step(4)
+        out.append([_in_batch(bt, i, s) for i, s in zip(ids, sc)])
+        bt.close()
+    for k, (x, y) in enumerate(zip(*out)):
+        _assert_same("scene %d" % k, x, y)

@@ -231,3 +231,47 @@ def test_set_predictions_find_every_pair(oracle, n, order, after):
     tol = max(RTOL, 2 * min(n, 27 * int((off[:, 1] - off[:, 0]).max())) * 2.0 ** -24)
     assert rho.max() > 1000.0
     assert_close("density_variation", got, np.maximum(rho - 1000.0, 0), scale=float(rho.max()), rtol=tol)
+
+
+# Predictions that outrun the skin lists before, at and after the building of the tight ones: few in a thousand, at speeds around
+# half the skin per step (they cross it within a step), a whole corner, or most, whose lists are then not built for some
+# sweeps or steps; skins narrower than the tight lists' margin; sizes on either side of the forms that mark by themselves, with
+# and without bucket order, boundary particles (and their skins), several steps
+@pytest.mark.parametrize("n,motion,speed,options", [
+    (1000, "few", 2.0, {}), (4096, "few", 4.0, {}), (8192, "few", 2.7, {}), (8193, "few", 2.7, {}), (20000, "few", 2.0, {}),
+    (20000, "few", 3.5, {"boundary": 1}), (20000, "few", 3.5, {"boundary": 1, "particle_skin": 0}), (6000, "few", 2.7, {"boundary": 1}),
+    (4096, "corner", 8.0, {}), (20000, "corner", 8.0, {}), (140000, "corner", 3.0, {}), (20000, "all", 1.2, {}), (5000, "all", 1.2, {}),
+    (20000, "all", 8.0, {}), (5000, "few", 2.0, {"list_skin": 0.03}), (9000, "few", 2.0, {"list_skin": 0.03}),
+    (9000, "few", 2.0, {"list_skin": 0.07}), (9000, "all", 0.6, {"list_skin": 0.1}), (9000, "few", 2.0, {"list_skin": 0.08, "boundary": 1}),
+    (200000, "few", 2.7, {}), (2100000, "few", 2.7, {}), (1000, "few", 4.6, {}), (4096, "few", 5.0, {}), (8192, "few", 4.8, {}),
+    (8193, "few", 4.8, {}), (20000, "few", 5.2, {}), (20000, "few", 4.8, {"boundary": 1}), (6000, "few", 5.0, {"boundary": 1}),
+    (140000, "corner", 5.0, {}), (20000, "all", 3.6, {}), (5000, "all", 3.6, {}), (200000, "few", 5.0, {}), (2100000, "few", 5.0, {})])
+def test_outrun_lists_change_no_bits(oracle, n, motion, speed, options):
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1 / 3)))
+    at = np.stack(np.unravel_index(np.arange(n), (side, side, side)), -1) + 0.5
+    pos = ((at + 0.15 * (2 * rng.random((n, 3)) - 1)) * D).astype(np.float32)
+    vel = (0.3 * rng.standard_normal((n, 3))).astype(np.float32)
+    who = {"few": rng.random(n) < 0.004, "corner": (at < 0.5 * side).all(1), "all": np.ones(n, bool)}[motion]
+    way = rng.standard_normal((n, 3))
+    vel[who] = (speed * way / np.linalg.norm(way, axis=1)[:, None] * (0.8 + 0.4 * rng.random((n, 1)))).astype(np.float32)[who]
+    floor = np.stack(np.meshgrid(np.arange(side), [-0.5], np.arange(side), indexing="ij"), -1).reshape(-1, 3) * D
+    walls = len(floor) if options.get("boundary") else 0
+    steps, iters = (2, 9) if n > 100000 else (5, 12)
+    p = oracle.derive_params(0.5 * D, 1000.0, n, walls, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    out = []
+    for loop_mode in (0, 1, 2):
+        f = fluid_like(p, min_iters=iters, max_iters=iters, loop_mode=loop_mode, spatial_order=2)
+        f.set_options(**{k: v for k, v in options.items() if k != "boundary"})
+        f.set_fluid_state(pos, vel)
+        if walls:
+            f.set_boundary_state(floor.astype(np.float32))
+        f.step(steps)
+        st = f.stats()
+        out.append(({k: f.get_field(k) for k in ("src", "density_variation", "pressure", "position", "velocity", "predicted_position")},
+                    (st.fast_particles, st.list_fallbacks, st.status_all)))
+        f.close()
+    for got in out[:2]:
+        assert got[1] == out[2][1]
+        for k in got[0]:
+            np.testing.assert_array_equal(got[0][k], out[2][0][k], err_msg=k)
