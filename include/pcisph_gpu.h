@@ -231,6 +231,11 @@ PCISPH_API int pcisph_sync_for(pcisph_ctx* ctx, int64_t timeout_ms);
 /* Synchronises, then reports the last step. */
 PCISPH_API int pcisph_last_stats(pcisph_ctx* ctx, pcisph_step_stats* out);
 PCISPH_API int pcisph_reset_stats(pcisph_ctx* ctx);
+/* The rebuilt neighbour lists of a context (variant 2; max_iterations 4 or more, not loop_mode 2): the device memory that they
+ * hold (276 bytes a particle; 0: none, or no room), and the pressure sweeps that read them since pcisph_reset_stats. The
+ * memory is spare: it is taken while an eighth of the device stays free, and given up when another allocation of this
+ * library finds no room; the scene's steps then read its other lists, with the same results. Synchronises. */
+PCISPH_API int pcisph_rebuilt_lists(pcisph_ctx* ctx, uint64_t* bytes, uint64_t* sweeps);
 
 /* Export. dst_bytes must cover count x layout; HOST copies synchronise. */
 PCISPH_API int pcisph_get_field(pcisph_ctx* ctx, int field, void* dst, size_t dst_bytes, int layout, int memory);

@@ -148,6 +148,7 @@ def load():
         "pcisph_sync_for": ([vp, C.c_int64], i32),
         "pcisph_last_stats": ([vp, C.POINTER(StepStats)], i32),
         "pcisph_reset_stats": ([vp], i32),
+        "pcisph_rebuilt_lists": ([vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)], i32),
         "pcisph_get_field": ([vp, i32, vp, sz, i32, i32], i32),
         "pcisph_get_fluid_state": ([vp, vp, vp, u32, i32, i32], i32),
         "pcisph_set_field": ([vp, i32, vp, sz, i32, i32], i32),

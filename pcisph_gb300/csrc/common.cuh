@@ -104,6 +104,7 @@ struct Control {
     unsigned int strays, moving_wait, moving_backoff;
     unsigned long long fast_before;  // fast_particles without those of the current round
     unsigned int tight_marked;   // the tight lists were built by a sweep that took marks, not flags
+    unsigned long long tight_sweeps;  // pressure sweeps that read tight lists
 };
 
 // Close a step after its last corrective iteration `it` (Fluid.cpp:301-306 decides the same way): status

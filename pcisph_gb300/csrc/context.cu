@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -105,7 +106,7 @@ struct pcisph_ctx {
     uint32_t *tight_list = nullptr, *tight_count = nullptr;  // null: no tight lists
     float4* tight_ref = nullptr;
     size_t tight_n = 0;
-    DeviceBlock tight_block;
+    host::SpareBlock tight_block;
     size_t list_n = 0;
     size_t list_b_n = 0;  // boundary particles the list block holds lists for
 
@@ -220,30 +221,36 @@ struct pcisph_ctx {
         const size_t n = params.fluid_count;
         if (n >= (1u << 31)) return fail(PCISPH_ERR_INVALID_ARG, "kernel variant 2 takes fewer than 2^31 particles");
         if (int rc = ensure_base_lists()) return rc;
-        // a scene whose tight lists find no memory does without
-        const bool want = P.tight_margin > 0.f && opts.loop_mode != 2;
-        if (want ? tight_n == n : !tight_list) return PCISPH_OK;  // tried once for a particle count
+        if (P.tight_margin > 0.f ? tight_list && tight_n == n : !tight_list) return PCISPH_OK;
+        // The tight lists take spare memory: a scene that finds none, or whose block was given up (begin_lists), does without
+        // until its parameters or options are set again. None are kept where none can be built.
         CUDA_TRY(cudaStreamSynchronize(stream()));
-        tight_list = nullptr;
-        tight_n = want ? n : 0;
         graph_valid = false;
-        if (!want) return PCISPH_OK;
         const size_t bytes = align256(n * kTightCap * 4) + align256(n * 4) + align256(n * 16);
-        size_t room = 0, total = 0;
-        if (bytes > tight_block.cap) {  // never the last of the memory: a scene that just fits keeps room for its exports
+        if (P.tight_margin == 0.f || !tight_block.acquire(bytes)) {
             tight_block.release();
-            CUDA_TRY(cudaMemGetInfo(&room, &total));
-            if (room < bytes + total / 8) return PCISPH_OK;
-        }
-        if (tight_block.ensure(bytes) != cudaSuccess) {
-            cudaGetLastError();
+            no_tight_lists();
             return PCISPH_OK;
         }
-        Carver c{static_cast<unsigned char*>(tight_block.p)};
+        Carver c{static_cast<unsigned char*>(tight_block.p())};
         tight_list = c.take<uint32_t>(n * kTightCap);
         tight_count = c.take<uint32_t>(n);
         tight_ref = c.take<float4>(n);
+        tight_n = n;
         return PCISPH_OK;
+    }
+    void no_tight_lists() {
+        tight_list = nullptr;
+        set_skins(false);
+        graph_valid = false;
+    }
+    // Before a step is submitted: its lists' memory is the context's until the lock goes.
+    std::unique_lock<std::mutex> begin_lists(cudaStream_t s) {
+        std::unique_lock<std::mutex> lock(tight_block.use);
+        if (tight_list && !tight_block.p()) no_tight_lists();  // given up for another allocation
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        if (tight_list && cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) tight_block.keep();
+        return lock;
     }
     int ensure_base_lists() {
         const size_t n = params.fluid_count;
@@ -390,8 +397,8 @@ struct pcisph_ctx {
         P.skin_factor = kSkinFactor;
         P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
         // (marks reach up to 2 kTightMargin h further where tight lists are built, see below)
-        set_tight_lists(&P, list_sweeps() && P.h + P.skin_max_half + 2.f * kTightMargin * P.h <= 1.9f * P.cell_size);
-        P.skin_min_half = std::min(kSkinMinHalf * P.h + P.tight_margin, P.skin_max_half);
+        set_skins(list_sweeps() && opts.loop_mode != 2 && opts.max_iterations >= kTightFrom &&
+                  P.h + P.skin_max_half + 2.f * kTightMargin * P.h <= 1.9f * P.cell_size);
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
         // cells (with a margin for the divisions of cell_of). With more than 1 in 8 fast nearly every warp holds walkers
@@ -402,6 +409,12 @@ struct pcisph_ctx {
                          : 0u;
         graph_valid = false;
         order_age = kNoOrder;
+    }
+
+    // With or without tight lists, for which the per-particle skins are wider.
+    void set_skins(bool tight) {
+        set_tight_lists(&P, tight);
+        P.skin_min_half = std::min(kSkinMinHalf * P.h + P.tight_margin, P.skin_max_half);
     }
 
     // update_deduced_attributes: derive, (re)allocate, zero velocities, mark the boundary for sorting.
@@ -720,6 +733,7 @@ struct pcisph_ctx {
             rc = boundary_sort(s);
             if (rc) return rc;
         }
+        const auto lists = begin_lists(s);
         if (opts.loop_mode != 1 && !profiling) {
             if (!graph_valid) {
                 rc = build_graph();
@@ -1345,6 +1359,20 @@ int pcisph_reset_stats(pcisph_ctx* ctx) {
     ctx->host_mode_iters = 0;
     Control zero{};
     CUDA_TRY(cudaMemcpy(ctx->ctl, &zero, sizeof(Control), cudaMemcpyHostToDevice));
+    return PCISPH_OK;
+}
+
+int pcisph_rebuilt_lists(pcisph_ctx* ctx, uint64_t* bytes, uint64_t* sweeps) {
+    if (!ctx) return fail(PCISPH_ERR_INVALID_ARG, "ctx is NULL");
+    DeviceGuard g(ctx->device);
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream()));
+    if (bytes) {
+        std::lock_guard<std::mutex> l(ctx->tight_block.use);
+        *bytes = ctx->tight_block.bytes();
+    }
+    unsigned long long n = 0;
+    CUDA_TRY(cudaMemcpy(&n, &ctx->ctl->tight_sweeps, sizeof n, cudaMemcpyDeviceToHost));
+    if (sweeps) *sweeps = n;
     return PCISPH_OK;
 }
 

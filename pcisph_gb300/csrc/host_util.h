@@ -12,6 +12,7 @@
 #include <thread>
 #include <vector>
 
+#include "spare_memory.h"
 #include "../../include/pcisph_gpu.h"
 #include "common.cuh"
 
@@ -235,7 +236,7 @@ struct DeviceBlock {
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        cudaError_t e = cudaMalloc(&p, std::max<size_t>(bytes, 256));
+        cudaError_t e = device_malloc(&p, std::max<size_t>(bytes, 256));
         if (e == cudaSuccess) cap = std::max<size_t>(bytes, 256);
         return e;
     }

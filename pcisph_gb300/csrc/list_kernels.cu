@@ -323,10 +323,11 @@ struct TightState {
     unsigned next, stray, age, wait, backoff, iter;
     int last;
     bool moves;
-    unsigned long long fast, before;
+    unsigned long long fast, before, sweeps;
     __device__ __forceinline__ TightState(const DevParams& P, const Control* c)
         : next(c->tight_next), stray(c->tight_stray), age(c->tight_age), wait(c->tight_wait), backoff(c->tight_backoff),
-          iter(c->iter), last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before) {}
+          iter(c->iter), last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before),
+          sweeps(c->tight_sweeps) {}
     __device__ __forceinline__ unsigned mode(const DevParams& P) const {
         if (next == kTightOff || (next == kTightUse && stray == 0u)) return next;
         const bool again = age != 0u && iter >= kTightAgain && (int)iter + 1 < P.max_iters;
@@ -358,6 +359,7 @@ __device__ __forceinline__ unsigned tight_advance(const DevParams& P, Control* c
     unsigned next = t.next;
     if (m == kTightUse) {
         ctl->tight_age = t.age + 1u;
+        ctl->tight_sweeps = t.sweeps + 1ull;
         if (t.age != 0u && t.backoff != 0u) ctl->tight_backoff = 0;
     } else if (m == kTightBuild) {
         next = kTightUse;

@@ -1,5 +1,6 @@
 // radix_sort.cu -- stable LSD radix sort (see radix_sort.cuh).
 #include "radix_sort.cuh"
+#include "spare_memory.h"
 
 #include <algorithm>
 
@@ -403,7 +404,7 @@ cudaError_t RadixSorter::sort(uint32_t* keys, uint32_t* values, size_t n, int bi
         if (scratch_) cudaFree(scratch_);
         scratch_ = nullptr;
         scratch_cap_ = 0;
-        cudaError_t e = cudaMalloc(&scratch_, need);
+        cudaError_t e = host::device_malloc(&scratch_, need);
         if (e != cudaSuccess) return e;
         scratch_cap_ = need;
         owns_ = true;

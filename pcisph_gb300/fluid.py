@@ -161,6 +161,12 @@ class Fluid:
     def reset_stats(self):
         check(self._L.pcisph_reset_stats(self._h))
 
+    def rebuilt_lists(self):
+        """(bytes held, pressure sweeps that read them) of the context's rebuilt neighbour lists."""
+        held, sweeps = C.c_uint64(), C.c_uint64()
+        check(self._L.pcisph_rebuilt_lists(self._h, C.byref(held), C.byref(sweeps)))
+        return held.value, sweeps.value
+
     def autotune(self, steps=3):
         """Pick the fastest list skin / working order / sort digit width, then the corrective-loop sweeps'
         block size, on the current state (results are unchanged by any choice); returns the choice and the

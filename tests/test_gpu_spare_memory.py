@@ -1,0 +1,179 @@
+"""GPU: the memory of the rebuilt neighbour lists is spare: taken where they can be built and an eighth of the device stays
+free, given up when another allocation of the library finds no room, with the same results either way."""
+import threading
+
+import numpy as np
+import pytest
+
+from gpu_util import fluid_like
+from pcisph_gb300 import Fluid, scenes, setup_scene
+
+pytestmark = pytest.mark.gpu
+
+PER_PARTICLE = 276
+
+
+def _block(oracle, n, seed=1, max_iters=7, **options):
+    d = 0.02
+    side = int(np.ceil(n ** (1 / 3)))
+    rng = np.random.default_rng(seed)
+    at = np.stack(np.unravel_index(np.arange(n), (side, side, side)), -1) + 0.5
+    pos = ((at + 0.1 * (2 * rng.random((n, 3)) - 1)) * d).astype(np.float32)
+    p = oracle.derive_params(0.5 * d, 1000.0, n, 0, 1e-3, -9.81, 0.2 * d ** 3, 0.5)
+    f = fluid_like(p, min_iters=min(6, max_iters), max_iters=max_iters, spatial_order=2)
+    f.set_options(**options)
+    f.set_fluid_state(pos)
+    return f
+
+
+def _state(f):
+    return [f.get_field(k) for k in ("src", "position", "velocity", "pressure")]
+
+
+def _same(a, b):
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x, y)
+
+
+def _leave(torch, room):
+    """A tensor that leaves `room` bytes of the device free."""
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(max(1, free - room), dtype=torch.uint8, device="cuda")
+
+
+def test_held_where_they_can_be_built(oracle):
+    n = 20000
+    f = _block(oracle, n)
+    f.step(2)
+    held, sweeps = f.rebuilt_lists()
+    assert PER_PARTICLE * n <= held <= PER_PARTICLE * n + 3 * 256 and sweeps >= 2 * 3
+    want = _state(f)
+    for options in ({"loop_mode": 2}, {"min_iterations": 3, "max_iterations": 3}, {"kernel_variant": 1}):
+        g = _block(oracle, n, **options)
+        g.step(2)
+        assert g.rebuilt_lists() == (0, 0), options
+        if "loop_mode" in options:
+            _same(_state(g), want)
+        g.close()
+    f.set_options(loop_mode=2)
+    f.step(1)
+    assert f.rebuilt_lists() == (0, sweeps)
+    f.set_options(loop_mode=0)
+    f.step(1)
+    assert f.rebuilt_lists()[0] == held and f.rebuilt_lists()[1] > sweeps
+    f.close()
+
+
+def test_a_scene_without_room_steps_the_same_and_asks_again(oracle):
+    torch = pytest.importorskip("torch")
+    n = 60000
+    f = _block(oracle, n)
+    f.step(3)
+    assert f.rebuilt_lists()[1] > 0
+    want = _state(f)
+    f.close()
+    _, total = torch.cuda.mem_get_info()
+    hold = _leave(torch, total // 10)
+    f = _block(oracle, n)
+    f.step(3)
+    assert f.rebuilt_lists() == (0, 0)
+    _same(_state(f), want)
+    del hold
+    torch.cuda.empty_cache()
+    f.step(1)
+    assert f.rebuilt_lists()[0] == 0  # asks when its options or parameters are set
+    f.set_options(restitution=0.5)
+    f.step(2)
+    held, sweeps = f.rebuilt_lists()
+    assert held >= PER_PARTICLE * n and sweeps > 0
+    f.close()
+
+
+@pytest.mark.parametrize("loop_mode", [0, 1])
+def test_given_up_for_another_context(oracle, loop_mode):
+    torch = pytest.importorskip("torch")
+    a = _block(oracle, 1500000, seed=2, loop_mode=loop_mode)
+    a.step(2)
+    assert a.rebuilt_lists()[0] >= PER_PARTICLE * 1500000
+    a.step(2)
+    want = _state(a)
+    a.close()
+    a = _block(oracle, 1500000, seed=2, loop_mode=loop_mode)
+    a.step(2)
+    a.get_field("velocity"), a.get_field("position")
+    hold = _leave(torch, 300 << 20)
+    b = _block(oracle, 500000, seed=3)  # needs more than is free
+    b.step(2)
+    got = _state(b)
+    assert a.rebuilt_lists()[0] == 0 and b.rebuilt_lists()[0] == 0
+    a.step(2)
+    del hold
+    torch.cuda.empty_cache()
+    _same(_state(a), want)
+    a.close()
+    b.close()
+    c = _block(oracle, 500000, seed=3)
+    c.step(2)
+    _same(got, _state(c))
+    c.close()
+
+
+def test_given_up_while_the_owner_steps(oracle):
+    """One thread steps a scene while another's allocations take its lists' memory back."""
+    torch = pytest.importorskip("torch")
+    a = _block(oracle, 1000000, seed=4)
+    a.step(12)
+    want = _state(a)
+    a.close()
+    a = _block(oracle, 1000000, seed=4)
+    a.step(1)
+    a.sync()
+    assert a.rebuilt_lists()[0] > 0
+    hold = _leave(torch, 200 << 20)
+    errors, go = [], threading.Event()
+
+    def owner():
+        try:
+            go.wait()
+            for _ in range(11):
+                a.step(1)
+            a.sync()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    t = threading.Thread(target=owner)
+    t.start()
+    go.set()
+    b = _block(oracle, 300000, seed=5)
+    b.step(1)
+    b.sync()
+    t.join()
+    assert not errors, errors
+    assert a.rebuilt_lists()[0] == 0
+    del hold
+    torch.cuda.empty_cache()
+    _same(_state(a), want)
+    a.close()
+    b.close()
+
+
+def test_tank_skins_without_rebuilt_lists(oracle):
+    """A tank stepped by the persistent loop and by the graph, and one without room: the same bits."""
+    torch = pytest.importorskip("torch")
+    out = []
+    _, total = torch.cuda.mem_get_info()
+    for loop_mode, leave in ((2, None), (0, None), (0, total // 10)):
+        hold = _leave(torch, leave) if leave else None
+        sc = scenes.small_dam(24, seed=6)
+        sc.boundary_pos = scenes.boundary_box((0.0, 0.0, 0.0), tuple(sc.box_hi), sc.spacing)
+        f = Fluid(0)
+        setup_scene(f, sc, loop_mode=loop_mode)
+        f.step(4)
+        assert (f.rebuilt_lists()[0] > 0) == (loop_mode == 0 and leave is None)
+        out.append(_state(f))
+        f.close()
+        del hold
+        torch.cuda.empty_cache()
+    _same(out[0], out[1])
+    _same(out[0], out[2])
