@@ -99,8 +99,10 @@ typedef struct pcisph_options {
                                       exported fields stay in the reference's sorted order); 0: sorted order;
                                       2 (default): 1 from 131,072 particles, else 0 */
     int32_t sweep_block;           /* variant 2: threads per block of the pressure and pressure-force sweeps
-                                      (the corrective loop's kernels): 128, 256 (default) or 512; scenes of at most
-                                      8,192 (pressure) and 49,152 particles (pressure force) have their own */
+                                      (the corrective loop's kernels): 128, 256 (default) or 512. Scenes of at most
+                                      8,192 (pressure) and 49,152 particles (pressure force) have their own; above
+                                      2,097,152 particles 256 stands for 128, which is faster there; the sweep that
+                                      builds the rebuilt lists takes 128 */
     int32_t particle_skin;         /* variant 2, per-particle skins. 1: particle i's fluid list takes the radius
                                       h + s_i + list_skin h / 2 and its boundary list h + s_i, s_i its own half
                                       skin (twice its largest predicted displacement of the previous step,

@@ -1614,8 +1614,15 @@ int pcisph_autotune(pcisph_ctx* ctx, uint32_t steps, pcisph_tune_result* out) {
             }
     // then the block size of the corrective-loop sweeps, on the best of the above
     int best_block = entry.sweep_block;
+    int timed_block = 0;  // one more that was timed
     for (int bl : {128, 256, 512}) {
         if (rc || bl == entry.sweep_block) continue;
+        const int used = sweep_block_used(N, bl);
+        if (used == sweep_block_used(N, entry.sweep_block) || (timed_block && used == sweep_block_used(N, timed_block))) {
+            ++n;  // the same launches as a block that was timed
+            continue;
+        }
+        timed_block = bl;
         float ms = 0.f;
         rc = apply(best_skin, best_order, best_bits, bl);
         if (!rc) rc = time_it(&ms);

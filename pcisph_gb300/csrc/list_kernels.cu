@@ -1948,9 +1948,13 @@ void launch_density_list(const DevParams& P, Control* ctl, const ListBuffers& b,
 //   64,000      19.5 / 21.0 / 29.8   16.2 / 16.3 / 26.4   15.1 / 16.2 / 25
 constexpr int kLanes = 8;
 constexpr uint32_t kDeepMax = 49152u;   // two chunks in flight, pressure force and normal
-// Past 2M particles the default block of the corrective sweeps is 128 threads instead of 256 (8.4M: pressure force 614 -> 588
+// Past 2M particles the default block of the corrective sweeps, 256, stands for 128 threads (8.4M: pressure force 614 -> 588
 // us, pressure 663 -> 658; equal at 1M).
 constexpr uint32_t kLargeScene = 1u << 21;
+int sweep_block_used(uint32_t n, int block) {
+    if (n <= kSharedMax) return 0;
+    return block == kBlock && n > kLargeScene ? 128 : block;
+}
 constexpr uint32_t kSms = 152u;  // of a GB300; launch shapes that fill it (results do not depend on them)
 
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
@@ -1994,7 +1998,7 @@ void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b
     };
     if (n <= kSharedMax) k_pressure_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b);
     else if (builds && b.tight) go(std::integral_constant<int, 128>{}, std::true_type{});
-    else if (block == 128 || (block == kBlock && n > kLargeScene)) go(std::integral_constant<int, 128>{}, std::false_type{});
+    else if (sweep_block_used(n, block) == 128) go(std::integral_constant<int, 128>{}, std::false_type{});
     else if (block == 512) go(std::integral_constant<int, 512>{}, std::false_type{});
     else go(std::integral_constant<int, kBlock>{}, std::false_type{});
 }
@@ -2011,7 +2015,7 @@ void launch_pressure_force_list(const DevParams& P, Control* ctl, const ListBuff
         k_pressure_force_list<OneScene, kBlock, kLanes><<<grid_for(n * kLanes), kBlock, 0, s>>>(ps, b, mode, cond, uc);
     else if (n <= kDeepMax)
         k_pressure_force_list<OneScene, 128, 1, 2><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
-    else if (block == 128 || (block == kBlock && n > kLargeScene))
+    else if (sweep_block_used(n, block) == 128)
         k_pressure_force_list<OneScene, 128><<<(n + 127) / 128, 128, 0, s>>>(ps, b, mode, cond, uc);
     else if (block == 512) k_pressure_force_list<OneScene, 512><<<(n + 511) / 512, 512, 0, s>>>(ps, b, mode, cond, uc);
     else k_pressure_force_list<OneScene, kBlock><<<grid_for(n), kBlock, 0, s>>>(ps, b, mode, cond, uc);

@@ -120,6 +120,8 @@ bool marks_inline(uint32_t n);
 // set): the particles whose next pressure sweep must walk. That sweep (launched with b.walk_stamp) closes
 // the round.
 void launch_mark_partners(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s);
+// The block that the corrective-loop sweeps of n particles run with when asked for `block` (0: their own, whatever is asked).
+int sweep_block_used(uint32_t n, int block);
 // block: threads per block of the two corrective-loop sweeps (128, 256 or 512). builds: this sweep is expected to build
 // the tight lists.
 void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b, int block, bool builds,

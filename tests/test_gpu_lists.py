@@ -275,3 +275,18 @@ def test_outrun_lists_change_no_bits(oracle, n, motion, speed, options):
         assert got[1] == out[2][1]
         for k in got[0]:
             np.testing.assert_array_equal(got[0][k], out[2][0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("n,block", [(8000, 256), (8000, 512), (2100000, 256), (2100000, 128)])
+def test_autotune_chooses_among_different_launches(oracle, n, block):
+    """The block stays what it was where another's launches are the same: scenes of at most 8,192 particles have their own,
+    and above 2,097,152 256 stands for 128."""
+    p = oracle.derive_params(0.5 * D, 1000.0, n, 0, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    for _ in range(3 if n < 10000 else 1):
+        f = fluid_like(p, spatial_order=1)
+        f.set_options(sweep_block=block)
+        f.set_fluid_state(_cloud(n, 8, seed=n))
+        r = f.autotune(steps=1)
+        assert r["candidates"] == 26
+        assert r["sweep_block"] in ((block,) if n < 10000 else (block, 512))
+        f.close()
