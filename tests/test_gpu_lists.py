@@ -290,3 +290,10 @@ def test_autotune_chooses_among_different_launches(oracle, n, block):
         assert r["candidates"] == 26
         assert r["sweep_block"] in ((block,) if n < 10000 else (block, 512))
         f.close()
+
+
+# the builder's second split (4 particles a warp up to 16,384, 8 beyond)
+@pytest.mark.parametrize("order", [0, 1])
+@pytest.mark.parametrize("n", [16384, 16385])
+def test_lists_at_the_builders_second_split(oracle, n, order):
+    test_lists_hold_the_walks_neighbours(oracle, n, 8, order)

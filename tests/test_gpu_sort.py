@@ -46,3 +46,34 @@ def test_sort_shapes(n, bits, kind, digit_bits):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(k.cpu().numpy().view(np.uint32), keys[order])
     np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[order])
+
+
+def _bucket_keys(x, h, buckets):
+    """The reference's bucket of each position (grid_utils.cl:9-19), whole numbers in wrapping 32-bit arithmetic."""
+    c = np.floor(x / np.float32(h)).astype(np.int64).astype(np.uint32)
+    with np.errstate(over="ignore"):
+        k = (c[:, 0] * np.uint32(19349663)) ^ (c[:, 1] * np.uint32(73856093)) ^ (c[:, 2] * np.uint32(83492791))
+        v = (k << np.uint32(6)) + (c[:, 0] & np.uint32(63)) + np.uint32(4) * (c[:, 1] & np.uint32(63)) + np.uint32(16) * (c[:, 2] & np.uint32(63))
+    return (v & np.uint32(0x7FFFFFFF)) % np.uint32(buckets)
+
+
+# A step sorts by the bits of its bucket count: digits narrower than the sorter's, tiles of 2,048 keys up to 65,536 particles
+# where these leave room for the counts, matches instead of ballots in the first pass. From shuffled particles, and again in the
+# order that the first sort left
+@pytest.mark.parametrize("n", [1, 2, 127, 4096, 4097, 8192, 8193, 10241, 16384, 16385, 20000, 32768, 33000, 40000, 65535, 65536,
+                               65537, 131072, 140001, 262144, 300000, 524288, 700001, 1048577])
+def test_a_steps_sort(oracle, n):
+    from gpu_util import fluid_like
+    d = 0.02
+    p = oracle.derive_params(0.5 * d, 1000.0, n, 0, 1e-3, -9.81, 0.2 * d ** 3, 0.5)
+    f = fluid_like(p, spatial_order=0)
+    x = (np.random.default_rng(n).random((n, 3)) * 2 * d * (n / 8) ** (1 / 3)).astype(np.float32)
+    for _ in range(2):
+        keys = _bucket_keys(x, p.cell_size, p.bucket_count)
+        order = np.argsort(keys, kind="stable")
+        f.set_fluid_state(x)
+        f.run_stage("sort")
+        np.testing.assert_array_equal(f.get_field("keys"), keys[order])
+        np.testing.assert_array_equal(f.get_field("src"), order.astype(np.uint32))
+        x = x[order]
+    f.close()
