@@ -371,7 +371,10 @@ struct pcisph_batch {
 
     int build_graph() {
         cudaGraph_t graph = nullptr;
+        const bool prof = profiling;
+        profiling = false;  // a captured launch is not timed
         int rc = capture(&graph);
+        profiling = prof;
         if (rc) return rc;
         if (graph_exec) {
             cudaGraphExecUpdateResultInfo info{};

@@ -293,3 +293,24 @@ def test_batch_outrun_lists_change_no_bits(skin):
         bt.close()
     for k, (x, y) in enumerate(zip(*out)):
         _assert_same("scene %d" % k, x, y)
+
+
+@pytest.mark.parametrize("mode", [0, 2])
+def test_profiling_from_the_first_step(mode):
+    sc = _mixed_scenes()[:2]
+    out = []
+    for profile in (True, False):
+        bt = Batch(0, max_particles=sum(s.fluid_count for s in sc), max_scenes=2, loop_mode=mode)
+        ids = [bt.add_scene(s) for s in sc]
+        if profile:
+            bt.profile(True)
+        bt.step(2)
+        if profile:
+            launches = bt.profile_read()
+            assert launches["density"][0] == 2 and launches["force"][0] == 2
+            bt.profile(False)
+        bt.step(1)
+        out.append([_in_batch(bt, i, s) for i, s in zip(ids, sc)])
+        bt.close()
+    for k, (x, y) in enumerate(zip(*out)):
+        _assert_same("scene %d" % k, x, y)
