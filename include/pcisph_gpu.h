@@ -105,8 +105,8 @@ typedef struct pcisph_options {
                                       builds the rebuilt lists takes 128 */
     int32_t particle_skin;         /* variant 2, per-particle skins. 1: particle i's fluid list takes the radius
                                       h + s_i + list_skin h / 2 and its boundary list h + s_i, s_i its own half
-                                      skin (twice its largest predicted displacement of the previous step,
-                                      within [0.02 h, list_skin h / 2]); a prediction past s_i makes that
+                                      skin (twice its largest predicted displacement of the previous step and
+                                      0.035 h, within [0.055 h, list_skin h / 2]); a prediction past s_i makes that
                                       particle walk. 0: s_i = list_skin h / 2 for every particle. 2 (default):
                                       1 for scenes with boundary particles (their boundary lists shrink; the
                                       boundary workload runs 6% faster), else 0 (fluid-only lists gain nothing

@@ -33,11 +33,11 @@ struct DevParams {
     float near_r2;      // within-h list radius^2: h^2 (1 + 1e-4), a margin far above rounding
     float list_r, list_r2, list_half_skin;
     // per-particle skins (one scene): particle i's lists take the radius h + sh_i + skin_max_half, sh_i its own
-    // half skin (twice its largest predicted displacement of the previous step, within [skin_min_half,
-    // skin_max_half]); a prediction past its own sh_i makes that particle walk, one past skin_max_half makes
+    // half skin (twice its largest predicted displacement of the previous step and skin_add more, within
+    // [skin_min_half, skin_max_half]); a prediction past its own sh_i makes that particle walk, one past skin_max_half makes
     // its neighbourhood walk (as with one skin). 0: every particle has skin_max_half (half the list skin).
     int particle_skin;
-    float skin_min_half, skin_max_half, skin_factor;
+    float skin_min_half, skin_max_half, skin_factor, skin_add;
     // partner marks (one scene, list sweeps): a prediction round with at most mark_cap fast predictions lists
     // them, and a kernel stamps the particles whose pressure sweep must walk because of them; 0: off (every
     // particle near a flagged bucket walks)

@@ -241,7 +241,7 @@ struct pcisph_ctx {
     }
     void no_tight_lists() {
         tight_list = nullptr;
-        set_skins(false);
+        set_tight_lists(&P, false);
         graph_valid = false;
     }
     // Before a step is submitted: its lists' memory is the context's until the lock goes.
@@ -395,10 +395,12 @@ struct pcisph_ctx {
         const bool skins = opts.particle_skin == 1 || (opts.particle_skin == 2 && params.boundary_count > 0);
         P.particle_skin = skins && list_sweeps() ? 1 : 0;
         P.skin_factor = kSkinFactor;
+        P.skin_add = kSkinAdd * P.h;
+        P.skin_min_half = std::min(kSkinMinHalf * P.h + P.skin_add, P.skin_max_half);
         P.moving_lists = list_sweeps() && params.boundary_count == 0 && !P.particle_skin ? 1 : 0;
         // (marks reach up to 2 kTightMargin h further where tight lists are built, see below)
-        set_skins(list_sweeps() && opts.loop_mode != 2 && opts.max_iterations >= kTightFrom &&
-                  P.h + P.skin_max_half + 2.f * kTightMargin * P.h <= 1.9f * P.cell_size);
+        set_tight_lists(&P, list_sweeps() && opts.loop_mode != 2 && opts.max_iterations >= kTightFrom &&
+                            P.h + P.skin_max_half + 2.f * kTightMargin * P.h <= 1.9f * P.cell_size);
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
         // cells (with a margin for the divisions of cell_of). With more than 1 in 8 fast nearly every warp holds walkers
@@ -409,12 +411,6 @@ struct pcisph_ctx {
                          : 0u;
         graph_valid = false;
         order_age = kNoOrder;
-    }
-
-    // With or without tight lists, for which the per-particle skins are wider.
-    void set_skins(bool tight) {
-        set_tight_lists(&P, tight);
-        P.skin_min_half = std::min(kSkinMinHalf * P.h + P.tight_margin, P.skin_max_half);
     }
 
     // update_deduced_attributes: derive, (re)allocate, zero velocities, mark the boundary for sorting.

@@ -47,6 +47,9 @@ inline constexpr int kIterationsAhead = 3;
 // per-particle skins: a particle's next half skin is kSkinFactor times its largest predicted displacement of
 // the step, at least kSkinMinHalf h (measured at 1M: 0.00-0.05% of the predictions then outrun their skin)
 inline constexpr float kSkinFactor = 2.0f;
+// kSkinAdd h is added to both: a particle that does not outrun its skin walks no buckets. (300,000 particles over a floor, their
+// state set anew every step, persistent loop: 1418 us without, 1129 with; a tank of 279,936 889 and 900.)
+inline constexpr float kSkinAdd = 0.035f;
 inline constexpr float kSkinMinHalf = 0.02f;
 
 // Wait up to timeout_ms for the work queued on s (0: look once). *done = false when it is still running at

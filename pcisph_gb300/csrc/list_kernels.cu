@@ -1643,7 +1643,7 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
     b.state_pos[o] = f4(x, 0.f);
     b.state_vel[o] = f4(v, 0.f);
     if (P.particle_skin)  // the next step's half skin: twice this step's largest predicted displacement
-        b.state_skin[o] = fminf(fmaxf(P.skin_factor * b.disp_max[i] + P.tight_margin, P.skin_min_half), P.skin_max_half);
+        b.state_skin[o] = fminf(fmaxf(P.skin_factor * b.disp_max[i] + P.skin_add, P.skin_min_half), P.skin_max_half);
     return false;
 }
 
