@@ -89,7 +89,9 @@ struct Control {
     unsigned int round;
     unsigned int moving;         // moving lists: the particles that fast (kMovingSpeed) when the step began
     // Every particle's pressure sweep reads these four, as one vector (list_state). Tight lists: how the next sweep finds its
-    // neighbours (kTightOff, kTightBuild or kTightUse), whether a prediction left their reach since they were built
+    // neighbours (kTightOff, kTightBuild or kTightUse; beside it kTightEarly: the lists in use, or the next ones, are built
+    // with the predictions flagged that came within tight_margin of half the skin), whether a prediction left their reach
+    // since they were built
     alignas(16) unsigned int tight_next;
     unsigned int tight_stray;
     unsigned int lists_outrun;   // some prediction of this step was fast (1), measured from the place that the step's
@@ -104,6 +106,7 @@ struct Control {
     unsigned int strays, moving_wait, moving_backoff;
     unsigned long long fast_before;  // fast_particles without those of the current round
     unsigned int tight_marked;   // the tight lists were built by a sweep that took marks, not flags
+    unsigned int tight_asked;    // the sweeps of this step that read tight lists and had to ask the marks or flags again
     unsigned long long tight_sweeps;  // pressure sweeps that read tight lists
 };
 
@@ -132,7 +135,11 @@ constexpr unsigned kTightAgain = 6;     // tight lists that were left behind are
 // Tight lists are built in a round in which at most 1 in kTightShare predictions outran the lists: of more, some leave the
 // tight lists, too, before these have paid for a building sweep in which as many walk.
 constexpr unsigned kTightShare = 16;
-constexpr unsigned kTightOff = 0, kTightBuild = 1, kTightUse = 2;
+// After so many sweeps that had to ask again, with so many iterations of the last step's number left, they are built anew with
+// predictions flagged early (half the skin less the margin): see the list sweeps.
+constexpr unsigned kTightAsked = 4, kTightEarlyLeft = 24;
+constexpr unsigned kTightOff = 0, kTightBuild = 1, kTightUse = 2, kTightEarly = 4;
+__device__ __forceinline__ unsigned tight_plan(unsigned tight_next) { return tight_next & 3u; }
 constexpr uint32_t kNearCap = 64;  // within-h list entries per particle
 constexpr uint32_t kSharedMax = 8192u;  // a scene of at most so many particles: eight lanes a particle in the list sweeps
 
@@ -143,6 +150,10 @@ constexpr unsigned kMovingShare = 8;
 // A particle counts as fast from this share of half the skin per step: pressure and gravity move a prediction further
 // (a sphere falling at 0.11 h a step outran a half skin of 0.125 h in every prediction).
 constexpr float kMovingSpeed = 0.75f;
+// After a step of kMovingLong iterations or more: a little slower bodies cross half the skin here and there, and a long loop pays
+// for that in most of its sweeps (186,000 particles falling at 0.09 h a step, 50 iterations: 3120 us a step, moving 2270).
+constexpr float kMovingSpeedLong = 0.69f;
+constexpr int kMovingLong = 30;
 __device__ __forceinline__ bool lists_move(const DevParams& P, const Control* ctl) {
     return P.moving_lists && ctl->moving > P.fluid_count / kMovingShare;
 }

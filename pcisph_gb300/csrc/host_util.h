@@ -32,7 +32,7 @@ inline float float_from_bits(uint32_t b) {
 }
 
 inline constexpr float kPi = 3.14159265358979323846f;  // utils/constants.h:4
-inline constexpr uint32_t kListCap = 96;           // neighbour-list entries per particle (multiple of 4)
+inline constexpr uint32_t kListCap = 96;           // neighbour-list entries per particle (a multiple of 8, as all of them)
 inline constexpr uint32_t kBoundaryListCap = 48;   // boundary particles within r_list per fluid particle
 inline constexpr uint32_t kBoundaryFluidCap = 64;  // fluid particles within r_list per boundary particle
 // partner marks: fast predictions a round may list (more: the round walks by bucket flags)

@@ -49,6 +49,7 @@ namespace pcisph {
 namespace {
 
 constexpr int kBlock = 256;
+constexpr uint32_t kSms = 152u;  // of a GB300: launch shapes that fill it (results do not depend on them)
 inline unsigned grid_for(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 
 // List layout: entries k = 8c .. 8c+7 of particle i (chunk c) are 32 contiguous bytes at uint4 offset
@@ -300,12 +301,18 @@ constexpr uint32_t kAll = 0xffffffffu;
 // one that read its skin list holds every such pair of the skin list, which is all of them unless the particle has to
 // walk by the rules of the skin lists (fast predictions' flags or marks). It does walk where these say so, and did not in the
 // building sweep. A fast prediction that was fast at the building, too, asks nobody again: there its partners within h + 2 m
-// were marked (or all near its bucket flagged), and walked. A particle with
+// were marked (or all near its bucket flagged), and walked. Where others keep crossing half the skin, sweep after sweep asks the
+// marks: a long loop builds the lists anew then, with the predictions flagged that came within m of it (99,768 to 186,000
+// particles that fall at 0.09 h a step, 50 iterations: 2640 to 3540 us a step without). A particle with
 // more than kTightCap entries walks in every sweep that would read them. One prediction out of reach (or NaN) puts the whole
 // scene back on the skin lists, and from iteration kTightAgain on rebuilds: a building sweep in the loop (it stores entry by
 // entry, 1670 us at 8.4M) pays from three sweeps that use it, which a loop of fewer iterations need not have left.
-// Margins at 1M / 8.4M / a 98,904-particle drop / a violently jittered block of 110,592, us a step: 0.02 2284 / 70510 /
-// 1880 / 5075, 0.03 1998 / 68148 / 1840 / 4793, 0.04 2018 / 67244 / 1821 / 4556.
+// Margins at 1M / 8.4M / a 98,904-particle drop, us a step: 0.02 2284 / 70510 / 1880, 0.03 1998 / 68148 / 1840, 0.04 2018 /
+// 67244 / 1821.
+//
+// A list that held the pairs without asking again (every prediction flagged that came within m of half the skin) cost more than
+// it spared wherever many did: 1,000,000 particles at 2 m/s 4480 us a step, 2770 now (3710 without tight lists); a tank at
+// list_skin 0.1 1240, 750 now.
 //
 // A step of 3 iterations gains nothing (378 us of sweeps at 1M, 399 with them): the lists are built where the previous step
 // took 4 or more. Batch of 32 scenes, 1.32M particles: 46.4 -> 44.6 ms for 16 steps (46.3 without that rule: its falling
@@ -320,13 +327,13 @@ __device__ __forceinline__ bool tight_by_walks(const DevParams& P) { return P.sk
 // The control fields that decide over the tight lists, loaded together: one thread decides at the end of a sweep, and small
 // scenes wait for it.
 struct TightState {
-    unsigned next, stray, age, wait, backoff, iter;
+    unsigned next, stray, age, wait, backoff, iter, outrun, asked, early;
     int last;
     bool moves;
     unsigned long long fast, before, sweeps;
     __device__ __forceinline__ TightState(const DevParams& P, const Control* c)
-        : next(c->tight_next), stray(c->tight_stray), age(c->tight_age), wait(c->tight_wait), backoff(c->tight_backoff),
-          iter(c->iter), last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before),
+        : next(tight_plan(c->tight_next)), stray(c->tight_stray), age(c->tight_age), wait(c->tight_wait), backoff(c->tight_backoff),
+          iter(c->iter), outrun(c->tight_outrun), asked(c->tight_asked), early(c->tight_next & kTightEarly), last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before),
           sweeps(c->tight_sweeps) {}
     __device__ __forceinline__ unsigned mode(const DevParams& P) const {
         if (next == kTightOff || (next == kTightUse && stray == 0u)) return next;
@@ -347,7 +354,7 @@ template <bool kTight>
 __device__ __forceinline__ ListState list_state(const DevParams& P, const Control* ctl, bool on) {
     const uint4 s = *reinterpret_cast<const uint4*>(&ctl->tight_next);  // next, stray, outrun, outrun since the building
     if (!kTight || !on) return ListState{kTightOff, s.z != 0u};
-    unsigned mode = s.x;
+    unsigned mode = tight_plan(s.x);
     if (mode == kTightBuild || (mode == kTightUse && s.y != 0u)) mode = TightState(P, ctl).mode(P);
     return ListState{mode, (mode == kTightUse ? s.w : s.z) != 0u};
 }
@@ -356,13 +363,20 @@ __device__ __forceinline__ unsigned tight_advance(const DevParams& P, Control* c
     if (!on) return kTightOff;
     const TightState t(P, ctl);
     const unsigned m = t.mode(P);
-    unsigned next = t.next;
+    unsigned next = t.next | t.early;
     if (m == kTightUse) {
         ctl->tight_age = t.age + 1u;
         ctl->tight_sweeps = t.sweeps + 1ull;
         if (t.age != 0u && t.backoff != 0u) ctl->tight_backoff = 0;
+        if (t.outrun != 0u && t.early == 0u) {
+            ctl->tight_asked = t.asked + 1u;
+            if (t.asked + 1u >= kTightAsked && t.last >= (int)(t.iter + kTightEarlyLeft)) {
+                next = kTightBuild | kTightEarly;
+            }
+        }
     } else if (m == kTightBuild) {
-        next = kTightUse;
+        // built at once, after a stray: nothing was flagged early
+        next = t.next == kTightUse ? kTightUse : kTightUse | t.early;
         ctl->tight_age = 0;
         ctl->tight_stray = 0;
         ctl->tight_marked = marks ? 1u : 0u;
@@ -376,9 +390,9 @@ __device__ __forceinline__ unsigned tight_advance(const DevParams& P, Control* c
         next = kTightBuild;
         ctl->tight_age = 0;
     }
-    if (next != t.next) ctl->tight_next = next;
+    if (next != (t.next | t.early)) ctl->tight_next = next;
     ctl->fast_before = t.fast;
-    return next;
+    return tight_plan(next);
 }
 // A lane's tight list in the making. kShared: two chunks staged in shared memory, a chunk written out when it is full (whole
 // sectors; 188 us at 1M). Otherwise entry by entry: the sweeps of the loop, which seldom build, keep the L1 (16 KB of
@@ -916,9 +930,9 @@ __global__ void __launch_bounds__(kBlock, DEEP == 1 ? 1 : 2) k_normal_list(PS ps
 // which gives the walk's sum. The round is the one the next pressure sweep reads (Control::round + 1); that sweep's last
 // block closes it.
 //
-// Where the next sweep may build tight lists, or reads some, partners count within h + 2 m.
-__device__ __forceinline__ float marks_ahead(const DevParams& P, const Control* ctl, const ListBuffers& b) {
-    return b.tight && ctl->tight_next != kTightOff ? 2.f * P.tight_margin : 0.f;
+// Where the next sweep may build tight lists, partners count within h + 2 m. watch: it reads some.
+__device__ __forceinline__ float marks_ahead(const DevParams& P, const Control* ctl, const ListBuffers& b, bool watch) {
+    return b.tight && tight_plan(ctl->tight_next) != kTightOff && !watch ? 2.f * P.tight_margin : 0.f;
 }
 // Cell o of the 5 x 5 x 5 cells around x*_j's cell c0, if particles in it can be partners: a particle that is not fast
 // lies within D = h + skin_max_half (< 2 cells, checked on the host) of such an x*_j, so its cell is among them, and its
@@ -946,13 +960,14 @@ __device__ __forceinline__ bool beyond_list(const DevParams& P, const float4& xi
 // nothing (the sweep then uses the bucket flags), nor does a step of moving lists. Grid-stride over the items, 4 blocks an
 // SM: a round of ~3,000 fast predictions at 1M takes 13 us (21 with one block an SM; 14 with a warp per prediction), a
 // round without any 2.5.
-constexpr unsigned kMarkBlocks = 608;
+constexpr unsigned kMarkBlocks = 4u * kSms;
 __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Control* ctl, ListBuffers b) {
     const unsigned long long n = ctl->fast_n;
     if (n == 0 || n > P.mark_cap) return;
-    const bool watch = b.tight && ctl->tight_next == kTightUse && ctl->tight_stray == 0u;  // the next sweep reads tight lists
+    const bool watch = b.tight && tight_plan(ctl->tight_next) == kTightUse && ctl->tight_stray == 0u;  // the next sweep reads tight lists
     if (watch && ctl->tight_outrun == 0u) return;  // and asks no marks
-    const float ahead = marks_ahead(P, ctl, b), far2 = ahead > 0.f ? P.tight_r2 : P.h2;
+    const float ahead = marks_ahead(P, ctl, b, watch), far2 = ahead > 0.f ? P.tight_r2 : P.h2;
+    const float threshold = built_threshold(P, ctl);
     const unsigned round = ctl->round + 1u;
     const unsigned long long items = n * 125ull;
     for (unsigned long long t = (unsigned long long)blockIdx.x * kBlock + threadIdx.x; t < items;
@@ -962,7 +977,7 @@ __global__ void __launch_bounds__(kBlock) k_mark_partners(DevParams P, const Con
         const float4 pj = b.pred[j];
         const float4 xj = b.pos[j];
         float disp;
-        if (watch && outruns<false>(P, ctl, xj, b.tight_ref[j], P.list_half_skin, make_float3(0.f, 0.f, 0.f), disp)) continue;
+        if (watch && outruns<false>(P, ctl, xj, b.tight_ref[j], threshold, make_float3(0.f, 0.f, 0.f), disp)) continue;
         if (o == 62u) b.walk_stamp[j] = round;  // the centre cell's thread: j itself walks
         Cell c;
         if (!partner_cell(P, pj, cell_of(pj.x, pj.y, pj.z, P), o, ahead, c)) continue;
@@ -999,7 +1014,7 @@ __device__ __noinline__ void mark_partners_inline(const DevParams& P, Control* c
     if (base >= P.mark_cap) return;  // past the cap: the sweep takes the bucket flags
     __syncwarp();                    // the lanes' predictions are stored
     const unsigned round = ctl->round + 1u;
-    const float ahead = marks_ahead(P, ctl, b);
+    const float ahead = marks_ahead(P, ctl, b, tight_plan(ctl->tight_next) == kTightUse);  // (else the sweep takes no marks)
     const float far = P.h + P.skin_max_half + ahead + 1e-4f * P.h;  // D, past the rounding of the distances
     for (; set; set &= set - 1u) {
         const uint32_t j = __shfl_sync(kAll, i, __ffs(set) - 1);
@@ -1211,7 +1226,7 @@ __device__ __forceinline__ PressurePlan plan_pressure(const PS& ps, const ListBu
         // the bucket flags: every particle near a fast one walks (marks by a predicting sweep that expected
         // tight lists to be read lack the predictions that were fast at their building)
         const unsigned long long fast_round = !PS::kBatched && b.walk_stamp ? ctl->fast_n : ~0ull;
-        if (fast_round <= P.mark_cap && (mode == kTightUse || b.fast_list || !b.tight || ctl->tight_next != kTightUse)) {
+        if (fast_round <= P.mark_cap && (mode == kTightUse || b.fast_list || !b.tight || tight_plan(ctl->tight_next) != kTightUse)) {
             p.walk = own_walk || (fast_round != 0 && b.walk_stamp[i] == ctl->round + 1u);
         } else {
             if (!all_lists_ok) p.c = cell_of(xi.x, xi.y, xi.z, P);
@@ -1597,7 +1612,8 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
     const float3 fp = make_float3(f.x * scale, f.y * scale, f.z * scale);
     b.f_press[i] = f4(fp, 0.f);
     const bool integrate = mode == 0 ? (ctl->done != 0u) : mode == 2;
-    const bool watch = b.tight && ctl->tight_next == kTightUse;
+    const unsigned plan = b.tight ? ctl->tight_next : kTightOff;
+    const bool watch = tight_plan(plan) == kTightUse;
     float4 r = xi;
     if (watch) r = b.tight_ref[i];  // with the loads below, not after them
     const float3 a = (f3(b.f_other[i]) + fp) / m;
@@ -1609,8 +1625,9 @@ __device__ __forceinline__ bool finish_pressure_force(const PS& ps, const ListBu
         const float4 xs = f4(x, 0.f);
         b.pred[i] = xs;
         bool fast;
-        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, P.list_half_skin, vi,
-                                                            watch ? &r : nullptr, fast, PS::kBatched ? nullptr : b.fast_list, i);
+        const float threshold = plan == (kTightBuild | kTightEarly) ? P.list_half_skin - P.tight_margin : P.list_half_skin;
+        const float disp = note_displacement<!PS::kBatched>(P, ctl, b.bucket_fast, xi, xs, threshold, vi, watch ? &r : nullptr,
+                                                            fast, PS::kBatched ? nullptr : b.fast_list, i);
         if (watch) {
             if (!(sqrtf(dist2(xs.x - r.x, xs.y - r.y, xs.z - r.z)) <= P.tight_reach) && ctl->tight_stray == 0u)
                 ctl->tight_stray = 1u;  // NaN strays
@@ -1874,6 +1891,7 @@ __global__ void k_batch_begin(DevParams* table, Control* ctls, uint32_t n_scenes
         c->tight_stray = 0;
         c->tight_age = 0;
         c->tight_outrun = 0;
+        c->tight_asked = 0;
         c->fast_before = c->fast_particles;
         c->status = 0;
     }
@@ -1955,10 +1973,9 @@ int sweep_block_used(uint32_t n, int block) {
     if (n <= kSharedMax) return 0;
     return block == kBlock && n > kLargeScene ? 128 : block;
 }
-constexpr uint32_t kSms = 152u;  // of a GB300; launch shapes that fill it (results do not depend on them)
 
 void launch_moving_lists(const DevParams& P, Control* ctl, const ListBuffers& b, cudaStream_t s) {
-    const unsigned blocks = std::min(grid_cells(P.fluid_count, 8), 5u * 152u);
+    const unsigned blocks = std::min(grid_cells(P.fluid_count, 8), 5u * kSms);
     if (P.fluid_count) k_moving_lists<<<blocks, kCellBlock, 0, s>>>(P, ctl, b);
 }
 
@@ -1987,11 +2004,10 @@ void launch_pressure_list(const DevParams& P, Control* ctl, const ListBuffers& b
         const unsigned blocks = (n + BS - 1) / BS;
         // 64 registers a thread (4 blocks of 256 per SM) against 48 (5 blocks), us per launch over the sweeps of a step (skin,
         // building and tight): 200,704 particles 35.5 / 36.8, 287,496 37.5 / 42.4, 405,224 52.5 / 55.8, 592,704 67.0 / 70.9,
-        // 1,048,576 112.3 / 113.5, 2.6M equal; below, 48 as long as they hold the scene in one wave (156,244: 27.6 / 23.9).
-        // Past 2M the walks in lane form, which need none of the spills of the inline form (skin list, before the lists were
-        // read past L1: 8.4M 1050 -> 1036).
-        // The building sweep with 64 registers, too, but where a wave of them just misses the scene: 156,244 particles 37
-        // us with 48, 43 with 64; 32,768 29 and 21.
+        // 1,048,576 112.3 / 113.5, 2.6M equal (few walkers in a function of their own then; inlined, a step of 200,000 to
+        // 2,000,000 takes 0.4 to 0.7% less). 48 where they hold a scene in one wave that 64 just miss (156,244: 27.6 / 23.9;
+        // the building sweep 43 / 37). Past 2M every lane walks by itself, which needs none of the spills of the other form
+        // (skin list, before the lists were read past L1: 8.4M 1050 -> 1036).
         if (n > kLargeScene) k_pressure_list<OneScene, BS, 1, false, S, 1280><<<blocks, BS, 0, s>>>(ps, b);
         else if (n > 1024u * kSms && n <= 1280u * kSms) k_pressure_list<OneScene, BS, 1, true, S, 1280><<<blocks, BS, 0, s>>>(ps, b);
         else k_pressure_list<OneScene, BS, 1, true, S><<<blocks, BS, 0, s>>>(ps, b);

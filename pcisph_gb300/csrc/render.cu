@@ -74,7 +74,8 @@ __device__ __forceinline__ float hit_ray(float rx, float ry, float3 s, float out
 // 145), of 262,144 95 -> 87 (1 lane 97, 8 108), of 64,000 82 -> 71 (1 lane 83), of 4,096 at 1920 x 721 312 -> 85 (1 lane 275); small
 // spheres keep one lane (262,144 at 320 x 240 43 -> 41).
 // The image depends on each sum's last bit where a sphere is grazed: as before, the first (columns mod 4) columns of a sphere
-// add rounded products, the others fuse.
+// add rounded products, the others fuse (the bytes of earlier images). k_shade finds the hit once more with its own rounding;
+// where that misses a sphere that was just grazed here (8 of 921,600 pixels of the 1M scene), the pixel is lit from the eye.
 constexpr int kStrip = 8;
 template <uint32_t kLanes>
 __global__ void __launch_bounds__(kBlock) k_splat(const float4* __restrict__ pos, uint32_t n, Camera c,

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(kBlock) k_hash(const float* __restrict__ pos, 
         if (i < n) {
             const float4 v = vel[i];
             const float dx = v.x * P.dt, dy = v.y * P.dt, dz = v.z * P.dt;
-            const float slow = kMovingSpeed * P.list_half_skin;
+            const float slow = (ctl->iterations_last >= kMovingLong ? kMovingSpeedLong : kMovingSpeed) * P.list_half_skin;
             moves = dist2(dx, dy, dz) > slow * slow;
         }
         const int m = __syncthreads_count(moves);  // one atomic per block that has any
@@ -128,6 +128,7 @@ __global__ void __launch_bounds__(kBlock) k_begin(Control* ctl, uint2* cells, ui
     ctl->tight_stray = 0;
     ctl->tight_age = 0;
     ctl->tight_outrun = 0;
+    ctl->tight_asked = 0;
     ctl->fast_before = fast_particles;
 }
 

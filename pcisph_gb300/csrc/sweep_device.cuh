@@ -39,13 +39,18 @@ __device__ __forceinline__ bool outruns(const DevParams& P, const Control* ctl, 
     return disp > threshold;
 }
 
+// The threshold past which predictions were flagged where the tight lists in use were built.
+__device__ __forceinline__ float built_threshold(const DevParams& P, const Control* ctl) {
+    return P.list_half_skin - (ctl->tight_next & kTightEarly ? P.tight_margin : 0.f);
+}
+
 // After predicting x*_i (stored as xs): a fast particle (moved more than half the skin) flags its bucket
 // and is counted (one atomic per warp that has one; no store otherwise: in a splash most predictions are
 // fast, and a flag stored by each of their warps measured slower than the counts alone); the predictions
 // past each adaptive skin level are counted. With a fast list (partner marks, one scene), a fast particle
 // also takes a slot of the round's list while the round holds at most P.mark_cap of them (one atomic per
 // warp that has one; none once the round is past the cap, which then falls back to the bucket flags).
-// Returns the displacement |x* - x|; threshold: the particle's fast_threshold; flag: whether it is past it. kOne: one
+// Returns the displacement |x* - x|; threshold: the particle's fast_threshold (or less); flag: whether it is past it. kOne: one
 // scene, whose lists may move with the particles (then the bucket is flagged when the prediction strays from y, and the
 // round's count is past the cap, so that nothing is listed); vi: the velocity at the step's start. ref (or null): the
 // prediction that the tight lists in use were built at; flag is then whether xs outran the lists and that one did not.
@@ -56,7 +61,7 @@ __device__ __forceinline__ float note_displacement(const DevParams& P, Control* 
                                                    bool& flag, uint32_t* __restrict__ fast_list = nullptr, uint32_t i = 0) {
     float disp;
     flag = outruns<kOne>(P, ctl, xi, xs, threshold, vi, disp);
-    warp_count(&ctl->fast_particles, disp > threshold);
+    warp_count(&ctl->fast_particles, disp > P.list_half_skin);
     if (flag && ctl->lists_outrun == 0u) ctl->lists_outrun = 1u;
     if (fast_list) {
         const unsigned act = __activemask();
@@ -82,7 +87,7 @@ __device__ __forceinline__ float note_displacement(const DevParams& P, Control* 
         unsigned char* mine = &bucket_fast[P.bucket_base + hash_key(c.x, c.y, c.z, P)];
         if (ref) {
             float at_ref;
-            flag = !outruns<kOne>(P, ctl, xi, *ref, threshold, vi, at_ref);
+            flag = !outruns<kOne>(P, ctl, xi, *ref, built_threshold(P, ctl), vi, at_ref);
             if (flag && (*mine == 0 || ctl->tight_marked) && ctl->tight_outrun == 0u) ctl->tight_outrun = 1u;
         }
         *mine = 1;

@@ -17,7 +17,7 @@ def _cloud(n, per_cell, seed):
 
 
 # sizes around the particles of a warp and of a block for each of the three splits (2, 4 and 8 particles a warp: up to
-# 8,192, up to 49,152, beyond), and dense clouds: more candidates than the 320 of one pass, more neighbours than the
+# 8,192, up to 16,384, beyond) and around the sweeps' own (8,192, 49,152), and dense clouds: more candidates than the 320 of one pass, more neighbours than the
 # near list (64), the skin list (96) and the staging area hold
 @pytest.mark.parametrize("order", [0, 1])
 @pytest.mark.parametrize("n,per_cell", [(1, 8), (2, 8), (7, 8), (9, 8), (33, 20), (1000, 40), (700, 300), (2000, 600),
@@ -297,3 +297,37 @@ def test_autotune_chooses_among_different_launches(oracle, n, block):
 @pytest.mark.parametrize("n", [16384, 16385])
 def test_lists_at_the_builders_second_split(oracle, n, order):
     test_lists_hold_the_walks_neighbours(oracle, n, 8, order)
+
+
+# Long loops in which particles keep crossing half the skin: after some sweeps the rebuilt lists are built once more, with
+# predictions flagged before they reach it
+@pytest.mark.parametrize("n,motion,speed,options", [
+    (6000, "few", 4.7, {}), (8193, "few", 4.7, {}), (30000, "few", 4.7, {}), (30000, "corner", 4.4, {}), (30000, "all", 2.2, {}),
+    (20000, "few", 4.7, {"boundary": 1}), (20000, "corner", 4.4, {"list_skin": 0.2}), (160000, "corner", 4.4, {})])
+def test_early_flags_change_no_bits(oracle, n, motion, speed, options):
+    rng = np.random.default_rng(n + 1)
+    side = int(np.ceil(n ** (1 / 3)))
+    at = np.stack(np.unravel_index(np.arange(n), (side, side, side)), -1) + 0.5
+    pos = ((at + 0.2 * (2 * rng.random((n, 3)) - 1)) * 0.95 * D).astype(np.float32)
+    vel = np.zeros((n, 3), np.float32)
+    who = {"few": rng.random(n) < 0.02, "corner": (at < 0.5 * side).all(1), "all": np.ones(n, bool)}[motion]
+    vel[who, 1] = (-speed * (0.95 + 0.1 * rng.random(n))).astype(np.float32)[who]
+    floor = np.stack(np.meshgrid(np.arange(side), [-0.5], np.arange(side), indexing="ij"), -1).reshape(-1, 3) * D
+    walls = len(floor) if options.get("boundary") else 0
+    p = oracle.derive_params(0.5 * D, 1000.0, n, walls, 1e-3, -9.81, 0.2 * D ** 3, 0.5)
+    out = []
+    for loop_mode in (0, 1, 2):
+        f = fluid_like(p, min_iters=40, max_iters=40, loop_mode=loop_mode, spatial_order=2)
+        f.set_options(**{k: v for k, v in options.items() if k != "boundary"})
+        f.set_fluid_state(pos, vel)
+        if walls:
+            f.set_boundary_state(floor.astype(np.float32))
+        f.step(3)
+        st = f.stats()
+        out.append(({k: f.get_field(k) for k in ("src", "density_variation", "pressure", "position", "velocity", "predicted_position")},
+                    (st.fast_particles, st.list_fallbacks, st.status_all)))
+        f.close()
+    for got in out[:2]:
+        assert got[1] == out[2][1]
+        for k in got[0]:
+            np.testing.assert_array_equal(got[0][k], out[2][0][k], err_msg=k)
