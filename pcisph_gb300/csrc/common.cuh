@@ -43,8 +43,9 @@ struct DevParams {
     // particle near a flagged bucket walks)
     uint32_t mark_cap;
     // moving lists (one scene without boundary particles or per-particle skins): in a step that begins with more than
-    // 1 in kMovingShare particles that move kMovingSpeed of half the skin or more per step, the skin lists are built around y = x + v dt
-    // (moving_place) and a prediction is measured from there: a body that moves as a whole keeps its lists
+    // 1 in kMovingShare particles that move kMovingSpeed of half the skin or more per step, the skin lists are built
+    // around y = x + v dt (moving_place) and a prediction is measured from there: a body that moves as a whole keeps its
+    // lists
     int moving_lists;
     // tight lists (see the list sweeps): the distance that a prediction may move from where they were built (0: none are),
     // the same less a margin for rounding, and their radius^2, (h + 2 tight_margin)^2
@@ -87,7 +88,7 @@ struct Control {
     // the current round's pressure sweep, whose last block closes the round)
     unsigned long long fast_n;
     unsigned int round;
-    unsigned int moving;         // moving lists: the particles that fast (kMovingSpeed) when the step began
+    unsigned int moving;         // moving lists: the particles that are that fast (kMovingSpeed) when the step begins
     // Every particle's pressure sweep reads these four, as one vector (list_state). Tight lists: how the next sweep finds its
     // neighbours (kTightOff, kTightBuild or kTightUse; beside it kTightEarly: the lists in use, or the next ones, are built
     // with the predictions flagged that came within tight_margin of half the skin), whether a prediction left their reach
@@ -151,7 +152,7 @@ constexpr unsigned kMovingShare = 8;
 // (a sphere falling at 0.11 h a step outran a half skin of 0.125 h in every prediction).
 constexpr float kMovingSpeed = 0.75f;
 // After a step of kMovingLong iterations or more: a little slower bodies cross half the skin here and there, and a long loop pays
-// for that in most of its sweeps (186,000 particles falling at 0.09 h a step, 50 iterations: 3120 us a step, moving 2270).
+// for that in most of its sweeps (186,000 particles falling at 0.09 h a step, 50 iterations: 3120 us a step, moving 2170).
 constexpr float kMovingSpeedLong = 0.69f;
 constexpr int kMovingLong = 30;
 __device__ __forceinline__ bool lists_move(const DevParams& P, const Control* ctl) {
