@@ -401,6 +401,10 @@ struct pcisph_ctx {
         // (marks reach up to 2 kTightMargin h further where tight lists are built, see below)
         set_tight_lists(&P, list_sweeps() && opts.loop_mode != 2 && opts.max_iterations >= kTightFrom &&
                             P.h + P.skin_max_half + 2.f * kTightMargin * P.h <= 1.9f * P.cell_size);
+        {
+            std::lock_guard<std::mutex> l(tight_block.use);
+            if (!tight_block.p()) tight_list = nullptr;  // refused or given up: the next step asks for room again
+        }
         // partner marks scan the 5 x 5 x 5 cells around a fast prediction: a particle that did not outrun its
         // skin lies within h + skin_max_half of a prediction within h of its own, which must stay below two
         // cells (with a margin for the divisions of cell_of). With more than 1 in 8 fast nearly every warp holds walkers

@@ -177,3 +177,21 @@ def test_tank_skins_without_rebuilt_lists(oracle):
         torch.cuda.empty_cache()
     _same(out[0], out[1])
     _same(out[0], out[2])
+
+
+def test_given_up_lists_are_asked_for_again(oracle):
+    torch = pytest.importorskip("torch")
+    a = _block(oracle, 1500000, seed=6)
+    a.step(1)
+    a.sync()
+    hold = _leave(torch, 300 << 20)
+    b = _block(oracle, 500000, seed=7)  # needs more than is free
+    b.step(1)
+    b.close()
+    del hold
+    torch.cuda.empty_cache()
+    assert a.rebuilt_lists()[0] == 0
+    a.set_options(restitution=0.5)
+    a.step(1)
+    assert a.rebuilt_lists()[0] >= PER_PARTICLE * 1500000
+    a.close()
