@@ -302,10 +302,10 @@ constexpr uint32_t kAll = 0xffffffffu;
 // walk by the rules of the skin lists (fast predictions' flags or marks). It does walk where these say so, and did not in the
 // building sweep. A fast prediction that was fast at the building, too, asks nobody again: there its partners within h + 2 m
 // were marked (or all near its bucket flagged), and walked. Where others keep crossing half the skin, sweep after sweep asks the
-// marks: a long loop builds the lists anew then, with the predictions flagged that came within m of it (99,768 to 186,000
-// particles that fall at 0.09 h a step, 50 iterations: 2640 to 3540 us a step without). A particle with
-// more than kTightCap entries walks in every sweep that would read them. One prediction out of reach (or NaN) puts the whole
-// scene back on the skin lists, and from iteration kTightAgain on rebuilds: a building sweep in the loop (it stores entry by
+// marks: a long loop builds the lists anew then, with the predictions flagged that came within m of it (99,768 / 150,000 /
+// 186,000 particles that fall at 0.09 h a step, 50 iterations, before moving lists took them: 2500 / 2910 / 3540 us a step
+// without, 2300 / 2510 / 3120 with). A particle with more than kTightCap entries walks in every sweep that would read them. One prediction
+// out of reach (or NaN) puts the whole scene back on the skin lists, and from iteration kTightAgain on rebuilds: a building sweep in the loop (it stores entry by
 // entry, 1670 us at 8.4M) pays from three sweeps that use it, which a loop of fewer iterations need not have left.
 // Margins at 1M / 8.4M / a 98,904-particle drop, us a step: 0.02 2284 / 70510 / 1880, 0.03 1998 / 68148 / 1840, 0.04 2018 /
 // 67244 / 1821.
@@ -322,7 +322,7 @@ constexpr uint32_t kAll = 0xffffffffu;
 // 862 -> 840. Eight lanes per particle: 4,096 particles at rest 159 -> 157 us, 8,000 violently jittered 985 -> 667.
 //
 // Skin lists narrower than this hold too few of the later pairs: the building sweep walks throughout, and every tight list is
-// complete. (list_skin 0.05, 4,096 particles 350 -> 183 us a step; from 0.07 on the lists are read, 182 -> 139.)
+// complete (list_skin 0.05, 4,096 particles 350 -> 183 us a step; from 0.08 on the lists are read, 140).
 __device__ __forceinline__ bool tight_by_walks(const DevParams& P) { return P.skin_max_half < 1.05f * P.tight_margin; }
 // The control fields that decide over the tight lists, loaded together: one thread decides at the end of a sweep, and small
 // scenes wait for it.
@@ -333,7 +333,8 @@ struct TightState {
     unsigned long long fast, before, sweeps;
     __device__ __forceinline__ TightState(const DevParams& P, const Control* c)
         : next(tight_plan(c->tight_next)), stray(c->tight_stray), age(c->tight_age), wait(c->tight_wait), backoff(c->tight_backoff),
-          iter(c->iter), outrun(c->tight_outrun), asked(c->tight_asked), early(c->tight_next & kTightEarly), last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before),
+          iter(c->iter), outrun(c->tight_outrun), asked(c->tight_asked), early(c->tight_next & kTightEarly),
+          last(c->iterations_last), moves(lists_move(P, c)), fast(c->fast_particles), before(c->fast_before),
           sweeps(c->tight_sweeps) {}
     __device__ __forceinline__ unsigned mode(const DevParams& P) const {
         if (next == kTightOff || (next == kTightUse && stray == 0u)) return next;
